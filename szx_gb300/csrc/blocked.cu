@@ -48,29 +48,18 @@ constexpr int kIdxItems = 8;   // items per thread in the index scans
 // ------------------------------------------------------------------ encode
 //
 // Per-block state a segment keeps in registers from its statistics pass to
-// its emission (szx/src/szx_float.cc:49-252 for one block).
-// Chunk-round byte totals of a segment are scanned packed, one field per
-// round: 8-bit fields for float up to 8 lanes (a round holds at most 8 x 16
-// bytes), 16-bit otherwise; in 32 bits whenever they fit.
-template <typename T, int G>
-struct RoundPack {
-    static constexpr int NC = EncCfg<T>::E / 4;
-    static constexpr int FB = (sizeof(T) == 4 && G <= 8) ? 8 : 16;
-    static constexpr uint32_t MASK = (1u << FB) - 1;
-    using P = typename std::conditional<NC * FB <= 32, uint32_t, unsigned long long>::type;
-};
-
+// its emission (szx/src/szx_float.cc:49-252 for one block).  A lane owns a run
+// of E consecutive values (64 bytes), whose stored bytes are one run of the
+// payload.
 template <typename T, int G>
 struct BlockEnc {
     using U = typename Elem<T>::U;
-    using P = typename RoundPack<T, G>::P;
     static constexpr int E = EncCfg<T>::E;
     static constexpr int NC = E / 4;
-    U cur[E];                        // shifted words
-    uint32_t cnt4[NC];               // stored bytes of the chunk's 4 values (byte i: value i)
-    uint32_t pre4[NC];               // exclusive offsets of those bytes within the chunk
-    uint32_t codes;                  // lead byte of chunk round k in byte k
-    P excl, tot;                     // per round (packed fields): bytes of earlier lanes, round total
+    U ev[E];                         // the value's required bytes (reqLength bits), right-aligned
+    uint32_t cnt8[NC];               // bits stored of each of the chunk's 4 values (byte i: value i)
+    uint32_t codes;                  // lead byte of chunk k in byte k
+    uint32_t excl;                   // mid bytes of earlier lanes
     int state;                       // 0 constant, 1 coded, 2 no block
     int reqLength;
     uint32_t med_bits;               // median as stored (payload or constant list)
@@ -92,22 +81,24 @@ struct EncArgs {
 // Statistics pass of one block by a G-lane segment: state, reqLength and
 // median (szx/src/szx_float.cc:314-371), the shifted words, lead codes
 // (szx/src/szx_float.cc:94-113) and stored-byte counts, all kept in registers.
+//
+// eb_key: the bound's rule for double radii (constant when the radius's bit
+// pattern, as an unsigned number, is below it; see eb_key_of).
 template <typename T, int G, bool FULL>
-__device__ __forceinline__ void enc_block_stats(const T* xs, int len, bool vec, float eb, int eb_exp, int omp_stats,
+__device__ __forceinline__ void enc_block_stats(const uint8_t* tile, uint32_t e0, int len, bool vec, float eb,
+                                                int eb_exp, unsigned long long eb_key, int omp_stats,
                                                 BlockEnc<T, G>& b) {
-    using C = Chunks<T, G>;
-    using RP = RoundPack<T, G>;
-    using P = typename RP::P;
     using EL = Elem<T>;
     using U = typename EL::U;
-    constexpr int E = C::E;
-    constexpr int NC = C::NC;
+    constexpr int W = EL::W;
+    constexpr int E = EncCfg<T>::E;
+    constexpr int NC = E / 4;
     const int sl = (int)(lane_id() & (G - 1));
     T v[E];
-    load_chunks<T, G>(xs, FULL ? G * E : len, vec, v);
+    load_run<T, G>(tile, e0, vec, v);
     T mn, mx;
     bool special;
-    seg_minmax<T, G, FULL>(v, len, mn, mx, special);
+    seg_minmax<T, G, FULL, Runs<T, G>>(v, len, mn, mx, special);
     int state;
     float radius_f, median_f;
     if constexpr (sizeof(T) == 4) {
@@ -120,7 +111,7 @@ __device__ __forceinline__ void enc_block_stats(const T* xs, int len, bool vec, 
         const double range = xsub(mx, mn);
         const double radius = xhalf(range);
         const double median = xadd(mn, radius);
-        state = (radius <= (double)eb) ? 0 : 1;
+        state = (unsigned long long)__double_as_longlong(radius) < eb_key ? 0 : 1;
         radius_f = xd2f(radius);
         median_f = xd2f(median);
     } else {
@@ -138,40 +129,52 @@ __device__ __forceinline__ void enc_block_stats(const T* xs, int len, bool vec, 
     T med;
     if constexpr (sizeof(T) == 4) med = __uint_as_float(payload_med);
     else med = xf2d(median_f);
-    // shifted words (szx/src/szx_float.cc:88-92); x86 NaN rules only where a NaN can arise
+    // differences from the median (szx/src/szx_float.cc:88-92); x86 NaN rules only where a NaN can arise
+    U d[E];
     if (__any_sync(0xffffffffu, special)) {
 #pragma unroll
-        for (int e = 0; e < E; e++) b.cur[e] = EL::bits(xsub(v[e], med)) >> s;
+        for (int e = 0; e < E; e++) d[e] = EL::bits(xsub(v[e], med));
     } else {
 #pragma unroll
-        for (int e = 0; e < E; e++) b.cur[e] = EL::bits(EL::sub(v[e], med)) >> s;
+        for (int e = 0; e < E; e++) d[e] = EL::bits(EL::sub(v[e], med));
     }
-    // lead codes: leading identical bytes with the previous value, capped at 3
-    uint32_t ldbs[NC];
-    seg_lead_bytes<T, G>(b.cur, ldbs);
-    P pk = 0;
-    uint32_t codes = 0;
+    // Lead codes: leading identical bytes of the words shifted right by s with
+    // the previous value's, capped at 3 -- (leading zeros of the XOR + s) / 8,
+    // with a guard bit that ends the count at 24 - s.  Only the top 32 bits
+    // decide; four counts are packed in a word before the division.
+    auto top = [](U u) { return (uint32_t)(u >> (8 * W - 32)); };
+    uint32_t prev = __shfl_up_sync(0xffffffffu, top(d[E - 1]), 1, G);
+    if (sl == 0) prev = 0u;   // zero before the block
+    const uint32_t guard = 0x80u << s, s4 = (uint32_t)s * 0x01010101u;
+    uint32_t codes = 0, mine = 0;
 #pragma unroll
     for (int k = 0; k < NC; k++) {
-        uint32_t ldb = ldbs[k];
+        uint32_t lz[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t h = top(d[4 * k + i]);
+            lz[i] = (uint32_t)__clz((h ^ prev) | guard);
+            prev = h;
+        }
+        const uint32_t p = __byte_perm(__byte_perm(lz[0], lz[1], 0x0040), __byte_perm(lz[2], lz[3], 0x0040), 0x5410);
+        uint32_t ldb = ((p + s4) >> 3) & 0x03030303u;
         uint32_t cnt4 = stored_counts(R, ldb);   // max(R - lead, 0) per value
         if constexpr (!FULL) {
-            const uint32_t m = low_bytes_mask(len - 4 * (sl + k * G));
+            const uint32_t m = low_bytes_mask(len - (E * sl + 4 * k));
             ldb &= m;
             cnt4 &= m;
         }
-        b.cnt4[k] = cnt4;
-        b.pre4[k] = cnt4 * 0x01010100u;
-        pk |= (P)((cnt4 * 0x01010101u) >> 24) << (RP::FB * k);
+        b.cnt8[k] = cnt4 << 3;
+        mine = __dp4a(cnt4, 0x01010101u, mine);
         codes |= ((ldb * 0x40100401u) >> 24) << (8 * k);   // 4 leads -> one byte, MSB first
     }
-    const P incl = seg_inclusive_sum<G>(pk);
-    b.tot = __shfl_sync(0xffffffffu, incl, G - 1, G);
-    b.excl = incl - pk;
+    const uint32_t incl = seg_inclusive_sum<G>(mine);
+    const uint32_t mid = __shfl_sync(0xffffffffu, incl, G - 1, G);
+    b.excl = incl - mine;
     b.codes = codes;
-    uint32_t mid = 0;
+    const int down = 8 * W - reqLength;   // drops the bits below the required ones
 #pragma unroll
-    for (int k = 0; k < NC; k++) mid += (uint32_t)((b.tot >> (RP::FB * k)) & RP::MASK);
+    for (int e = 0; e < E; e++) b.ev[e] = d[e] >> down;
     const int Lb = FULL ? G * NC : (len + 3) / 4;
     b.size = 5 + (uint32_t)Lb + mid;
     b.state = len ? state : 2;
@@ -179,50 +182,90 @@ __device__ __forceinline__ void enc_block_stats(const T* xs, int len, bool vec, 
     b.med_bits = state == 1 ? payload_med : __float_as_uint(median_f);
 }
 
-// Emission of one coded block into the tile's staging buffer: header and lead
-// bytes, then each value's stored bytes with predicated byte stores.  Every
-// byte of [loc, loc + size) is written exactly once, so the staging buffer
-// needs no clearing and no atomics (a value's bytes are contiguous, values
-// follow each other without gaps).
-template <typename T, int G, bool FULL>
-__device__ __forceinline__ void enc_block_emit(uint8_t* stg, uint32_t loc, int len, const BlockEnc<T, G>& b) {
-    using RP = RoundPack<T, G>;
-    using C = Chunks<T, G>;
-    using EL = Elem<T>;
-    using U = typename EL::U;
-    constexpr int W = EL::W;
-    constexpr int NC = C::NC;
-    const int sl = (int)(lane_id() & (G - 1));
-    uint8_t* p = stg + loc;
-    if (sl == 0) {
-        p[0] = (uint8_t)b.reqLength;
-        p[1] = (uint8_t)(b.med_bits >> 24);
-        p[2] = (uint8_t)(b.med_bits >> 16);
-        p[3] = (uint8_t)(b.med_bits >> 8);
-        p[4] = (uint8_t)b.med_bits;
+// A double block is constant when radius <= (double)eb.  The radius is a
+// non-negative number or a NaN, so the test is one on unsigned bit patterns:
+// pattern < eb_key, with key 0 (never) for negative and NaN bounds; a NaN's
+// pattern of either sign is above every bound's.
+__device__ __forceinline__ unsigned long long eb_key_of(float eb) {
+    if (!(eb >= 0.0f)) return 0ull;
+    return (unsigned long long)__double_as_longlong(xf2d(fabsf(eb))) + 1ull;
+}
+
+// Byte-wise appending to a payload in shared memory.  A lane appends its
+// run's values one after the other: `last` holds the four bytes written last
+// (the newest on top), so the word that a value completes is a funnel shift of
+// (last, value) by the position's bit offset and the next `last` one by the
+// value's bits -- no masks, no byte stores, and whole words leave with one
+// predicated store each.  The first word a lane completes carries stale
+// bytes below the run's start; what belongs there (the lane before's last
+// bytes, or the block's lead codes) is stored after it, bytewise.
+struct RunOut {
+    uint32_t last, q8, sp;   // last four bytes, bit position, shared address of the word being filled
+    __device__ __forceinline__ void append(uint32_t v, uint32_t n8) {   // the low n8 / 8 (0..4) bytes of v
+        const uint32_t w = __funnelshift_l(last, v, q8);
+        last = __funnelshift_rc(last, v, n8);
+        const uint32_t q = q8 + n8;
+        if ((q ^ q8) & ~31u) {
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(sp), "r"(w) : "memory");
+            sp += 4;
+        }
+        q8 = q;
     }
+};
+
+// Emission of the coded blocks of a warp (act: this segment has one) into the
+// tile's staging buffer: every lane's whole words, then headers, lead bytes
+// and the bytes of the words that lanes share.  Every byte of a block's
+// [loc, loc + size) ends up as the stream wants it; bytes outside are not
+// touched (a lane's first word starts at most 3 bytes early, inside the
+// block's own header and lead bytes).  ~8 instructions and one 4-byte store
+// per float value, where a store per byte took ~15 and up to four.
+template <typename T, int G, bool FULL>
+__device__ __forceinline__ void enc_block_emit(uint8_t* stg, uint32_t loc, int len, bool act, const BlockEnc<T, G>& b) {
+    constexpr int E = EncCfg<T>::E;
+    constexpr int NC = E / 4;
+    const int sl = (int)(lane_id() & (G - 1));
     const int Lb = FULL ? G * NC : (len + 3) / 4;
-    int R, s;
-    split_reqlen(b.reqLength, &R, &s);
-    (void)s;
-    const int low = 8 * (W - R);
-    uint32_t before = loc + 5 + (uint32_t)Lb;
+    const uint32_t q0 = loc + 5 + (uint32_t)Lb + b.excl;
+    RunOut o;
+    o.last = 0;
+    o.q8 = 8 * q0;
+    o.sp = smem_u32(stg) + (q0 & ~3u);
+    if (act) {
 #pragma unroll
-    for (int k = 0; k < NC; k++) {
-        const int c = sl + k * G;
+        for (int k = 0; k < NC; k++) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t n8 = byte_of(b.cnt8[k], i);
+                if constexpr (sizeof(T) == 4) {
+                    o.append((uint32_t)b.ev[4 * k + i], n8);
+                } else {
+                    const uint32_t nl = n8 < 32u ? n8 : 32u;
+                    o.append((uint32_t)b.ev[4 * k + i], nl);
+                    o.append((uint32_t)(b.ev[4 * k + i] >> 32), n8 - nl);
+                }
+            }
+        }
+    }
+    __syncwarp();
+    if (act) {
+        // the last, partial word: its bytes from the run's start (if that lies in it) to the run's end
+        const uint32_t w = __funnelshift_l(o.last, 0u, o.q8);
+        const uint32_t end = (o.q8 >> 3) & 3u, beg = (o.sp ^ smem_u32(stg + q0)) < 4u ? q0 & 3u : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 3; j++)
+            if (j >= beg && j < end) asm volatile("st.shared.u8 [%0], %1;" ::"r"(o.sp + j), "r"(w >> (8 * j)) : "memory");
+        uint8_t* p = stg + loc;
         // lead codes: 4 per byte, MSB first (szx/src/szx_TypeManager.cc:198-273)
-        if (FULL || c < Lb) p[5 + c] = (uint8_t)(b.codes >> (8 * k));
-        const uint32_t qb = before + (uint32_t)((b.excl >> (RP::FB * k)) & RP::MASK);
-        before += (uint32_t)((b.tot >> (RP::FB * k)) & RP::MASK);
-        // mid bytes: bytes [W-R .. W-1-lead] of each shifted word, ascending
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t n = byte_of(b.cnt4[k], i);
-            uint8_t* d = stg + qb + byte_of(b.pre4[k], i);
-            const U ev = b.cur[4 * k + i] >> low;
-#pragma unroll
-            for (int j = 0; j < W; j++)
-                if ((uint32_t)j < n) d[j] = (uint8_t)(ev >> (8 * j));
+        for (int k = 0; k < NC; k++)
+            if (FULL || NC * sl + k < Lb) p[5 + NC * sl + k] = (uint8_t)(b.codes >> (8 * k));
+        if (sl == 0) {
+            p[0] = (uint8_t)b.reqLength;
+            p[1] = (uint8_t)(b.med_bits >> 24);
+            p[2] = (uint8_t)(b.med_bits >> 16);
+            p[3] = (uint8_t)(b.med_bits >> 8);
+            p[4] = (uint8_t)b.med_bits;
         }
     }
 }
@@ -248,7 +291,8 @@ struct EncTile {
     static_assert(kGroups <= 8 && kBlocks % kBpw == 0, "one block group per warp");
     static_assert(kBlocks <= 64, "a tile's sizes are scanned as two warp-wide halves");
     static_assert(kBlocks * kMaxPay < 65535, "a tile's byte count + 1 fits the 16-bit aggregate words");
-    static_assert(kIn % 16 == 0 && kBuf % 16 == 0, "TMA destinations stay 16-byte aligned");
+    static_assert(kIn % 512 == 0 && kBuf % 16 == 0, "swizzled chunks stay inside the tile, buffers 16-byte aligned");
+    static_assert(kThreads % 32 == 0, "a thread's chunks keep one swizzle phase");
 };
 
 // One pass over the input.  A CTA works through its tiles T_j in a ring of
@@ -276,7 +320,6 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     constexpr int BPW = TL::kBpw;
     constexpr int NGRP = TB / BPW;
     extern __shared__ __align__(128) uint8_t dsm[];
-    __shared__ unsigned long long bar[4];
     __shared__ __align__(16) uint16_t s_w16[2][kLbWin + 8];   // look-back windows (16-bit aggregates)
     __shared__ long long s_an_t, s_wlo[2];                     // placement anchor tile; window first tiles
     __shared__ unsigned long long s_an_incl;                   // the anchor's inclusive prefix
@@ -298,8 +341,6 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     auto field_of = [&](long long g) { return (int)a.tile_field[g]; };
     auto buf_ptr = [&](int r) { return dsm + r * TL::kBuf; };
     if (threadIdx.x == 0) {
-        for (int r = 0; r < 4; r++) mbar_init(&bar[r], 1);
-        mbar_fence_init();
         for (int r = 0; r < 2; r++) {
             s_tile[r] = (long long)atomicAdd(a.tile_ctr, 1ull);
             s_fld[r] = (MULTI && s_tile[r] < nt) ? field_of(s_tile[r]) : 0;
@@ -309,35 +350,35 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     // a field's members: from the kernel parameters for one field, from the table for a batch
     auto fld = [&](int f) -> const BlkField* { return MULTI ? a.fields + f : nullptr; };
 #define FV(F_, m) (MULTI ? (F_)->m : a.one.m)
-    uint32_t phase = 0;   // bit r: parity to wait for on ring buffer r
 
     auto tile_count = [&](const BlkField* F, long long t) {
         const unsigned long long start = (unsigned long long)t * tile_elems;
         const unsigned long long rem = FV(F, n) - start;
         return rem < tile_elems ? rem : tile_elems;
     };
-    // all threads: TMA of the 16-byte part by thread 0, the rest by plain copies
+    // all threads: the tile's values into ring buffer r, swizzled in 16-byte
+    // chunks, by cp.async (one group; completed before the next iteration's
+    // first barrier)
     auto issue = [&](long long g, int f, int r) {
         const BlkField* F = fld(f);
         const long long t = g - (long long)FV(F, enc_tile0);
-        const T* x = (const T*)FV(F, x);
-        const bool tma_ok = ((uintptr_t)x & 15) == 0;
-        const unsigned long long cnt = tile_count(F, t);
-        const uint32_t bytes = (uint32_t)(cnt * sizeof(T));
-        const uint32_t tbytes = tma_ok ? (bytes & ~15u) : 0u;
-        T* dst = (T*)buf_ptr(r);
-        const T* src = x + (unsigned long long)t * tile_elems;
-        if (threadIdx.x == 0 && tbytes) {
-            fence_proxy_async();   // the buffer's last generic accesses come before the async write
-            mbar_arrive_expect_tx(&bar[r], tbytes);
-            tma_load_1d(dst, src, tbytes, &bar[r]);
-        }
-        for (unsigned long long i = tbytes / sizeof(T) + threadIdx.x; i < cnt; i += TL::kThreads) dst[i] = src[i];
-    };
-    auto wait_buf = [&](const BlkField* F, long long t, int r) {
-        if (((uintptr_t)FV(F, x) & 15) == 0 && ((tile_count(F, t) * sizeof(T)) & ~15ull)) {
-            if (!mbar_wait(&bar[r], (phase >> r) & 1u) && threadIdx.x == 0) atomicExch(a.err, kErrLookback);
-            phase ^= 1u << r;
+        const uint32_t cnt = (uint32_t)tile_count(F, t);
+        const uint8_t* src = (const uint8_t*)((const T*)FV(F, x) + (unsigned long long)t * tile_elems);
+        uint8_t* dst = buf_ptr(r);
+        if (((uintptr_t)src & 15) == 0) {
+            constexpr uint32_t VN = 16 / sizeof(T);
+            const uint32_t nch = cnt / VN;
+            // chunks threadIdx.x + k * kThreads: the swizzle phase is the same for all of them
+            const uint8_t* sp = src + 16 * threadIdx.x;
+            uint8_t* dp = dst + 16 * swz16(threadIdx.x);
+#pragma unroll
+            for (int k = 0; k < (TL::kIn / 16 + TL::kThreads - 1) / TL::kThreads; k++)
+                if (threadIdx.x + k * TL::kThreads < nch) cp_async16(dp + 16 * k * TL::kThreads, sp + 16 * k * TL::kThreads);
+            const uint32_t i = nch * VN + threadIdx.x;
+            if (i < cnt) cp_async_small<sizeof(T)>(dst + swz_off<T>(i), src + i * sizeof(T));
+        } else {
+            for (uint32_t i = threadIdx.x; i < cnt; i += TL::kThreads)
+                cp_async_small<sizeof(T)>(dst + swz_off<T>(i), src + i * sizeof(T));
         }
     };
     auto block_len = [&](const BlkField* F, long long t, int lb) {
@@ -433,12 +474,13 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
                 base = an_incl;
                 placed = true;
             } else if (ok == 1) {
+                // (the window's group; the next tile's values, issued after it, stay in flight)
+                cp_async_wait_group<1>();
+                __syncwarp();
                 // a window with aggregates not yet published is copied again
                 // (one round trip each) a few times before the global walk
                 const int units = (int)((t - lo + 7) >> 3);
                 for (int attempt = 0;; attempt++) {
-                    cp_async_wait_all();
-                    __syncwarp();
                     unsigned long long sum = 0;
                     bool ready = true;
                     for (long long i = an_t + 1 + lane; i < t; i += 32) {
@@ -453,8 +495,9 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
                     }
                     if (attempt == kWinRepolls) break;
                     __nanosleep(128);
-                    const uint16_t* src = agg16_of(F) + lo;
-                    for (int u = lane; u < units; u += 32) cp_async16(&s_w16[buf][8 * u], src + 8 * u);
+                    const uint32_t* src = (const uint32_t*)(agg16_of(F) + lo);
+                    for (int u = lane; u < units; u += 32) *(uint4*)&s_w16[buf][8 * u] = ld_volatile_v4(src + 4 * u);
+                    __syncwarp();
                 }
             }
             if (!placed) base = prefix_resolve(FV(F, st_enc), t, agg, a.err);   // publishes t's inclusive prefix
@@ -473,20 +516,25 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     };
 
     if (s_tile[0] < nt) issue(s_tile[0], s_fld[0], 0);
+    cp_async_commit();
+    cp_async_commit();   // (an empty group in the window's place)
     const bool taker = warp == TL::kWarps - 1 && lane == 0;
     long long t1 = -1, t2 = -1;   // T_{j-1}, T_{j-2} (field-local), -1: none
     int eb_f = -1, eb_exp = 0;    // field whose bound is loaded, the bound's exponent
     float eb = 0.f;
+    unsigned long long eb_key = 0;   // and its key for double radii
     int f1 = 0, f2 = 0;
     int j = 0;
     for (;; j++) {
         const int r = j & 3;
+        cp_async_wait_group<1>();   // T_j's values are in (the window issued after them may still be on its way)
         __syncthreads();   // ring position j+1 claimed, copy-out of T_{j-3} done
         {
             const int rn = (j + 1) & 3;
             const long long gn = s_tile[rn];
             if (gn < nt) issue(gn, s_fld[rn], rn);
         }
+        cp_async_commit();
         if (warp == 0 && t2 >= 0) place(fld(f2), f2, t2, (j - 2) & 3, (j - 1) & 1);
         const long long g = s_tile[r];
         if (g >= nt) break;
@@ -496,7 +544,6 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
         // the last warp takes the tile of ring position j+2; the reply is used after the statistics
         unsigned long long gc = 0;
         if (taker) gc = atomicAdd(a.tile_ctr, 1ull);
-        wait_buf(F, t, r);
         // ---- statistics of the tile's blocks, one block per segment
         const int lb = warp * BPW + seg;
         const bool mine = warp < NGRP;
@@ -507,13 +554,14 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
         if (f != eb_f) {   // the field's bound and its exponent, once per field
             eb = FV(F, params) ? FV(F, params)->eb : FV(F, eb);
             eb_exp = exponent_f64_of_f32(eb);
+            if constexpr (sizeof(T) == 8) eb_key = eb_key_of(eb);
             eb_f = f;
         }
         BlockEnc<T, G> b;
         if (mine) {
-            const T* xs = (const T*)buf_ptr(r) + (size_t)lb * a.bs;
-            if (full) enc_block_stats<T, G, true>(xs, len, vec, eb, eb_exp, a.omp_stats, b);
-            else enc_block_stats<T, G, false>(xs, len, vec, eb, eb_exp, a.omp_stats, b);
+            const uint32_t e0 = (uint32_t)(lb * a.bs);
+            if (full) enc_block_stats<T, G, true>(buf_ptr(r), e0, len, vec, eb, eb_exp, eb_key, a.omp_stats, b);
+            else enc_block_stats<T, G, false>(buf_ptr(r), e0, len, vec, eb, eb_exp, eb_key, a.omp_stats, b);
             if (sl == 0) {
                 s_state[r][lb] = (uint8_t)b.state;
                 s_size[r][lb] = b.state == 1 ? b.size : 0;
@@ -528,6 +576,7 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
         __syncthreads();   // statistics in (T_j's input is dead), T_{j-2} placed
         // warp 0: T_{j-1}'s look-back window, in flight until the next iteration
         if (warp == 0 && t1 >= 0) win_issue(fld(f1), f1, t1, j & 1);
+        cp_async_commit();   // the window's group (empty in the other warps)
         // every warp: the tile's block offsets (two warp-wide halves)
         const bool in0 = lane < TB;
         const uint32_t sz0 = in0 ? s_size[r][lane] : 0;
@@ -548,10 +597,10 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
             }
             prefix_publish(FV(F, st_enc), t, agg);
         }
-        if (mine && b.state == 1) {
+        if (mine) {
             const uint32_t loc = lb < 32 ? loc_lo : loc_hi;
-            if (full) enc_block_emit<T, G, true>(buf_ptr(r), loc, len, b);
-            else enc_block_emit<T, G, false>(buf_ptr(r), loc, len, b);
+            if (full) enc_block_emit<T, G, true>(buf_ptr(r), loc, len, b.state == 1, b);
+            else enc_block_emit<T, G, false>(buf_ptr(r), loc, len, b.state == 1, b);
         }
         if (t2 >= 0) copy_out(fld(f2), (j - 2) & 3);
         t2 = t1;
@@ -569,6 +618,8 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
         __syncthreads();   // s_base is free again
         if (warp == 0) {
             win_issue(fld(f1), f1, t1, j & 1);
+            cp_async_commit();
+            cp_async_commit();   // (place() leaves the newest group in flight)
             place(fld(f1), f1, t1, (j - 1) & 3, j & 1);
         }
         __syncthreads();

@@ -78,8 +78,30 @@ __device__ __forceinline__ float xsub(float a, float b) { float r = __fsub_rn(a,
 __device__ __forceinline__ float xadd(float a, float b) { float r = __fadd_rn(a, b); return r == r ? r : nan_rule(a, b); }
 __device__ __forceinline__ float xmul(float a, float b) { float r = __fmul_rn(a, b); return r == r ? r : nan_rule(a, b); }
 __device__ __forceinline__ float xdiv(float a, float b) { float r = __fdiv_rn(a, b); return r == r ? r : nan_rule(a, b); }
-__device__ __forceinline__ double xsub(double a, double b) { double r = __dsub_rn(a, b); return r == r ? r : nan_rule(a, b); }
-__device__ __forceinline__ double xadd(double a, double b) { double r = __dadd_rn(a, b); return r == r ? r : nan_rule(a, b); }
+// The FP64 pipe of this GPU retires two lanes a clock on an SM (a warp
+// instruction holds it for 16 clocks), 1/32 of what the integer pipe does, so
+// double code spends it on the additions alone: tests, halving and conversions
+// work on the bit pattern, with the plain operation for the rare patterns
+// (infinities, NaNs, subnormals) they leave out.
+__device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)((unsigned long long)__double_as_longlong(v) >> 32); }
+__device__ __forceinline__ uint32_t lo32(double v) { return (uint32_t)(unsigned long long)__double_as_longlong(v); }
+__device__ __forceinline__ double from_hi_lo(uint32_t hi, uint32_t lo) {
+    return __longlong_as_double((long long)(((unsigned long long)hi << 32) | lo));
+}
+__device__ __forceinline__ bool inf_or_nan(double v) { return (hi32(v) & 0x7FF00000u) == 0x7FF00000u; }
+__device__ __forceinline__ bool inf_or_nan(float v) { return (__float_as_uint(v) & 0x7F800000u) == 0x7F800000u; }
+__device__ __forceinline__ bool is_zero(double v) { return ((hi32(v) << 1) | lo32(v)) == 0u; }
+__device__ __forceinline__ bool is_zero(float v) { return v == 0.0f; }
+__device__ __forceinline__ double xsub(double a, double b) {
+    const double r = __dsub_rn(a, b);
+    if (!inf_or_nan(r)) return r;
+    return r == r ? r : nan_rule(a, b);
+}
+__device__ __forceinline__ double xadd(double a, double b) {
+    const double r = __dadd_rn(a, b);
+    if (!inf_or_nan(r)) return r;
+    return r == r ? r : nan_rule(a, b);
+}
 __device__ __forceinline__ double xmul(double a, double b) { double r = __dmul_rn(a, b); return r == r ? r : nan_rule(a, b); }
 __device__ __forceinline__ double xdiv(double a, double b) { double r = __ddiv_rn(a, b); return r == r ? r : nan_rule(a, b); }
 // x / 2 as a multiplication: both are the correctly rounded value of the same
@@ -87,16 +109,31 @@ __device__ __forceinline__ double xdiv(double a, double b) { double r = __ddiv_r
 // way, so the result is bit-identical to the division at a fraction of its
 // cost.
 __device__ __forceinline__ float xhalf(float x) { return xmul(x, 0.5f); }
-__device__ __forceinline__ double xhalf(double x) { return xmul(x, 0.5); }
+// (double: the exponent less one, where both x and the half are normal numbers)
+__device__ __forceinline__ double xhalf(double x) {
+    const uint32_t hi = hi32(x), e = (hi >> 20) & 0x7FFu;
+    if (e - 2u <= 2044u) return from_hi_lo(hi - 0x00100000u, lo32(x));
+    if (is_zero(x)) return x;
+    return xmul(x, 0.5);
+}
 // cvtsd2ss / cvtss2sd
 __device__ __forceinline__ float xd2f(double d) {
+    const uint32_t hi = hi32(d), lo = lo32(d), e = (hi >> 20) & 0x7FFu;
+    if (e - 897u <= 253u) {   // a normal float (or the overflow to infinity that rounding up makes of it)
+        uint32_t u = __funnelshift_l(lo, hi, 3) - 0xC0000000u;       // exponent less 896, the top 23 fraction bits
+        u += ((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (u & 1u)) >> 29;    // to nearest, ties to even
+        return __uint_as_float((u & 0x7FFFFFFFu) | (hi & 0x80000000u));
+    }
+    if (is_zero(d)) return __uint_as_float(hi);
     if (d == d) return __double2float_rn(d);
     unsigned long long b = (unsigned long long)__double_as_longlong(d);
     return __uint_as_float((uint32_t)(b >> 32 & 0x80000000u) | 0x7FC00000u | (uint32_t)(b >> 29 & 0x7FFFFFu));
 }
 __device__ __forceinline__ double xf2d(float f) {
+    const uint32_t b = __float_as_uint(f), e = (b >> 23) & 0xFFu;
+    if (e - 1u <= 253u) return from_hi_lo((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u), b << 29);
+    if ((b << 1) == 0u) return from_hi_lo(b, 0u);
     if (f == f) return (double)f;
-    uint32_t b = __float_as_uint(f);
     return __longlong_as_double((long long)(((unsigned long long)(b & 0x80000000u) << 32) | 0x7FF8000000000000ull |
                                             ((unsigned long long)(b & 0x7FFFFFu) << 29)));
 }
@@ -689,24 +726,43 @@ __device__ __forceinline__ unsigned long long prefix_resolve_win(unsigned long l
     return pa;
 }
 
-// Copy n bytes from a 16-aligned staging buffer (data at offset 0) to global
-// dst of any alignment with the whole CTA: 16-byte aligned stores, the
-// staging words realigned with funnel shifts; byte copies at the ragged ends.
+// One pass of cta_copy_realign for a word phase of WS: 16 destination bytes
+// are words WS .. WS+4 of two 16-byte staging chunks, shifted by rs bits.
+template <int WS>
+__device__ __forceinline__ void copy_realign_chunks(const uint8_t* stg, uint8_t* gbase, uint32_t sh, uint32_t end,
+                                                    uint32_t nch, uint32_t rs) {
+    for (uint32_t c = threadIdx.x; c < nch; c += blockDim.x) {
+        const uint32_t lo = c << 4;
+        if (lo >= sh && lo + 16 <= end) {
+            const uint4* sp = (const uint4*)(stg + ((lo - sh) & ~15u));
+            const uint4 p = sp[0], q = sp[1];
+            const uint32_t a[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+            *(uint4*)(gbase + lo) =
+                make_uint4(__funnelshift_r(a[WS], a[WS + 1], rs), __funnelshift_r(a[WS + 1], a[WS + 2], rs),
+                           __funnelshift_r(a[WS + 2], a[WS + 3], rs), __funnelshift_r(a[WS + 3], a[WS + 4], rs));
+        }
+    }
+}
+
+// Copy n bytes from a 16-aligned staging buffer (data at offset 0, 32 bytes
+// of slack behind it) to global dst of any alignment with the whole CTA:
+// 16-byte aligned stores, the staging bytes realigned with funnel shifts;
+// byte copies at the ragged ends.  The staging side is read as aligned
+// 16-byte chunks (8 shared-memory wavefronts per warp and 512 bytes; five
+// 4-byte reads at a 16-byte stride take 20): the phase between the two sides
+// is the same for every chunk, so its word part is a branch of the whole CTA.
 __device__ __forceinline__ void cta_copy_realign(const uint8_t* stg, uint32_t n, uint8_t* dst) {
     if (n == 0) return;
     const uint32_t sh = (uint32_t)((uintptr_t)dst & 15);
     uint8_t* gbase = dst - sh;
     const uint32_t end = sh + n, nch = (end + 15) >> 4;
-    const uint32_t* sw = (const uint32_t*)stg;
-    const uint32_t rs = ((16u - sh) & 3u) * 8u;   // byte phase of staging vs. destination words
-    for (uint32_t c = threadIdx.x; c < nch; c += blockDim.x) {
-        const uint32_t lo = c << 4;
-        if (lo >= sh && lo + 16 <= end) {
-            const uint32_t so = lo - sh, w = so >> 2;
-            const uint32_t a0 = sw[w], a1 = sw[w + 1], a2 = sw[w + 2], a3 = sw[w + 3], a4 = sw[w + 4];
-            *(uint4*)(gbase + lo) = make_uint4(__funnelshift_r(a0, a1, rs), __funnelshift_r(a1, a2, rs),
-                                               __funnelshift_r(a2, a3, rs), __funnelshift_r(a3, a4, rs));
-        }
+    const uint32_t ph = (16u - sh) & 15u;   // byte phase of staging chunks vs. destination chunks
+    const uint32_t rs = (ph & 3u) * 8u;
+    switch (ph >> 2) {
+        case 0: copy_realign_chunks<0>(stg, gbase, sh, end, nch, rs); break;
+        case 1: copy_realign_chunks<1>(stg, gbase, sh, end, nch, rs); break;
+        case 2: copy_realign_chunks<2>(stg, gbase, sh, end, nch, rs); break;
+        default: copy_realign_chunks<3>(stg, gbase, sh, end, nch, rs); break;
     }
     if (threadIdx.x < 32) {
         const uint32_t last = nch - 1;
@@ -721,6 +777,10 @@ __device__ __forceinline__ void cta_copy_realign(const uint8_t* stg, uint32_t n,
 // do not queue behind the TMA unit's bulk copies), L2 only.
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
+}
+template <int BYTES>   // 4 or 8, for data that is not 16-byte aligned
+__device__ __forceinline__ void cp_async_small(void* smem, const void* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(smem)), "l"(gmem), "n"(BYTES) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }

@@ -44,6 +44,53 @@ struct Chunks {
     static __device__ __forceinline__ int first(int sl, int k) { return 4 * (sl + k * G); }
 };
 
+// Run layout: lane sl owns the E consecutive values from E*sl on (64 bytes).
+template <typename T, int G>
+struct Runs {
+    static constexpr int E = EncCfg<T>::E;
+    static __device__ __forceinline__ int first(int sl, int k) { return E * sl + 4 * k; }
+};
+
+// Tiles of values in shared memory hold their 16-byte chunks swizzled: chunk c
+// lies at chunk c ^ ((c >> 3) & 3), so that the eight lanes of a quarter warp
+// that read one chunk each of eight consecutive 64-byte runs touch all 32
+// banks (unswizzled, such a read is 4-way conflicted).
+__device__ __forceinline__ uint32_t swz16(uint32_t c) { return c ^ ((c >> 3) & 3u); }
+// byte offset of value i in a swizzled tile
+template <typename T>
+__device__ __forceinline__ uint32_t swz_off(uint32_t i) {
+    constexpr uint32_t VN = 16 / sizeof(T);
+    return swz16(i / VN) * 16 + (i % VN) * (uint32_t)sizeof(T);
+}
+
+// A lane's run of the block that starts at value e0 of a swizzled tile.  vec:
+// blocks start on 16-byte boundaries.  Values past the block's end are what
+// lies there (the caller masks them); the reads stay inside a tile of
+// G*E-value blocks.
+template <typename T, int G>
+__device__ __forceinline__ void load_run(const uint8_t* tile, uint32_t e0, bool vec, T (&v)[EncCfg<T>::E]) {
+    constexpr int E = EncCfg<T>::E;
+    constexpr uint32_t VN = 16 / sizeof(T);
+    const uint32_t f = e0 + E * (lane_id() & (G - 1));
+    if (vec) {
+        const uint32_t c0 = f / VN;
+#pragma unroll
+        for (uint32_t j = 0; j < E / VN; j++) {
+            const uint8_t* p = tile + swz16(c0 + j) * 16;
+            if constexpr (sizeof(T) == 4) {
+                const float4 q = *(const float4*)p;
+                v[4 * j] = q.x; v[4 * j + 1] = q.y; v[4 * j + 2] = q.z; v[4 * j + 3] = q.w;
+            } else {
+                const double2 q = *(const double2*)p;
+                v[2 * j] = q.x; v[2 * j + 1] = q.y;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < E; e++) v[e] = *(const T*)(tile + swz_off<T>(f + e));
+    }
+}
+
 template <typename T, int G>
 __device__ __forceinline__ void load_chunks(const T* xs, int len, bool vec, T (&v)[EncCfg<T>::E]) {
     using C = Chunks<T, G>;
@@ -110,10 +157,10 @@ __device__ __forceinline__ uint32_t low_bytes_mask(int n) {
 // (szx/src/szx_float.cc:322-345): the first value reaching an extreme wins,
 // NaNs are skipped unless the block's first value is NaN.  `special` is set
 // (segment-uniform) when the block holds a NaN or an infinity, where the
-// x86 NaN rules of the subtraction matter.
-template <typename T, int G, bool FULL>
+// x86 NaN rules of the subtraction matter.  C: the lanes' layout (Chunks or
+// Runs).
+template <typename T, int G, bool FULL, typename C = Chunks<T, G>>
 __device__ __forceinline__ void seg_minmax(const T (&v)[EncCfg<T>::E], int len, T& mn, T& mx, bool& special) {
-    using C = Chunks<T, G>;
     constexpr int E = C::E;
     const int sl = (int)(lane_id() & (G - 1));
     if constexpr (sizeof(T) == 4) {
@@ -147,6 +194,44 @@ __device__ __forceinline__ void seg_minmax(const T (&v)[EncCfg<T>::E], int len, 
         const unsigned segmask = G == 32 ? 0xffffffffu : (((1u << G) - 1) << seg0);
         special = (__ballot_sync(0xffffffffu, isnan(hn)) & segmask) != 0 || isinf(lo) || isinf(hi);
     } else {
+        // Order-preserving integer keys, high words first: the extremes of
+        // the 32-bit high keys, then of the low words beside them -- 32-bit
+        // operations throughout, about half of what 64-bit keys cost.  Any
+        // infinity or NaN shows in the high extremes.
+        auto key_hi = [](uint32_t h) { return (int)(h ^ ((uint32_t)((int)h >> 31) & 0x7FFFFFFFu)); };
+        int khn = 0x7FFFFFFF, khx = (int)0x80000000;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int k = key_hi(hi32(v[e]));
+            const bool in = FULL || C::first(sl, e / 4) + (e & 3) < len;
+            khn = in ? min(khn, k) : khn;
+            khx = in ? max(khx, k) : khx;
+        }
+#pragma unroll
+        for (int d = G / 2; d > 0; d >>= 1) {
+            khn = min(khn, __shfl_xor_sync(0xffffffffu, khn, d, G));
+            khx = max(khx, __shfl_xor_sync(0xffffffffu, khx, d, G));
+        }
+        const bool odd = khx >= 0x7FF00000 || khn <= (int)0x800FFFFF;
+        if (!__any_sync(0xffffffffu, odd)) {
+            uint32_t kln = 0xFFFFFFFFu, klx = 0u;
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const uint32_t h = hi32(v[e]), l = lo32(v[e]) ^ (uint32_t)((int)h >> 31);
+                const int k = key_hi(h);
+                const bool in = FULL || C::first(sl, e / 4) + (e & 3) < len;
+                if (in && k == khn) kln = min(kln, l);
+                if (in && k == khx) klx = max(klx, l);
+            }
+#pragma unroll
+            for (int d = G / 2; d > 0; d >>= 1) {
+                kln = min(kln, __shfl_xor_sync(0xffffffffu, kln, d, G));
+                klx = max(klx, __shfl_xor_sync(0xffffffffu, klx, d, G));
+            }
+            mn = from_hi_lo((uint32_t)key_hi((uint32_t)khn), kln ^ (uint32_t)(khn >> 31));
+            mx = from_hi_lo((uint32_t)key_hi((uint32_t)khx), klx ^ (uint32_t)(khx >> 31));
+            special = false;
+        } else {
         long long lo = 0x7FFFFFFFFFFFFFFFll, hi = (long long)0x8000000000000000ull;
         bool nan = false;
 #pragma unroll
@@ -177,16 +262,17 @@ __device__ __forceinline__ void seg_minmax(const T (&v)[EncCfg<T>::E], int len, 
         const unsigned seg0 = lane_id() & ~(unsigned)(G - 1);
         const unsigned segmask = G == 32 ? 0xffffffffu : (((1u << G) - 1) << seg0);
         special = (nm & segmask) != 0 || isinf(mn) || isinf(mx);
+        }
     }
     // a zero extreme takes the sign of the block's first zero; only warps
     // that met one pay for the search
-    if (__any_sync(0xffffffffu, mn == (T)0 || mx == (T)0)) {
+    if (__any_sync(0xffffffffu, is_zero(mn) || is_zero(mx))) {
         int zi = 1 << 30;
         T zv = 0;
 #pragma unroll
         for (int e = E - 1; e >= 0; e--) {
             const int idx = C::first(sl, e / 4) + (e & 3);
-            if ((FULL || idx < len) && v[e] == (T)0 && idx < zi) { zi = idx; zv = v[e]; }
+            if ((FULL || idx < len) && is_zero(v[e]) && idx < zi) { zi = idx; zv = v[e]; }
         }
         int best = zi;
 #pragma unroll
@@ -197,8 +283,8 @@ __device__ __forceinline__ void seg_minmax(const T (&v)[EncCfg<T>::E], int len, 
         const unsigned mm = m & segmask;
         const T first = __shfl_sync(0xffffffffu, zv, mm ? __ffs(mm) - 1 : (int)seg0);
         if (mm) {
-            if (mn == (T)0) mn = first;
-            if (mx == (T)0) mx = first;
+            if (is_zero(mn)) mn = first;
+            if (is_zero(mx)) mx = first;
         }
     }
     // a NaN first value pins both extremes; only a block holding a NaN can have one
