@@ -78,6 +78,159 @@ struct EncArgs {
     int* err;
 };
 
+// A double block is constant when radius <= (double)eb.  The radius is a
+// non-negative number or a NaN, so the test is one on unsigned bit patterns:
+// pattern < eb_key, with key 0 (never) for negative and NaN bounds; a NaN's
+// pattern of either sign is above every bound's.
+__device__ __forceinline__ unsigned long long eb_key_of(float eb) {
+    if (!(eb >= 0.0f)) return 0ull;
+    return (unsigned long long)__double_as_longlong(xf2d(fabsf(eb))) + 1ull;
+}
+
+// Extremes of a lane's block, for blocks without infinities, NaNs and (beside
+// a zero extreme) negative zeros; true where the block has one of these and
+// the exact rules below decide.
+template <typename T, int G, bool FULL>
+__device__ __forceinline__ bool enc_minmax_fast(const T (&v)[EncCfg<T>::E], int len, T& mn, T& mx) {
+    constexpr int E = EncCfg<T>::E;
+    const int f = E * (int)(lane_id() & (G - 1));
+    bool odd;
+    if constexpr (sizeof(T) == 4) {
+        // (three-input forms where whole runs are compared; hn: NaN if any value is one)
+        float lo = __builtin_huge_valf(), hi = -__builtin_huge_valf(), hn = -__builtin_huge_valf();
+        if constexpr (FULL) {
+#pragma unroll
+            for (int e = 0; e < E; e += 2) {
+                lo = fmin3(lo, v[e], v[e + 1]);
+                hi = fmax3(hi, v[e], v[e + 1]);
+                hn = fmax3_nan(hn, v[e], v[e + 1]);
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                if (f + e < len) {
+                    lo = fminf(lo, v[e]);
+                    hi = fmaxf(hi, v[e]);
+                    hn = fmax_nan(hn, v[e]);
+                }
+            }
+        }
+        odd = isnan(hn);
+#pragma unroll
+        for (int d = G / 2; d > 0; d >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, d, G));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, d, G));
+        }
+        mn = lo;
+        mx = hi;
+        odd = odd || (len > 0 && (inf_or_nan(lo) || inf_or_nan(hi)));
+    } else {
+        // Order-preserving integer keys, high words first: the extremes of
+        // the 32-bit high keys, then of the low words beside them -- 32-bit
+        // operations throughout, about half of what 64-bit keys cost.  Any
+        // infinity or NaN shows in the high extremes.
+        int khn = 0x7FFFFFFF, khx = (int)0x80000000;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int k = dkey_hi(hi32(v[e]));
+            const bool in = FULL || f + e < len;
+            khn = in ? min(khn, k) : khn;
+            khx = in ? max(khx, k) : khx;
+        }
+#pragma unroll
+        for (int d = G / 2; d > 0; d >>= 1) {
+            khn = min(khn, __shfl_xor_sync(0xffffffffu, khn, d, G));
+            khx = max(khx, __shfl_xor_sync(0xffffffffu, khx, d, G));
+        }
+        odd = khx >= 0x7FF00000 || khn <= (int)0x800FFFFF;
+        uint32_t kln = 0xFFFFFFFFu, klx = 0u;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const uint32_t h = hi32(v[e]), l = lo32(v[e]) ^ (uint32_t)((int)h >> 31);
+            const int k = dkey_hi(h);
+            const bool in = FULL || f + e < len;
+            if (in && k == khn) kln = min(kln, l);
+            if (in && k == khx) klx = max(klx, l);
+        }
+#pragma unroll
+        for (int d = G / 2; d > 0; d >>= 1) {
+            kln = min(kln, __shfl_xor_sync(0xffffffffu, kln, d, G));
+            klx = max(klx, __shfl_xor_sync(0xffffffffu, klx, d, G));
+        }
+        mn = from_hi_lo((uint32_t)dkey_hi((uint32_t)khn), kln ^ (uint32_t)(khn >> 31));
+        mx = from_hi_lo((uint32_t)dkey_hi((uint32_t)khx), klx ^ (uint32_t)(khx >> 31));
+    }
+    // a zero extreme has the sign of the block's first zero: plus, unless there is a negative one
+    if (__any_sync(0xffffffffu, is_zero(mn) || is_zero(mx))) {
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            if constexpr (sizeof(T) == 4) odd = odd || __float_as_uint(v[e]) == 0x80000000u;
+            else odd = odd || (hi32(v[e]) == 0x80000000u && lo32(v[e]) == 0u);
+        }
+    }
+    return odd;
+}
+
+// The same with every rule of the reference's sequential scan
+// (szx/src/szx_float.cc:322-345), for the warps that met an odd value: NaNs
+// are skipped unless the block's first value is one, a zero extreme has the
+// sign of the first zero.  Values come from shared memory again, one at a
+// time: this is the rare path, and small code beside the encoder's loop
+// matters more than its speed.  Returns whether the block holds a NaN or an
+// infinity.
+template <typename T, int G>
+__device__ __forceinline__ bool enc_minmax_exact(const uint8_t* tile, uint32_t e0, int len, T& mn, T& mx) {
+    using U = typename Elem<T>::U;
+    using K = typename std::make_signed<U>::type;   // order-preserving key of a non-NaN pattern
+    constexpr int E = EncCfg<T>::E;
+    constexpr int B = 8 * (int)sizeof(T) - 1;
+    constexpr U MAG = (U)~(U)0 >> 1;
+    const U inf = Elem<T>::bits((T)__builtin_huge_val());
+    const int f = E * (int)(lane_id() & (G - 1));
+    auto key = [](U u) { return (K)(u ^ ((U)((K)u >> B) & MAG)); };
+    K lo = (K)MAG, hi = (K)~MAG;
+    int zi = 1 << 30;   // 2 * index + sign of the first zero
+    bool nan = false;
+#pragma unroll 1
+    for (int i = f; i < f + E && i < len; i++) {
+        const U u = *(const U*)(tile + swz_off<T>(e0 + i)), m = u & MAG;
+        if (m > inf) { nan = true; continue; }
+        lo = min(lo, key(u));
+        hi = max(hi, key(u));
+        if (m == 0) zi = min(zi, 2 * i + (int)(u >> B));
+    }
+#pragma unroll 1
+    for (int d = G / 2; d > 0; d >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, d, G));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, d, G));
+        zi = min(zi, __shfl_xor_sync(0xffffffffu, zi, d, G));
+        nan = __shfl_xor_sync(0xffffffffu, (int)nan, d, G) || nan;
+    }
+    U ulo = (U)lo ^ ((U)(lo >> B) & MAG), uhi = (U)hi ^ ((U)(hi >> B) & MAG);
+    const U zero = (U)(zi & 1) << B;
+    if ((ulo & MAG) == 0) ulo = zero;
+    if ((uhi & MAG) == 0) uhi = zero;
+    if (len > 0) {
+        const U u = *(const U*)(tile + swz_off<T>(e0));
+        if ((u & MAG) > inf) ulo = uhi = u;
+    }
+    mn = Elem<T>::of(ulo);
+    mx = Elem<T>::of(uhi);
+    return nan || (ulo & MAG) >= inf || (uhi & MAG) >= inf;
+}
+// A run's differences from the median under the x86 NaN rules, in place.
+template <typename T, int G>
+__device__ __forceinline__ void enc_diff_exact(uint8_t* tile, uint32_t e0, int len, T med) {
+    constexpr int E = EncCfg<T>::E;
+    const int f = E * (int)(lane_id() & (G - 1));
+#pragma unroll 1
+    for (int i = f; i < f + E && i < len; i++) {
+        T* p = (T*)(tile + swz_off<T>(e0 + i));
+        *p = xsub(*p, med);
+    }
+    __syncwarp();
+}
+
 // Statistics pass of one block by a G-lane segment: state, reqLength and
 // median (szx/src/szx_float.cc:314-371), the shifted words, lead codes
 // (szx/src/szx_float.cc:94-113) and stored-byte counts, all kept in registers.
@@ -85,7 +238,7 @@ struct EncArgs {
 // eb_key: the bound's rule for double radii (constant when the radius's bit
 // pattern, as an unsigned number, is below it; see eb_key_of).
 template <typename T, int G, bool FULL>
-__device__ __forceinline__ void enc_block_stats(const uint8_t* tile, uint32_t e0, int len, bool vec, float eb,
+__device__ __forceinline__ void enc_block_stats(uint8_t* tile, uint32_t e0, int len, bool vec, float eb,
                                                 int eb_exp, unsigned long long eb_key, int omp_stats,
                                                 BlockEnc<T, G>& b) {
     using EL = Elem<T>;
@@ -95,10 +248,11 @@ __device__ __forceinline__ void enc_block_stats(const uint8_t* tile, uint32_t e0
     constexpr int NC = E / 4;
     const int sl = (int)(lane_id() & (G - 1));
     T v[E];
-    load_run<T, G>(tile, e0, vec, v);
+    if constexpr (FULL) load_run_full<T>(smem_u32(tile), e0 / E + sl, v);
+    else load_run<T, G>(tile, e0, vec, v);
     T mn, mx;
-    bool special;
-    seg_minmax<T, G, FULL, Runs<T, G>>(v, len, mn, mx, special);
+    bool special = enc_minmax_fast<T, G, FULL>(v, len, mn, mx);
+    if (__any_sync(0xffffffffu, special)) special = enc_minmax_exact<T, G>(tile, e0, len, mn, mx);
     int state;
     float radius_f, median_f;
     if constexpr (sizeof(T) == 4) {
@@ -132,33 +286,36 @@ __device__ __forceinline__ void enc_block_stats(const uint8_t* tile, uint32_t e0
     // differences from the median (szx/src/szx_float.cc:88-92); x86 NaN rules only where a NaN can arise
     U d[E];
     if (__any_sync(0xffffffffu, special)) {
+        enc_diff_exact<T, G>(tile, e0, len, med);
+        load_run<T, G>(tile, e0, vec, v);
 #pragma unroll
-        for (int e = 0; e < E; e++) d[e] = EL::bits(xsub(v[e], med));
+        for (int e = 0; e < E; e++) d[e] = EL::bits(v[e]);
     } else {
-#pragma unroll
-        for (int e = 0; e < E; e++) d[e] = EL::bits(EL::sub(v[e], med));
+        sub_run(v, med, d);
     }
     // Lead codes: leading identical bytes of the words shifted right by s with
     // the previous value's, capped at 3 -- (leading zeros of the XOR + s) / 8,
     // with a guard bit that ends the count at 24 - s.  Only the top 32 bits
-    // decide; four counts are packed in a word before the division.
+    // decide; four leading-bit positions (31 - zeros) are packed in a word,
+    // by multiplications the idle FMA pipe takes, before the division.
     auto top = [](U u) { return (uint32_t)(u >> (8 * W - 32)); };
     uint32_t prev = __shfl_up_sync(0xffffffffu, top(d[E - 1]), 1, G);
     if (sl == 0) prev = 0u;   // zero before the block
-    const uint32_t guard = 0x80u << s, s4 = (uint32_t)s * 0x01010101u;
+    const uint32_t guard = 0x80u << s, s4 = (uint32_t)(31 + s) * 0x01010101u;
     uint32_t codes = 0, mine = 0;
 #pragma unroll
     for (int k = 0; k < NC; k++) {
-        uint32_t lz[4];
+        uint32_t lb[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const uint32_t h = top(d[4 * k + i]);
-            lz[i] = (uint32_t)__clz((h ^ prev) | guard);
+            asm("bfind.u32 %0, %1;" : "=r"(lb[i]) : "r"((h ^ prev) | guard));
             prev = h;
         }
-        const uint32_t p = __byte_perm(__byte_perm(lz[0], lz[1], 0x0040), __byte_perm(lz[2], lz[3], 0x0040), 0x5410);
-        uint32_t ldb = ((p + s4) >> 3) & 0x03030303u;
-        uint32_t cnt4 = stored_counts(R, ldb);   // max(R - lead, 0) per value
+        const uint32_t p = (lb[3] * 256u + lb[2]) * 65536u + (lb[1] * 256u + lb[0]);
+        uint32_t ldb = ((s4 - p) >> 3) & 0x03030303u;
+        // max(R - lead, 0) per value; R is at least 2 here, so only lead 3 at R = 2 needs raising
+        uint32_t cnt4 = (uint32_t)R * 0x01010101u + (R == 2 ? (ldb >> 1) & ldb & 0x01010101u : 0u) - ldb;
         if constexpr (!FULL) {
             const uint32_t m = low_bytes_mask(len - (E * sl + 4 * k));
             ldb &= m;
@@ -182,37 +339,6 @@ __device__ __forceinline__ void enc_block_stats(const uint8_t* tile, uint32_t e0
     b.med_bits = state == 1 ? payload_med : __float_as_uint(median_f);
 }
 
-// A double block is constant when radius <= (double)eb.  The radius is a
-// non-negative number or a NaN, so the test is one on unsigned bit patterns:
-// pattern < eb_key, with key 0 (never) for negative and NaN bounds; a NaN's
-// pattern of either sign is above every bound's.
-__device__ __forceinline__ unsigned long long eb_key_of(float eb) {
-    if (!(eb >= 0.0f)) return 0ull;
-    return (unsigned long long)__double_as_longlong(xf2d(fabsf(eb))) + 1ull;
-}
-
-// Byte-wise appending to a payload in shared memory.  A lane appends its
-// run's values one after the other: `last` holds the four bytes written last
-// (the newest on top), so the word that a value completes is a funnel shift of
-// (last, value) by the position's bit offset and the next `last` one by the
-// value's bits -- no masks, no byte stores, and whole words leave with one
-// predicated store each.  The first word a lane completes carries stale
-// bytes below the run's start; what belongs there (the lane before's last
-// bytes, or the block's lead codes) is stored after it, bytewise.
-struct RunOut {
-    uint32_t last, q8, sp;   // last four bytes, bit position, shared address of the word being filled
-    __device__ __forceinline__ void append(uint32_t v, uint32_t n8) {   // the low n8 / 8 (0..4) bytes of v
-        const uint32_t w = __funnelshift_l(last, v, q8);
-        last = __funnelshift_rc(last, v, n8);
-        const uint32_t q = q8 + n8;
-        if ((q ^ q8) & ~31u) {
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(sp), "r"(w) : "memory");
-            sp += 4;
-        }
-        q8 = q;
-    }
-};
-
 // Emission of the coded blocks of a warp (act: this segment has one) into the
 // tile's staging buffer: every lane's whole words, then headers, lead bytes
 // and the bytes of the words that lanes share.  Every byte of a block's
@@ -228,9 +354,7 @@ __device__ __forceinline__ void enc_block_emit(uint8_t* stg, uint32_t loc, int l
     const int Lb = FULL ? G * NC : (len + 3) / 4;
     const uint32_t q0 = loc + 5 + (uint32_t)Lb + b.excl;
     RunOut o;
-    o.last = 0;
-    o.q8 = 8 * q0;
-    o.sp = smem_u32(stg) + (q0 & ~3u);
+    o.start(stg, q0);
     if (act) {
 #pragma unroll
         for (int k = 0; k < NC; k++) {
@@ -249,12 +373,7 @@ __device__ __forceinline__ void enc_block_emit(uint8_t* stg, uint32_t loc, int l
     }
     __syncwarp();
     if (act) {
-        // the last, partial word: its bytes from the run's start (if that lies in it) to the run's end
-        const uint32_t w = __funnelshift_l(o.last, 0u, o.q8);
-        const uint32_t end = (o.q8 >> 3) & 3u, beg = (o.sp ^ smem_u32(stg + q0)) < 4u ? q0 & 3u : 0u;
-#pragma unroll
-        for (uint32_t j = 0; j < 3; j++)
-            if (j >= beg && j < end) asm volatile("st.shared.u8 [%0], %1;" ::"r"(o.sp + j), "r"(w >> (8 * j)) : "memory");
+        o.finish(stg, q0);
         uint8_t* p = stg + loc;
         // lead codes: 4 per byte, MSB first (szx/src/szx_TypeManager.cc:198-273)
 #pragma unroll
@@ -268,6 +387,15 @@ __device__ __forceinline__ void enc_block_emit(uint8_t* stg, uint32_t loc, int l
             p[4] = (uint8_t)b.med_bits;
         }
     }
+}
+
+// Lane-predicated claim of the next tile: the reply is waited for where `next`
+// is used, not at the end of a branch.
+__device__ __forceinline__ void claim_tile(unsigned long long& next, unsigned long long* ctr, bool take) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p atom.relaxed.gpu.global.add.u64 %0, [%1], 1;\n\t}"
+                 : "+l"(next)
+                 : "l"(ctr), "r"((uint32_t)take)
+                 : "memory");
 }
 
 template <typename T, int G, int TBYTES = kEncTileBytes>
@@ -284,14 +412,15 @@ struct EncTile {
     static constexpr int kIn = kBlocks * kBsMax * (int)sizeof(T);      // input bytes per buffer
     static constexpr int kMaxPay = 5 + (kBsMax + 3) / 4 + (int)sizeof(T) * kBsMax;
     // payloads of a tile + slack for the word-wise reads of the realigning copy
-    static constexpr int kStage = ((kBlocks * kMaxPay + 32 + 15) / 16) * 16;
+    // (a multiple of 64: a run's address is swizzled by exclusive-or)
+    static constexpr int kStage = ((kBlocks * kMaxPay + 32 + 63) / 64) * 64;
     // a ring buffer holds a tile's input, then (in place) its payloads
     static constexpr int kBuf = kIn > kStage ? kIn : kStage;
     static constexpr int kDynSmem = 4 * kBuf;
     static_assert(kGroups <= 8 && kBlocks % kBpw == 0, "one block group per warp");
     static_assert(kBlocks <= 64, "a tile's sizes are scanned as two warp-wide halves");
-    static_assert(kBlocks * kMaxPay < 65535, "a tile's byte count + 1 fits the 16-bit aggregate words");
-    static_assert(kIn % 512 == 0 && kBuf % 16 == 0, "swizzled chunks stay inside the tile, buffers 16-byte aligned");
+    static_assert(kBlocks * kMaxPay < 32767, "a tile's byte count + 1 fits 15 bits of the aggregate words");
+    static_assert(kIn % 512 == 0 && kBuf % 64 == 0, "swizzled chunks stay inside the tile, runs on 64-byte boundaries");
     static_assert(kThreads % 32 == 0, "a thread's chunks keep one swizzle phase");
 };
 
@@ -320,30 +449,30 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     constexpr int BPW = TL::kBpw;
     constexpr int NGRP = TB / BPW;
     extern __shared__ __align__(128) uint8_t dsm[];
-    __shared__ __align__(16) uint16_t s_w16[2][kLbWin + 8];   // look-back windows (16-bit aggregates)
-    __shared__ long long s_an_t, s_wlo[2];                     // placement anchor tile; window first tiles
-    __shared__ unsigned long long s_an_incl;                   // the anchor's inclusive prefix
-    __shared__ int s_an_f, s_wok[2];                           // its field; window states
-    __shared__ uint32_t s_size[4][TB], s_med[4][TB];
-    __shared__ uint8_t s_state[4][TB];
+    __shared__ __align__(16) uint16_t s_w16[kLbWin + 8];   // look-back window (16-bit aggregates)
+    __shared__ int s_an_t, s_wlo;                          // placement anchor tile; window's first tile
+    __shared__ unsigned long long s_an_incl;               // the anchor's inclusive prefix
+    __shared__ int s_an_f, s_wok;                          // its field; window state
+    __shared__ uint32_t s_size[TB], s_med[TB];
+    __shared__ uint8_t s_state[TB];
     __shared__ uint32_t s_agg[4];
-    __shared__ long long s_tile[4];     // launch-wide tile index of each ring position
+    __shared__ int s_tile[4];           // launch-wide tile index of each ring position (-1: none left)
     __shared__ int s_fld[4];            // its field
-    __shared__ unsigned long long s_base;
-    __shared__ int s_skip;
+    __shared__ unsigned long long s_base[2];
+    __shared__ int s_skip[2];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int seg = lane / G, sl = lane & (G - 1);
-    const long long nt = (long long)a.total_tiles;
-    const unsigned long long tile_elems = (unsigned long long)TB * a.bs;
+    const uint32_t tile_elems = (uint32_t)(TB * a.bs);
     const bool vec = ((a.bs * (int)sizeof(T)) & 15) == 0;   // every block starts 16-byte aligned
     // field of a launch-wide tile: one load from the plan's tile map
-    auto field_of = [&](long long g) { return (int)a.tile_field[g]; };
+    auto field_of = [&](int g) { return (int)a.tile_field[g]; };
     auto buf_ptr = [&](int r) { return dsm + r * TL::kBuf; };
     if (threadIdx.x == 0) {
         for (int r = 0; r < 2; r++) {
-            s_tile[r] = (long long)atomicAdd(a.tile_ctr, 1ull);
-            s_fld[r] = (MULTI && s_tile[r] < nt) ? field_of(s_tile[r]) : 0;
+            const unsigned long long g = atomicAdd(a.tile_ctr, 1ull);
+            s_tile[r] = g < a.total_tiles ? (int)g : -1;
+            s_fld[r] = (MULTI && s_tile[r] >= 0) ? field_of(s_tile[r]) : 0;
         }
     }
     __syncthreads();
@@ -351,29 +480,31 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     auto fld = [&](int f) -> const BlkField* { return MULTI ? a.fields + f : nullptr; };
 #define FV(F_, m) (MULTI ? (F_)->m : a.one.m)
 
-    auto tile_count = [&](const BlkField* F, long long t) {
-        const unsigned long long start = (unsigned long long)t * tile_elems;
-        const unsigned long long rem = FV(F, n) - start;
-        return rem < tile_elems ? rem : tile_elems;
+    auto tile_count = [&](const BlkField* F, int t) {
+        if (t + 1 < (int)FV(F, enc_tiles)) return tile_elems;
+        return (uint32_t)(FV(F, n) - (unsigned long long)t * tile_elems);
     };
     // all threads: the tile's values into ring buffer r, swizzled in 16-byte
     // chunks, by cp.async (one group; completed before the next iteration's
     // first barrier)
-    auto issue = [&](long long g, int f, int r) {
+    auto issue = [&](int g, int f, int r) {
         const BlkField* F = fld(f);
-        const long long t = g - (long long)FV(F, enc_tile0);
-        const uint32_t cnt = (uint32_t)tile_count(F, t);
+        const int t = g - (int)FV(F, enc_tile0);
+        const uint32_t cnt = tile_count(F, t);
         const uint8_t* src = (const uint8_t*)((const T*)FV(F, x) + (unsigned long long)t * tile_elems);
         uint8_t* dst = buf_ptr(r);
         if (((uintptr_t)src & 15) == 0) {
             constexpr uint32_t VN = 16 / sizeof(T);
             const uint32_t nch = cnt / VN;
-            // chunks threadIdx.x + k * kThreads: the swizzle phase is the same for all of them
             const uint8_t* sp = src + 16 * threadIdx.x;
-            uint8_t* dp = dst + 16 * swz16(threadIdx.x);
+            uint8_t* dp = dst + 16 * swz16(threadIdx.x);   // the threads' later chunks share its swizzle phase
+            if (TL::kIn % (16 * TL::kThreads) == 0 && nch == TL::kIn / 16) {   // a whole tile of the largest blocks
 #pragma unroll
-            for (int k = 0; k < (TL::kIn / 16 + TL::kThreads - 1) / TL::kThreads; k++)
-                if (threadIdx.x + k * TL::kThreads < nch) cp_async16(dp + 16 * k * TL::kThreads, sp + 16 * k * TL::kThreads);
+                for (int k = 0; k < TL::kIn / 16 / TL::kThreads; k++)
+                    cp_async16(dp + 16 * k * TL::kThreads, sp + 16 * k * TL::kThreads);
+                return;
+            }
+            for (uint32_t c = threadIdx.x; c < nch; c += TL::kThreads) cp_async16(dst + 16 * swz16(c), src + 16 * c);
             const uint32_t i = nch * VN + threadIdx.x;
             if (i < cnt) cp_async_small<sizeof(T)>(dst + swz_off<T>(i), src + i * sizeof(T));
         } else {
@@ -381,14 +512,14 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
                 cp_async_small<sizeof(T)>(dst + swz_off<T>(i), src + i * sizeof(T));
         }
     };
-    auto block_len = [&](const BlkField* F, long long t, int lb) {
+    auto block_len = [&](const BlkField* F, int t, int lb) {
         const unsigned long long b = (unsigned long long)t * TB + lb;
         if (b >= FV(F, nb)) return 0;
         const unsigned long long rem = FV(F, n) - b * (unsigned long long)a.bs;
         return rem < (unsigned long long)a.bs ? (int)rem : a.bs;
     };
 
-    unsigned long long nnc_cta = 0;   // warp 0 lane 0, single field: non-constant blocks of this CTA's tiles
+    unsigned long long nnc_cta = 0;   // warp kMetaWarp lane 0, single field: non-constant blocks of this CTA's tiles
     // Placement (warp 0).  A tile's offset is the inclusive prefix of this
     // CTA's previous tile (the anchor, known here) plus the aggregates of the
     // tiles claimed between the two, read from the field's 16-bit aggregate
@@ -406,42 +537,40 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     auto agg16_of = [&](const BlkField* F) {
         return (uint16_t*)(FV(F, st_enc) + enc_tile_words(FV(F, nb)));
     };
-    auto win_issue = [&](const BlkField* F, int f, long long t, int buf) {
+    auto win_issue = [&](const BlkField* F, int f, int t) {
         int ok = 0;
-        long long lo = 0;
-        const long long an_t = s_an_t;
+        int lo = 0;
+        const int an_t = s_an_t;
         if (t > 0 && an_t >= 0 && s_an_f == f && an_t < t && t - an_t - 1 <= kLbWin) {
             if (t - an_t == 1) {
                 ok = 2;
             } else {
-                lo = (an_t + 1) & ~7ll;
-                const int units = (int)((t - lo + 7) >> 3);
+                lo = (an_t + 1) & ~7;
+                const int units = (t - lo + 7) >> 3;
                 const uint16_t* src = agg16_of(F) + lo;
-                for (int u = lane; u < units; u += 32) cp_async16(&s_w16[buf][8 * u], src + 8 * u);
+                for (int u = lane; u < units; u += 32) cp_async16(&s_w16[8 * u], src + 8 * u);
                 ok = 1;
             }
         }
         if (lane == 0) {
-            s_wlo[buf] = lo;
-            s_wok[buf] = ok;
+            s_wlo = lo;
+            s_wok = ok;
         }
         __syncwarp();
     };
-    // warp 0: tile t of field F (metadata set r) placed at `base`: its sizes /
-    // medians / state bits by block, the capacity check, the field's totals
-    auto meta = [&](const BlkField* F, long long t, int r, unsigned long long base) {
-        const uint32_t agg = s_agg[r];
-        const bool cap_ok = base + agg <= FV(F, payload_cap);
+    // one warp: sizes, medians and state bits of tile t's blocks, by block
+    constexpr int kMetaWarp = TL::kWarps - 2;
+    auto meta = [&](const BlkField* F, int t) {
         const unsigned long long tb0 = (unsigned long long)t * TB;
         uint32_t m01[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int lb = lane + 32 * h;
             const bool in = lb < TB;
-            const int st = in ? s_state[r][lb] : 2;
+            const int st = in ? s_state[lb] : 2;
             if (in && st != 2) {
-                FV(F, size_blk)[tb0 + lb] = (uint16_t)s_size[r][lb];
-                FV(F, med_blk)[tb0 + lb] = s_med[r][lb];
+                FV(F, size_blk)[tb0 + lb] = (uint16_t)s_size[lb];
+                FV(F, med_blk)[tb0 + lb] = s_med[lb];
             }
             m01[h] = __ballot_sync(0xffffffffu, in && st == 1);
         }
@@ -451,75 +580,89 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
             const uint32_t r0 = __brev(m01[0]), r1 = __brev(m01[1]);
 #pragma unroll
             for (int k = 0; k < TB / 8; k++) sbp[k] = (uint8_t)((k < 4 ? r0 : r1) >> (24 - 8 * (k & 3)));
-            if (!cap_ok) atomicExch(a.err, kErrCapacity);
             const unsigned long long k = (unsigned long long)(__popc(m01[0]) + __popc(m01[1]));
             if (!MULTI) nnc_cta += k;
             else if (k) atomicAdd(&FV(F, tot)->nnc, k);
-            if (t == (long long)FV(F, enc_tiles) - 1) FV(F, tot)->payload_bytes = base + agg;
-            s_base = base;
-            s_skip = !cap_ok;
         }
     };
-    // warp 0: place tile t of field f (metadata set r; its window in buffer buf)
-    auto place = [&](const BlkField* F, int f, long long t, int r, int buf) {
+    // warp 0: place tile t of field f, ring position r: its offset in the payload, the capacity check, the field's payload total
+    auto place = [&](const BlkField* F, int f, int t, int r) {
         const uint32_t agg = s_agg[r];
         unsigned long long base = 0;
         if (t > 0) {
-            const int ok = s_wok[buf];
-            const long long lo = s_wlo[buf];
-            const long long an_t = s_an_t;
+            const int ok = s_wok;
+            const int an_t = s_an_t;
             const unsigned long long an_incl = s_an_incl;
             bool placed = false;
             if (ok == 2) {
                 base = an_incl;
                 placed = true;
             } else if (ok == 1) {
-                // (the window's group; the next tile's values, issued after it, stay in flight)
-                cp_async_wait_group<1>();
+                // Sum of the aggregates an_t + 1 .. t - 1, eight to a 16-byte
+                // read (two reads a lane at most) and a redux across the warp;
+                // the words outside that range count as 1, published and empty.
+                const int lo = s_wlo;
+                const int units = (t - lo + 7) >> 3;
+                const int first = an_t + 1 - lo, last = t - lo;
+                cp_async_wait_all();
                 __syncwarp();
-                // a window with aggregates not yet published is copied again
-                // (one round trip each) a few times before the global walk
-                const int units = (int)((t - lo + 7) >> 3);
                 for (int attempt = 0;; attempt++) {
-                    unsigned long long sum = 0;
-                    bool ready = true;
-                    for (long long i = an_t + 1 + lane; i < t; i += 32) {
-                        const uint32_t v = s_w16[buf][i - lo];
-                        ready = ready && v != 0;
-                        sum += v - 1;
+                    uint32_t sum = 0, pub = 0x80008000u;
+                    for (int u = lane; u < units; u += 32) {
+                        const uint4 q = *(const uint4*)&s_w16[8 * u];
+                        uint32_t w[4] = {q.x, q.y, q.z, q.w};
+                        if (u == 0 || u == units - 1) {
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                const int at = 8 * u + i, sh = 16 * (i & 1);
+                                if (at < first || at >= last) w[i >> 1] = (w[i >> 1] & ~(0xFFFFu << sh)) | (1u << sh);
+                            }
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            sum += (w[i] & 0xFFFFu) + (w[i] >> 16);
+                            pub &= w[i] + 0x7FFF7FFFu;   // bit 15 of a half: it is not zero
+                        }
+                        sum -= 8;
                     }
-                    if (__all_sync(0xffffffffu, ready)) {
-                        base = an_incl + warp_sum(sum);
+                    if (__all_sync(0xffffffffu, (pub & 0x80008000u) == 0x80008000u)) {
+                        base = an_incl + __reduce_add_sync(0xffffffffu, sum);
                         placed = true;
                         break;
                     }
+                    // a window with aggregates not yet published is copied again
+                    // (one round trip each) a few times before the global walk
                     if (attempt == kWinRepolls) break;
-                    __nanosleep(128);
+                    __nanosleep(64);
                     const uint32_t* src = (const uint32_t*)(agg16_of(F) + lo);
-                    for (int u = lane; u < units; u += 32) *(uint4*)&s_w16[buf][8 * u] = ld_volatile_v4(src + 4 * u);
+                    __syncwarp();
+                    for (int u = lane; u < units; u += 32) *(uint4*)&s_w16[8 * u] = ld_volatile_v4(src + 4 * u);
                     __syncwarp();
                 }
             }
             if (!placed) base = prefix_resolve(FV(F, st_enc), t, agg, a.err);   // publishes t's inclusive prefix
             else if (lane == 0) st_volatile64(&FV(F, st_enc)[t], kS64Inc | ((base + agg) & kS64Val));
         }
-        meta(F, t, r, base);
         if (lane == 0) {
+            const bool cap_ok = base + agg <= FV(F, payload_cap);
+            if (!cap_ok) atomicExch(a.err, kErrCapacity);
+            if (t == (int)FV(F, enc_tiles) - 1) FV(F, tot)->payload_bytes = base + agg;
+            s_base[r & 1] = base;
+            s_skip[r & 1] = !cap_ok;
             s_an_t = t;
             s_an_f = f;
             s_an_incl = base + agg;
         }
         __syncwarp();
     };
-    auto copy_out = [&](const BlkField* F, int r) {
-        if (!s_skip) cta_copy_realign(buf_ptr(r), s_agg[r], FV(F, payload) + s_base);
+    // threads tid of nthr: the placed tile of ring position r to its place
+    auto copy_out = [&](const BlkField* F, int r, uint32_t tid, uint32_t nthr) {
+        if (!s_skip[r & 1]) cta_copy_realign(buf_ptr(r), s_agg[r], FV(F, payload) + s_base[r & 1], tid, nthr);
     };
 
-    if (s_tile[0] < nt) issue(s_tile[0], s_fld[0], 0);
-    cp_async_commit();
-    cp_async_commit();   // (an empty group in the window's place)
+    if (s_tile[0] >= 0) issue(s_tile[0], s_fld[0], 0);
     const bool taker = warp == TL::kWarps - 1 && lane == 0;
-    long long t1 = -1, t2 = -1;   // T_{j-1}, T_{j-2} (field-local), -1: none
+    int t1 = -1, t2 = -1;         // T_{j-1}, T_{j-2} (field-local), -1: none
     int eb_f = -1, eb_exp = 0;    // field whose bound is loaded, the bound's exponent
     float eb = 0.f;
     unsigned long long eb_key = 0;   // and its key for double radii
@@ -527,31 +670,30 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     int j = 0;
     for (;; j++) {
         const int r = j & 3;
-        cp_async_wait_group<1>();   // T_j's values are in (the window issued after them may still be on its way)
+        // (after the last tile two more iterations place and copy out what is staged)
+        cp_async_wait_all();   // T_j's values are in
         __syncthreads();   // ring position j+1 claimed, copy-out of T_{j-3} done
         {
             const int rn = (j + 1) & 3;
-            const long long gn = s_tile[rn];
-            if (gn < nt) issue(gn, s_fld[rn], rn);
+            const int gn = s_tile[rn];
+            if (gn >= 0) issue(gn, s_fld[rn], rn);
         }
-        cp_async_commit();
-        if (warp == 0 && t2 >= 0) place(fld(f2), f2, t2, (j - 2) & 3, (j - 1) & 1);
-        const long long g = s_tile[r];
-        if (g >= nt) break;
-        const int f = s_fld[r];
+        const int g = s_tile[r];
+        const bool live = g >= 0;
+        if (!live && t1 < 0 && t2 < 0) break;
+        const int f = live ? s_fld[r] : 0;
         const BlkField* F = fld(f);
-        const long long t = g - (long long)FV(F, enc_tile0);
-        // the last warp takes the tile of ring position j+2; the reply is used after the statistics
-        unsigned long long gc = 0;
-        if (taker) gc = atomicAdd(a.tile_ctr, 1ull);
+        const int t = live ? g - (int)FV(F, enc_tile0) : -1;
+        // the last warp takes the tile of ring position j+2; the reply is used at the iteration's end
+        unsigned long long gc = ~0ull;
+        claim_tile(gc, a.tile_ctr, taker && live);
         // ---- statistics of the tile's blocks, one block per segment
         const int lb = warp * BPW + seg;
-        const bool mine = warp < NGRP;
+        const bool mine = live && warp < NGRP;
         // every tile but a field's last holds whole blocks only
-        const bool whole = (unsigned long long)(t + 1) * tile_elems <= FV(F, n);
-        const int len = !mine ? 0 : (whole ? a.bs : block_len(F, t, lb));
+        const int len = !mine ? 0 : (t + 1 < (int)FV(F, enc_tiles) ? a.bs : block_len(F, t, lb));
         const bool full = __all_sync(0xffffffffu, len == TL::kBsMax);
-        if (f != eb_f) {   // the field's bound and its exponent, once per field
+        if (live && f != eb_f) {   // the field's bound and its exponent, once per field
             eb = FV(F, params) ? FV(F, params)->eb : FV(F, eb);
             eb_exp = exponent_f64_of_f32(eb);
             if constexpr (sizeof(T) == 8) eb_key = eb_key_of(eb);
@@ -563,33 +705,27 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
             if (full) enc_block_stats<T, G, true>(buf_ptr(r), e0, len, vec, eb, eb_exp, eb_key, a.omp_stats, b);
             else enc_block_stats<T, G, false>(buf_ptr(r), e0, len, vec, eb, eb_exp, eb_key, a.omp_stats, b);
             if (sl == 0) {
-                s_state[r][lb] = (uint8_t)b.state;
-                s_size[r][lb] = b.state == 1 ? b.size : 0;
-                s_med[r][lb] = b.med_bits;
+                s_state[lb] = (uint8_t)b.state;
+                s_size[lb] = b.state == 1 ? b.size : 0;
+                s_med[lb] = b.med_bits;
             }
         }
-        if (taker) {
-            const int rc = (j + 2) & 3;   // T_{j-2}'s position: its id was read two barriers ago
-            s_tile[rc] = (long long)gc;
-            s_fld[rc] = (MULTI && (long long)gc < nt) ? field_of((long long)gc) : 0;
-        }
-        __syncthreads();   // statistics in (T_j's input is dead), T_{j-2} placed
-        // warp 0: T_{j-1}'s look-back window, in flight until the next iteration
-        if (warp == 0 && t1 >= 0) win_issue(fld(f1), f1, t1, j & 1);
-        cp_async_commit();   // the window's group (empty in the other warps)
+        __syncthreads();   // statistics in (T_j's input is dead)
+        // warp 0: T_{j-1}'s look-back window, in flight during the emission
+        if (warp == 0 && t1 >= 0) win_issue(fld(f1), f1, t1);
         // every warp: the tile's block offsets (two warp-wide halves)
         const bool in0 = lane < TB;
-        const uint32_t sz0 = in0 ? s_size[r][lane] : 0;
+        const uint32_t sz0 = in0 ? s_size[lane] : 0;
         const uint32_t i0 = warp_inclusive_sum(sz0);
         const uint32_t loc_lo = __shfl_sync(0xffffffffu, i0 - sz0, lb & 31);
         uint32_t i1 = i0, loc_hi = 0;   // tiles of up to 32 blocks have no second half
         if constexpr (TB > 32) {
             const bool in1 = lane + 32 < TB;
-            const uint32_t sz1 = in1 ? s_size[r][lane + 32] : 0;
+            const uint32_t sz1 = in1 ? s_size[lane + 32] : 0;
             i1 = warp_inclusive_sum(sz1) + __shfl_sync(0xffffffffu, i0, 31);
             loc_hi = __shfl_sync(0xffffffffu, i1 - sz1, lb & 31);
         }
-        if (warp == 0) {
+        if (live && warp == 0) {
             const uint32_t agg = __shfl_sync(0xffffffffu, i1, 31);
             if (lane == 0) {
                 s_agg[r] = agg;
@@ -602,30 +738,24 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
             if (full) enc_block_emit<T, G, true>(buf_ptr(r), loc, len, b.state == 1, b);
             else enc_block_emit<T, G, false>(buf_ptr(r), loc, len, b.state == 1, b);
         }
-        if (t2 >= 0) copy_out(fld(f2), (j - 2) & 3);
+        // T_{j-2} to its place by all warps but warp 0, which places T_{j-1} meanwhile
+        if (warp == 0) {
+            if (t1 >= 0) place(fld(f1), f1, t1, (j - 1) & 3);
+        } else {
+            if (live && warp == kMetaWarp) meta(F, t);
+            if (t2 >= 0) copy_out(fld(f2), (j - 2) & 3, threadIdx.x - 32, TL::kThreads - 32);
+        }
+        if (taker) {
+            const int rc = (j + 2) & 3;   // T_{j-2}'s position: its id was read two barriers ago
+            s_tile[rc] = gc < a.total_tiles ? (int)gc : -1;
+            s_fld[rc] = (MULTI && gc < a.total_tiles) ? field_of((int)gc) : 0;
+        }
         t2 = t1;
         f2 = f1;
         t1 = t;
         f1 = f;
     }
-    // this CTA's last two tiles: T_{j-2} was placed at the top of the final
-    // iteration, T_{j-1} still needs its window and placement
-    if (t2 >= 0) {
-        __syncthreads();
-        copy_out(fld(f2), (j - 2) & 3);
-    }
-    if (t1 >= 0) {
-        __syncthreads();   // s_base is free again
-        if (warp == 0) {
-            win_issue(fld(f1), f1, t1, j & 1);
-            cp_async_commit();
-            cp_async_commit();   // (place() leaves the newest group in flight)
-            place(fld(f1), f1, t1, (j - 1) & 3, j & 1);
-        }
-        __syncthreads();
-        copy_out(fld(f1), (j - 1) & 3);
-    }
-    if (threadIdx.x == 0 && nnc_cta) atomicAdd(&a.one.tot->nnc, nnc_cta);
+    if (warp == kMetaWarp && lane == 0 && nnc_cta) atomicAdd(&a.one.tot->nnc, nnc_cta);
 #undef FV
 }
 
@@ -866,7 +996,7 @@ cudaError_t launch_blocked_encode_fields(int layout, int dtype, int bs, int nf, 
                                          unsigned long long enc_total, unsigned long long asm_total,
                                          unsigned long long* counters, int* err, cudaStream_t s,
                                          const LaunchShape& shape) {
-    if (nf < 1 || enc_total == 0 || (nf > 1 && !d_tile_field)) return cudaErrorInvalidValue;
+    if (nf < 1 || enc_total == 0 || enc_total > 0x7FFFFFFFull || (nf > 1 && !d_tile_field)) return cudaErrorInvalidValue;
     EncArgs a;
     a.one = one;
     a.fields = d_fields;

@@ -689,7 +689,7 @@ __device__ __forceinline__ unsigned long long prefix_resolve(unsigned long long*
 // or an empty word before it, falls back to the global look-back (which then
 // waits); either way the tile's inclusive value is published and its
 // exclusive prefix returned.
-constexpr int kLbWin = 512;   // status words per window (4 KiB)
+constexpr int kLbWin = 1024;   // status words per window (4 KiB)
 __device__ __forceinline__ unsigned long long prefix_resolve_win(unsigned long long* st, long long tile,
                                                                 unsigned long long agg, int* err,
                                                                 const unsigned long long* win, long long lo) {
@@ -728,48 +728,48 @@ __device__ __forceinline__ unsigned long long prefix_resolve_win(unsigned long l
 
 // One pass of cta_copy_realign for a word phase of WS: 16 destination bytes
 // are words WS .. WS+4 of two 16-byte staging chunks, shifted by rs bits.
+// sp: shared address of the first of n full destination chunks' staging chunk.
 template <int WS>
-__device__ __forceinline__ void copy_realign_chunks(const uint8_t* stg, uint8_t* gbase, uint32_t sh, uint32_t end,
-                                                    uint32_t nch, uint32_t rs) {
-    for (uint32_t c = threadIdx.x; c < nch; c += blockDim.x) {
-        const uint32_t lo = c << 4;
-        if (lo >= sh && lo + 16 <= end) {
-            const uint4* sp = (const uint4*)(stg + ((lo - sh) & ~15u));
-            const uint4 p = sp[0], q = sp[1];
-            const uint32_t a[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
-            *(uint4*)(gbase + lo) =
-                make_uint4(__funnelshift_r(a[WS], a[WS + 1], rs), __funnelshift_r(a[WS + 1], a[WS + 2], rs),
-                           __funnelshift_r(a[WS + 2], a[WS + 3], rs), __funnelshift_r(a[WS + 3], a[WS + 4], rs));
-        }
+__device__ __forceinline__ void copy_realign_chunks(uint32_t sp, uint8_t* gp, uint32_t n, uint32_t rs, uint32_t tid,
+                                                    uint32_t nthr) {
+    sp += 16 * tid;
+    gp += 16 * tid;
+    for (uint32_t c = tid; c < n; c += nthr, sp += 16 * nthr, gp += 16 * nthr) {
+        uint32_t a[8];
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(sp) : "memory");
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4+16];"
+                     : "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]) : "r"(sp) : "memory");
+        *(uint4*)gp = make_uint4(__funnelshift_r(a[WS], a[WS + 1], rs), __funnelshift_r(a[WS + 1], a[WS + 2], rs),
+                                 __funnelshift_r(a[WS + 2], a[WS + 3], rs), __funnelshift_r(a[WS + 3], a[WS + 4], rs));
     }
 }
 
 // Copy n bytes from a 16-aligned staging buffer (data at offset 0, 32 bytes
-// of slack behind it) to global dst of any alignment with the whole CTA:
-// 16-byte aligned stores, the staging bytes realigned with funnel shifts;
-// byte copies at the ragged ends.  The staging side is read as aligned
-// 16-byte chunks (8 shared-memory wavefronts per warp and 512 bytes; five
-// 4-byte reads at a 16-byte stride take 20): the phase between the two sides
-// is the same for every chunk, so its word part is a branch of the whole CTA.
-__device__ __forceinline__ void cta_copy_realign(const uint8_t* stg, uint32_t n, uint8_t* dst) {
+// of slack behind it) to global dst of any alignment with threads tid = 0 ..
+// nthr - 1 of the CTA (nthr a multiple of 32): 16-byte aligned stores, the
+// staging bytes realigned with funnel shifts; byte copies at the ragged ends.
+// The staging side is read as aligned 16-byte chunks (8 shared-memory
+// wavefronts per warp and 512 bytes; five 4-byte reads at a 16-byte stride
+// take 20): the phase between the two sides is the same for every chunk, so
+// its word part is a branch of the whole CTA.
+__device__ __forceinline__ void cta_copy_realign(const uint8_t* stg, uint32_t n, uint8_t* dst, uint32_t tid,
+                                                 uint32_t nthr) {
     if (n == 0) return;
-    const uint32_t sh = (uint32_t)((uintptr_t)dst & 15);
-    uint8_t* gbase = dst - sh;
-    const uint32_t end = sh + n, nch = (end + 15) >> 4;
-    const uint32_t ph = (16u - sh) & 15u;   // byte phase of staging chunks vs. destination chunks
-    const uint32_t rs = (ph & 3u) * 8u;
-    switch (ph >> 2) {
-        case 0: copy_realign_chunks<0>(stg, gbase, sh, end, nch, rs); break;
-        case 1: copy_realign_chunks<1>(stg, gbase, sh, end, nch, rs); break;
-        case 2: copy_realign_chunks<2>(stg, gbase, sh, end, nch, rs); break;
-        default: copy_realign_chunks<3>(stg, gbase, sh, end, nch, rs); break;
+    const uint32_t head = (0u - (uint32_t)(uintptr_t)dst) & 15u;   // bytes before dst's first 16-byte boundary
+    const uint32_t h = head < n ? head : n, full = (n - h) >> 4, tail = h + 16 * full;
+    const uint32_t sp = smem_u32(stg), rs = (head & 3u) * 8u;
+    uint8_t* gp = dst + h;
+    switch (head >> 2) {
+        case 0: copy_realign_chunks<0>(sp, gp, full, rs, tid, nthr); break;
+        case 1: copy_realign_chunks<1>(sp, gp, full, rs, tid, nthr); break;
+        case 2: copy_realign_chunks<2>(sp, gp, full, rs, tid, nthr); break;
+        default: copy_realign_chunks<3>(sp, gp, full, rs, tid, nthr); break;
     }
-    if (threadIdx.x < 32) {
-        const uint32_t last = nch - 1;
-        const uint32_t c = threadIdx.x < 16 ? 0 : last;
-        const bool part = threadIdx.x < 16 ? (sh > 0 || end < 16) : (last > 0 && (end & 15) != 0);
-        const uint32_t gb = (c << 4) + (threadIdx.x & 15);
-        if (part && gb >= sh && gb < end) gbase[gb] = stg[gb - sh];
+    // lanes 0-15 the bytes before the first full chunk, lanes 16-31 those after the last
+    if (tid < 32) {
+        const uint32_t k = tid < 16 ? tid : tail + tid - 16;
+        if (k < (tid < 16 ? h : n)) dst[k] = stg[k];
     }
 }
 

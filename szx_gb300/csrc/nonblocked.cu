@@ -21,6 +21,7 @@
 // (stream offset 17) starts 16-byte aligned.
 #include "common.cuh"
 #include "kernels.h"
+#include "segment.cuh"
 
 namespace szxg {
 
@@ -192,7 +193,8 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
     uint8_t* mid = lead + L;
     const unsigned long long mid_cap = a.cap - (kNbShift + 17 + L);
     const int lane = threadIdx.x & 31;
-    const int low = 8 * (W - R);
+    const int down = 8 * W - reqLength;
+    const uint32_t guard = 0x80u << s, s4 = (uint32_t)(31 + s) * 0x01010101u, R4 = (uint32_t)R * 0x01010101u;
     const long long nt = (long long)a.ntiles;
     // warp 0's placement state: anchor tile and its inclusive prefix; window
     long long an_t = -1;
@@ -232,25 +234,36 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
             base = an_incl;
             placed = true;
         } else if (!placed && w_ok == 1) {
+            // counts of tiles an_t + 1 .. t - 1, four status words to a read
             const int units = (int)((t - w_lo + 3) >> 2);
+            const int lo = (int)(an_t + 1 - w_lo), hi = (int)(t - w_lo);
+            cp_async_wait_all();
+            __syncwarp();
             for (int attempt = 0;; attempt++) {
-                cp_async_wait_all();
-                __syncwarp();
-                unsigned long long sum = 0;
+                uint32_t sum = 0;
                 bool ready = true;
-                for (long long i = an_t + 1 + lane; i < t; i += 32) {
-                    const uint32_t w = s_win[i - w_lo];
-                    ready = ready && (w & 0xC0000000u) != 0;
-                    sum += w & 0x7FFFFFu;
+                for (int u = lane; u < units; u += 32) {
+                    const uint4 q = *(const uint4*)&s_win[4 * u];
+                    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int at = 4 * u + i;
+                        if (at >= lo && at < hi) {
+                            ready = ready && w[i] >= kSt32Agg;
+                            sum += w[i] & 0x7FFFFFu;
+                        }
+                    }
                 }
                 if (__all_sync(0xffffffffu, ready)) {
-                    base = an_incl + warp_sum(sum);
+                    base = an_incl + __reduce_add_sync(0xffffffffu, sum);
                     placed = true;
                     break;
                 }
                 if (attempt == kNbRepolls) break;
                 __nanosleep(128);
-                for (int u = lane; u < units; u += 32) cp_async16(&s_win[4 * u], a.st.st + w_lo + 4 * u);
+                __syncwarp();
+                for (int u = lane; u < units; u += 32) *(uint4*)&s_win[4 * u] = ld_volatile_v4(a.st.st + w_lo + 4 * u);
+                __syncwarp();
             }
         }
         if (!placed) {
@@ -301,43 +314,48 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
         // the next tile, claimed now and read after the scan's barriers
         if (threadIdx.x == 0) s_tile[(it + 1) & 1] = (long long)atomicAdd(a.tile_ctr, 1ull);
         const unsigned long long first = (unsigned long long)tile * kNbTile + threadIdx.x * kNbPer;
-        U cur[kNbPer];
-        bool bad = false;
-#pragma unroll
-        for (int e = 0; e < kNbPer; e++) {
-            T d = EL::sub(v[e], med);
-            bad |= d != d;
-            cur[e] = EL::bits(d) >> s;
-        }
+        U d[kNbPer];
         const T dprev = EL::sub(before, med);
-        U prev_l0 = first > 0 ? (EL::bits(dprev) >> s) : (U)0;
-        if (__any_sync(0xffffffffu, bad || (lane == 0 && first > 0 && dprev != dprev))) {
+        U d_l0 = first > 0 ? EL::bits(dprev) : (U)0;   // lane 0: the value before its first one
+        sub_run(v, med, d);
+        bool bad = lane == 0 && first > 0 && inf_or_nan(dprev);
+        if constexpr (sizeof(T) == 4) {
+            float hn = __uint_as_float(d[0]);
 #pragma unroll
-            for (int e = 0; e < kNbPer; e++) cur[e] = EL::bits(xsub(v[e], med)) >> s;
-            if (lane == 0 && first > 0) prev_l0 = EL::bits(xsub(before, med)) >> s;
+            for (int e = 1; e + 1 < kNbPer; e += 2) hn = fmax3_nan(hn, __uint_as_float(d[e]), __uint_as_float(d[e + 1]));
+            bad = bad || isnan(fmax_nan(hn, __uint_as_float(d[kNbPer - 1])));
+        } else {
+#pragma unroll
+            for (int e = 0; e < kNbPer; e++) bad = bad || inf_or_nan(EL::of(d[e]));
         }
-        U prev = __shfl_up_sync(0xffffffffu, cur[kNbPer - 1], 1);
-        if (lane == 0) prev = prev_l0;
-        uint32_t codes = 0, mine = 0, cnt4[kNbPer / 4];
+        if (__any_sync(0xffffffffu, bad)) {
+#pragma unroll
+            for (int e = 0; e < kNbPer; e++) d[e] = EL::bits(xsub(v[e], med));
+            if (lane == 0 && first > 0) d_l0 = EL::bits(xsub(before, med));
+        }
+        // lead codes from the top 32 bits, as in the blocked encoder
+        auto top = [](U u) { return (uint32_t)(u >> (8 * W - 32)); };
+        uint32_t prev = __shfl_up_sync(0xffffffffu, top(d[kNbPer - 1]), 1);
+        if (lane == 0) prev = top(d_l0);
+        const int rem = first >= a.n ? 0 : (a.n - first < kNbPer ? (int)(a.n - first) : kNbPer);   // values of this thread
+        uint32_t codes = 0, mine = 0, cnt8[kNbPer / 4];
 #pragma unroll
         for (int k = 0; k < kNbPer / 4; k++) {
-            uint32_t c4 = 0;
+            uint32_t lb[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int e = 4 * k + i;
-                const U xr = cur[e] ^ (e ? cur[e - 1] : prev);
-                int lz;
-                if constexpr (sizeof(T) == 4) lz = __clz(xr) >> 3;
-                else lz = __clzll((long long)xr) >> 3;
-                const int ld = lz < 3 ? lz : 3;
-                if (first + e < a.n) {
-                    codes |= (uint32_t)ld << (8 * k + 6 - 2 * i);
-                    const int c = R - ld;
-                    c4 |= (uint32_t)(c > 0 ? c : 0) << (8 * i);
-                }
+                const uint32_t h = top(d[4 * k + i]);
+                asm("bfind.u32 %0, %1;" : "=r"(lb[i]) : "r"((h ^ prev) | guard));
+                prev = h;
             }
-            cnt4[k] = c4;
-            mine += (c4 * 0x01010101u) >> 24;
+            const uint32_t p = (lb[3] * 256u + lb[2]) * 65536u + (lb[1] * 256u + lb[0]);
+            const uint32_t keep = low_bytes_mask(rem - 4 * k);
+            const uint32_t ldb = ((s4 - p) >> 3) & 0x03030303u & keep;
+            // max(R - lead, 0) per value, R >= 2
+            const uint32_t c4 = (R4 + (R == 2 ? (ldb >> 1) & ldb & 0x01010101u : 0u) - ldb) & keep;
+            cnt8[k] = c4 << 3;
+            mine = __dp4a(c4, 0x01010101u, mine);
+            codes |= ((ldb * 0x40100401u) >> 24) << (8 * k);   // 4 leads -> one byte, MSB first
         }
         uint32_t total;
         const uint32_t ex = cta_excl_sum32(mine, &total, s_sum);   // one barrier
@@ -351,29 +369,34 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
         else
             for (int j = 0; j < 4; j++)
                 if (lb + j < L) lead[lb + j] = (uint8_t)(codes >> (8 * j));
-        // mid bytes: each value's low (R - lead) bytes of its word shifted down
-        // to the stored range, at tile-local offsets (every byte written once)
-        uint8_t* stg = stage(it);
-        uint32_t q = ex;
+        // mid bytes: each value's low (R - lead) bytes of its required bits, at
+        // tile-local offsets: whole words now, the bytes of the words that
+        // threads share after the barrier below
+        RunOut o;
+        o.start(stage(it), ex);
 #pragma unroll
         for (int k = 0; k < kNbPer / 4; k++) {
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const uint32_t c = byte_of(cnt4[k], i);
-                const U ev = cur[4 * k + i] >> low;
-#pragma unroll
-                for (int j = 0; j < W; j++)
-                    if ((uint32_t)j < c) stg[q + j] = (uint8_t)(ev >> (8 * j));
-                q += c;
+                const uint32_t n8 = byte_of(cnt8[k], i);
+                const U ev = d[4 * k + i] >> down;
+                if constexpr (sizeof(T) == 4) {
+                    o.append((uint32_t)ev, n8);
+                } else {
+                    const uint32_t nl = n8 < 32u ? n8 : 32u;
+                    o.append((uint32_t)ev, nl);
+                    o.append((uint32_t)(ev >> 32), n8 - nl);
+                }
             }
         }
         // the next tile's values are in flight during the placement
         const long long next = s_tile[(it + 1) & 1];
         if (next < nt) fetch(next);
         if (threadIdx.x < 32 && t2 >= 0) place(t2, s_total[(it - 2) % 3]);
-        __syncthreads();   // T_j staged; T_{j-2}'s offset known
+        __syncthreads();   // T_j's whole words staged; T_{j-2}'s offset known
+        o.finish(stage(it), ex);   // (read by T_j's copy-out, two iterations on)
         if (threadIdx.x < 32) publish();
-        if (t2 >= 0 && !s_skip) cta_copy_realign(stage(it - 2), s_total[(it - 2) % 3], mid + s_base);
+        if (t2 >= 0 && !s_skip) cta_copy_realign(stage(it - 2), s_total[(it - 2) % 3], mid + s_base, threadIdx.x, kNbThreads);
         // no barrier here: the next writes of T_{j-2}'s buffer (T_{j+1}'s
         // emission), of s_base / s_skip (the next placement) and of s_sum /
         // s_total all come after the next iteration's scan barrier
@@ -392,7 +415,7 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
         }
         __syncthreads();
         if (threadIdx.x < 32) publish();
-        if (!s_skip) cta_copy_realign(stage(it - back), s_total[(it - back) % 3], mid + s_base);
+        if (!s_skip) cta_copy_realign(stage(it - back), s_total[(it - back) % 3], mid + s_base, threadIdx.x, kNbThreads);
     }
 }
 

@@ -14,6 +14,9 @@ template <typename T> struct EncCfg;
 template <> struct EncCfg<float> { static constexpr int E = 16; };    // values per lane
 template <> struct EncCfg<double> { static constexpr int E = 8; };
 
+// high word of a double's order-preserving signed key (its own inverse)
+__device__ __forceinline__ int dkey_hi(uint32_t h) { return (int)(h ^ ((uint32_t)((int)h >> 31) & 0x7FFFFFFFu)); }
+
 template <int G, typename V>
 __device__ __forceinline__ V seg_sum(V v) {
 #pragma unroll
@@ -61,6 +64,23 @@ template <typename T>
 __device__ __forceinline__ uint32_t swz_off(uint32_t i) {
     constexpr uint32_t VN = 16 / sizeof(T);
     return swz16(i / VN) * 16 + (i % VN) * (uint32_t)sizeof(T);
+}
+
+// Run `row` (64 bytes) of a swizzled tile at shared address `tile`, a multiple
+// of 64: the swizzle is one exclusive-or on the address per 16-byte chunk.
+template <typename T>
+__device__ __forceinline__ void load_run_full(uint32_t tile, uint32_t row, T (&v)[EncCfg<T>::E]) {
+    const uint32_t p = tile + 64 * row + 8 * (row & 6u);   // chunk 0 of the run: chunk (row >> 1) & 3 of its 64 bytes
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if constexpr (sizeof(T) == 4)
+            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                         : "=f"(v[4 * j]), "=f"(v[4 * j + 1]), "=f"(v[4 * j + 2]), "=f"(v[4 * j + 3])
+                         : "r"(p ^ (16u * j))
+                         : "memory");
+        else
+            asm volatile("ld.shared.v2.f64 {%0,%1}, [%2];" : "=d"(v[2 * j]), "=d"(v[2 * j + 1]) : "r"(p ^ (16u * j)) : "memory");
+    }
 }
 
 // A lane's run of the block that starts at value e0 of a swizzled tile.  vec:
@@ -198,11 +218,10 @@ __device__ __forceinline__ void seg_minmax(const T (&v)[EncCfg<T>::E], int len, 
         // the 32-bit high keys, then of the low words beside them -- 32-bit
         // operations throughout, about half of what 64-bit keys cost.  Any
         // infinity or NaN shows in the high extremes.
-        auto key_hi = [](uint32_t h) { return (int)(h ^ ((uint32_t)((int)h >> 31) & 0x7FFFFFFFu)); };
         int khn = 0x7FFFFFFF, khx = (int)0x80000000;
 #pragma unroll
         for (int e = 0; e < E; e++) {
-            const int k = key_hi(hi32(v[e]));
+            const int k = dkey_hi(hi32(v[e]));
             const bool in = FULL || C::first(sl, e / 4) + (e & 3) < len;
             khn = in ? min(khn, k) : khn;
             khx = in ? max(khx, k) : khx;
@@ -218,7 +237,7 @@ __device__ __forceinline__ void seg_minmax(const T (&v)[EncCfg<T>::E], int len, 
 #pragma unroll
             for (int e = 0; e < E; e++) {
                 const uint32_t h = hi32(v[e]), l = lo32(v[e]) ^ (uint32_t)((int)h >> 31);
-                const int k = key_hi(h);
+                const int k = dkey_hi(h);
                 const bool in = FULL || C::first(sl, e / 4) + (e & 3) < len;
                 if (in && k == khn) kln = min(kln, l);
                 if (in && k == khx) klx = max(klx, l);
@@ -228,8 +247,8 @@ __device__ __forceinline__ void seg_minmax(const T (&v)[EncCfg<T>::E], int len, 
                 kln = min(kln, __shfl_xor_sync(0xffffffffu, kln, d, G));
                 klx = max(klx, __shfl_xor_sync(0xffffffffu, klx, d, G));
             }
-            mn = from_hi_lo((uint32_t)key_hi((uint32_t)khn), kln ^ (uint32_t)(khn >> 31));
-            mx = from_hi_lo((uint32_t)key_hi((uint32_t)khx), klx ^ (uint32_t)(khx >> 31));
+            mn = from_hi_lo((uint32_t)dkey_hi((uint32_t)khn), kln ^ (uint32_t)(khn >> 31));
+            mx = from_hi_lo((uint32_t)dkey_hi((uint32_t)khx), klx ^ (uint32_t)(khx >> 31));
             special = false;
         } else {
         long long lo = 0x7FFFFFFFFFFFFFFFll, hi = (long long)0x8000000000000000ull;
@@ -325,5 +344,64 @@ __device__ __forceinline__ void seg_lead_bytes(const typename Elem<T>::U (&cur)[
         ldb[k] = b;
     }
 }
+
+// Differences of a run from the median, as bit patterns: floats two to an
+// instruction (add.f32x2 rounds each half like the scalar addition of -med).
+template <int N>
+__device__ __forceinline__ void sub_run(const float (&v)[N], float med, uint32_t (&d)[N]) {
+    const float nm = -med;
+#pragma unroll
+    for (int e = 0; e < N; e += 2)
+        asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tadd.rn.f32x2 a, a, b;\n\t"
+            "mov.b64 {%0, %1}, a;\n\t}"
+            : "=r"(d[e]), "=r"(d[e + 1])
+            : "f"(v[e]), "f"(v[e + 1]), "f"(nm));
+}
+template <int N>
+__device__ __forceinline__ void sub_run(const double (&v)[N], double med, unsigned long long (&d)[N]) {
+#pragma unroll
+    for (int e = 0; e < N; e++) d[e] = Elem<double>::bits(__dsub_rn(v[e], med));
+}
+
+// Byte-wise appending to a payload in shared memory.  A lane appends its
+// run's values one after the other: `last` holds the four bytes written last
+// (the newest on top), so the word that a value completes is a funnel shift of
+// (last, value) by the position's bit offset and the next `last` one by the
+// value's bits -- no masks, no byte stores, and whole words leave with one
+// predicated store each: ~8 instructions a float value, where a store per
+// byte took ~15 and up to four stores.  The first word a lane completes
+// carries stale bytes below the run's start; what belongs there (the lane
+// before's last bytes, or the block's lead codes) has to be stored after it:
+// finish(), the bytes of the run's last, partial word, comes after a
+// synchronisation of all lanes whose runs may share a word.
+struct RunOut {
+    uint32_t last, q8, sp;   // last four bytes, bit position, shared address of the word being filled
+    // run of bytes at offset q0 of a staging buffer (16-byte aligned shared memory)
+    __device__ __forceinline__ void start(const uint8_t* stg, uint32_t q0) {
+        last = 0;
+        q8 = 8 * q0;
+        sp = smem_u32(stg) + (q0 & ~3u);
+    }
+    __device__ __forceinline__ void append(uint32_t v, uint32_t n8) {   // the low n8 / 8 (0..4) bytes of v
+        const uint32_t w = __funnelshift_l(last, v, q8);
+        last = __funnelshift_rc(last, v, n8);
+        const uint32_t q = q8 + n8;
+        // predicated, not branched over: the position crosses a word boundary
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tlop3.or.b32 t|p, %1, %2, -32, 0x28, 0;\n\t"
+                     "@p st.shared.u32 [%0], %3;\n\t@p add.u32 %0, %0, 4;\n\t}"
+                     : "+r"(sp)
+                     : "r"(q), "r"(q8), "r"(w)
+                     : "memory");
+        q8 = q;
+    }
+    // the bytes of the last word from the run's start (if that lies in it) to its end
+    __device__ __forceinline__ void finish(const uint8_t* stg, uint32_t q0) const {
+        const uint32_t w = __funnelshift_l(last, 0u, q8);
+        const uint32_t end = (q8 >> 3) & 3u, beg = (sp ^ smem_u32(stg + q0)) < 4u ? q0 & 3u : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 3; j++)
+            if (j >= beg && j < end) asm volatile("st.shared.u8 [%0], %1;" ::"r"(sp + j), "r"(w >> (8 * j)) : "memory");
+    }
+};
 
 }  // namespace szxg

@@ -57,3 +57,22 @@ def test_streams_at_emission_edges(szx, dt, bs):
                     assert got == O.compress(mode, x, eb, bs), (name, n, off, mode)
                     if off == 0:
                         break   # the other layouts share the encoder: one of them suffices there
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 4095, 4097, 5 * 4096 + 37])
+def test_non_blocked_streams_at_emission_edges(szx, dt, n):
+    """The one-chain layout: runs that share words across lanes and warps, a
+    last thread with 1..16 values, NaNs beside the run's start."""
+    import torch
+    codec = szx.DeviceCodec(1, dt, n + 4)
+    cases = list(fields(dt, n))
+    x = np.random.default_rng(3).normal(size=n).astype(dt)
+    x[n // 2::511] = np.nan
+    cases.append(("nan", x, 1e-3))
+    for name, x, eb in cases:
+        for off in (0, 1):
+            buf = torch.zeros(n + 4, dtype=torch.float32 if dt == np.float32 else torch.float64, device="cuda")
+            buf[off:off + n] = torch.from_numpy(x).cuda()
+            codec.compress(buf[off:off + n], szx.ABS, eb)
+            assert codec.stream_bytes().cpu().numpy().tobytes() == O.compress(1, x, eb, 128), (name, off)
