@@ -1278,23 +1278,6 @@ __global__ void __launch_bounds__(kIdxThreads) k_blocked_index_fields(const DecF
 
 // ------------------------------------------------------------------ decode, per block
 //
-// A segment of G lanes decodes one non-constant block with the encoder's
-// chunk layout: lane sl owns the 4-value chunks sl, sl+G, sl+2G, ... (chunk c
-// = lead byte c of the payload).  Stored bytes are read from the staged
-// payload in shared memory; every value is first rebuilt with a zero carry
-// (its top `lead` bytes come from its predecessor, szx/src/szxd_float.cc:
-// 431-470), then the bytes still inherited from before the chunk are filled in
-// from a "last writer" scan over chunk summaries in block order.
-
-// Chunk summary: [25:24] the smallest lead in the chunk (it wrote the top-3
-// bytes at indices >= that lead), [23:0] the top three bytes of its last value.
-__device__ __forceinline__ uint32_t lw_op(uint32_t a, uint32_t b) {
-    const uint32_t ma = a >> 24, mb = b >> 24;
-    const uint32_t mask = 0xFFFFFFu >> (8 * mb);
-    return ((ma < mb ? ma : mb) << 24) | (a & 0xFFFFFFu & ~mask) | (b & mask);
-}
-constexpr uint32_t kLwNone = 3u << 24;   // writes nothing; the value before a block is zero
-
 // Lead-byte tables (a lead byte holds 4 codes, MSB first): the four leads as
 // bytes (value 0 in byte 0), and their running minimum from a start of 3
 // (the byte lanes a value still inherits from before its chunk).
@@ -1310,121 +1293,6 @@ __device__ __forceinline__ void lead_tables_init(uint32_t* lut_ld, uint32_t* lut
         lut_ld[c] = ldb;
         lut_cm[c] = cmb;
     }
-}
-
-// FULL: every segment of the warp decodes a whole block of G*E values (no
-// range checks); otherwise values at or past len are ignored.
-template <typename T, int G, bool FULL>
-__device__ __forceinline__ void dec_segment(const uint8_t* p, int len, T* ob, bool vec, const uint32_t* lut_ld,
-                                            const uint32_t* lut_cm) {
-    using C = Chunks<T, G>;
-    using EL = Elem<T>;
-    using U = typename EL::U;
-    constexpr int W = EL::W;
-    constexpr int E = C::E;
-    constexpr int NC = C::NC;
-    constexpr int TOPSH = 8 * (W - 3);
-    const int sl = (int)(lane_id() & (G - 1));
-    const int reqLength = p[0];
-    const uint32_t mb = ((uint32_t)p[1] << 24) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 8) | p[4];
-    int R, s;
-    split_reqlen(reqLength, &R, &s);
-    R = R < 1 ? 1 : (R > W ? W : R);   // a no-op for valid streams; keeps the shifts defined otherwise
-    const int low = 8 * (W - R);
-    const int Lb = FULL ? G * NC : (len + 3) / 4;
-    // per chunk: leads, running minima, stored-byte counts and their offsets (bytes of a word)
-    uint32_t ldb[NC], cmb[NC], pre[NC];
-    unsigned long long pk = 0;
-#pragma unroll
-    for (int k = 0; k < NC; k++) {
-        const int c = sl + k * G;
-        const uint32_t code = (FULL || c < Lb) ? (uint32_t)p[5 + c] : 0u;
-        ldb[k] = lut_ld[code];
-        cmb[k] = lut_cm[code];
-        uint32_t cnt4 = stored_counts(R, ldb[k]);   // max(R - lead, 0) per value
-        if constexpr (!FULL) {
-            const int nin = len - 4 * c;
-            cnt4 &= nin >= 4 ? 0xFFFFFFFFu : (nin <= 0 ? 0u : 0xFFFFFFFFu >> (32 - 8 * nin));
-        }
-        pre[k] = cnt4 * 0x01010100u;   // byte i: bytes of values 0..i-1
-        pk |= (unsigned long long)((cnt4 * 0x01010101u) >> 24) << (16 * k);
-    }
-    const unsigned long long incl = seg_inclusive_sum<G>(pk);
-    const unsigned long long tot = __shfl_sync(0xffffffffu, incl, G - 1, G);
-    const unsigned long long excl = incl - pk;
-    const uint32_t ph = (uint32_t)((uintptr_t)p & 15);
-    const uint32_t* buf = (const uint32_t*)(p - ph);
-    U cur[E];
-    uint32_t sum[NC];
-    uint32_t before = ph + 5 + (uint32_t)Lb;
-#pragma unroll
-    for (int k = 0; k < NC; k++) {
-        const uint32_t qb = before + (uint32_t)((excl >> (16 * k)) & 0xFFFF);
-        before += (uint32_t)((tot >> (16 * k)) & 0xFFFF);
-        const uint32_t ld8 = ldb[k] << 3;
-        U run = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t q = qb + byte_of(pre[k], i);
-            const uint32_t* wp = buf + (q >> 2);
-            const uint32_t w0 = wp[0], w1 = wp[1];
-            const uint32_t inh = top_bytes_mask(byte_of(ld8, i));   // top lead bytes: from the predecessor
-            // stored bytes land at [W-R, W-lead); the bytes above them are inherited
-            if constexpr (sizeof(T) == 4) {
-                const uint32_t sp = __funnelshift_r(w0, w1, q << 3) << low;
-                run = (run & inh) | (sp & ~inh);
-            } else {
-                const uint32_t w2 = wp[2];
-                const uint32_t lo = __funnelshift_r(w0, w1, q << 3), hi = __funnelshift_r(w1, w2, q << 3);
-                const unsigned long long sp = (((unsigned long long)hi << 32) | lo) << low;
-                const unsigned long long ih = (unsigned long long)inh << 32;
-                run = (run & ih) | (sp & ~ih);
-            }
-            cur[4 * k + i] = run;
-        }
-        sum[k] = (byte_of(cmb[k], 3) << 24) | ((uint32_t)(run >> TOPSH) & 0xFFFFFFu);
-    }
-    // last-writer scans: one per chunk round (independent), then the round carries
-    uint32_t inc[NC];
-#pragma unroll
-    for (int k = 0; k < NC; k++) inc[k] = sum[k];
-#pragma unroll
-    for (int d = 1; d < G; d <<= 1) {
-#pragma unroll
-        for (int k = 0; k < NC; k++) {
-            const uint32_t o = __shfl_up_sync(0xffffffffu, inc[k], d, G);
-            if (sl >= d) inc[k] = lw_op(o, inc[k]);
-        }
-    }
-    uint32_t carry_in = kLwNone;
-    const T med = widen_median<T>(__uint_as_float(mb));
-    T v[E];
-    bool bad = false;
-#pragma unroll
-    for (int k = 0; k < NC; k++) {
-        uint32_t ex = __shfl_up_sync(0xffffffffu, inc[k], 1, G);
-        if (sl == 0) ex = kLwNone;
-        const uint32_t fin = lw_op(carry_in, ex);
-        carry_in = lw_op(carry_in, __shfl_sync(0xffffffffu, inc[k], G - 1, G));
-        const uint32_t carry = (fin & 0xFFFFFFu) << 8;   // top three bytes of a 32-bit word
-        const uint32_t cm8 = cmb[k] << 3;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t keep = top_bytes_mask(byte_of(cm8, i));   // byte lanes inherited from before the chunk
-            U u = cur[4 * k + i];
-            if constexpr (sizeof(T) == 4) u |= carry & keep;
-            else u |= (unsigned long long)(carry & keep) << 32;
-            u <<= s;
-            cur[4 * k + i] = u;
-            v[4 * k + i] = EL::add(EL::of(u), med);
-            bad |= v[4 * k + i] != v[4 * k + i];
-        }
-    }
-    if (__any_sync(0xffffffffu, bad)) {
-#pragma unroll
-        for (int e = 0; e < E; e++) v[e] = xadd(EL::of(cur[e]), med);
-    }
-    store_chunks<T, G>(ob, len, vec, v);
 }
 
 // Consecutive layout: lane sl of the segment decodes the E consecutive values
@@ -1559,9 +1427,10 @@ __device__ __forceinline__ void dec_segment_seq(const uint8_t* p, int len, T* ob
         hn = fmax_nan(hn, v[E - 1]);
         bad = hn != hn;
     } else {
+        // (integer test, infinities too: a compare costs the FP64 pipe as much as the addition)
         bad = false;
 #pragma unroll
-        for (int e = 0; e < E; e++) bad |= v[e] != v[e];
+        for (int e = 0; e < E; e++) bad |= inf_or_nan(v[e]);
     }
     if (__any_sync(0xffffffffu, bad)) {
 #pragma unroll
@@ -1604,8 +1473,11 @@ __device__ __forceinline__ void dec_segment_seq(const uint8_t* p, int len, T* ob
 constexpr int kDecWarps = 8;
 constexpr int kDecThreadsP = (kDecWarps + 1) * 32;
 constexpr int kDecStages = 3;
-// 4 CTAs of 9 warps per SM (56 registers, three ring stages of shared memory)
+// 4 CTAs of 9 warps per SM (56 registers, three ring stages of shared memory,
+// or two of the largest blocks': 2^28 float64 in blocks of 256 took 1010 us
+// with three stages, which left three resident CTAs to a grid of four)
 constexpr int kDecCtasPerSm = 4;
+constexpr int kSmemPerSm = 233472;   // bytes
 
 template <typename T, int G>
 struct DecTileV {
@@ -1617,7 +1489,10 @@ struct DecTileV {
     // a valid tile's payloads fit kBlocks * kMaxPay; one more kMaxPay + 32
     // keeps the reads of a corrupt block inside the buffer
     static constexpr int kStage = (((kBlocks + 1) * kMaxPay + 32) + 15) / 16 * 16;
-    static constexpr int kDynSmem = kDecStages * kStage;
+    // two stages where three would leave shared memory for three CTAs an SM only
+    static constexpr int kStatic = 2048 + 128 + 17 * kBlocks + 1024;   // lead tables, block tables, the reserved part
+    static constexpr int kStages = kDecStages * kStage + kStatic <= kSmemPerSm / kDecCtasPerSm ? kDecStages : kDecStages - 1;
+    static constexpr int kDynSmem = kStages * kStage;
 };
 
 struct DecArgs {
@@ -1641,7 +1516,7 @@ template <typename T, int G, bool MULTI>
 __global__ void __launch_bounds__(kDecThreadsP, kDecCtasPerSm) k_blocked_decode(DecArgs a) {
     using TL = DecTileV<T, G>;
     constexpr int TB = TL::kBlocks;
-    constexpr int NS = kDecStages;
+    constexpr int NS = TL::kStages;
     extern __shared__ __align__(128) uint8_t dsm[];
     __shared__ unsigned long long full[NS], empty[NS];
     __shared__ uint32_t s_info[NS][TB];    // coded: payload position in the stage; constant: median bits

@@ -83,8 +83,18 @@ __device__ __forceinline__ float xdiv(float a, float b) { float r = __fdiv_rn(a,
 // double code spends it on the additions alone: tests, halving and conversions
 // work on the bit pattern, with the plain operation for the rare patterns
 // (infinities, NaNs, subnormals) they leave out.
-__device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)((unsigned long long)__double_as_longlong(v) >> 32); }
-__device__ __forceinline__ uint32_t lo32(double v) { return (uint32_t)(unsigned long long)__double_as_longlong(v); }
+// (the halves are taken by PTX moves: from casts the compiler recognises a
+// test for infinity or NaN and makes a double comparison of it)
+__device__ __forceinline__ uint32_t hi32(double v) {
+    uint32_t r;
+    asm("{\n\t.reg .b32 t;\n\tmov.b64 {t, %0}, %1;\n\t}" : "=r"(r) : "d"(v));
+    return r;
+}
+__device__ __forceinline__ uint32_t lo32(double v) {
+    uint32_t r;
+    asm("{\n\t.reg .b32 t;\n\tmov.b64 {%0, t}, %1;\n\t}" : "=r"(r) : "d"(v));
+    return r;
+}
 __device__ __forceinline__ double from_hi_lo(uint32_t hi, uint32_t lo) {
     return __longlong_as_double((long long)(((unsigned long long)hi << 32) | lo));
 }
@@ -679,52 +689,11 @@ __device__ __forceinline__ unsigned long long prefix_resolve(unsigned long long*
     return pa;
 }
 
-// The look-back from a window of status words that a TMA bulk copy has put
-// in shared memory: win[i] holds the word of tile lo + i, for every tile in
-// [lo, tile).  Lane l reads the words of tiles tile-1-l-32k (k = 0..15, rows
-// of 32 consecutive tiles, conflict-free) all at once; the nearest inclusive
-// prefix is the lowest (row, lane) holding one, found with two warp
-// reductions, so the walk is a handful of independent instructions rather
-// than a chain of dependent rows.  A window that holds no inclusive prefix,
-// or an empty word before it, falls back to the global look-back (which then
-// waits); either way the tile's inclusive value is published and its
-// exclusive prefix returned.
-constexpr int kLbWin = 1024;   // status words per window (4 KiB)
-__device__ __forceinline__ unsigned long long prefix_resolve_win(unsigned long long* st, long long tile,
-                                                                unsigned long long agg, int* err,
-                                                                const unsigned long long* win, long long lo) {
-    if (tile == 0) return 0;
-    constexpr int R = kLbWin / 32;
-    const unsigned lane = lane_id();
-    unsigned long long w[R];
-    unsigned first = R;   // this lane's first row holding an inclusive word
-#pragma unroll
-    for (int k = 0; k < R; k++) {
-        const long long j = tile - 1 - 32 * (long long)k - (long long)lane;
-        w[k] = j >= lo ? win[j - lo] : 0ull;   // outside the window reads as empty
-        if (first == R && (w[k] & ~kS64Val) == kS64Inc) first = k;
-    }
-    const unsigned K = __reduce_min_sync(0xffffffffu, first);
-    bool ok = K < R;
-    unsigned long long sa = 0;
-    if (ok) {
-        const unsigned stop = __ffs(__ballot_sync(0xffffffffu, first == K)) - 1;
-        bool ready = true;
-#pragma unroll
-        for (int k = 0; k < R; k++) {
-            const bool take = (unsigned)k < K || ((unsigned)k == K && lane <= stop);
-            if (take) {
-                ready = ready && (w[k] & ~kS64Val) != 0;
-                sa += w[k] & kS64Val;
-            }
-        }
-        ok = __all_sync(0xffffffffu, ready);
-    }
-    if (!ok) return prefix_resolve(st, tile, agg, err);
-    const unsigned long long pa = warp_sum(sa);
-    if (lane == 0) st_volatile64(&st[tile], kS64Inc | ((pa + agg) & kS64Val));
-    return pa;
-}
+// Tiles a placement window of the blocked encoder reaches back (2 KiB of
+// 16-bit counts): a CTA's previous tile is one launch's CTAs back on average
+// (456), further for a CTA that lags; 512 sent a third of the lagging CTAs'
+// tiles to the global walk.
+constexpr int kLbWin = 1024;
 
 // One pass of cta_copy_realign for a word phase of WS: 16 destination bytes
 // are words WS .. WS+4 of two 16-byte staging chunks, shifted by rs bits.

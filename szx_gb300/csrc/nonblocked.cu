@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 3 : 2)
             const U cur = (sp[e] & ~inh) | (prev & inh);
             sp[e] = cur << sft;
             v[e] = EL::add(EL::of(sp[e]), med);
-            if constexpr (sizeof(T) != 4) bad |= v[e] != v[e];
+            if constexpr (sizeof(T) != 4) bad |= inf_or_nan(v[e]);   // (integer test, infinities too)
             prev = cur;
         }
         if constexpr (sizeof(T) == 4) {   // a NaN anywhere: three-input max with NaN propagation
