@@ -1278,30 +1278,24 @@ __global__ void __launch_bounds__(kIdxThreads) k_blocked_index_fields(const DecF
 
 // ------------------------------------------------------------------ decode, per block
 //
-// Lead-byte tables (a lead byte holds 4 codes, MSB first): the four leads as
-// bytes (value 0 in byte 0), and their running minimum from a start of 3
-// (the byte lanes a value still inherits from before its chunk).
-__device__ __forceinline__ void lead_tables_init(uint32_t* lut_ld, uint32_t* lut_cm) {
-    for (int c = threadIdx.x; c < 256; c += blockDim.x) {
-        uint32_t ldb = 0, cmb = 0, m = 3;
-        for (int i = 0; i < 4; i++) {
-            const uint32_t ld = (c >> (6 - 2 * i)) & 3;
-            m = ld < m ? ld : m;
-            ldb |= ld << (8 * i);
-            cmb |= m << (8 * i);
-        }
-        lut_ld[c] = ldb;
-        lut_cm[c] = cmb;
-    }
+// Lead-byte table (a lead byte holds 4 codes, MSB first): the four leads as
+// bytes, value 0 in byte 0.
+__device__ __forceinline__ void lead_table_init(uint32_t* lut_ld) {
+    for (int c = threadIdx.x; c < 256; c += blockDim.x)
+        lut_ld[c] = (uint32_t)(c >> 6) | (uint32_t)(c >> 4 & 3) << 8 | (uint32_t)(c >> 2 & 3) << 16 | (uint32_t)(c & 3) << 24;
 }
 
-// Consecutive layout: lane sl of the segment decodes the E consecutive values
-// [E*sl, E*sl + E) of the block (chunks NC*sl .. NC*sl + NC-1).  Each value is
-// rebuilt in order with one running word per lane, so inheritance from
-// earlier values of the same lane (szx/src/szxd_float.cc:431-470: the top
-// `lead` bytes come from the predecessor) is resolved as it goes; only the
-// bytes inherited from before the lane's first value are unknown, and one
-// "last writer" scan over the G lane summaries per block supplies them.
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t lds8(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+
 // 32-byte stores (sm_100 and later): a lane's 8 floats / 4 doubles at a
 // 32-byte aligned address, so that lanes writing consecutive 64-byte runs fill
 // whole 32-byte sectors.
@@ -1315,84 +1309,63 @@ __device__ __forceinline__ void st_v8(double* p, const double* v) {
                  : "memory");
 }
 
+// One block by a segment of G lanes; p: its payload (shared address).  Lane
+// sl decodes the E consecutive values [E*sl, E*sl + E).
+//
+// A value's top `lead` bytes are its predecessor's (szx/src/szxd_float.cc:
+// 431-470).  What a lane inherits from before its run is found first, from
+// its lead codes alone: per top byte lane the last value that stored it and
+// where, three byte loads, and a "last writer" scan over the G lanes.  Then one
+// pass over the run finishes the values in order: the four (eight) payload
+// bytes that END with a value's last one hold its stored bytes on top, so two
+// funnel shifts put them under the bytes kept from the previous value -- no
+// masks, and no second pass to merge what was inherited.
+//
+// FULL: every segment of the warp decodes a whole block of G*E values (no
+// range checks); otherwise values at or past len are ignored.
 // vec: 0 scalar stores, 1 16-byte stores, 2 32-byte stores (the output's
 // alignment and the block's byte size allow them).
 template <typename T, int G, bool FULL>
-__device__ __forceinline__ void dec_segment_seq(const uint8_t* p, int len, T* ob, int vec, const uint32_t* lut_ld,
-                                                const uint32_t* lut_cm) {
+__device__ __forceinline__ void dec_segment(uint32_t p, int len, T* ob, int vec, const uint32_t* lut_ld) {
     using EL = Elem<T>;
     using U = typename EL::U;
     constexpr int W = EL::W;
     constexpr int E = EncCfg<T>::E;
     constexpr int NC = E / 4;
-    constexpr int TOPSH = 8 * (W - 3);
     const int sl = (int)(lane_id() & (G - 1));
-    const int reqLength = p[0];
-    const uint32_t mb = ((uint32_t)p[1] << 24) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 8) | p[4];
-    int R, s;
-    split_reqlen(reqLength, &R, &s);
+    const int reqLength = (int)lds8(p);
+    const uint32_t mb = (lds8(p + 1) << 24) | (lds8(p + 2) << 16) | (lds8(p + 3) << 8) | lds8(p + 4);
+    int R = (reqLength + 7) >> 3;
     R = R < 1 ? 1 : (R > W ? W : R);   // a no-op for valid streams; keeps the shifts defined otherwise
-    const int low = 8 * (W - R);
     const int Lb = FULL ? G * NC : (len + 3) / 4;
-    const int c0 = sl * NC;            // the lane's first chunk
-    uint32_t ldb[NC], cmb[NC], cnt[NC];
-    uint32_t mine = 0;
-#pragma unroll
-    for (int k = 0; k < NC; k++) {
-        const int c = c0 + k;
-        const uint32_t code = (FULL || c < Lb) ? (uint32_t)p[5 + c] : 0u;
-        ldb[k] = lut_ld[code];
-        cmb[k] = lut_cm[code];
-        uint32_t cnt4 = stored_counts(R, ldb[k]);   // max(R - lead, 0) per value
-        if constexpr (!FULL) {
-            const int nin = len - 4 * c;
-            cnt4 &= nin >= 4 ? 0xFFFFFFFFu : (nin <= 0 ? 0u : 0xFFFFFFFFu >> (32 - 8 * nin));
-        }
-        cnt[k] = cnt4;
-        mine += (cnt4 * 0x01010101u) >> 24;
-    }
+    const int nv = FULL ? E : (len - E * sl < 0 ? 0 : (len - E * sl < E ? len - E * sl : E));   // the lane's values
+    // the lane's lead bytes, chunk k in byte k
+    const uint32_t lp = p + 5 + NC * sl;
+    uint32_t codes = __funnelshift_r(lds32(lp & ~3u), lds32((lp & ~3u) + 4), 8 * lp);
+    if constexpr (NC == 2) codes &= 0xFFFFu;
+    // masks with one bit per value, value e's at bit 2e + 1: lead <= 0, 1, 2
+    const uint32_t c2 = vorder(codes & 0x55555555u), c1 = vorder((codes >> 1) & 0x55555555u);
+    const uint32_t valid = nv ? 0xAAAAAAAAu >> (32 - 2 * nv) : 0u;
+    const uint32_t v0 = ~(c1 | c2) & valid, v1 = ~c1 & valid, v2 = ~(c1 & c2) & valid;
+    const uint32_t m1 = R >= 2 ? v1 : 0u, m2 = R >= 3 ? v2 : 0u;
+    const uint32_t below3 = R > 3 ? (uint32_t)(R - 3) : 0u;   // bytes every value stores below the top three
+    const uint32_t mine = __popc(v0) + __popc(m1) + __popc(m2) + below3 * (uint32_t)nv;
     const uint32_t incl = seg_inclusive_sum<G>(mine);
-    const uint32_t ph = (uint32_t)((uintptr_t)p & 15);
-    const uint32_t* buf = (const uint32_t*)(p - ph);
-    uint32_t q = ph + 5 + (uint32_t)Lb + incl - mine;
-    U cur[E];
-    U run = 0;
-    uint32_t mlead = 3;   // smallest lead so far in the lane: its top bytes still come from before the lane
-    uint32_t keep8[NC];   // per value (byte i of chunk k): 8 * bytes inherited from before the lane
+    const uint32_t q0 = p + 5 + (uint32_t)Lb + incl - mine;   // the run's first byte
+    // lane summary: the top three bytes as the lane leaves them (sv) and which of them it wrote (sw)
+    uint32_t sv = 0, sw = 0;
 #pragma unroll
-    for (int k = 0; k < NC; k++) {
-        // byte-wise min(running minimum within the chunk, minimum before it):
-        // all values are <= 3, so bit 7 of a byte of (c | 0x80..) - m says c >= m
-        const uint32_t M = mlead * 0x01010101u;
-        const uint32_t ge = (((cmb[k] | 0x80808080u) - M) & 0x80808080u) >> 7;
-        const uint32_t kb = (M & (ge * 0xFFu)) | (cmb[k] & ~(ge * 0xFFu));
-        keep8[k] = kb << 3;
-        mlead = kb >> 24;
-        const uint32_t ld8 = ldb[k] << 3;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t* wp = buf + (q >> 2);
-            const uint32_t w0 = wp[0], w1 = wp[1];
-            const uint32_t inh = top_bytes_mask(byte_of(ld8, i));   // top lead bytes: from the predecessor
-            if constexpr (sizeof(T) == 4) {
-                const uint32_t sp = __funnelshift_r(w0, w1, q << 3) << low;
-                run = (run & inh) | (sp & ~inh);
-            } else {
-                const uint32_t w2 = wp[2];
-                const uint32_t lo = __funnelshift_r(w0, w1, q << 3), hi = __funnelshift_r(w1, w2, q << 3);
-                const unsigned long long sp = (((unsigned long long)hi << 32) | lo) << low;
-                const unsigned long long ih = (unsigned long long)inh << 32;
-                run = (run & ih) | (sp & ~ih);
-            }
-            cur[4 * k + i] = run;
-            q += byte_of(cnt[k], i);
+    for (int k = 0; k < 3; k++) {
+        const uint32_t vk = k == 0 ? v0 : k == 1 ? m1 : m2;
+        const int top = 31 - __clz(vk);   // -1: none
+        const uint32_t before = top < 0 ? 0u : (1u << top) - 1u;
+        const uint32_t at = q0 + __popc(v0 & before) + __popc(m1 & before) + __popc(m2 & before) +
+                            below3 * (uint32_t)(top >> 1) + (uint32_t)(R - 1 - k);
+        if (top >= 0) {
+            sv |= lds8(at) << (16 - 8 * k);
+            sw |= 0xFFu << (16 - 8 * k);
         }
     }
-    // lane summary: the top three bytes of its last value, scanned over the
-    // segment as (top three bytes, byte mask of the ones the lane wrote): a later
-    // lane's written bytes win; bytes no lane wrote stay zero (the chain of
-    // every lane starts at zero)
-    uint32_t sv = (uint32_t)(run >> TOPSH) & 0xFFFFFFu, sw = 0xFFFFFFu >> (8 * mlead);
 #pragma unroll
     for (int d = 1; d < G; d <<= 1) {
         const uint32_t ov = __shfl_up_sync(0xffffffffu, sv, d, G), ow = __shfl_up_sync(0xffffffffu, sw, d, G);
@@ -1402,20 +1375,54 @@ __device__ __forceinline__ void dec_segment_seq(const uint8_t* p, int len, T* ob
         }
     }
     const uint32_t ex = __shfl_up_sync(0xffffffffu, sv, 1, G);
-    const uint32_t carry = sl ? ex << 8 : 0u;   // top three bytes of a 32-bit word
+    const uint32_t carry = sl ? ex << 8 : 0u;   // top three bytes of a 32-bit word (zero before the block)
     const T med = widen_median<T>(__uint_as_float(mb));
+    uint32_t q8 = 8 * q0;   // bit address of the next stored byte
+    U cur[E];
     T v[E];
+    if constexpr (sizeof(T) == 4) {
+        const int down = reqLength > 32 ? 0 : (reqLength < 1 ? 31 : 32 - reqLength);   // `run` ends in the value's required bits
+        uint32_t run = carry >> (32 - 8 * R);
 #pragma unroll
-    for (int k = 0; k < NC; k++) {
+        for (int k = 0; k < NC; k++) {
+            const uint32_t ldb = lut_ld[byte_of(codes, k)];
+            uint32_t cnt8 = stored_counts(R, ldb) << 3;
+            if constexpr (!FULL) cnt8 &= low_bytes_mask(nv - 4 * k);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t keep = top_bytes_mask(byte_of(keep8[k], i));
-            U u = cur[4 * k + i];
-            if constexpr (sizeof(T) == 4) u |= carry & keep;
-            else u |= (unsigned long long)(carry & keep) << 32;
-            u <<= s;
-            cur[4 * k + i] = u;
-            v[4 * k + i] = EL::add(EL::of(u), med);
+            for (int i = 0; i < 4; i++) {
+                const uint32_t n8 = byte_of(cnt8, i);
+                q8 += n8;
+                const uint32_t a = (q8 >> 3) & ~3u;
+                const uint32_t y = __funnelshift_r(lds32(a - 4), lds32(a), q8);   // the four bytes before q8
+                run = __funnelshift_lc(y, __funnelshift_rc(run, 0u, n8), n8);
+                cur[4 * k + i] = run << down;
+                v[4 * k + i] = EL::add(EL::of(cur[4 * k + i]), med);
+            }
+        }
+    } else {
+        const int s = reqLength & 7 ? 8 - (reqLength & 7) : 0;
+        const U keep = ~(U)0 << (8 * (W - R));
+        uint32_t prev = carry;   // the previous value's top 32 bits
+#pragma unroll
+        for (int k = 0; k < NC; k++) {
+            const uint32_t ldb = lut_ld[byte_of(codes, k)];
+            uint32_t cnt8 = stored_counts(R, ldb) << 3;
+            if constexpr (!FULL) cnt8 &= low_bytes_mask(nv - 4 * k);
+            const uint32_t ld8 = ldb << 3;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                q8 += byte_of(cnt8, i);
+                const uint32_t l8 = byte_of(ld8, i);
+                const uint32_t a = (q8 >> 3) & ~3u;
+                const uint32_t w0 = lds32(a - 8), w1 = lds32(a - 4), w2 = lds32(a);
+                const uint32_t ylo = __funnelshift_r(w0, w1, q8), yhi = __funnelshift_r(w1, w2, q8);   // the eight bytes before q8
+                const uint32_t hi = __funnelshift_r(yhi, __funnelshift_l(prev, 0u, l8), l8);
+                const uint32_t lo = __funnelshift_r(ylo, yhi, l8);
+                const U u = (((U)hi << 32) | lo) & keep;
+                prev = hi;
+                cur[4 * k + i] = u << s;
+                v[4 * k + i] = EL::add(EL::of(cur[4 * k + i]), med);
+            }
         }
     }
     // a NaN result anywhere (three-input max with NaN propagation, float)
@@ -1488,9 +1495,10 @@ struct DecTileV {
     static constexpr int kMaxPay = 5 + (kBsMax + 3) / 4 + (int)sizeof(T) * kBsMax;
     // a valid tile's payloads fit kBlocks * kMaxPay; one more kMaxPay + 32
     // keeps the reads of a corrupt block inside the buffer
-    static constexpr int kStage = (((kBlocks + 1) * kMaxPay + 32) + 15) / 16 * 16;
+    static constexpr int kFront = 16;   // the decoder reads up to eight bytes before a value
+    static constexpr int kStage = (kFront + ((kBlocks + 1) * kMaxPay + 32) + 15) / 16 * 16;
     // two stages where three would leave shared memory for three CTAs an SM only
-    static constexpr int kStatic = 2048 + 128 + 17 * kBlocks + 1024;   // lead tables, block tables, the reserved part
+    static constexpr int kStatic = 1024 + 128 + 17 * kBlocks + 1024;   // lead tables, block tables, the reserved part
     static constexpr int kStages = kDecStages * kStage + kStatic <= kSmemPerSm / kDecCtasPerSm ? kDecStages : kDecStages - 1;
     static constexpr int kDynSmem = kStages * kStage;
 };
@@ -1524,7 +1532,7 @@ __global__ void __launch_bounds__(kDecThreadsP, kDecCtasPerSm) k_blocked_decode(
     __shared__ uint8_t s_ok[NS];
     __shared__ int s_fld[NS];              // a batch: the tile's field
     __shared__ uint16_t s_rank[TB];        // producer scratch: rank within the tile
-    __shared__ uint32_t lut_ld[256], lut_cm[256];
+    __shared__ uint32_t lut_ld[256];
     BlockedHdr h = {};
     if constexpr (!MULTI) {
         h = *a.hdr;
@@ -1542,15 +1550,141 @@ __global__ void __launch_bounds__(kDecThreadsP, kDecCtasPerSm) k_blocked_decode(
         }
         mbar_fence_init();
     }
-    lead_tables_init(lut_ld, lut_cm);
+    lead_table_init(lut_ld);
     __syncthreads();
     const long long ntiles = MULTI ? (long long)a.total_tiles : (long long)((h.nb + TB - 1) / TB);
     const int bs = MULTI ? a.bs : (int)h.bs;
     // field of a launch-wide tile (batch): one load from the plan's tile map
     auto field_of = [&](long long g) { return (int)a.tile_field[g]; };
 
+    // The producer's copy of a tile's payload range [sa, sa + nbytes) of the
+    // stream [sbeg, send): one TMA copy of the 16-byte chunks it touches, and
+    // plain copies of the ends where a chunk would pass the stream's.  Byte x
+    // goes to stage + kFront + (x - (sa & ~15)).
+    auto copy_range = [&](uint8_t* stage, const uint8_t* src, unsigned long long nbytes, const uint8_t* sbeg,
+                          const uint8_t* send, int slot) {
+        if (nbytes == 0) return;
+        const uintptr_t sa = (uintptr_t)src, se = sa + nbytes, base = sa & ~(uintptr_t)15;
+        const uintptr_t a0 = base < (uintptr_t)sbeg ? base + 16 : base;
+        uintptr_t a1 = (se + 15) & ~(uintptr_t)15;
+        if (a1 > (uintptr_t)send) a1 -= 16;
+        if (a1 > a0 && lane == 0) {
+            fence_proxy_async();
+            mbar_expect_tx(&full[slot], (uint32_t)(a1 - a0));
+            tma_load_1d(stage + TL::kFront + (a0 - base), (const void*)a0, (uint32_t)(a1 - a0), &full[slot]);
+        }
+        uint8_t* d = stage + TL::kFront;
+        const uintptr_t head = a0 < se ? a0 : se, tail = a1 > head ? a1 : head;   // plain: [sa, head) and [tail, se)
+        for (uintptr_t x = sa + lane; x < head; x += 32) d[x - base] = *(const uint8_t*)x;
+        for (uintptr_t x = tail + lane; x < se; x += 32) d[x - base] = *(const uint8_t*)x;
+    };
+    if (!MULTI && TB <= 32 && warp == kDecWarps) {
+        // ---------------------------------------------------------- producer, one stream, at most 32 blocks a tile
+        // Pipelined: iteration i issues the loads of tile i+2's state bits and
+        // rank word and of tile i+1's offsets and medians, and stages tile i
+        // from what the iteration before loaded.  (Loaded when needed, the
+        // three dependent round trips took 3.2 us of a tile's 3.9, and the
+        // decoders waited for them.)  Lane l holds block l of the tile's
+        // 32-block state word; the tile's blocks are lanes bit0 .. bit0 + TB - 1.
+        const uint8_t* S = a.s;
+        auto load_a = [&](long long t, uint32_t& st, uint32_t& rw) {
+            const unsigned long long w = (unsigned long long)t * TB >> 5, bi = 4 * w + (lane >> 3);
+            st = bi < h.sb ? (uint32_t)S[h.s_off + bi] : 0u;
+            rw = a.RW[w];
+        };
+        // tile t's coded blocks (bit per block), first rank, and this lane's block lb = lane
+        auto blocks_of = [&](long long t) { const unsigned long long left = h.nb - (unsigned long long)t * TB; return left < (unsigned long long)TB ? (int)left : TB; };
+        auto load_b = [&](long long t, uint32_t st, uint32_t rw, uint32_t& mt, uint32_t (&x)[4], uint32_t& good) {
+            const unsigned long long b0 = (unsigned long long)t * TB;
+            const int bit0 = (int)(b0 & 31), nblk = blocks_of(t);
+            const uint32_t m = __ballot_sync(0xffffffffu, (st >> (7 - (lane & 7))) & 1u);
+            const uint32_t rank0 = rw + __popc(m & ((1u << bit0) - 1u));
+            mt = m >> bit0 & (nblk < 32 ? (1u << nblk) - 1u : 0xFFFFFFFFu);
+            const uint32_t r = __popc(mt & ((1u << lane) - 1u));
+            good = rank0 + __popc(mt) <= h.nnc;
+            x[0] = x[1] = x[2] = x[3] = 0;
+            if (lane < nblk) {
+                if (mt >> lane & 1u) {
+                    if (good) {
+                        const unsigned long long k = (unsigned long long)rank0 + r, p0 = a.P[k], p1 = a.P[k + 1];
+                        x[0] = (uint32_t)p0; x[1] = (uint32_t)(p0 >> 32);
+                        x[2] = (uint32_t)p1; x[3] = (uint32_t)(p1 >> 32);
+                    }
+                } else {
+                    const unsigned long long b = b0 + lane, rk = (unsigned long long)rank0 + r, mo = h.m_off + 4 * (b - rk);
+                    if (b >= rk && mo + 4 <= h.q_off) {
+#pragma unroll
+                        for (int c = 0; c < 4; c++) x[c] = S[mo + c];
+                    } else {
+                        good = 0;
+                    }
+                }
+            }
+        };
+        long long t = blockIdx.x, i = 0;
+        const long long gs = gridDim.x;
+        uint32_t stA = 0, rwA = 0, mtB = 0, xB[4] = {0, 0, 0, 0}, goodB = 0;
+        if (t < ntiles) {
+            load_a(t, stA, rwA);
+            load_b(t, stA, rwA, mtB, xB, goodB);
+        }
+        if (t + gs < ntiles) load_a(t + gs, stA, rwA);
+        for (; t < ntiles; t += gs, i++) {
+            uint32_t stN = 0, rwN = 0, mtN = 0, xN[4] = {0, 0, 0, 0}, goodN = 0;
+            if (t + 2 * gs < ntiles) load_a(t + 2 * gs, stN, rwN);
+            if (t + gs < ntiles) load_b(t + gs, stA, rwA, mtN, xN, goodN);
+            const int slot = (int)(i % NS);
+            if (i >= NS && !mbar_wait(&empty[slot], (uint32_t)((i / NS - 1) & 1))) {
+                if (lane == 0) atomicExch(a.err, kErrLookback);
+                break;
+            }
+            uint8_t* stage = dsm + slot * TL::kStage;
+            const int nblk = blocks_of(t);
+            const unsigned long long p0 = ((unsigned long long)xB[1] << 32) | xB[0], p1 = ((unsigned long long)xB[3] << 32) | xB[2];
+            const int first = mtB ? __ffs(mtB) - 1 : 0, last = mtB ? 31 - __clz(mtB) : 0;
+            const unsigned long long pa = __shfl_sync(0xffffffffu, p0, first), pb = __shfl_sync(0xffffffffu, p1, last);
+            uint32_t ok = goodB;
+            if (mtB && (pb < pa || pb - pa > (unsigned long long)TB * TL::kMaxPay || h.q_off + pb > a.len)) ok = 0;
+            ok = __all_sync(0xffffffffu, ok);
+            const unsigned long long nbytes = ok && mtB ? pb - pa : 0;
+            const uint8_t* src = S + h.q_off + pa;
+            const uint32_t ph = (uint32_t)((uintptr_t)src & 15);
+            copy_range(stage, src, nbytes, S, S + a.len, slot);
+            if (lane < TB) {
+                const bool in = lane < nblk, coded = mtB >> lane & 1u;
+                uint32_t info;
+                if (coded) {
+                    const unsigned long long rem = h.n - ((unsigned long long)t * TB + lane) * h.bs;
+                    const int blen = rem < h.bs ? (int)rem : bs;
+                    const unsigned long long minsz = 5 + (unsigned long long)((blen + 3) / 4);
+                    if (p0 < pa || p1 > pb || p1 < p0 + minsz || p1 - p0 > (unsigned long long)TL::kMaxPay) ok = 0;
+                    info = TL::kFront + ph + (uint32_t)(p0 - pa);
+                } else {
+                    info = a.native_medians ? (xB[0] | (xB[1] << 8) | (xB[2] << 16) | (xB[3] << 24))
+                                            : ((xB[0] << 24) | (xB[1] << 16) | (xB[2] << 8) | xB[3]);
+                }
+                s_info[slot][lane] = info;
+                s_kind[slot][lane] = !in ? kBlkNone : (coded ? kBlkCoded : kBlkConst);
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) {
+                s_ok[slot] = (uint8_t)ok;
+                if (!ok) atomicExch(a.err, kErrStream);
+                mbar_arrive(&full[slot]);
+            }
+            stA = stN; rwA = rwN;
+            mtB = mtN; goodB = goodN;
+#pragma unroll
+            for (int c = 0; c < 4; c++) xB[c] = xN[c];
+        }
+        // copies still in flight finish before the CTA exits
+        for (long long k = i > NS ? i - NS : 0; k < i; k++) mbar_wait(&full[k % NS], (uint32_t)((k / NS) & 1));
+        return;
+    }
     if (warp == kDecWarps) {
-        // ---------------------------------------------------------- producer
+        // ---------------------------------------------------------- producer, any tile
         long long i = 0;
         for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, i++) {
             const int slot = (int)(i % NS);
@@ -1616,21 +1750,8 @@ __global__ void __launch_bounds__(kDecThreadsP, kDecCtasPerSm) k_blocked_decode(
             const uint8_t* src = S + hh.q_off + pa;
             const uint32_t ph = (uint32_t)((uintptr_t)src & 15);
             const unsigned long long nbytes = ok ? pb - pa : 0;
-            const uintptr_t sa = (uintptr_t)src;
-            const uintptr_t a0 = (sa + 15) & ~(uintptr_t)15, a1 = (sa + nbytes) & ~(uintptr_t)15;
-            uint32_t tx = 0;
-            uintptr_t head_end = sa + nbytes, tail_beg = sa + nbytes;
-            if (a1 > a0) {
-                tx = (uint32_t)(a1 - a0);
-                head_end = a0;
-                tail_beg = a1;
-            }
             __syncwarp();
-            if (lane == 0 && tx) {
-                fence_proxy_async();
-                mbar_expect_tx(&full[slot], tx);
-                tma_load_1d(stage + ph + (a0 - sa), (const void*)a0, tx, &full[slot]);
-            }
+            copy_range(stage, src, nbytes, S, S + L, slot);
             // medians of the constant blocks, payload offsets of the coded ones
             for (int j = 0; j < TB; j += 32) {
                 const int lb = j + lane;
@@ -1658,15 +1779,12 @@ __global__ void __launch_bounds__(kDecThreadsP, kDecCtasPerSm) k_blocked_decode(
                     const int blen = rem < hh.bs ? (int)rem : bs;
                     const unsigned long long minsz = 5 + (unsigned long long)((blen + 3) / 4);
                     if (p0 < pa || p1 > pb || p1 < p0 + minsz || p1 - p0 > (unsigned long long)TL::kMaxPay) ok = 0;
-                    s_info[slot][lb] = ph + (uint32_t)(p0 - pa);
+                    s_info[slot][lb] = TL::kFront + ph + (uint32_t)(p0 - pa);
                 } else {
                     ok = 0;   // a coded block without a valid payload range
                 }
             }
             ok = __all_sync(0xffffffffu, ok);
-            // ragged ends of the payload range by the lanes
-            for (uintptr_t x = sa + lane; x < head_end; x += 32) stage[ph + (x - sa)] = *(const uint8_t*)x;
-            for (uintptr_t x = tail_beg + lane; x < sa + nbytes; x += 32) stage[ph + (x - sa)] = *(const uint8_t*)x;
             __threadfence_block();
             __syncwarp();
             if (lane == 0) {
@@ -1723,12 +1841,12 @@ __global__ void __launch_bounds__(kDecThreadsP, kDecCtasPerSm) k_blocked_decode(
             store_chunks<T, G>(ob, blen, vec, v);
         }
         const bool coded = kind == kBlkCoded && s_ok[slot];
-        const uint8_t* stage = dsm + slot * TL::kStage;
+        const uint32_t pay = smem_u32(dsm + slot * TL::kStage) + (coded ? info : (uint32_t)TL::kFront);
         // the whole warp takes one path: segments that decode nothing store nothing either way
         if (__all_sync(0xffffffffu, !coded || blen == TL::kBsMax))
-            dec_segment_seq<T, G, true>(stage + (coded ? info : 0u), coded ? blen : 0, ob, vec, lut_ld, lut_cm);
+            dec_segment<T, G, true>(pay, coded ? blen : 0, ob, vec, lut_ld);
         else
-            dec_segment_seq<T, G, false>(stage + (coded ? info : 0u), coded ? blen : 0, ob, vec, lut_ld, lut_cm);
+            dec_segment<T, G, false>(pay, coded ? blen : 0, ob, vec, lut_ld);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[slot]);
     }

@@ -200,6 +200,9 @@ __device__ __forceinline__ void split_reqlen(int reqLength, int* R, int* s) {
 }
 
 __device__ __forceinline__ uint32_t bswap32(uint32_t v) { return __byte_perm(v, 0, 0x0123); }
+// 16 lead codes as stored (4 to a byte, MSB first), one bit of each pair set:
+// moved to value order, value e's bit (its pair's low one) to position 2e+1
+__device__ __forceinline__ uint32_t vorder(uint32_t m) { return __byte_perm(__brev(m), 0, 0x0123); }
 // byte i of x, zero-extended
 __device__ __forceinline__ uint32_t byte_of(uint32_t x, int i) { return __byte_perm(x, 0, 0x4440 | i); }
 // top `n8 / 8` bytes of a 32-bit word set (n8 = 8 * bytes, 0..24)

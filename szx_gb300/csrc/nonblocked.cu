@@ -510,8 +510,6 @@ __device__ __forceinline__ uint32_t lead_word(const uint8_t* lead, unsigned long
 // 2*(e%4)), as masks with one bit per value: m_k has the low bit of value
 // e's pair set when its lead code is <= k, i.e. when its byte lane W-1-k is
 // stored.  vorder() moves value e's bit to position 2e+1 (value order).
-__device__ __forceinline__ uint32_t vorder(uint32_t m) { return __byte_perm(__brev(m), 0, 0x0123); }
-
 // Valid-value mask (pair low bits) of a word whose first value is `first`.
 __device__ __forceinline__ uint32_t valid_pairs(unsigned long long first, unsigned long long n) {
     if (first + 16 <= n) return 0x55555555u;
