@@ -1278,37 +1278,6 @@ __global__ void __launch_bounds__(kIdxThreads) k_blocked_index_fields(const DecF
 
 // ------------------------------------------------------------------ decode, per block
 //
-// Lead-byte table (a lead byte holds 4 codes, MSB first): the four leads as
-// bytes, value 0 in byte 0.
-__device__ __forceinline__ void lead_table_init(uint32_t* lut_ld) {
-    for (int c = threadIdx.x; c < 256; c += blockDim.x)
-        lut_ld[c] = (uint32_t)(c >> 6) | (uint32_t)(c >> 4 & 3) << 8 | (uint32_t)(c >> 2 & 3) << 16 | (uint32_t)(c & 3) << 24;
-}
-
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ uint32_t lds8(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return v;
-}
-
-// 32-byte stores (sm_100 and later): a lane's 8 floats / 4 doubles at a
-// 32-byte aligned address, so that lanes writing consecutive 64-byte runs fill
-// whole 32-byte sectors.
-__device__ __forceinline__ void st_v8(float* p, const float* v) {
-    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
-                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-                 : "memory");
-}
-__device__ __forceinline__ void st_v8(double* p, const double* v) {
-    asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
-                 : "memory");
-}
-
 // One block by a segment of G lanes; p: its payload (shared address).  Lane
 // sl decodes the E consecutive values [E*sl, E*sl + E).
 //
@@ -1329,43 +1298,23 @@ template <typename T, int G, bool FULL>
 __device__ __forceinline__ void dec_segment(uint32_t p, int len, T* ob, int vec, const uint32_t* lut_ld) {
     using EL = Elem<T>;
     using U = typename EL::U;
-    constexpr int W = EL::W;
     constexpr int E = EncCfg<T>::E;
     constexpr int NC = E / 4;
     const int sl = (int)(lane_id() & (G - 1));
     const int reqLength = (int)lds8(p);
     const uint32_t mb = (lds8(p + 1) << 24) | (lds8(p + 2) << 16) | (lds8(p + 3) << 8) | lds8(p + 4);
-    int R = (reqLength + 7) >> 3;
-    R = R < 1 ? 1 : (R > W ? W : R);   // a no-op for valid streams; keeps the shifts defined otherwise
+    const int R = run_bytes<T>(reqLength);
     const int Lb = FULL ? G * NC : (len + 3) / 4;
     const int nv = FULL ? E : (len - E * sl < 0 ? 0 : (len - E * sl < E ? len - E * sl : E));   // the lane's values
     // the lane's lead bytes, chunk k in byte k
     const uint32_t lp = p + 5 + NC * sl;
     uint32_t codes = __funnelshift_r(lds32(lp & ~3u), lds32((lp & ~3u) + 4), 8 * lp);
     if constexpr (NC == 2) codes &= 0xFFFFu;
-    // masks with one bit per value, value e's at bit 2e + 1: lead <= 0, 1, 2
-    const uint32_t c2 = vorder(codes & 0x55555555u), c1 = vorder((codes >> 1) & 0x55555555u);
-    const uint32_t valid = nv ? 0xAAAAAAAAu >> (32 - 2 * nv) : 0u;
-    const uint32_t v0 = ~(c1 | c2) & valid, v1 = ~c1 & valid, v2 = ~(c1 & c2) & valid;
-    const uint32_t m1 = R >= 2 ? v1 : 0u, m2 = R >= 3 ? v2 : 0u;
-    const uint32_t below3 = R > 3 ? (uint32_t)(R - 3) : 0u;   // bytes every value stores below the top three
-    const uint32_t mine = __popc(v0) + __popc(m1) + __popc(m2) + below3 * (uint32_t)nv;
-    const uint32_t incl = seg_inclusive_sum<G>(mine);
-    const uint32_t q0 = p + 5 + (uint32_t)Lb + incl - mine;   // the run's first byte
-    // lane summary: the top three bytes as the lane leaves them (sv) and which of them it wrote (sw)
-    uint32_t sv = 0, sw = 0;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const uint32_t vk = k == 0 ? v0 : k == 1 ? m1 : m2;
-        const int top = 31 - __clz(vk);   // -1: none
-        const uint32_t before = top < 0 ? 0u : (1u << top) - 1u;
-        const uint32_t at = q0 + __popc(v0 & before) + __popc(m1 & before) + __popc(m2 & before) +
-                            below3 * (uint32_t)(top >> 1) + (uint32_t)(R - 1 - k);
-        if (top >= 0) {
-            sv |= lds8(at) << (16 - 8 * k);
-            sw |= 0xFFu << (16 - 8 * k);
-        }
-    }
+    const RunLeads<E> leads(codes, nv, R);
+    const uint32_t incl = seg_inclusive_sum<G>(leads.bytes());
+    const uint32_t q0 = p + 5 + (uint32_t)Lb + incl - leads.bytes();   // the run's first byte
+    uint32_t sv, sw;   // the top three bytes as the lane leaves them, and which of them it wrote
+    leads.summary(q0, sv, sw);
 #pragma unroll
     for (int d = 1; d < G; d <<= 1) {
         const uint32_t ov = __shfl_up_sync(0xffffffffu, sv, d, G), ow = __shfl_up_sync(0xffffffffu, sw, d, G);
@@ -1377,69 +1326,10 @@ __device__ __forceinline__ void dec_segment(uint32_t p, int len, T* ob, int vec,
     const uint32_t ex = __shfl_up_sync(0xffffffffu, sv, 1, G);
     const uint32_t carry = sl ? ex << 8 : 0u;   // top three bytes of a 32-bit word (zero before the block)
     const T med = widen_median<T>(__uint_as_float(mb));
-    uint32_t q8 = 8 * q0;   // bit address of the next stored byte
     U cur[E];
     T v[E];
-    if constexpr (sizeof(T) == 4) {
-        const int down = reqLength > 32 ? 0 : (reqLength < 1 ? 31 : 32 - reqLength);   // `run` ends in the value's required bits
-        uint32_t run = carry >> (32 - 8 * R);
-#pragma unroll
-        for (int k = 0; k < NC; k++) {
-            const uint32_t ldb = lut_ld[byte_of(codes, k)];
-            uint32_t cnt8 = stored_counts(R, ldb) << 3;
-            if constexpr (!FULL) cnt8 &= low_bytes_mask(nv - 4 * k);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint32_t n8 = byte_of(cnt8, i);
-                q8 += n8;
-                const uint32_t a = (q8 >> 3) & ~3u;
-                const uint32_t y = __funnelshift_r(lds32(a - 4), lds32(a), q8);   // the four bytes before q8
-                run = __funnelshift_lc(y, __funnelshift_rc(run, 0u, n8), n8);
-                cur[4 * k + i] = run << down;
-                v[4 * k + i] = EL::add(EL::of(cur[4 * k + i]), med);
-            }
-        }
-    } else {
-        const int s = reqLength & 7 ? 8 - (reqLength & 7) : 0;
-        const U keep = ~(U)0 << (8 * (W - R));
-        uint32_t prev = carry;   // the previous value's top 32 bits
-#pragma unroll
-        for (int k = 0; k < NC; k++) {
-            const uint32_t ldb = lut_ld[byte_of(codes, k)];
-            uint32_t cnt8 = stored_counts(R, ldb) << 3;
-            if constexpr (!FULL) cnt8 &= low_bytes_mask(nv - 4 * k);
-            const uint32_t ld8 = ldb << 3;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                q8 += byte_of(cnt8, i);
-                const uint32_t l8 = byte_of(ld8, i);
-                const uint32_t a = (q8 >> 3) & ~3u;
-                const uint32_t w0 = lds32(a - 8), w1 = lds32(a - 4), w2 = lds32(a);
-                const uint32_t ylo = __funnelshift_r(w0, w1, q8), yhi = __funnelshift_r(w1, w2, q8);   // the eight bytes before q8
-                const uint32_t hi = __funnelshift_r(yhi, __funnelshift_l(prev, 0u, l8), l8);
-                const uint32_t lo = __funnelshift_r(ylo, yhi, l8);
-                const U u = (((U)hi << 32) | lo) & keep;
-                prev = hi;
-                cur[4 * k + i] = u << s;
-                v[4 * k + i] = EL::add(EL::of(cur[4 * k + i]), med);
-            }
-        }
-    }
-    // a NaN result anywhere (three-input max with NaN propagation, float)
-    bool bad;
-    if constexpr (sizeof(T) == 4) {
-        float hn = v[0];
-#pragma unroll
-        for (int e = 1; e + 1 < E; e += 2) hn = fmax3_nan(hn, v[e], v[e + 1]);
-        hn = fmax_nan(hn, v[E - 1]);
-        bad = hn != hn;
-    } else {
-        // (integer test, infinities too: a compare costs the FP64 pipe as much as the addition)
-        bad = false;
-#pragma unroll
-        for (int e = 0; e < E; e++) bad |= inf_or_nan(v[e]);
-    }
-    if (__any_sync(0xffffffffu, bad)) {
+    const bool bad = run_decode<T, E, FULL>(codes, nv, R, reqLength, q0, carry, med, lut_ld, cur, v);
+    if (__any_sync(0xffffffffu, bad && len > 0)) {
 #pragma unroll
         for (int e = 0; e < E; e++) v[e] = xadd(EL::of(cur[e]), med);
     }
@@ -1498,7 +1388,7 @@ struct DecTileV {
     static constexpr int kFront = 16;   // the decoder reads up to eight bytes before a value
     static constexpr int kStage = (kFront + ((kBlocks + 1) * kMaxPay + 32) + 15) / 16 * 16;
     // two stages where three would leave shared memory for three CTAs an SM only
-    static constexpr int kStatic = 1024 + 128 + 17 * kBlocks + 1024;   // lead tables, block tables, the reserved part
+    static constexpr int kStatic = 2048 + 128 + 17 * kBlocks + 1024;   // lead tables, block tables, the reserved part
     static constexpr int kStages = kDecStages * kStage + kStatic <= kSmemPerSm / kDecCtasPerSm ? kDecStages : kDecStages - 1;
     static constexpr int kDynSmem = kStages * kStage;
 };
@@ -1532,7 +1422,7 @@ __global__ void __launch_bounds__(kDecThreadsP, kDecCtasPerSm) k_blocked_decode(
     __shared__ uint8_t s_ok[NS];
     __shared__ int s_fld[NS];              // a batch: the tile's field
     __shared__ uint16_t s_rank[TB];        // producer scratch: rank within the tile
-    __shared__ uint32_t lut_ld[256];
+    __shared__ uint32_t lut_ld[512];
     BlockedHdr h = {};
     if constexpr (!MULTI) {
         h = *a.hdr;

@@ -107,7 +107,11 @@ __device__ __forceinline__ void load16(const T* p, unsigned long long first, uns
 template <typename T>
 __device__ __forceinline__ void store16(T* p, unsigned long long first, unsigned long long n, const T (&v)[kNbPer]) {
     const bool full = first + kNbPer <= n;
-    if (full && ((uintptr_t)(p + first) % 16) == 0) {
+    if (full && ((uintptr_t)(p + first) % 32) == 0) {   // whole 32-byte sectors
+        constexpr int V8 = 32 / (int)sizeof(T);
+#pragma unroll
+        for (int i = 0; i < kNbPer / V8; i++) st_v8(p + first + V8 * i, v + V8 * i);
+    } else if (full && ((uintptr_t)(p + first) % 16) == 0) {
         uint4* q = (uint4*)(p + first);
 #pragma unroll
         for (int i = 0; i < kNbPer * (int)sizeof(T) / 16; i++) {
@@ -506,19 +510,6 @@ __device__ __forceinline__ uint32_t lead_word(const uint8_t* lead, unsigned long
     return w;
 }
 
-// Lead codes of 16 values in one 32-bit word (value e at bits 8*(e/4) + 6 -
-// 2*(e%4)), as masks with one bit per value: m_k has the low bit of value
-// e's pair set when its lead code is <= k, i.e. when its byte lane W-1-k is
-// stored.  vorder() moves value e's bit to position 2e+1 (value order).
-// Valid-value mask (pair low bits) of a word whose first value is `first`.
-__device__ __forceinline__ uint32_t valid_pairs(unsigned long long first, unsigned long long n) {
-    if (first + 16 <= n) return 0x55555555u;
-    uint32_t v = 0;
-    for (int e = 0; e < 16; e++)
-        if (first + e < n) v |= 1u << (8 * (e >> 2) + 6 - 2 * (e & 3));
-    return v;
-}
-
 // Lead word of values [first, first + 16): one 4-byte load when aligned.
 __device__ __forceinline__ uint32_t lead_word16(const uint8_t* lead, unsigned long long first,
                                                 unsigned long long L) {
@@ -529,11 +520,12 @@ __device__ __forceinline__ uint32_t lead_word16(const uint8_t* lead, unsigned lo
 
 // Per tile (one warp): its mid-byte count (tcnt[t]) and, for each of the top
 // three byte lanes, where in the tile's mid bytes the last value storing that
-// lane put it (aux[3t+2], 3x21 bits, position+1, 0 = none).  A lane takes the
-// tile's 16-code words lane, lane+32, ... so that every load of the warp reads
-// 128 consecutive lead bytes; a warp scan per round orders the words.  Counts
-// and positions come from population counts of the per-lane masks:
-// a value stores max(R - lead, 0) bytes = the number of k < R with lead <= k.
+// lane put it (aux[3t+2], 3x21 bits, position+1, 0 = none).  A lane takes 8
+// consecutive 16-code words (two 16-byte loads), so the tile takes one warp
+// scan; each word costs its three masks, their population counts (a value
+// stores max(R - lead, 0) bytes = the number of k < R with lead <= k) and the
+// last word of each mask that is not empty.  (One word per lane and eight
+// scans a tile: 59 us at 2^27 values.)
 // The CTA's eight tiles form a group: aux[3t] / aux[3t+1] get the tile's
 // exclusive prefix within its group (bytes; latest writer tiles, 3x21 bits,
 // tile+1), gsum[g] / gwr[g] the group's totals.  Independent per group: no
@@ -546,54 +538,59 @@ __global__ void __launch_bounds__(kNbThreads) k_nb_count(const uint8_t* __restri
                                                          unsigned long long* __restrict__ gwr) {
     constexpr int W = Elem<T>::W;
     constexpr int kTpg = kNbThreads / 32;   // tiles per group
+    constexpr int kWords = kNbTile / (32 * kNbPer);   // words per lane
     __shared__ uint32_t s_cnt[kTpg];
     __shared__ unsigned long long s_own[kTpg];
     const NonBlockedHdr h = *hp;
-    if (!h.ok) return;
-    int R, sft;
-    split_reqlen(h.reqLength, &R, &sft);
-    if (R > W) return;
+    if (!h.ok || h.reqLength > 8 * W) return;
+    const int R = run_bytes<T>(h.reqLength);
     const unsigned long long ntiles = (h.n + kNbTile - 1) / kNbTile;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long tile = (long long)blockIdx.x * kTpg + warp;
     const uint8_t* lead = s + 17;
-    const uint32_t full = R > 3 ? (uint32_t)(R - 3) : 0u;   // bytes every value stores below the top three lanes
     uint32_t run = 0;
     int gpos[3] = {-1, -1, -1};
     if (tile < (long long)ntiles) {
-#pragma unroll 2
-        for (int j = 0; j < kNbTile / (32 * kNbPer); j++) {
-            const unsigned long long first =
-                (unsigned long long)tile * kNbTile + (unsigned long long)kNbPer * (32 * j + lane);
-            const uint32_t codes = lead_word16(lead, first, h.L);
-            const uint32_t valid = valid_pairs(first, h.n);
-            const uint32_t lo = codes & 0x55555555u, hi = (codes >> 1) & 0x55555555u;
-            const uint32_t m0 = ~(lo | hi) & valid, m1 = ~hi & valid, m2 = ~(lo & hi) & valid;
-            const uint32_t nv = __popc(valid);
-            const uint32_t mine = __popc(m0) + (R >= 2 ? __popc(m1) : 0u) + (R >= 3 ? __popc(m2) : 0u) + full * nv;
-            const uint32_t incl = warp_inclusive_sum(mine);
-            const uint32_t ex = run + incl - mine;
-            const uint32_t v0 = vorder(m0), v1 = vorder(m1), v2 = vorder(m2);
+        const unsigned long long first = (unsigned long long)tile * kNbTile + (unsigned long long)(kWords * kNbPer) * lane;
+        uint32_t cw[kWords];
+        const uint8_t* lp = lead + (first >> 2);
+        if (first + kWords * kNbPer <= h.n && ((uintptr_t)lp & 15) == 0) {
+            const uint4 a = __ldg((const uint4*)lp), b = __ldg((const uint4*)lp + 1);
+            cw[0] = a.x; cw[1] = a.y; cw[2] = a.z; cw[3] = a.w;
+            cw[4] = b.x; cw[5] = b.y; cw[6] = b.z; cw[7] = b.w;
+        } else {
 #pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const uint32_t vk = k == 0 ? v0 : k == 1 ? v1 : v2;
-                if (k <= R - 1 && vk) {   // later words hold later positions
-                    const int e = (31 - __clz(vk)) >> 1;
-                    const uint32_t below = (1u << (2 * e)) - 1;
-                    const uint32_t before = __popc(v0 & below) + (R >= 2 ? __popc(v1 & below) : 0u) +
-                                            (R >= 3 ? __popc(v2 & below) : 0u) + full * (uint32_t)e;
-                    gpos[k] = (int)(ex + before) + (R - 1 - k);
-                }
-            }
-            run += __shfl_sync(0xffffffffu, incl, 31);
+            for (int j = 0; j < kWords; j++) cw[j] = lead_word16(lead, first + kNbPer * j, h.L);
         }
+        uint32_t mine = 0, lastw[3] = {0, 0, 0}, lastc[3] = {0, 0, 0};   // per byte lane: its last word and the bytes before it
+        int lastn[3] = {0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < kWords; j++) {
+            const unsigned long long f = first + kNbPer * j;
+            const int nv = f >= h.n ? 0 : (h.n - f < kNbPer ? (int)(h.n - f) : kNbPer);
+            const RunLeads<kNbPer> l(cw[j], nv, R);
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                if (k == 0 ? l.v0 : k == 1 ? l.v1 : l.v2) {
+                    lastw[k] = cw[j];
+                    lastc[k] = mine;
+                    lastn[k] = nv;
+                }
+            mine += l.bytes();
+        }
+        const uint32_t incl = warp_inclusive_sum(mine);
+        run = __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            if (lastn[k]) {
+                const RunLeads<kNbPer> l(lastw[k], lastn[k], R);
+                gpos[k] = (int)(incl - mine + lastc[k] + l.last_at(k));
+            }
     }
     unsigned long long own = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        int p = gpos[k];
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) p = max(p, __shfl_xor_sync(0xffffffffu, p, d));
+        const int p = __reduce_max_sync(0xffffffffu, gpos[k]);
         own |= (unsigned long long)(p + 1) << (21 * k);
     }
     if (lane == 0) {
@@ -601,25 +598,34 @@ __global__ void __launch_bounds__(kNbThreads) k_nb_count(const uint8_t* __restri
         s_own[warp] = own;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long pa = 0, pb = 0;
-        for (int w = 0; w < kTpg; w++) {
-            const long long t = (long long)blockIdx.x * kTpg + w;
-            if (t >= (long long)ntiles) break;
-            const unsigned long long o = s_own[w];
-            aux[3 * t] = pa;
-            aux[3 * t + 1] = pb;
-            aux[3 * t + 2] = o;
-            tcnt[t] = s_cnt[w];
-            pa += s_cnt[w];
-            unsigned long long wr = 0;
+    if (threadIdx.x < 32) {   // the group's prefixes: lane w holds tile w (0 past the last)
+        const long long t = (long long)blockIdx.x * kTpg + lane;
+        const bool in = lane < kTpg && t < (long long)ntiles;
+        const unsigned long long o = in ? s_own[lane] : 0ull;
+        const uint32_t c = in ? s_cnt[lane] : 0u;
+        unsigned long long pa = c, pb = 0;
 #pragma unroll
-            for (int k = 0; k < 3; k++)
-                if ((o >> (21 * k)) & 0x1FFFFF) wr |= (unsigned long long)(t + 1) << (21 * k);
-            pb = Max3x21Op::op(pb, wr);
+        for (int k = 0; k < 3; k++)
+            if ((o >> (21 * k)) & 0x1FFFFF) pb |= (unsigned long long)(t + 1) << (21 * k);
+#pragma unroll
+        for (int d = 1; d < kTpg; d <<= 1) {
+            const unsigned long long oa = __shfl_up_sync(0xffffffffu, pa, d), ob = __shfl_up_sync(0xffffffffu, pb, d);
+            if (lane >= d) {
+                pa += oa;
+                pb = Max3x21Op::op(ob, pb);
+            }
         }
-        gsum[blockIdx.x] = pa;
-        gwr[blockIdx.x] = pb;
+        if (lane == kTpg - 1) {
+            gsum[blockIdx.x] = pa;
+            gwr[blockIdx.x] = pb;
+        }
+        const unsigned long long eb = __shfl_up_sync(0xffffffffu, pb, 1);
+        if (in) {
+            aux[3 * t] = pa - c;
+            aux[3 * t + 1] = lane ? eb : 0ull;
+            aux[3 * t + 2] = o;
+            tcnt[t] = c;
+        }
     }
 }
 
@@ -733,10 +739,11 @@ __global__ void k_nb_carry(const uint8_t* __restrict__ s, unsigned long long len
 // iteration and its mid bytes copied with cp.async into the second staging
 // buffer while the current tile decodes.
 template <typename T>
-constexpr int nb_dec_stage_bytes() { return ((kNbTile * (int)sizeof(T) + 48) + 15) / 16 * 16; }
+constexpr int nb_dec_stage_bytes() { return ((kNbTile * (int)sizeof(T) + 64) + 15) / 16 * 16; }
+constexpr uint32_t kNbFront = 16;   // bytes before a tile's (the run decoder reads up to eight back)
 
 template <typename T>
-__global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 3 : 2)
+__global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2)
     k_nb_decode(const uint8_t* __restrict__ s, unsigned long long len, const NonBlockedHdr* hp,
                 const uint32_t* __restrict__ tcnt, const unsigned long long* __restrict__ aux,
                 const unsigned long long* __restrict__ gsum, T* out) {
@@ -744,18 +751,18 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 3 : 2)
     using EL = Elem<T>;
     using U = typename EL::U;
     constexpr int W = EL::W;
-    constexpr int TOPSH = 8 * (W - 3);
     extern __shared__ __align__(16) uint8_t nb_dyn[];   // two staging buffers of nb_dec_stage_bytes<T>()
     __shared__ uint32_t s_sum[8];
     __shared__ uint32_t s_wv[8], s_wm[8];   // per warp: last written top bytes, their byte mask
+    __shared__ uint32_t lut_ld[512];
     const NonBlockedHdr h = *hp;
     if (!h.ok) return;
-    int R, sft;
-    split_reqlen(h.reqLength, &R, &sft);
-    if (R > W) return;
+    if (h.reqLength > 8 * W) return;
+    const int R = run_bytes<T>(h.reqLength);
     const long long ntiles = (long long)((h.n + kNbTile - 1) / kNbTile);
     long long tile = blockIdx.x;
     if (tile >= ntiles) return;
+    lead_table_init(lut_ld);   // (the first tile's barriers come before its use)
     const uint8_t* lead = s + 17;
     const uint8_t* mid = s + h.mid_off;
     const uint8_t* send = s + len;
@@ -769,7 +776,7 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 3 : 2)
         const uint32_t sh = (uint32_t)((uintptr_t)src & 15);
         const uint8_t* gbase = src - sh;
         const uint32_t nch = (sh + tot + 15) >> 4;
-        uint8_t* stg = stage(k);
+        uint8_t* stg = stage(k) + kNbFront;
         for (uint32_t c = threadIdx.x; c < nch; c += kNbThreads) {
             const uint8_t* lo = gbase + (c << 4);
             if (lo >= s && lo + 16 <= send) cp_async16(stg + (c << 4), lo);
@@ -794,7 +801,6 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 3 : 2)
     words(tile, cd0, ga0, la0, cy0, tot0);
     if (tile + G < ntiles) words(tile + G, cd1, ga1, la1, cy1, tot1);
     copy_in(0, ga0 + la0, tot0);
-    const uint32_t full = R > 3 ? (uint32_t)(R - 3) : 0u;
     for (int it = 0;; it++) {
         const bool more = tile + G < ntiles;
         // the words of the tile after next, in flight during this tile
@@ -804,52 +810,20 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 3 : 2)
         const uint32_t codes = cd0, carry = cy0;
         const unsigned long long base = ga0 + la0;
         const unsigned long long first = (unsigned long long)tile * kNbTile + threadIdx.x * kNbPer;
-        // lanes written by this thread's values: lane W-1-k by a value with lead <= k
-        uint32_t mine, sm;
-        {
-            const uint32_t valid = valid_pairs(first, h.n);
-            const uint32_t lo = codes & 0x55555555u, hi = (codes >> 1) & 0x55555555u;
-            const uint32_t m0 = ~(lo | hi) & valid, m1 = ~hi & valid, m2 = ~(lo & hi) & valid;
-            mine = __popc(m0) + (R >= 2 ? __popc(m1) : 0u) + (R >= 3 ? __popc(m2) : 0u) + full * __popc(valid);
-            sm = (m2 ? 0xFFu : 0u) | (m1 ? 0xFF00u : 0u) | (m0 ? 0xFF0000u : 0u);
-        }
+        const int nv = first >= h.n ? 0 : (h.n - first < kNbPer ? (int)(h.n - first) : kNbPer);
+        const RunLeads<kNbPer> leads(codes, nv, R);
+        const uint32_t mine = leads.bytes();
         uint32_t total;
         const uint32_t ex = cta_excl_sum32(mine, &total, s_sum);   // one barrier
         if (more) copy_in(it + 1, ga1 + la1, tot1);
         else cp_async_commit();   // an empty group: the wait below still means "this tile's copy"
         cp_async_wait_group<1>();
         __syncthreads();   // this tile's bytes are staged
-        const uint32_t* buf = (const uint32_t*)stage(it);
-        uint32_t q = (uint32_t)((uintptr_t)(mid + base) & 15) + ex;
-        // Values past the end of the field (codes 0) are decoded like the
-        // others and never stored: they follow every real value, so nothing
-        // they change reaches one.
-        U sp[kNbPer];
-        U prev0 = 0;   // the thread's chain from an all-zero start: its top bytes summarise the thread
-#pragma unroll
-        for (int e = 0; e < kNbPer; e++) {
-            const uint32_t ld = (codes >> (8 * (e >> 2) + 6 - 2 * (e & 3))) & 3;
-            const int c0 = R - (int)ld;
-            const uint32_t c = c0 > 0 ? (uint32_t)c0 : 0u;
-            const uint32_t w0 = buf[q >> 2], w1 = buf[(q >> 2) + 1];
-            const uint32_t lo = __funnelshift_r(w0, w1, q << 3);   // the shift wraps: (q & 3) * 8
-            // the value's c bytes moved to the top of its R-byte window; the
-            // bytes that follow them (the next values') land in the top `ld`
-            // bytes, which the chain below takes from the previous value
-            if constexpr (sizeof(T) == 4) {
-                sp[e] = lo << (8 * (W - R));
-            } else {
-                const uint32_t w2 = buf[(q >> 2) + 2];
-                const uint32_t hi = __funnelshift_r(w1, w2, q << 3);
-                sp[e] = (((unsigned long long)hi << 32) | lo) << (8 * (W - R));
-            }
-            q += c;
-            const U inh = ~((~(U)0) >> (8 * ld));   // the top `ld` bytes come from the previous value
-            prev0 = (sp[e] & ~inh) | (prev0 & inh);
-        }
+        const uint32_t q0 = smem_u32(stage(it)) + kNbFront + (uint32_t)((uintptr_t)(mid + base) & 15) + ex;
         // (top bytes, byte mask) pairs: a later pair's masked bytes win,
         // masks accumulate -- one three-input logic op each
-        uint32_t sv = (uint32_t)(prev0 >> TOPSH) & 0xFFFFFFu, sw = sm;
+        uint32_t sv, sw;
+        leads.summary(q0, sv, sw);
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const uint32_t ov = __shfl_up_sync(0xffffffffu, sv, d), ow = __shfl_up_sync(0xffffffffu, sw, d);
@@ -870,26 +844,10 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 3 : 2)
         }
         const uint32_t ev = __shfl_up_sync(0xffffffffu, sv, 1), ew = __shfl_up_sync(0xffffffffu, sw, 1);
         if (lane) pv = (pv & ~ew) | (ev & ew);
-        U prev = (U)pv << TOPSH;
+        // (values past the end of the field are decoded like the others and never stored)
+        U sp[kNbPer];
         T v[kNbPer];
-        bool bad = false;
-#pragma unroll
-        for (int e = 0; e < kNbPer; e++) {
-            const uint32_t ld = (codes >> (8 * (e >> 2) + 6 - 2 * (e & 3))) & 3;
-            const U inh = ~((~(U)0) >> (8 * ld));
-            const U cur = (sp[e] & ~inh) | (prev & inh);
-            sp[e] = cur << sft;
-            v[e] = EL::add(EL::of(sp[e]), med);
-            if constexpr (sizeof(T) != 4) bad |= inf_or_nan(v[e]);   // (integer test, infinities too)
-            prev = cur;
-        }
-        if constexpr (sizeof(T) == 4) {   // a NaN anywhere: three-input max with NaN propagation
-            float hn = v[0];
-#pragma unroll
-            for (int e = 1; e + 1 < kNbPer; e += 2) hn = fmax3_nan(hn, v[e], v[e + 1]);
-            hn = fmax_nan(hn, v[kNbPer - 1]);
-            bad = hn != hn;
-        }
+        const bool bad = run_decode<T, kNbPer, true>(codes, nv, R, h.reqLength, q0, pv << 8, med, lut_ld, sp, v);
         if (__any_sync(0xffffffffu, bad)) {
 #pragma unroll
             for (int e = 0; e < kNbPer; e++) v[e] = xadd(EL::of(sp[e]), med);

@@ -404,4 +404,185 @@ struct RunOut {
     }
 };
 
+// 32-byte stores (sm_100 and later): a lane's 8 floats / 4 doubles at a
+// 32-byte aligned address, so that lanes writing consecutive 64-byte runs fill
+// whole 32-byte sectors.
+__device__ __forceinline__ void st_v8(float* p, const float* v) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void st_v8(double* p, const double* v) {
+    asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+                 : "memory");
+}
+
+// ------------------------------------------------------------------ runs, decoded
+
+// Lead-byte tables (a lead byte holds 4 codes, MSB first): 8 * the four leads
+// as bytes, value 0 in byte 0; at 256 + c the same with leads cut at 2.  A
+// value stores max(R - lead, 0) bytes, so 8 * R less the entry is its stored
+// bits, from the second table where R is 2 (no stream has a smaller one).
+__device__ __forceinline__ void lead_table_init(uint32_t* lut) {
+    for (int c = threadIdx.x; c < 256; c += blockDim.x) {
+        uint32_t a = 0, b = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t ld = (uint32_t)c >> (6 - 2 * i) & 3u;
+            a |= 8 * ld << (8 * i);
+            b |= 8 * (ld < 2 ? ld : 2u) << (8 * i);
+        }
+        lut[c] = a;
+        lut[256 + c] = b;
+    }
+}
+
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t lds8(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// Stored bytes of a value at lead 0, kept in range for streams that are not valid.
+template <typename T>
+__device__ __forceinline__ int run_bytes(int reqLength) {
+    const int R = (reqLength + 7) >> 3;
+    return R < 2 ? 2 : (R > Elem<T>::W ? Elem<T>::W : R);
+}
+
+// The lead codes of a run of up to E (at most 16) values as masks, value e's
+// bit at position 2e + 1: values with lead <= 0, 1, 2, i.e. those that store
+// byte lane W-1, W-2, W-3.
+template <int E>
+struct RunLeads {
+    uint32_t v0, v1, v2, low;   // low: bytes every value stores below the top three
+    int nv, R;
+    // codes: 4 to a byte, MSB first, chunk k in byte k; nv values
+    __device__ __forceinline__ RunLeads(uint32_t codes, int nv_, int R_) : nv(nv_), R(R_) {
+        const uint32_t c2 = vorder(codes & 0x55555555u), c1 = vorder((codes >> 1) & 0x55555555u);
+        const uint32_t valid = nv ? 0xAAAAAAAAu >> (32 - 2 * nv) : 0u;
+        v0 = ~(c1 | c2) & valid;
+        v1 = ~c1 & valid;
+        v2 = R >= 3 ? ~(c1 & c2) & valid : 0u;
+        low = R > 3 ? (uint32_t)(R - 3) : 0u;
+    }
+    // bytes the run stores
+    __device__ __forceinline__ uint32_t bytes() const { return __popc(v0) + __popc(v1) + __popc(v2) + low * (uint32_t)nv; }
+    // the top three bytes as the run leaves them (v, zero where it wrote none)
+    // and a mask of the ones it wrote (w); q0: shared address of its first byte
+    __device__ __forceinline__ void summary(uint32_t q0, uint32_t& v, uint32_t& w) const {
+        v = 0;
+        w = 0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            if (k == 0 ? v0 : k == 1 ? v1 : v2) {
+                v |= lds8(q0 + last_at(k)) << (16 - 8 * k);
+                w |= 0xFFu << (16 - 8 * k);
+            }
+        }
+    }
+    // where in the run's bytes the last value that stored byte lane W-1-k put it (there is one)
+    __device__ __forceinline__ uint32_t last_at(int k) const {
+        const int top = 31 - __clz(k == 0 ? v0 : k == 1 ? v1 : v2);
+        const uint32_t before = (1u << top) - 1u;
+        return __popc(v0 & before) + __popc(v1 & before) + __popc(v2 & before) + low * (uint32_t)(top >> 1) +
+               (uint32_t)(R - 1 - k);
+    }
+};
+
+// One pass over a run: cur, the values' bits less the median, and v, their
+// sums with it.  q0: shared address of the run's first stored byte (the reads
+// start up to eight bytes before it); carry: the top 32 bits of the value before
+// (three bytes of them count).  Returns whether a sum may be a NaN: the x86
+// rules then decide (nan_rule).  FULL: nv is E.
+template <typename T, int E, bool FULL>
+__device__ __forceinline__ bool run_decode(uint32_t codes, int nv, int R, int reqLength, uint32_t q0, uint32_t carry,
+                                           T med, const uint32_t* lut_ld, typename Elem<T>::U (&cur)[E], T (&v)[E]) {
+    using EL = Elem<T>;
+    using U = typename EL::U;
+    constexpr int W = EL::W;
+    constexpr int NC = E / 4;
+    uint32_t q8 = 8 * q0;   // bit address of the next stored byte
+    const uint32_t* lut_cnt = lut_ld + (R == 2 ? 256 : 0);
+    const uint32_t R8 = (uint32_t)R * 0x08080808u;
+    unsigned long long nan2 = 0;
+    if constexpr (sizeof(T) == 4) {
+        const int down = reqLength > 32 ? 0 : (reqLength < 1 ? 31 : 32 - reqLength);   // `run` ends in the value's required bits
+        // (the shift by `down` is a multiplication: the integer pipe sets the pace, the FMA pipe has room)
+        const uint32_t scale = 1u << down;
+        uint32_t run = carry >> (32 - 8 * R);
+        // the word before the one the position lies in, and that word
+        uint32_t sp = q0 & ~3u;
+        uint32_t wa = lds32(sp - 4), wb = lds32(sp);
+#pragma unroll
+        for (int k = 0; k < NC; k++) {
+            uint32_t cnt8 = R8 - lut_cnt[byte_of(codes, k)];
+            if constexpr (!FULL) cnt8 &= low_bytes_mask(nv - 4 * k);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t n8 = byte_of(cnt8, i);
+                const uint32_t qn = q8 + n8;
+                // (predicated: the position crosses into the next word)
+                asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tlop3.or.b32 t|p, %3, %4, -32, 0x28, 0;\n\t"
+                             "@p mov.b32 %0, %1;\n\t@p ld.shared.u32 %1, [%2+4];\n\t@p add.u32 %2, %2, 4;\n\t}"
+                             : "+r"(wa), "+r"(wb), "+r"(sp)
+                             : "r"(qn), "r"(q8)
+                             : "memory");
+                q8 = qn;
+                const uint32_t y = __funnelshift_r(wa, wb, q8);   // the four bytes before q8
+                run = __funnelshift_lc(y, __funnelshift_rc(run, 0u, n8), n8);
+                asm("mul.lo.u32 %0, %1, %2;" : "=r"(cur[4 * k + i]) : "r"(run), "r"(scale));
+            }
+        }
+        // the sums, two to an instruction, and a word that is NaN if any sum is one (or an infinity)
+        asm("mov.b64 %0, {%1, %1};" : "=l"(nan2) : "f"(0.0f));
+#pragma unroll
+        for (int e = 0; e < E; e += 2)
+            asm("{\n\t.reg .b64 a, b, z;\n\tmov.b64 a, {%3, %4};\n\tmov.b64 b, {%5, %5};\n\tmov.b64 z, {%6, %6};\n\t"
+                "add.rn.f32x2 a, a, b;\n\tfma.rn.f32x2 %2, a, z, %2;\n\tmov.b64 {%0, %1}, a;\n\t}"
+                : "=f"(v[e]), "=f"(v[e + 1]), "+l"(nan2)
+                : "r"(cur[e]), "r"(cur[e + 1]), "f"(med), "f"(0.0f));
+    } else {
+        const int s = reqLength & 7 ? 8 - (reqLength & 7) : 0;
+        const U keep = ~(U)0 << (8 * (W - R));
+        uint32_t prev = carry;   // the previous value's top 32 bits
+#pragma unroll
+        for (int k = 0; k < NC; k++) {
+            const uint32_t code = byte_of(codes, k), ld8 = lut_ld[code];
+            uint32_t cnt8 = R8 - lut_cnt[code];
+            if constexpr (!FULL) cnt8 &= low_bytes_mask(nv - 4 * k);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                q8 += byte_of(cnt8, i);
+                const uint32_t l8 = byte_of(ld8, i);
+                const uint32_t a = (q8 >> 3) & ~3u;
+                const uint32_t w0 = lds32(a - 8), w1 = lds32(a - 4), w2 = lds32(a);
+                const uint32_t ylo = __funnelshift_r(w0, w1, q8), yhi = __funnelshift_r(w1, w2, q8);   // the eight bytes before q8
+                const uint32_t hi = __funnelshift_r(yhi, __funnelshift_l(prev, 0u, l8), l8);
+                const uint32_t lo = __funnelshift_r(ylo, yhi, l8);
+                const U u = (((U)hi << 32) | lo) & keep;
+                prev = hi;
+                cur[4 * k + i] = u << s;
+                v[4 * k + i] = EL::add(EL::of(cur[4 * k + i]), med);
+            }
+        }
+    }
+    // a NaN (or infinite) result anywhere
+    if constexpr (sizeof(T) == 4) {
+        const float a = __uint_as_float((uint32_t)nan2) + __uint_as_float((uint32_t)(nan2 >> 32));   // zero, or NaN
+        return a != a;
+    } else {
+        // (integer test: a compare costs the FP64 pipe as much as the addition)
+        bool bad = false;
+#pragma unroll
+        for (int e = 0; e < E; e++) bad |= inf_or_nan(v[e]);
+        return bad;
+    }
+}
+
 }  // namespace szxg
