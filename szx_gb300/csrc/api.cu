@@ -167,6 +167,7 @@ size_t bound_for(int mode, int dtype, size_t n, int bs) {
 }
 
 __global__ void k_ws_clear(ClearList c) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t nthr = (size_t)gridDim.x * blockDim.x;
     for (int r = 0; r < c.n; r++) {
@@ -189,7 +190,7 @@ cudaError_t launch_ws_clear(const ClearList& c, cudaStream_t s) {
 }
 
 // Enqueue compress; the result record lands in res_out (device; default
-// ws.result).  One launch clears what the passes expect zeroed (the
+// ws.result).  One launch (for a small field the value-range pass itself) clears what the passes expect zeroed (the
 // value-range pass's ticket and the result record among it), so the
 // value-range pass and the encoder skip their own clears.
 static int enqueue_compress(int mode, int dtype, const void* d_x, size_t n, int bs, int err_mode, float abs_eb,
@@ -203,17 +204,20 @@ static int enqueue_compress(int mode, int dtype, const void* d_x, size_t n, int 
         c.bytes[c.n] = sizeof(StreamResult);
         c.n++;
     }
-    if ((e = launch_ws_clear(c, s)) != cudaSuccess) return cuda_fail(e);
+    const bool ranged = mode == kNonBlocked || err_mode == REL;
+    if (ranged && range_is_small(dtype, n)) {
+        if ((e = launch_range_small(dtype, d_x, n, err_mode, abs_eb, rel, ws, c, s)) != cudaSuccess) return cuda_fail(e);
+    } else {
+        if ((e = launch_ws_clear(c, s)) != cudaSuccess) return cuda_fail(e);
+        if (ranged && (e = launch_range(dtype, d_x, n, err_mode, abs_eb, rel, ws, s, true)) != cudaSuccess)
+            return cuda_fail(e);
+    }
     if (mode == kNonBlocked) {
-        if ((e = launch_range(dtype, d_x, n, err_mode, abs_eb, rel, ws, s, true)) != cudaSuccess) return cuda_fail(e);
         if ((e = launch_nonblocked_encode(dtype, d_x, n, d_out, cap, ws, s, true, res_out)) != cudaSuccess)
             return cuda_fail(e);
         return SZXG_OK;
     }
-    bool use_params = err_mode == REL;
-    if (use_params && (e = launch_range(dtype, d_x, n, err_mode, abs_eb, rel, ws, s, true)) != cudaSuccess)
-        return cuda_fail(e);
-    if ((e = launch_blocked_encode(mode, dtype, d_x, n, bs, use_params, abs_eb, d_out, cap, ws, s, true, res_out)) !=
+    if ((e = launch_blocked_encode(mode, dtype, d_x, n, bs, ranged, abs_eb, d_out, cap, ws, s, true, res_out)) !=
         cudaSuccess)
         return cuda_fail(e);
     return SZXG_OK;

@@ -444,6 +444,7 @@ struct EncTile {
 template <typename T, int G, bool MULTI, int TBYTES = kEncTileBytes>
 __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G, TBYTES>::kMinCtas)
     k_blocked_encode(EncArgs a) {
+    pdl_start();
     using TL = EncTile<T, G, TBYTES>;
     constexpr int TB = TL::kBlocks;
     constexpr int BPW = TL::kBpw;
@@ -804,6 +805,7 @@ __device__ __forceinline__ void asm_header(const BlkField* F, int layout, unsign
 }
 
 __global__ void __launch_bounds__(kAsmThreads) k_blocked_assemble(AsmArgs a) {
+    pdl_start();
     __shared__ uint32_t s_word[kAsmWords], s_pre[kAsmWords];
     __shared__ uint32_t s_wsum[kAsmThreads / 32];
     __shared__ long long s_t;
@@ -927,7 +929,8 @@ size_t blocked_bound(int layout, int dtype, size_t n, int bs) {
 
 // ctas_per_sm: 0 as many as fit, else at most that many.
 template <typename T, int G, int TBYTES = kEncTileBytes>
-static cudaError_t run_encode(EncArgs a, int ctas_per_sm, cudaStream_t s) {
+static cudaError_t run_encode(EncArgs a, const LaunchShape& shape, cudaStream_t s) {
+    const int ctas_per_sm = shape.enc_ctas_per_sm;
     using TL = EncTile<T, G, TBYTES>;
     static bool attr_set[64] = {false};
     static int per_sm[64] = {0};
@@ -954,8 +957,10 @@ static cudaError_t run_encode(EncArgs a, int ctas_per_sm, cudaStream_t s) {
     const size_t g = (size_t)sm_count() * cps;
     const int grid = (int)(a.total_tiles < g ? a.total_tiles : g);
     TraceScope tr("blocked_encode", s);
-    if (a.nf > 1) k_blocked_encode<T, G, true, TBYTES><<<grid, TL::kThreads, TL::kDynSmem, s>>>(a);
-    else k_blocked_encode<T, G, false, TBYTES><<<grid, TL::kThreads, TL::kDynSmem, s>>>(a);
+    if (a.nf == 1 && shape.after_kernel)
+        return launch_after(k_blocked_encode<T, G, false, TBYTES>, grid, TL::kThreads, TL::kDynSmem, s, a);
+    if (a.nf == 1) k_blocked_encode<T, G, false, TBYTES><<<grid, TL::kThreads, TL::kDynSmem, s>>>(a);
+    else k_blocked_encode<T, G, true, TBYTES><<<grid, TL::kThreads, TL::kDynSmem, s>>>(a);
     return cudaGetLastError();
 }
 // The one encoder tile variant a launch shape can pick besides the default:
@@ -1011,24 +1016,24 @@ cudaError_t launch_blocked_encode_fields(int layout, int dtype, int bs, int nf, 
     const int G = lanes_for_bs(dtype, bs);
     if (dtype == 0) {
         switch (G) {
-            case 1: e = run_encode<float, 1>(a, shape.enc_ctas_per_sm, s); break;
-            case 2: e = run_encode<float, 2>(a, shape.enc_ctas_per_sm, s); break;
-            case 4: e = run_encode<float, 4>(a, shape.enc_ctas_per_sm, s); break;
+            case 1: e = run_encode<float, 1>(a, shape, s); break;
+            case 2: e = run_encode<float, 2>(a, shape, s); break;
+            case 4: e = run_encode<float, 4>(a, shape, s); break;
             case 8:
                 e = shape.enc_tile_variant == 1
-                        ? run_encode<float, 8, kEncTileBytesSmall>(a, shape.enc_ctas_per_sm, s)
-                        : run_encode<float, 8>(a, shape.enc_ctas_per_sm, s);
+                        ? run_encode<float, 8, kEncTileBytesSmall>(a, shape, s)
+                        : run_encode<float, 8>(a, shape, s);
                 break;
-            default: e = run_encode<float, 16>(a, shape.enc_ctas_per_sm, s); break;
+            default: e = run_encode<float, 16>(a, shape, s); break;
         }
     } else {
         switch (G) {
-            case 1: e = run_encode<double, 1>(a, shape.enc_ctas_per_sm, s); break;
-            case 2: e = run_encode<double, 2>(a, shape.enc_ctas_per_sm, s); break;
-            case 4: e = run_encode<double, 4>(a, shape.enc_ctas_per_sm, s); break;
-            case 8: e = run_encode<double, 8>(a, shape.enc_ctas_per_sm, s); break;
-            case 16: e = run_encode<double, 16>(a, shape.enc_ctas_per_sm, s); break;
-            default: e = run_encode<double, 32>(a, shape.enc_ctas_per_sm, s); break;
+            case 1: e = run_encode<double, 1>(a, shape, s); break;
+            case 2: e = run_encode<double, 2>(a, shape, s); break;
+            case 4: e = run_encode<double, 4>(a, shape, s); break;
+            case 8: e = run_encode<double, 8>(a, shape, s); break;
+            case 16: e = run_encode<double, 16>(a, shape, s); break;
+            default: e = run_encode<double, 32>(a, shape, s); break;
         }
     }
     if (e != cudaSuccess) return e;
@@ -1044,8 +1049,7 @@ cudaError_t launch_blocked_encode_fields(int layout, int dtype, int bs, int nf, 
     const size_t gmax = (size_t)sm_count() * 4;
     const int ag = (int)(asm_total < gmax ? (asm_total ? asm_total : 1) : gmax);
     TraceScope tr("blocked_assemble", s);
-    k_blocked_assemble<<<ag, kAsmThreads, 0, s>>>(m);
-    return cudaGetLastError();
+    return launch_after(k_blocked_assemble, ag, kAsmThreads, 0, s, m);
 }
 
 ClearList blocked_enc_clear(const Workspace& ws, size_t nb) {
@@ -1085,8 +1089,10 @@ cudaError_t launch_blocked_encode(int layout, int dtype, const void* x, size_t n
     F.size_blk = ws.o_scr; F.med_blk = ws.m_scr; F.s_scr = ws.s_scr;
     F.tot = ws.totals;
     F.res = res_out ? res_out : ws.result;
+    LaunchShape shape;
+    shape.after_kernel = true;   // the clear, or the value-range pass
     return launch_blocked_encode_fields(layout, dtype, bs, 1, F, nullptr, nullptr, F.enc_tiles, F.asm_tiles,
-                                        ws.counters, ws.err, s, LaunchShape{});
+                                        ws.counters, ws.err, s, shape);
 }
 
 // ------------------------------------------------------------------ decode
@@ -1122,11 +1128,109 @@ __device__ BlockedHdr parse_blocked(const uint8_t* s, unsigned long long len, un
     return r;
 }
 
-__global__ void k_blocked_parse(const uint8_t* s, unsigned long long len, unsigned long long n,
-                                unsigned long long bs_expect, BlockedHdr* h, int* err) {
-    const BlockedHdr r = parse_blocked(s, len, n, bs_expect);
-    *h = r;
-    *err = r.ok ? kErrNone : kErrStream;
+// Parse and validate the mode-2 header (szx/src/szxd_float.cc:247-270).
+__device__ BlockedHdr parse_m2(const uint8_t* s, unsigned long long len, unsigned long long n,
+                               unsigned long long bs_expect) {
+    BlockedHdr r = {};
+    r.n = n;
+    r.ok = 0;
+    if (len >= 13 && s[3] == 0) {
+        r.bs = s[4];
+        r.nc = be64(s + 5);
+        if (r.bs >= 1 && (bs_expect == 0 || r.bs == bs_expect)) {
+            r.nb = (n + r.bs - 1) / r.bs;
+            r.sb = (r.nb + 7) / 8;
+            if (r.nc <= r.nb) {
+                r.nnc = r.nb - r.nc;
+                r.o_off = 13;
+                r.s_off = 13;
+                r.m_off = r.s_off + r.sb;
+                r.q_off = r.m_off + 4 * r.nc;
+                r.ok = r.q_off <= len;
+            }
+        }
+    }
+    return r;
+}
+
+// First kernel of a decode: the index kernel's counter and status words
+// cleared, the header parsed (thread 0) into *h and the error word set.
+__global__ void k_blocked_begin(ClearList c, const uint8_t* s, unsigned long long len, unsigned long long n,
+                                unsigned long long bs_expect, int m2, BlockedHdr* h, int* err) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (tid == 0) {
+        const BlockedHdr r = m2 ? parse_m2(s, len, n, bs_expect) : parse_blocked(s, len, n, bs_expect);
+        *h = r;
+        *err = r.ok ? kErrNone : kErrStream;
+    }
+    for (int r = 0; r < c.n; r++)
+        for (size_t i = tid; i < c.bytes[r] / 4; i += (size_t)gridDim.x * blockDim.x) ((uint32_t*)c.p[r])[i] = 0u;
+}
+
+// The whole of it for a stream of at most kIdxSmallBlocks blocks: header,
+// payload offsets and rank words by one CTA, without counter, status words or
+// their clearing.  (The parse, clear and index kernels took three launches.)
+constexpr int kIdxSmallThreads = 1024, kIdxSmallPer = 16;
+constexpr size_t kIdxSmallBlocks = (size_t)kIdxSmallThreads * kIdxSmallPer;
+__global__ void __launch_bounds__(kIdxSmallThreads) k_blocked_index_small(const uint8_t* s, unsigned long long len,
+                                                                          unsigned long long n,
+                                                                          unsigned long long bs_expect, int m2,
+                                                                          BlockedHdr* hp, int* err,
+                                                                          unsigned long long* P, uint32_t* RW) {
+    __shared__ uint32_t s_w[2][32];
+    __shared__ BlockedHdr s_h;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        const BlockedHdr r = m2 ? parse_m2(s, len, n, bs_expect) : parse_blocked(s, len, n, bs_expect);
+        s_h = r;
+        *hp = r;
+        *err = r.ok ? kErrNone : kErrStream;
+    }
+    __syncthreads();
+    const BlockedHdr h = s_h;
+    if (!h.ok || h.nb > kIdxSmallBlocks) {
+        if (h.ok && tid == 0) *err = kErrStream;   // (not reached: the host sized the launch by the same count)
+        return;
+    }
+    // payload sizes of ranks 16 tid .. (no size index in fastMode 2), population of state word tid
+    const uint32_t nnc = m2 ? 0u : (uint32_t)h.nnc, nw = (uint32_t)((h.nb + 31) / 32);
+    uint32_t v[kIdxSmallPer], mine = 0, pc = 0;
+#pragma unroll
+    for (int i = 0; i < kIdxSmallPer; i++) {
+        const uint32_t k = kIdxSmallPer * tid + i;
+        v[i] = k < nnc ? (uint32_t)s[h.o_off + 2 * k] | (uint32_t)s[h.o_off + 2 * k + 1] << 8 : 0u;
+        mine += v[i];
+    }
+    if ((uint32_t)tid < nw)
+        for (int j = 0; j < 4; j++) {
+            const uint32_t bi = 4 * tid + j;
+            if (bi < h.sb) pc += __popc((uint32_t)s[h.s_off + bi]);
+        }
+    const uint32_t ia = warp_inclusive_sum(mine), ib = warp_inclusive_sum(pc);
+    if (lane == 31) {
+        s_w[0][warp] = ia;
+        s_w[1][warp] = ib;
+    }
+    __syncthreads();
+    if (warp < 2) {
+        const uint32_t w = s_w[warp][lane];
+        s_w[warp][lane] = warp_inclusive_sum(w) - w;
+    }
+    __syncthreads();
+    unsigned long long run = (unsigned long long)s_w[0][warp] + ia - mine;   // < 16384 * 65536
+#pragma unroll
+    for (int i = 0; i < kIdxSmallPer; i++) {
+        const uint32_t k = kIdxSmallPer * tid + i;
+        if (k < nnc) P[k] = run;
+        run += v[i];
+        if (k + 1 == nnc) {
+            P[nnc] = run;
+            if (h.q_off + run > len) *err = kErrStream;
+        }
+    }
+    if ((uint32_t)tid < nw) RW[tid] = s_w[1][warp] + ib - pc;
 }
 
 // Every stream of a batch: one thread per field.
@@ -1219,6 +1323,7 @@ __global__ void __launch_bounds__(kIdxThreads) k_blocked_index(const uint8_t* s,
                                                                TileStatus stA, TileStatus stB,
                                                                unsigned long long* ctr, int* err,
                                                                unsigned long long len, int famA) {
+    pdl_start();
     __shared__ unsigned long long sm[8];
     __shared__ long long s_tile;
     __shared__ unsigned long long s_base;
@@ -1412,6 +1517,7 @@ enum : uint8_t { kBlkConst = 0, kBlkCoded = 1, kBlkNone = 2 };
 
 template <typename T, int G, bool MULTI>
 __global__ void __launch_bounds__(kDecThreadsP, kDecCtasPerSm) k_blocked_decode(DecArgs a) {
+    pdl_start();
     using TL = DecTileV<T, G>;
     constexpr int TB = TL::kBlocks;
     constexpr int NS = TL::kStages;
@@ -1769,8 +1875,7 @@ static cudaError_t run_decode(const uint8_t* s, size_t len, size_t nb, const Wor
     a.s = s; a.len = len; a.hdr = ws.bhdr; a.P = ws.p_off; a.RW = ws.rank_w; a.out = out;
     a.native_medians = native; a.err = ws.err;
     TraceScope tr("blocked_decode", st);
-    k_blocked_decode<T, G, false><<<grid, kDecThreadsP, TL::kDynSmem, st>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_blocked_decode<T, G, false>, grid, kDecThreadsP, TL::kDynSmem, st, a);
 }
 
 template <typename T, int G>
@@ -1866,36 +1971,42 @@ cudaError_t launch_blocked_decode(int layout, int dtype, const uint8_t* d_stream
     if (bs < 1 || bs > 256 || n == 0) return cudaErrorInvalidValue;
     const bool m2 = layout == kBlocked;
     cudaError_t e;
-    {
-        ClearList c{};   // the index kernel's tile counter and both look-backs' status words
-        c.p[0] = ws.counters;
-        c.bytes[0] = sizeof(unsigned long long);
-        c.p[1] = ws.st_word;
-        c.bytes[1] = sizeof(unsigned long long) * ws.status_tiles;
-        c.p[2] = ws.st2_word;
-        c.bytes[2] = sizeof(unsigned long long) * ws.status2_tiles;
-        c.n = 3;
-        if ((e = launch_ws_clear(c, s)) != cudaSuccess) return e;
-    }
-    {
-        TraceScope tr("blocked_parse", s);
-        if (m2) k_m2_parse<<<1, 1, 0, s>>>(d_stream, len, n, (unsigned long long)bs, ws.bhdr, ws.err);
-        else k_blocked_parse<<<1, 1, 0, s>>>(d_stream, len, n, (unsigned long long)bs, ws.bhdr, ws.err);
-    }
-    {
-        int ig = sm_count() * 4;
+    const size_t nb = (n + bs - 1) / bs;
+    if (nb <= kIdxSmallBlocks) {
         TraceScope tr("blocked_index", s);
-        k_blocked_index<<<ig, kIdxThreads, 0, s>>>(d_stream, ws.bhdr, ws.p_off, ws.rank_w,
-                                                    TileStatus{ws.st_word, ws.st_agg2, ws.st_inc2},
-                                                    TileStatus{ws.st2_word, ws.st2_agg2, ws.st2_inc2},
-                                                    &ws.counters[0], ws.err, len, m2 ? 0 : 1);
+        k_blocked_index_small<<<1, kIdxSmallThreads, 0, s>>>(d_stream, len, n, (unsigned long long)bs, m2 ? 1 : 0,
+                                                             ws.bhdr, ws.err, ws.p_off, ws.rank_w);
+    } else {
+        {
+            // the index kernel's tile counter and both look-backs' status words
+            const size_t ta = (nb + kIdxPerTile - 1) / kIdxPerTile, tb = ((nb + 31) / 32 + kIdxPerTile - 1) / kIdxPerTile;
+            ClearList c{};
+            c.p[0] = ws.counters;
+            c.bytes[0] = sizeof(unsigned long long);
+            c.p[1] = ws.st_word;
+            c.bytes[1] = sizeof(unsigned long long) * ta;
+            c.p[2] = ws.st2_word;
+            c.bytes[2] = sizeof(unsigned long long) * tb;
+            c.n = 3;
+            TraceScope tr("blocked_parse", s);
+            k_blocked_begin<<<(unsigned)((2 * ta + 255) / 256), 256, 0, s>>>(c, d_stream, len, n, (unsigned long long)bs,
+                                                                            m2 ? 1 : 0, ws.bhdr, ws.err);
+        }
+        const size_t tiles = (m2 ? 0 : (nb + kIdxPerTile - 1) / kIdxPerTile) + ((nb + 31) / 32 + kIdxPerTile - 1) / kIdxPerTile;
+        const size_t cap = (size_t)sm_count() * 4;
+        TraceScope tr("blocked_index", s);
+        if ((e = launch_after(k_blocked_index, (unsigned)(tiles < cap ? tiles : cap), kIdxThreads, 0, s, d_stream, ws.bhdr,
+                              ws.p_off, ws.rank_w, TileStatus{ws.st_word, ws.st_agg2, ws.st_inc2},
+                              TileStatus{ws.st2_word, ws.st2_agg2, ws.st2_inc2}, &ws.counters[0], ws.err,
+                              (unsigned long long)len, m2 ? 0 : 1)) != cudaSuccess)
+            return e;
     }
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (m2 && (e = launch_m2_offsets(dtype, d_stream, len, n, bs, ws.m2, ws.m2_bytes, ws, s)) != cudaSuccess)
         return e;
     // bs comes from the stream header (read by the caller); the device header
     // is validated again by every kernel and a mismatch is reported, not used.
     const int native = layout == kRandomAccessNative;
-    const size_t nb = (n + bs - 1) / bs;
     const int G = dec_lanes(dtype, bs);
     if (dtype == 0) {
         switch (G) {

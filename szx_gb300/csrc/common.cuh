@@ -13,6 +13,16 @@ namespace szxg {
 
 constexpr int kWarp = 32;
 
+// Programmatic dependent launch: a kernel launched by launch_after() may be
+// scheduled while the kernel before it in the stream still runs; it waits here,
+// before its first access to memory, until that kernel has finished, and then
+// lets its own successor be scheduled.  (After a plain launch the wait returns
+// at once.)
+__device__ __forceinline__ void pdl_start() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ------------------------------------------------------------------ element traits
 
 template <typename T> struct Elem;

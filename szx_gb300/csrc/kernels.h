@@ -187,8 +187,6 @@ size_t m2_ws_bytes(int dtype, size_t n, int bs, size_t len);
 // (header already parsed into ws.bhdr).
 cudaError_t launch_m2_offsets(int dtype, const uint8_t* d_stream, size_t len, size_t n, int bs, void* m2ws,
                               size_t m2wsb, const Workspace& ws, cudaStream_t s);
-__global__ void k_m2_parse(const uint8_t* s, unsigned long long len, unsigned long long n,
-                           unsigned long long bs_expect, BlockedHdr* h, int* err);
 
 size_t ws_bytes(int layout, int dtype, size_t n, int bs);
 Workspace ws_carve(void* base, int layout, int dtype, size_t n, int bs);
@@ -209,6 +207,12 @@ cudaError_t launch_ws_clear(const ClearList& c, cudaStream_t s);
 // cleared: the caller has zeroed counters[3] (the CTA ticket) already.
 cudaError_t launch_range(int dtype, const void* x, size_t n, int err_mode, float abs_eb, float rel,
                          const Workspace& ws, cudaStream_t s, bool cleared = false);
+
+// The same for a small field (range_is_small), clearing the listed regions in
+// the same launch.
+bool range_is_small(int dtype, size_t n);
+cudaError_t launch_range_small(int dtype, const void* x, size_t n, int err_mode, float abs_eb, float rel,
+                               const Workspace& ws, const ClearList& c, cudaStream_t s);
 
 // Blocked encode (layouts 2, 3, 4): stats + encode + placement + header assembly.
 // d_out must hold blocked_bound() bytes; the stream lands at d_out + result.offset.
@@ -236,6 +240,7 @@ struct LaunchShape {
     int enc_tile_variant = 0;
     int enc_ctas_per_sm = 0;
     int dec_ctas_per_sm = 0;
+    bool after_kernel = false;   // the encoder follows another kernel of the same call (launch_after)
 };
 int blocked_tile_blocks(int dtype, int bs, int tile_variant = 0);
 cudaError_t launch_blocked_encode_fields(int layout, int dtype, int bs, int nf, const BlkField& one,
@@ -274,6 +279,24 @@ cudaError_t launch_nonblocked_decode(int dtype, const uint8_t* d_stream, size_t 
                                      const Workspace& ws, cudaStream_t s);
 
 int sm_count();
+
+// Launch of a kernel that begins with pdl_start() right behind another one of
+// this library's kernels on the stream: its launch overlaps that kernel's end
+// (2-3 us less between two dependent kernels).
+template <typename... K, typename... A>
+inline cudaError_t launch_after(void (*k)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k, static_cast<K>(args)...);
+}
 
 // Records CUDA events around one kernel launch when tracing is enabled
 // (SZxG_trace_enable); a no-op otherwise.

@@ -50,12 +50,6 @@ struct M2Geom {
     int list;                  // words of a segment's block list
 };
 
-__device__ __forceinline__ unsigned long long be64d(const uint8_t* p) {
-    unsigned long long v = 0;
-    for (int i = 0; i < 8; i++) v = (v << 8) | p[i];
-    return v;
-}
-
 // Payload bytes of a block of blen values from the sums over its lead codes
 // (l: of the codes, n3: how many are 3).  A value stores max(R - lead, 0)
 // bytes; R is at least 2 (reqLength >= 9), so only lead 3 at R = 2 clips.
@@ -197,32 +191,6 @@ __device__ __forceinline__ void m2_lut_init(uint8_t* lut) {
 
 }  // namespace
 
-// Parse and validate the mode-2 header (szx/src/szxd_float.cc:247-270).
-__global__ void k_m2_parse(const uint8_t* s, unsigned long long len, unsigned long long n,
-                           unsigned long long bs_expect, BlockedHdr* h, int* err) {
-    BlockedHdr r = {};
-    r.n = n;
-    r.ok = 0;
-    if (len >= 13 && s[3] == 0) {
-        r.bs = s[4];
-        r.nc = be64d(s + 5);
-        if (r.bs >= 1 && (bs_expect == 0 || r.bs == bs_expect)) {
-            r.nb = (n + r.bs - 1) / r.bs;
-            r.sb = (r.nb + 7) / 8;
-            if (r.nc <= r.nb) {
-                r.nnc = r.nb - r.nc;
-                r.o_off = 13;
-                r.s_off = 13;
-                r.m_off = r.s_off + r.sb;
-                r.q_off = r.m_off + 4 * r.nc;
-                r.ok = r.q_off <= len;
-            }
-        }
-    }
-    *h = r;
-    *err = r.ok ? kErrNone : kErrStream;
-}
-
 // Pass 1: one CTA per segment.  The candidate starts (offsets c < maxsize) with
 // a valid reqLength are gathered, and each is walked by one thread until it
 // has passed kM2Reach maximal blocks; that ends nearly all walks that are not
@@ -239,6 +207,7 @@ constexpr uint32_t kM2Reach = 4;
 __global__ void __launch_bounds__(kM2Threads) k_m2_walk(const uint8_t* s, const BlockedHdr* hp, M2Geom g, int W,
                                                         unsigned short* cnt_tab, unsigned long long* exit_lo,
                                                         unsigned long long* exit_hi, uint32_t* lists) {
+    pdl_start();
     extern __shared__ __align__(16) uint8_t m2_dyn[];
     __shared__ uint32_t s_lo, s_hi;
     __shared__ int s_n, s_places;
@@ -361,6 +330,7 @@ __global__ void __launch_bounds__(kM2Threads) k_m2_walk(const uint8_t* s, const 
 __global__ void k_m2_link(const BlockedHdr* hp, M2Geom g, const unsigned short* cnt_tab,
                           const unsigned long long* exit_lo, const unsigned long long* exit_hi,
                           unsigned long long* entry, unsigned int* cnt, unsigned int* ambiguous, unsigned int* redo) {
+    pdl_start();
     const unsigned long long j = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (j == 0) *redo = 0;
     const BlockedHdr h = *hp;
@@ -391,6 +361,7 @@ __global__ void k_m2_link(const BlockedHdr* hp, M2Geom g, const unsigned short* 
 constexpr int kM2ScanPer = 8;
 __global__ void __launch_bounds__(1024) k_m2_scan(unsigned long long nseg, const unsigned int* cnt,
                                                   unsigned long long* base) {
+    pdl_start();
     __shared__ unsigned long long s_w[32];
     unsigned long long carry = 0;
     for (unsigned long long j0 = 0; j0 < nseg; j0 += 1024 * kM2ScanPer) {
@@ -428,6 +399,7 @@ __global__ void __launch_bounds__(kM2Threads) k_m2_replay(const uint8_t* s, cons
                                                           const unsigned long long* base,
                                                           const unsigned int* ambiguous, const uint32_t* lists,
                                                           unsigned long long* Poff, unsigned int* redo) {
+    pdl_start();
     const BlockedHdr h = *hp;
     if (!h.ok) return;
     const unsigned long long j = ((unsigned long long)blockIdx.x * kM2Threads + threadIdx.x) >> 5;
@@ -484,6 +456,7 @@ __global__ void __launch_bounds__(kM2Threads) k_m2_replay(const uint8_t* s, cons
 // Fallback when the parallel passes disagree: the serial walk (one thread).
 __global__ void k_m2_serial(const uint8_t* s, const BlockedHdr* hp, M2Geom g, int W, const unsigned int* redo,
                             unsigned long long* Poff, int* err) {
+    pdl_start();
     __shared__ uint8_t lut[9 * 256];
     m2_lut_init(lut);
     __syncthreads();
@@ -572,19 +545,20 @@ cudaError_t launch_m2_offsets(int dtype, const uint8_t* d_stream, size_t len, si
     }
     {
         TraceScope tr("m2_walk", s);
-        k_m2_walk<<<(unsigned)g.nseg, kM2Threads, dyn, s>>>(d_stream, ws.bhdr, g, W, cnt_tab, exit_lo, exit_hi,
-                                                            lists);
+        e = launch_after(k_m2_walk, (unsigned)g.nseg, kM2Threads, dyn, s, d_stream, ws.bhdr, g, W, cnt_tab, exit_lo, exit_hi,
+                         lists);
     }
-    k_m2_link<<<(unsigned)((g.nseg + 255) / 256), 256, 0, s>>>(ws.bhdr, g, cnt_tab, exit_lo, exit_hi, entry, cnt, amb,
-                                                               redo);
-    k_m2_scan<<<1, 1024, 0, s>>>(g.nseg, cnt, base);
-    {
+    if (e == cudaSuccess)
+        e = launch_after(k_m2_link, (unsigned)((g.nseg + 255) / 256), 256, 0, s, ws.bhdr, g, cnt_tab, exit_lo, exit_hi, entry,
+                         cnt, amb, redo);
+    if (e == cudaSuccess) e = launch_after(k_m2_scan, 1, 1024, 0, s, g.nseg, cnt, base);
+    if (e == cudaSuccess) {
         TraceScope tr("m2_replay", s);
-        k_m2_replay<<<(unsigned)((g.nseg + kM2Threads / 32 - 1) / (kM2Threads / 32)), kM2Threads, 0, s>>>(
-            d_stream, ws.bhdr, g, W, entry, base, amb, lists, ws.p_off, redo);
+        e = launch_after(k_m2_replay, (unsigned)((g.nseg + kM2Threads / 32 - 1) / (kM2Threads / 32)), kM2Threads, 0, s,
+                         d_stream, ws.bhdr, g, W, entry, base, amb, lists, ws.p_off, redo);
     }
-    k_m2_serial<<<1, 256, 0, s>>>(d_stream, ws.bhdr, g, W, redo, ws.p_off, ws.err);
-    return cudaGetLastError();
+    if (e == cudaSuccess) e = launch_after(k_m2_serial, 1, 256, 0, s, d_stream, ws.bhdr, g, W, redo, ws.p_off, ws.err);
+    return e;
 }
 
 }  // namespace szxg

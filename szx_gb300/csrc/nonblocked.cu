@@ -170,6 +170,7 @@ constexpr int nb_stage_bytes() { return ((kNbTile * (int)sizeof(T) + 48) + 15) /
 
 template <typename T>
 __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encode(NbEncArgs a) {
+    pdl_start();
     using EL = Elem<T>;
     using U = typename EL::U;
     constexpr int W = EL::W;
@@ -474,18 +475,13 @@ cudaError_t launch_nonblocked_encode(int dtype, const void* x, size_t n, uint8_t
     int grid = (int)(ntiles < g ? ntiles : g);
     {
         TraceScope tr("nonblocked_encode", s);
-        if (dtype == 0) k_nb_encode<float><<<grid, kNbThreads, dyn, s>>>(a);
-        else k_nb_encode<double><<<grid, kNbThreads, dyn, s>>>(a);
+        return launch_after(dtype == 0 ? k_nb_encode<float> : k_nb_encode<double>, grid, kNbThreads, dyn, s, a);
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    // fold the error word into the result
-    return cudaSuccess;
 }
 
 // ------------------------------------------------------------------ decode
 
-__global__ void k_nb_parse(const uint8_t* s, unsigned long long len, unsigned long long n, NonBlockedHdr* h,
-                           int* err) {
+__device__ NonBlockedHdr parse_nb(const uint8_t* s, unsigned long long len, unsigned long long n) {
     NonBlockedHdr r = {};
     r.n = n;
     r.ok = 0;
@@ -499,8 +495,7 @@ __global__ void k_nb_parse(const uint8_t* s, unsigned long long len, unsigned lo
         r.ok = L == (n + 3) / 4 && r.mid_off <= len && r.reqLength >= 1 && r.reqLength <= 64;
         r.mid_len = r.ok ? len - r.mid_off : 0;
     }
-    *h = r;
-    *err = r.ok ? kErrNone : kErrStream;
+    return r;
 }
 
 __device__ __forceinline__ uint32_t lead_word(const uint8_t* lead, unsigned long long lb, unsigned long long L) {
@@ -531,7 +526,8 @@ __device__ __forceinline__ uint32_t lead_word16(const uint8_t* lead, unsigned lo
 // tile+1), gsum[g] / gwr[g] the group's totals.  Independent per group: no
 // look-back.
 template <typename T>
-__global__ void __launch_bounds__(kNbThreads) k_nb_count(const uint8_t* __restrict__ s, const NonBlockedHdr* hp,
+__global__ void __launch_bounds__(kNbThreads) k_nb_count(const uint8_t* __restrict__ s, unsigned long long len,
+                                                         unsigned long long n, NonBlockedHdr* hp, int* err,
                                                          uint32_t* __restrict__ tcnt,
                                                          unsigned long long* __restrict__ aux,
                                                          unsigned long long* __restrict__ gsum,
@@ -541,7 +537,12 @@ __global__ void __launch_bounds__(kNbThreads) k_nb_count(const uint8_t* __restri
     constexpr int kWords = kNbTile / (32 * kNbPer);   // words per lane
     __shared__ uint32_t s_cnt[kTpg];
     __shared__ unsigned long long s_own[kTpg];
-    const NonBlockedHdr h = *hp;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const NonBlockedHdr h = parse_nb(s, len, n);   // (every thread: the same loads, from cache)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {     // for the kernels that follow
+        *hp = h;
+        *err = h.ok ? kErrNone : kErrStream;
+    }
     if (!h.ok || h.reqLength > 8 * W) return;
     const int R = run_bytes<T>(h.reqLength);
     const unsigned long long ntiles = (h.n + kNbTile - 1) / kNbTile;
@@ -637,6 +638,7 @@ constexpr int kScanThreads = 512, kScanPer = 8;
 
 __global__ void __launch_bounds__(kScanThreads) k_nb_scan(const NonBlockedHdr* hp, unsigned long long* gsum,
                                                           unsigned long long* gwr, int* err) {
+    pdl_start();
     __shared__ unsigned long long s_a[kScanThreads / 32], s_b[kScanThreads / 32];
     const NonBlockedHdr h = *hp;
     if (!h.ok) return;
@@ -709,8 +711,9 @@ __global__ void __launch_bounds__(kScanThreads) k_nb_scan(const NonBlockedHdr* h
 // thread rewrites only its own tile's aux[3t+1] and reads only the other two
 // words of other tiles.
 __global__ void k_nb_carry(const uint8_t* __restrict__ s, unsigned long long len, const NonBlockedHdr* hp,
-                           unsigned long long* aux, const unsigned long long* __restrict__ gsum,
-                           const unsigned long long* __restrict__ gwr) {
+                           unsigned long long* aux, const unsigned long long* gsum,
+                           const unsigned long long* gwr) {
+    pdl_start();
     constexpr int kTpg = kNbThreads / 32;
     const NonBlockedHdr h = *hp;
     if (!h.ok) return;
@@ -745,8 +748,9 @@ constexpr uint32_t kNbFront = 16;   // bytes before a tile's (the run decoder re
 template <typename T>
 __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2)
     k_nb_decode(const uint8_t* __restrict__ s, unsigned long long len, const NonBlockedHdr* hp,
-                const uint32_t* __restrict__ tcnt, const unsigned long long* __restrict__ aux,
-                const unsigned long long* __restrict__ gsum, T* out) {
+                const uint32_t* tcnt, const unsigned long long* aux,
+                const unsigned long long* gsum, T* out) {
+    pdl_start();
     constexpr int kTpg = kNbThreads / 32;
     using EL = Elem<T>;
     using U = typename EL::U;
@@ -875,21 +879,20 @@ cudaError_t launch_nonblocked_decode(int dtype, const uint8_t* d_stream, size_t 
     unsigned long long* gsum = ws.st_word;                     // [ng] group byte totals, then prefixes
     unsigned long long* gwr = ws.st_word + ws.status_tiles;    // [ng] group latest writers, then prefixes
     {
-        TraceScope tr("nonblocked_parse", s);
-        k_nb_parse<<<1, 1, 0, s>>>(d_stream, len, n, ws.nhdr, ws.err);
-    }
-    {
         TraceScope tr("nonblocked_count", s);
-        if (dtype == 0) k_nb_count<float><<<(int)ng, kNbThreads, 0, s>>>(d_stream, ws.nhdr, tcnt, ws.tile_aux, gsum, gwr);
-        else k_nb_count<double><<<(int)ng, kNbThreads, 0, s>>>(d_stream, ws.nhdr, tcnt, ws.tile_aux, gsum, gwr);
+        if (dtype == 0) k_nb_count<float><<<(int)ng, kNbThreads, 0, s>>>(d_stream, len, n, ws.nhdr, ws.err, tcnt, ws.tile_aux, gsum, gwr);
+        else k_nb_count<double><<<(int)ng, kNbThreads, 0, s>>>(d_stream, len, n, ws.nhdr, ws.err, tcnt, ws.tile_aux, gsum, gwr);
     }
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     {
         TraceScope tr("nonblocked_scan", s);
-        k_nb_scan<<<1, kScanThreads, 0, s>>>(ws.nhdr, gsum, gwr, ws.err);
+        if ((e = launch_after(k_nb_scan, 1, kScanThreads, 0, s, ws.nhdr, gsum, gwr, ws.err)) != cudaSuccess) return e;
     }
     {
         TraceScope tr("nonblocked_carry", s);
-        k_nb_carry<<<(int)((ntiles + 255) / 256), 256, 0, s>>>(d_stream, len, ws.nhdr, ws.tile_aux, gsum, gwr);
+        if ((e = launch_after(k_nb_carry, (unsigned)((ntiles + 255) / 256), 256, 0, s, d_stream, (unsigned long long)len,
+                              ws.nhdr, ws.tile_aux, gsum, gwr)) != cudaSuccess)
+            return e;
     }
     static int per_sm[2][64] = {{0}};
     int dev = 0;
@@ -915,13 +918,11 @@ cudaError_t launch_nonblocked_decode(int dtype, const uint8_t* d_stream, size_t 
     {
         TraceScope tr("nonblocked_decode", s);
         if (dtype == 0)
-            k_nb_decode<float><<<grid, kNbThreads, dyn, s>>>(d_stream, len, ws.nhdr, tcnt, ws.tile_aux, gsum,
-                                                             (float*)d_out);
-        else
-            k_nb_decode<double><<<grid, kNbThreads, dyn, s>>>(d_stream, len, ws.nhdr, tcnt, ws.tile_aux, gsum,
-                                                              (double*)d_out);
+            return launch_after(k_nb_decode<float>, grid, kNbThreads, dyn, s, d_stream, (unsigned long long)len, ws.nhdr, tcnt,
+                                ws.tile_aux, gsum, (float*)d_out);
+        return launch_after(k_nb_decode<double>, grid, kNbThreads, dyn, s, d_stream, (unsigned long long)len, ws.nhdr, tcnt,
+                            ws.tile_aux, gsum, (double*)d_out);
     }
-    return cudaGetLastError();
 }
 
 }  // namespace szxg

@@ -1,0 +1,82 @@
+"""Call paths whose launches depend on the size: the one-cluster value range
+and the ticketed one, the one-CTA stream index and the persistent one, at and
+around the sizes where they change over; and compress and decompress captured
+in a CUDA graph and replayed on new values.  Streams and values equal the
+oracle's."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def szx():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for the gpu tests")
+    import szx_gb300
+    from szx_gb300 import build
+    build.build()
+    return szx_gb300
+
+
+def field(dt, n, seed):
+    rng = np.random.default_rng(seed)
+    x = np.sin(np.arange(n) / 300.0) + 0.01 * rng.normal(size=n)
+    for b in range(0, n - 300, 5000):
+        x[b:b + 300] = 0.25
+    x[n // 3] = -7.5
+    return x.astype(dt)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("mode", [1, 2, 3, 4])
+def test_sizes_around_the_changeovers(szx, dt, mode):
+    import torch
+    es = np.dtype(dt).itemsize
+    for n, bs in (((2 << 20) // es, 128), ((2 << 20) // es + 1, 128), (16384 * 32, 32), (16384 * 32 + 1, 32),
+                  (16384 * 4 - 3, 4), (16385 * 4, 4), (16384, 1), (16385, 1)):
+        x = field(dt, n, n % 97)
+        for off in (0, 1):
+            codec = szx.DeviceCodec(mode, dt, n, bs)
+            buf = torch.zeros(n + 1, dtype=torch.float32 if dt == np.float32 else torch.float64, device="cuda")
+            buf[off:off + n] = torch.from_numpy(x).cuda()
+            codec.ws.random_(0, 256)   # a workspace holds anything before a call
+            codec.compress(buf[off:off + n], szx.REL, 0.0, 1e-3)
+            s = codec.stream_bytes()
+            want = O.fast_compress_args(mode, x, 1, 0.0, 1e-3, bs)
+            assert s.cpu().numpy().tobytes() == want, (n, bs, off)
+            codec.ws.random_(0, 256)
+            y = codec.decompress(s, n)
+            assert codec.status() == 0, (n, bs, off)
+            z = O.decompress(mode, dt, want, n)
+            assert np.array_equal(y.cpu().numpy().view(np.uint8), z.view(np.uint8)), (n, bs, off)
+
+
+@pytest.mark.parametrize("mode", [1, 2, 3])
+@pytest.mark.parametrize("n", [50_000, 3_000_001])
+def test_captured_in_a_graph(szx, mode, n):
+    import torch
+    x = torch.from_numpy(field(np.float32, n, 1)).cuda()
+    codec = szx.DeviceCodec(mode, np.float32, n)
+    codec.compress(x, szx.REL, 0.0, 1e-3)
+    s = codec.stream_bytes().clone()
+    y = torch.empty(n, dtype=torch.float32, device="cuda")
+    dec = szx.DeviceCodec(mode, np.float32, n)
+    dec.decompress(s, n, y)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        codec.compress(x, szx.REL, 0.0, 1e-3)
+        dec.decompress(s, n, y)
+    for seed in (2, 3):
+        v = field(np.float32, n, seed)
+        x.copy_(torch.from_numpy(v))
+        y.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert codec.stream_bytes().cpu().numpy().tobytes() == O.fast_compress_args(mode, v, 1, 0.0, 1e-3, 128)
+        z = O.decompress(mode, np.float32, s.cpu().numpy().tobytes(), n)
+        assert dec.status() == 0 and np.array_equal(y.cpu().numpy().view(np.uint8), z.view(np.uint8))
