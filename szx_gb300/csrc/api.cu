@@ -173,7 +173,12 @@ __global__ void k_ws_clear(ClearList c) {
     for (int r = 0; r < c.n; r++) {
         uint32_t* p = (uint32_t*)c.p[r];
         const size_t words = c.bytes[r] / 4;
-        for (size_t i = tid; i < words; i += nthr) p[i] = 0u;
+        size_t i0 = 0;
+        if (((uintptr_t)p & 15) == 0) {
+            for (size_t i = tid; i < words / 4; i += nthr) ((uint4*)p)[i] = make_uint4(0u, 0u, 0u, 0u);
+            i0 = words / 4 * 4;
+        }
+        for (size_t i = i0 + tid; i < words; i += nthr) p[i] = 0u;
     }
 }
 

@@ -11,7 +11,8 @@
 // counter, so a field's tiles are always acquired before any later field's,
 // which is all the per-field look-back needs to make progress.
 //
-// Fields are grouped by size class (a table of value-count bounds, each with
+// Fields are grouped by size class, and neighbouring classes of one launch
+// shape share a launch (a table of value-count bounds, each with
 // its launch shape: encoder tile size and CTAs per SM of the encoder and the
 // decoder), and each class is one persistent launch per kernel with its own
 // shape.  The table comes from the tuning file written by the project's
@@ -113,8 +114,16 @@ LaunchShape batch_class_shape(int k) {
     return g_shapes[(size_t)k < g_shapes.size() ? (size_t)k : g_shapes.size() - 1].shape;
 }
 
+static bool same_shape(const LaunchShape& x, const LaunchShape& y) {
+    return x.enc_tile_variant == y.enc_tile_variant && x.enc_ctas_per_sm == y.enc_ctas_per_sm &&
+           x.dec_ctas_per_sm == y.dec_ctas_per_sm;
+}
+
 // The fields a compress run codes, grouped by class in a stable order, their
-// device table and tile map (per class: tiles numbered from 0, field
+// device table and tile map.  Neighbouring classes of one launch shape are one
+// part, i.e. one launch per kernel: each launch of a persistent kernel ends in
+// a tail of partly idle SMs (48 fields of 2^14..2^24 values in three launches
+// of one shape: 319 us).  (Per part: tiles numbered from 0, field
 // indices relative to the class's first table entry).
 cudaError_t batch_select(SZxG_Batch* b, int nActive, const int* h_idx, const float* h_eb, cudaStream_t s) {
     if (b->direction != 0 || nActive < 1 || nActive > b->nf) return cudaErrorInvalidValue;
@@ -132,23 +141,23 @@ cudaError_t batch_select(SZxG_Batch* b, int nActive, const int* h_idx, const flo
     b->h_tile_field.clear();
     for (int c = 0; c < ncls; c++) {
         if (by[c].empty()) continue;
-        BatchPart P;
-        P.shape = b->class_shape[c];
-        P.i0 = (int)b->run.size();
-        P.map0 = b->h_tile_field.size();
-        unsigned long long et = 0, at = 0;
+        // classes of one shape share a launch
+        if (b->parts.empty() || !same_shape(b->parts.back().shape, b->class_shape[c])) {
+            BatchPart P;
+            P.shape = b->class_shape[c];
+            P.i0 = (int)b->run.size();
+            P.map0 = b->h_tile_field.size();
+            b->parts.push_back(P);
+        }
+        BatchPart& P = b->parts.back();
         for (int f : by[c]) {
             BlkField F = b->tab[f];   // enc_tiles already for this class's tile size
-            F.enc_tile0 = et; et += F.enc_tiles;
-            F.asm_tile0 = at; at += F.asm_tiles;
-            for (unsigned long long t = 0; t < F.enc_tiles; t++)
-                b->h_tile_field.push_back((uint32_t)(b->run.size() - P.i0));
+            F.enc_tile0 = P.enc_total; P.enc_total += F.enc_tiles;
+            F.asm_tile0 = P.asm_total; P.asm_total += F.asm_tiles;
+            b->h_tile_field.insert(b->h_tile_field.end(), (size_t)F.enc_tiles, (uint32_t)(b->run.size() - P.i0));
             b->run.push_back(F);
         }
         P.i1 = (int)b->run.size();
-        P.enc_total = et;
-        P.asm_total = at;
-        b->parts.push_back(P);
     }
     // pageable sources: each copy is staged before the call returns, ordered after earlier runs on s
     cudaError_t e = cudaMemcpyAsync(b->d_fields, b->run.data(), sizeof(BlkField) * b->run.size(),
@@ -273,11 +282,15 @@ static SZxG_Batch* create_decode(int fastMode, int dataType, int blockSize, int 
     std::vector<DecField> tab(nf);
     for (size_t c = 0, k = 0; c < by.size(); c++) {
         if (by[c].empty()) continue;
-        BatchPart P;
-        P.shape = batch_class_shape((int)c);
-        P.i0 = (int)k;
-        P.map0 = b->h_tile_field.size();
-        unsigned long long it = 0, dt = 0;
+        const LaunchShape shape = batch_class_shape((int)c);
+        if (b->parts.empty() || !same_shape(b->parts.back().shape, shape)) {
+            BatchPart P;
+            P.shape = shape;
+            P.i0 = (int)k;
+            P.map0 = b->h_tile_field.size();
+            b->parts.push_back(P);
+        }
+        BatchPart& P = b->parts.back();
         for (size_t f : by[c]) {
             const SZxG_Field& S = fields[f];
             DecField& D = tab[k];
@@ -293,18 +306,15 @@ static SZxG_Batch* create_decode(int fastMode, int dataType, int blockSize, int 
             st += 3 * ta[f];
             for (int q = 0; q < 3; q++) D.stB[q] = st + q * tbw[f];
             D.idxA_tiles = ta[f]; D.idxB_tiles = tbw[f];
-            D.idx_tile0 = it; it += ta[f] + tbw[f];
+            D.idx_tile0 = P.idx_total; P.idx_total += ta[f] + tbw[f];
             D.dec_tiles = (D.nb + tb - 1) / tb;
-            D.dec_tile0 = dt; dt += D.dec_tiles;
+            D.dec_tile0 = P.dec_total; P.dec_total += D.dec_tiles;
             D.err = (int*)(base + o_err) + f;
             D.res = b->results + f;
             for (unsigned long long t = 0; t < D.dec_tiles; t++) b->h_tile_field.push_back((uint32_t)(k - P.i0));
             k++;
         }
         P.i1 = (int)k;
-        P.idx_total = it;
-        P.dec_total = dt;
-        b->parts.push_back(P);
     }
     b->d_dec = (DecField*)(base + o_tab);
     b->d_tile_field = (uint32_t*)(base + o_map);
@@ -421,20 +431,26 @@ SZxG_Batch* SZxG_batch_create(int direction, int fastMode, int dataType, int blo
 int SZxG_batch_run(SZxG_Batch* b, SZxG_StreamInfo* d_info, void* stream) {
     if (!b) { set_last_error(SZXG_ERR_ARG); return SZXG_ERR_ARG; }
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(b->zero, 0, b->zero_bytes, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b->counters, 0, 32 * kMaxBatchParts, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b->err, 0, sizeof(int), s);
+    // status words and totals, tile counters, error word: one clearing launch
+    ClearList c{};
+    c.p[0] = b->zero; c.bytes[0] = b->zero_bytes;
+    c.p[1] = b->counters; c.bytes[1] = 32 * kMaxBatchParts;
+    c.p[2] = b->err; c.bytes[2] = sizeof(int);
+    c.n = 3;
+    cudaError_t e = launch_ws_clear(c, s);
     for (size_t k = 0; k < b->parts.size() && e == cudaSuccess; k++) {
         const BatchPart& P = b->parts[k];
         const int n = P.i1 - P.i0;
         unsigned long long* ctr = b->counters + 4 * k;
+        LaunchShape shape = P.shape;
+        shape.after_kernel = true;   // the clear, or the part before
         if (b->direction == 1)
             e = launch_blocked_decode_fields(b->mode, b->dtype, b->bs, n, b->d_dec + P.i0, b->d_tile_field + P.map0,
                                              P.idx_total, P.dec_total, ctr, b->results, b->err, s, P.shape);
         else
             e = launch_blocked_encode_fields(b->mode, b->dtype, b->bs, n, b->run[(size_t)P.i0],
                                              n > 1 ? b->d_fields + P.i0 : nullptr, b->d_tile_field + P.map0,
-                                             P.enc_total, P.asm_total, ctr, b->err, s, P.shape);
+                                             P.enc_total, P.asm_total, ctr, b->err, s, shape);
     }
     if (e == cudaSuccess && d_info)
         e = cudaMemcpyAsync(d_info, b->results, sizeof(StreamResult) * b->nf, cudaMemcpyDeviceToDevice, s);

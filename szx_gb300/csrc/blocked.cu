@@ -41,6 +41,7 @@ namespace szxg {
 // save.
 constexpr int kEncTileBytes = 16384;
 constexpr int kEncWarpsPerSm = 24;
+constexpr int kSizeThreads = 256;
 constexpr int kWinRepolls = 32;   // window re-reads before the global look-back walk
 constexpr int kIdxThreads = 256;
 constexpr int kIdxItems = 8;   // items per thread in the index scans
@@ -760,6 +761,107 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
 #undef FV
 }
 
+// Exact stream sizes of float fields in blocks of 128 at given bounds, without
+// coding them: the encoder's statistics alone, every warp on its own over a
+// contiguous range of 4-block steps (2 KiB, copied a step ahead into its own
+// two buffers), no placement, no barriers.  An item is a field and a bound;
+// acc[2 i] / [2 i + 1] gain its coded blocks' payload bytes and their number.
+__global__ void __launch_bounds__(kSizeThreads) k_blocked_sizes(const SizeItem* items, int ni,
+                                                                unsigned long long steps, unsigned long long* acc) {
+    constexpr int G = 8, BS = 128, STEP = 4 * BS;   // values per step
+    __shared__ __align__(512) uint8_t buf[kSizeThreads / 32][2][STEP * 4];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, seg = lane / G, sl = lane & (G - 1);
+    const unsigned long long w = (unsigned long long)blockIdx.x * (kSizeThreads / 32) + warp,
+                             nw = (unsigned long long)gridDim.x * (kSizeThreads / 32);
+    const unsigned long long u0 = steps * w / nw, u1 = steps * (w + 1) / nw;
+    if (u0 >= u1) return;
+    // item of step u0: the last one that starts at or before it
+    int lo = 0, hi = ni - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (items[mid].step0 <= u0) lo = mid;
+        else hi = mid - 1;
+    }
+    int it = lo, itl = lo;   // items of the step in work and of the step being copied
+    SizeItem cur = items[it], nxt = cur;
+    auto load = [&](unsigned long long u, int b) {
+        while (itl + 1 < ni && items[itl + 1].step0 <= u) nxt = items[++itl];
+        const unsigned long long v0 = (u - nxt.step0) * STEP;
+        const uint32_t cnt = nxt.n - v0 < STEP ? (uint32_t)(nxt.n - v0) : (uint32_t)STEP;
+        const float* src = nxt.x + v0;
+        uint8_t* d = buf[warp][b];
+        if (((uintptr_t)src & 15) == 0 && cnt == STEP) {
+#pragma unroll
+            for (int k = 0; k < STEP / 128; k++) cp_async16(d + 16 * swz16(lane) + 512 * k, src + 4 * lane + 128 * k);
+        } else {
+            for (uint32_t i = lane; i < cnt; i += 32) cp_async_small<4>(d + swz_off<float>(i), src + i);
+        }
+        cp_async_commit();
+    };
+    unsigned long long pay = 0;
+    uint32_t nnc = 0;
+    auto flush = [&]() {
+        const unsigned long long p = warp_sum(pay);
+        const uint32_t c = __reduce_add_sync(0xffffffffu, nnc);
+        if (lane == 0 && c) {
+            atomicAdd(&acc[2 * it], p);
+            atomicAdd(&acc[2 * it + 1], (unsigned long long)c);
+        }
+        pay = 0;
+        nnc = 0;
+    };
+    int eb_exp = exponent_f64_of_f32(cur.eb);
+    load(u0, 0);
+    for (unsigned long long u = u0; u < u1; u++) {
+        const int b = (int)(u - u0) & 1;
+        if (u + 1 < u1) {
+            load(u + 1, b ^ 1);
+            cp_async_wait_group<1>();
+        } else {
+            cp_async_wait_all();
+        }
+        __syncwarp();
+        if (it + 1 < ni && items[it + 1].step0 <= u) {
+            flush();
+            while (it + 1 < ni && items[it + 1].step0 <= u) it++;
+            cur = items[it];
+            eb_exp = exponent_f64_of_f32(cur.eb);
+        }
+        const unsigned long long v = (u - cur.step0) * STEP + (unsigned long long)(seg * BS);
+        const int len = v >= cur.n ? 0 : (cur.n - v < BS ? (int)(cur.n - v) : BS);
+        BlockEnc<float, G> e;
+        if (__all_sync(0xffffffffu, len == BS))
+            enc_block_stats<float, G, true>(buf[warp][b], seg * BS, len, true, cur.eb, eb_exp, 0ull, 0, e);
+        else
+            enc_block_stats<float, G, false>(buf[warp][b], seg * BS, len, true, cur.eb, eb_exp, 0ull, 0, e);
+        if (sl == 0 && e.state == 1) {
+            pay += e.size;
+            nnc++;
+        }
+        __syncwarp();   // (the buffer is copied into again by the next step)
+    }
+    flush();
+}
+
+cudaError_t launch_blocked_sizes(const SizeItem* d_items, int ni, unsigned long long steps, unsigned long long* d_acc,
+                                 cudaStream_t s) {
+    if (ni < 1 || steps == 0) return cudaErrorInvalidValue;
+    static int per_sm[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!per_sm[dev]) {
+        int occ = 0;
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_blocked_sizes, kSizeThreads, 0);
+        if (e != cudaSuccess) return e;
+        per_sm[dev] = occ < 1 ? 1 : occ;
+    }
+    const unsigned long long cap = (unsigned long long)sm_count() * per_sm[dev], want = (steps + 15) / 16;   // >= 2 steps a warp
+    TraceScope tr("blocked_sizes", s);
+    k_blocked_sizes<<<(unsigned)(want < cap ? want : cap), kSizeThreads, 0, s>>>(d_items, ni, steps, d_acc);
+    return cudaGetLastError();
+}
+
 // Header, size index, state bits and medians (szx/src/szx_float.cc:1437-1483).
 // The encoder leaves payload sizes and medians by block index; this kernel
 // compacts them: an assemble tile covers kAsmWords state words (32 blocks
@@ -957,10 +1059,9 @@ static cudaError_t run_encode(EncArgs a, const LaunchShape& shape, cudaStream_t 
     const size_t g = (size_t)sm_count() * cps;
     const int grid = (int)(a.total_tiles < g ? a.total_tiles : g);
     TraceScope tr("blocked_encode", s);
-    if (a.nf == 1 && shape.after_kernel)
-        return launch_after(k_blocked_encode<T, G, false, TBYTES>, grid, TL::kThreads, TL::kDynSmem, s, a);
-    if (a.nf == 1) k_blocked_encode<T, G, false, TBYTES><<<grid, TL::kThreads, TL::kDynSmem, s>>>(a);
-    else k_blocked_encode<T, G, true, TBYTES><<<grid, TL::kThreads, TL::kDynSmem, s>>>(a);
+    auto k = a.nf == 1 ? k_blocked_encode<T, G, false, TBYTES> : k_blocked_encode<T, G, true, TBYTES>;
+    if (shape.after_kernel) return launch_after(k, grid, TL::kThreads, TL::kDynSmem, s, a);
+    k<<<grid, TL::kThreads, TL::kDynSmem, s>>>(a);
     return cudaGetLastError();
 }
 // The one encoder tile variant a launch shape can pick besides the default:

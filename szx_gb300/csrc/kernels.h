@@ -248,6 +248,18 @@ cudaError_t launch_blocked_encode_fields(int layout, int dtype, int bs, int nf, 
                                          unsigned long long enc_total, unsigned long long asm_total,
                                          unsigned long long* counters, int* err, cudaStream_t s,
                                          const LaunchShape& shape = LaunchShape{});
+// A field (float, blocks of 128 values) at a bound whose exact stream size is
+// asked for; step0: the first launch-wide step of 512 values, ascending.
+struct SizeItem {
+    const float* x;
+    unsigned long long n, step0;
+    float eb;
+    int pad;
+};
+// Adds item i's coded payload bytes and coded blocks to d_acc[2 i], d_acc[2 i + 1]
+// (zeroed by the caller); steps: all items' steps.
+cudaError_t launch_blocked_sizes(const SizeItem* d_items, int ni, unsigned long long steps, unsigned long long* d_acc,
+                                 cudaStream_t s);
 // Blocked decode of nf streams (layouts 3, 4) in one launch per kernel: the
 // headers are parsed into the fields' hdr, counters[0] and every field's
 // look-back words and error word zeroed by the caller; res[f] receives field

@@ -74,13 +74,18 @@ constexpr int kH = 64;              // hidden width
 constexpr int kProbes = 16;         // coarse probes, y = -1.5 j (j = 1..16)
 constexpr int kFine = 16;           // fine probes, y = yq + (k - 8) / 4
 constexpr int kRate = 10;           // every 10th block sampled
-constexpr int kTileBlocks = 32;     // sampled blocks per warp tile
+constexpr int kTileBlocks = 8;      // sampled blocks per warp tile (a multiple of kCoarseStep): with 32 the few, long
+                                    // tiles of 24 fields of 2^18..2^23 values left the passes waiting on latency
 constexpr int kCoarseStep = 4;      // the coarse curve uses every 4th sampled block (every 40th block)
 constexpr int kAcc = 18;            // per field, over the coarse blocks: count, bytes[16], radius-0 blocks
 constexpr int A_NS = 0, A_BYTES = 1, A_ZERO = 17;
 constexpr int kRowAcc = 48;         // per row: quarter-step bytes[16], 1/64-step bytes[16], second sample's [16]
 constexpr int kOff2 = 5;            // the second sample: blocks 5, 15, 25, ...
 constexpr int kQMin = -100, kQMax = 4;   // quarter-step window centre, quarters of y
+constexpr int kSizeAhead = 7;           // sizes a pass measures of one field: the next bound's, and those of the two bounds after it
+constexpr int kAheadFrom = 2;           // passes of a field before its later bounds are measured ahead
+constexpr unsigned long long kAheadSteps = 1ull << 17;   // steps of 512 values a launch with such bounds may have
+                                                         // (2^26 values: ~55 us, about what another pass's round trip costs)
 constexpr double kBracketStop = 1.0 / 1024;   // searches stop on a measured bracket this narrow
 
 // parameter offsets
@@ -115,6 +120,8 @@ struct LfxWork {
     unsigned long long* rtile0 = nullptr;   // [cap_rows + 1] first (row, tile) item of each row
     float* X = nullptr;                  // [cap_rows][kF]
     float* pred = nullptr;               // [cap_rows]
+    uint8_t* size_in = nullptr;          // [cap_items] SizeItem, then [cap_items][2] sums: one copy up clears them
+    size_t cap_items = 0;
     size_t cap_rows = 0;
     unsigned long long tiles = 0;
     std::vector<unsigned long long> ftiles;   // tiles of each field
@@ -982,6 +989,8 @@ cudaError_t lfx_prepare(SZxG_Batch* b, size_t rows) {
     const size_t o_rt = off; off += a256(8 * (cr + 1));
     const size_t o_X = off; off += a256(4 * kF * cr);
     const size_t o_pred = off; off += a256(4 * cr);
+    const size_t ci = (size_t)kSizeAhead * nf;   // a pass asks for at most so many sizes
+    const size_t o_size = off; off += a256((sizeof(SizeItem) + 16) * ci);
     cudaError_t e = cudaMalloc(&w->dev, off);
     if (e != cudaSuccess) {
         delete w;
@@ -1000,6 +1009,8 @@ cudaError_t lfx_prepare(SZxG_Batch* b, size_t rows) {
     w->rtile0 = (unsigned long long*)(base + o_rt);
     w->X = (float*)(base + o_X);
     w->pred = (float*)(base + o_pred);
+    w->size_in = base + o_size;
+    w->cap_items = ci;
     e = cudaMemcpy(w->d_f, tab.data(), sizeof(LfxField) * nf, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         lfx_free(w);
@@ -1223,15 +1234,15 @@ int SZxG_batch_fixed_rate(SZxG_Batch* b, const SZxG_Mlp* mlp, const float* targe
     if (e != cudaSuccess) return fail_code(e);
 
     const double lo0 = -28.0, hi0 = 1.0;
-    std::vector<double> lo(nf, lo0), hi(nf, hi0), y(nf), yprev(nf, 0.0), step(nf, 0.0), best_y(nf, 0),
-        best_err(nf, 1e300), best_cr(nf, 0);
-    // done: 1 converged, 2 stopped on a jump over the target band
-    std::vector<int> passes(nf, 0), done(nf, 0), stage(nf, 0), last_is_best(nf, 0), lo_m(nf, 0), hi_m(nf, 0);
-    std::vector<float> ebk(nf);
-    for (int f = 0; f < nf; f++) ebk[f] = b->tab[f].eb;
-    // bounds of the bracket's measured ends, of the best pass, and a bound
-    // to code exactly in the next pass (0: from y)
-    std::vector<float> lo_eb(nf, 0.f), hi_eb(nf, 0.f), best_eb(nf, 0.f), ebx(nf, 0.f);
+    // One field's search.  done: 1 converged, 2 stopped on a jump over the
+    // target band; lo_eb / hi_eb / best_eb: bounds of the bracket's measured
+    // ends and of the best pass; ebx: a bound to measure exactly next (0: from y).
+    struct Search {
+        double lo, hi, y, yprev = 0, step = 0, best_err = 1e300, best_cr = 0;
+        float lo_eb = 0, hi_eb = 0, best_eb = 0, ebx = 0, ebk = 0;
+        int passes = 0, done = 0, stage = 0;
+        bool last_is_best = false, lo_m = false, hi_m = false;
+    };
     // one power of two P between the bracket's ends: the side of P to code
     // next, -1 when both sides are measured (the ratio jumps over the band
     // at P), 0 when the ends hold none or several
@@ -1244,138 +1255,196 @@ int SZxG_batch_fixed_rate(SZxG_Batch* b, const SZxG_Mlp* mlp, const float* targe
         if (le == Pm && he == P) return -1.f;
         return he > P ? P : Pm;
     };
-    std::vector<StreamResult> res(nf);
-    auto eb_of = [&](int f, double yy) {
-        const float r = range[f] > 0.f ? range[f] : 1.f;
-        return (float)((double)r * exp2(yy));
-    };
     auto clampy = [&](double v) { return std::min(std::max(v, lo0), hi0); };
-    // next bound of a field that missed, from its bracket
-    auto next_y = [&](int f) {
-        if (!mlp || (lo_m[f] && hi_m[f])) return 0.5 * (lo[f] + hi[f]);
-        step[f] = step[f] > 0 ? 2.0 * step[f] : std::max(2.0 * fabs(y[f] - yprev[f]), 0.25);
-        return lo_m[f] ? std::min(lo[f] + step[f], hi[f]) : std::max(hi[f] - step[f], lo[f]);
+    auto safe_range = [&](int f) { return range[f] > 0.f ? range[f] : 1.f; };
+    auto bound_of = [&](int f, const Search& S) {
+        return S.ebx > 0.f ? S.ebx : (float)((double)safe_range(f) * exp2(S.y));
     };
-    for (int f = 0; f < nf; f++) y[f] = mlp ? clampy(ys[f]) : 0.5 * (lo0 + hi0);
-    int err_code = SZXG_OK;
-    for (int pass = 0; pass < maxPasses; pass++) {
-        std::vector<int> act;
-        std::vector<float> ebs;
-        for (int f = 0; f < nf; f++)
-            if (!done[f]) {
-                act.push_back(f);
-                ebs.push_back(ebx[f] > 0.f ? ebx[f] : eb_of(f, y[f]));
-                ebx[f] = 0.f;
-            }
-        if (act.empty()) break;
-        e = batch_select(b, (int)act.size(), act.data(), ebs.data(), s);
-        if (e == cudaSuccess) {
-            const int rc = SZxG_batch_run(b, nullptr, stream);
-            if (rc) { err_code = rc; break; }
-            e = cudaMemcpyAsync(res.data(), b->results, sizeof(StreamResult) * nf, cudaMemcpyDeviceToHost, s);
+    // next bound of a field that missed, from its bracket
+    auto next_y = [&](Search& S) {
+        if (!mlp || (S.lo_m && S.hi_m)) return 0.5 * (S.lo + S.hi);
+        S.step = S.step > 0 ? 2.0 * S.step : std::max(2.0 * fabs(S.y - S.yprev), 0.25);
+        return S.lo_m ? std::min(S.lo + S.step, S.hi) : std::max(S.hi - S.step, S.lo);
+    };
+    // A measured ratio at bound eb.  True when the field goes on by re-aiming
+    // its sampled crossing (stage 1), else its next bound is set.
+    auto judge = [&](int f, Search& S, float eb, double cr) {
+        S.passes++;
+        S.ebk = eb;
+        S.ebx = 0.f;
+        const double rel = fabs(cr / tgt[f] - 1.0);
+        S.last_is_best = false;
+        if (rel < S.best_err) {
+            S.best_err = rel;
+            S.best_eb = eb;
+            S.best_cr = cr;
+            S.last_is_best = true;
         }
+        if (rel <= tolerance) { S.done = 1; return false; }
+        if (cr < tgt[f]) {
+            if (!S.lo_m || eb > S.lo_eb) S.lo_eb = eb;
+            S.lo = std::max(S.lo, S.y);
+            S.lo_m = true;
+        } else {
+            if (!S.hi_m || eb < S.hi_eb) S.hi_eb = eb;
+            S.hi = std::min(S.hi, S.y);
+            S.hi_m = true;
+        }
+        // the ratio jumps over the target band inside a bracket this narrow: nothing to find
+        if (S.lo_m && S.hi_m && S.hi - S.lo < kBracketStop) { S.done = 2; return false; }
+        const double ycur = S.y;
+        bool refine = false;
+        if (mlp && S.stage == 0) {
+            S.stage = 1;
+            refine = true;
+        } else {
+            const float pr = mlp && S.lo_m && S.hi_m ? jump_probe(S.lo_eb, S.hi_eb) : 0.f;
+            if (pr < 0.f) { S.done = 2; return false; }
+            if (pr > 0.f) {
+                S.ebx = pr;
+                S.y = log2((double)pr / (double)safe_range(f));
+            } else {
+                S.y = next_y(S);
+            }
+        }
+        S.yprev = ycur;
+        return refine;
+    };
+    std::vector<Search> st(nf);
+    for (int f = 0; f < nf; f++) {
+        st[f].lo = lo0;
+        st[f].hi = hi0;
+        st[f].y = mlp ? clampy(ys[f]) : 0.5 * (lo0 + hi0);
+        st[f].ebk = b->tab[f].eb;
+    }
+    // Passes measure exact stream sizes (launch_blocked_sizes) and code
+    // nothing; the streams are coded once, at the chosen bounds.  Beside the
+    // next bound of a field that has missed twice a pass measures the bounds
+    // that would follow either outcome, two deep, while that stays a small part
+    // of a launch (kAheadSteps): a search that runs on then takes three
+    // decisions per launch and round trip.  Decisions, bounds and pass counts
+    // are those of the one-by-one search.  (24 fields of 2^18..2^23 values,
+    // ratio 16: up to ten passes, each of which coded its fields, 2267 us.)
+    const unsigned long long hdr = b->mode == kBlocked ? 13 : 20, per_nnc = b->mode == kBlocked ? 0 : 2;
+    struct Asked { float eb; double cr; };
+    auto same = [](float x, float y) { return memcmp(&x, &y, sizeof x) == 0; };   // (a NaN bound is found again too)
+    std::vector<std::vector<Asked>> known(nf);
+    auto find = [&](int f, float eb) -> const Asked* {
+        for (const Asked& a : known[f])
+            if (same(a.eb, eb)) return &a;
+        return nullptr;
+    };
+    std::vector<uint8_t> up;
+    std::vector<unsigned long long> sums;
+    std::vector<SizeItem> items;
+    std::vector<int> owner;
+    for (;;) {
+        items.clear();
+        owner.clear();
+        unsigned long long steps = 0;
+        auto ask = [&](int f, float eb) {
+            for (size_t k = 0; k < items.size(); k++)
+                if (owner[k] == f && same(items[k].eb, eb)) return;
+            const unsigned long long n = b->tab[f].n;
+            items.push_back({(const float*)b->tab[f].x, n, steps, eb, 0});
+            owner.push_back(f);
+            steps += (n + 511) / 512;
+        };
+        for (int f = 0; f < nf; f++) {
+            if (st[f].done || st[f].passes >= maxPasses) continue;
+            ask(f, bound_of(f, st[f]));
+        }
+        for (int f = 0; f < nf; f++) {
+            if (st[f].done || st[f].passes < kAheadFrom || st[f].passes + 1 >= maxPasses) continue;
+            const unsigned long long own = (b->tab[f].n + 511) / 512;
+            const int deep = steps + 6 * own <= kAheadSteps ? 2 : steps + 2 * own <= kAheadSteps ? 1 : 0;
+            // both outcomes of this bound, and both of each of those (a miss is a miss, by any factor)
+            std::vector<Search> level{st[f]};
+            for (int d = 0; d < deep; d++) {
+                std::vector<Search> next;
+                for (const Search& S : level)
+                    for (int side = 0; side < 2; side++) {
+                        Search Q = S;
+                        judge(f, Q, bound_of(f, S), (double)tgt[f] * (side ? 8.0 * (1.0 + tolerance) : 0.125 / (1.0 + tolerance)));
+                        if (Q.done || Q.passes >= maxPasses) continue;
+                        ask(f, bound_of(f, Q));
+                        next.push_back(Q);
+                    }
+                level.swap(next);
+            }
+        }
+        if (items.empty()) break;
+        const size_t ni = items.size(), ib = sizeof(SizeItem) * ni;
+        up.assign(ib + 16 * ni, 0);
+        memcpy(up.data(), items.data(), ib);
+        unsigned long long* d_acc = (unsigned long long*)(b->lfx->size_in + ib);
+        sums.resize(2 * ni);
+        e = cudaMemcpyAsync(b->lfx->size_in, up.data(), up.size(), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = launch_blocked_sizes((const SizeItem*)b->lfx->size_in, (int)ni, steps, d_acc, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(sums.data(), d_acc, 16 * ni, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return fail_code(e);
-        bool need_refine = false;
+        for (size_t k = 0; k < ni; k++) {
+            const int f = owner[k];
+            const unsigned long long n = b->tab[f].n, nb = b->tab[f].nb, pay = sums[2 * k], nnc = sums[2 * k + 1];
+            const unsigned long long size = hdr + per_nnc * nnc + (nb + 7) / 8 + 4 * (nb - nnc) + pay;
+            known[f].push_back({items[k].eb, (double)n * 4.0 / (double)size});
+        }
+        // every field as far as its measured bounds take it
+        std::vector<int> fl, fw;
         std::vector<float> t2 = tgt;
-        for (size_t k = 0; k < act.size(); k++) {
-            const int f = act[k];
-            passes[f]++;
-            ebk[f] = ebs[k];
-            const StreamResult& r = res[f];
-            if (r.status) { err_code = r.status; done[f] = 1; continue; }
-            const double cr = (double)b->tab[f].n * 4.0 / (double)r.size;
-            const double rel = fabs(cr / tgt[f] - 1.0);
-            last_is_best[f] = 0;
-            if (rel < best_err[f]) {
-                best_err[f] = rel;
-                best_y[f] = y[f];
-                best_eb[f] = ebs[k];
-                best_cr[f] = cr;
-                last_is_best[f] = 1;
-            }
-            if (rel <= tolerance) { done[f] = 1; continue; }
-            if (cr < tgt[f]) {
-                if (!lo_m[f] || ebs[k] > lo_eb[f]) lo_eb[f] = ebs[k];
-                lo[f] = std::max(lo[f], y[f]);
-                lo_m[f] = 1;
-            } else {
-                if (!hi_m[f] || ebs[k] < hi_eb[f]) hi_eb[f] = ebs[k];
-                hi[f] = std::min(hi[f], y[f]);
-                hi_m[f] = 1;
-            }
-            // the ratio jumps over the target band inside a bracket this narrow: nothing to find
-            if (lo_m[f] && hi_m[f] && hi[f] - lo[f] < kBracketStop) { done[f] = 2; continue; }
-            const double ycur = y[f];
-            if (mlp && stage[f] == 0) {
+        for (int f = 0; f < nf; f++) {
+            Search& S = st[f];
+            while (!S.done && S.passes < maxPasses) {
+                const float eb = bound_of(f, S);
+                const Asked* a = find(f, eb);
+                if (!a) break;
+                if (!judge(f, S, eb, a->cr)) continue;
                 // re-aim the sampled crossing by the miss this pass measured
-                stage[f] = 1;
-                t2[f] = (float)((double)aim[f] * std::min(std::max((double)tgt[f] / cr, 0.25), 4.0));
-                need_refine = true;
-            } else {
-                const float pr = mlp && lo_m[f] && hi_m[f] ? jump_probe(lo_eb[f], hi_eb[f]) : 0.f;
-                if (pr < 0.f) { done[f] = 2; continue; }
-                if (pr > 0.f) {
-                    ebx[f] = pr;
-                    y[f] = log2((double)pr / (double)(range[f] > 0.f ? range[f] : 1.f));
+                t2[f] = (float)((double)aim[f] * std::min(std::max((double)tgt[f] / a->cr, 0.25), 4.0));
+                if (!(t2[f] > 0.f) || !std::isfinite(t2[f])) t2[f] = aim[f];
+                double yw;
+                if (window_crossing(f, t2[f], yw)) {
+                    ys[f] = yw;
+                    fw.push_back(f);
                 } else {
-                    y[f] = next_y(f);
+                    fl.push_back(f);
                 }
+                break;
             }
-            yprev[f] = ycur;
         }
-        if (err_code) break;
-        if (need_refine) {
-            std::vector<int> fl, fw;
-            for (int f = 0; f < nf; f++)
-                if (!done[f] && stage[f] == 1) {
-                    if (!(t2[f] > 0.f) || !std::isfinite(t2[f])) t2[f] = aim[f];
-                    double yw;
-                    if (window_crossing(f, t2[f], yw)) {
-                        ys[f] = yw;
-                        fw.push_back(f);
-                    } else {
-                        fl.push_back(f);
-                    }
-                }
-            if ((e = crossing(fl, t2, ys, false)) != cudaSuccess) return fail_code(e);
-            fl.insert(fl.end(), fw.begin(), fw.end());
-            for (int f : fl) {
-                stage[f] = 2;
-                y[f] = (ys[f] > lo[f] && ys[f] < hi[f]) ? ys[f] : next_y(f);
-            }
+        if (!fl.empty() && (e = crossing(fl, t2, ys, false)) != cudaSuccess) return fail_code(e);
+        fl.insert(fl.end(), fw.begin(), fw.end());
+        for (int f : fl) {
+            Search& S = st[f];
+            S.stage = 2;
+            S.y = (ys[f] > S.lo && ys[f] < S.hi) ? ys[f] : next_y(S);
         }
     }
-    // a field that stopped unconverged gets its best bound back
-    if (!err_code) {
-        std::vector<int> act;
-        std::vector<float> ebs;
-        for (int f = 0; f < nf; f++)
-            if (done[f] != 1 && !last_is_best[f] && best_err[f] < 1e300) {
-                act.push_back(f);
-                ebs.push_back(best_eb[f]);
-                passes[f]++;
-                ebk[f] = ebs.back();
-            }
-        if (!act.empty()) {
-            e = batch_select(b, (int)act.size(), act.data(), ebs.data(), s);
-            if (e == cudaSuccess) {
-                const int rc = SZxG_batch_run(b, nullptr, stream);
-                if (rc) err_code = rc;
-            }
-            if (e != cudaSuccess) return fail_code(e);
+    std::vector<float> ebk(nf);
+    for (int f = 0; f < nf; f++) {
+        Search& S = st[f];
+        // a field that stopped unconverged gets its best bound back
+        if (S.done != 1 && !S.last_is_best && S.best_err < 1e300) {
+            S.passes++;
+            S.ebk = S.best_eb;
         }
+        ebk[f] = S.ebk;
     }
-    // leave the plan coding every field, at the chosen bounds
+    // code every field at its chosen bound, and leave the plan doing so
+    std::vector<StreamResult> res(nf);
     e = batch_select(b, nf, nullptr, ebk.data(), s);
-    if (e == cudaSuccess && d_info)
-        e = cudaMemcpyAsync(d_info, b->results, sizeof(StreamResult) * nf, cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) return fail_code(e);
+    int err_code = SZxG_batch_run(b, d_info, stream);
+    if (err_code) return err_code;
+    e = cudaMemcpyAsync(res.data(), b->results, sizeof(StreamResult) * nf, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail_code(e);
     for (int f = 0; f < nf; f++) {
+        if (res[f].status && !err_code) err_code = res[f].status;
         if (h_eb) h_eb[f] = ebk[f];
-        if (h_ratio) h_ratio[f] = (float)best_cr[f];
-        if (h_passes) h_passes[f] = passes[f];
+        if (h_ratio) h_ratio[f] = (float)st[f].best_cr;
+        if (h_passes) h_passes[f] = st[f].passes;
     }
     set_last_error(err_code);
     return err_code;
