@@ -6,6 +6,7 @@ and nothing here computes anything itself.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 
 from . import build as _build
@@ -134,6 +135,7 @@ def lib() -> C.CDLL:
     return _lib
 
 
+@functools.cache
 def libc() -> C.CDLL:
     c = C.CDLL(None)
     c.free.argtypes = [C.c_void_p]

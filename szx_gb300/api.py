@@ -10,6 +10,7 @@ workspace and output buffers owned by the caller.
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 
 import numpy as np
 
@@ -56,6 +57,14 @@ def _take(ptr: int, nbytes: int) -> bytes:
     b = C.string_at(ptr, nbytes)
     libc().free(ptr)
     return b
+
+
+def _take_array(ptr: int, n: int, dtype: np.dtype) -> np.ndarray:
+    """The library's malloc'd values as an array, without a copy: freed with the last view of it.  (Two copies into
+    fresh pages took 1.8 of the 2.1 ms of a 16 MiB decompress.)"""
+    buf = (C.c_ubyte * (n * dtype.itemsize)).from_address(ptr)
+    weakref.finalize(buf, libc().free, ptr).atexit = False   # (an array may outlive the exit handlers)
+    return np.frombuffer(buf, dtype)
 
 
 # ------------------------------------------------------------------ reference interface
@@ -108,7 +117,7 @@ def fast_decompress(fastMode: int, dtype, stream: bytes, n: int | None = None, d
     if not p:
         raise SZxError(last_error(), "SZx_fast_decompress")
     nd = np.dtype(_np_dtype(code))
-    return np.frombuffer(_take(p, n * nd.itemsize), nd).copy()
+    return _take_array(p, n, nd)
 
 
 def estimate_error_bound(data: np.ndarray, compressionRatio: float, tolerance: float, initErrorBound: float,
@@ -189,7 +198,7 @@ def decompress_host(fastMode: int, dtype, stream: bytes, n: int) -> np.ndarray:
     if not p:
         raise SZxError(last_error(), "SZxG_decompress_host")
     nd = np.dtype(_np_dtype(code))
-    return np.frombuffer(_take(p, n * nd.itemsize), nd).copy()
+    return _take_array(p, n, nd)
 
 
 # ------------------------------------------------------------------ device interface
