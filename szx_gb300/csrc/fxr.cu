@@ -19,6 +19,9 @@
 #include <math.h>
 #include <string.h>
 
+#include <utility>
+#include <vector>
+
 #include "../../include/szx_gb300.h"
 #include "kernels.h"
 #include "segment.cuh"
@@ -43,7 +46,7 @@ struct FxWs {
 size_t fx_a256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 size_t fx_bytes(size_t ns) {
-    return fx_a256(4 * ns) * 2 + fx_a256(8 * ns) * 3 + 256;
+    return fx_a256(4 * ns) * 2 + fx_a256(8 * ns) * 3 + 1024;
 }
 
 FxWs fx_carve(void* base, size_t ns) {
@@ -55,7 +58,7 @@ FxWs fx_carve(void* base, size_t ns) {
     w.bmin = b; b += fx_a256(8 * ns);
     w.bmax = b; b += fx_a256(8 * ns);
     w.acc = (unsigned long long*)b;
-    w.range = (float*)(b + 64);
+    w.range = (float*)(b + 768);   // (behind kFxBounds triples of sums)
     return w;
 }
 
@@ -162,10 +165,23 @@ __global__ void __launch_bounds__(1024) k_fxr_range(const T* x, const T* bmin, c
 // required bytes per coded block, and min(lead, required bytes) summed over
 // the coded blocks' values.  The subtraction uses the median the reference
 // hands to the value loop: zeroed when the required length is clamped.
+// Several bounds a launch (blockIdx.y): the search asks for the ones it may
+// need next along with the next one, and a round trip costs as much as many
+// evaluations of a sample.
+constexpr int kFxBounds = 24;
+// Sampled values a launch with such bounds may evaluate: 2^23 take about 10 us,
+// a round trip 15.
+constexpr size_t kFxAheadValues = size_t(1) << 23;
+struct FxBounds {
+    float eb[kFxBounds];
+};
 template <typename T, int G>
 __global__ void __launch_bounds__(kFxThreads) k_fxr_eval(const T* x, unsigned long long ns, unsigned long long stride,
                                                          int bs, const float* rads, const float* meds,
-                                                         const double* rads_d, float eb, unsigned long long* acc) {
+                                                         const double* rads_d, FxBounds bounds,
+                                                         unsigned long long* acc) {
+    const float eb = bounds.eb[blockIdx.y];
+    acc += 3 * blockIdx.y;
     using EL = Elem<T>;
     using U = typename EL::U;
     constexpr int E = EncCfg<T>::E;
@@ -316,17 +332,50 @@ struct FxSample {
         return e;
     }
 
-    // ratio estimate at eb; the integer sums in *sr, *sl, *sc
-    cudaError_t eval(float eb, float* cr, size_t* sr, size_t* sl, size_t* sc) {
-        cudaError_t e = cudaMemsetAsync(w.acc, 0, 3 * sizeof(unsigned long long), s);
+    // Ratio estimate at eb; the integer sums in *sr, *sl, *sc.  When eb has not
+    // been evaluated yet, the bounds in `ahead` (what the search may ask for
+    // next) are evaluated by the same launch.
+    cudaError_t eval(float eb, float* cr, size_t* sr, size_t* sl, size_t* sc, const std::vector<float>& ahead = {}) {
+        auto find = [&](float v) -> const Known* {
+            for (const Known& k : known)
+                if (memcmp(&k.eb, &v, sizeof v) == 0) return &k;
+            return nullptr;
+        };
+        const Known* k = find(eb);
+        if (!k) {
+            FxBounds B;
+            int nb = 0;
+            B.eb[nb++] = eb;
+            const size_t room = ns ? kFxAheadValues / (ns * (size_t)bs) : 0;
+            for (float v : ahead)
+                if (nb < kFxBounds && (size_t)nb < room && v != eb && !find(v)) B.eb[nb++] = v;
+            const cudaError_t e = eval_bounds(B, nb);
+            if (e != cudaSuccess) return e;
+            k = find(eb);
+        }
+        *sc = (size_t)k->sums[0];
+        *sr = (size_t)k->sums[1];
+        *sl = (size_t)k->sums[2];
+        *cr = fx_model(dtype, bs, n, nden, *sc, *sr, *sl);
+        return cudaSuccess;
+    }
+
+    struct Known {
+        float eb;
+        unsigned long long sums[3];   // constant blocks, required bytes, leading bytes
+    };
+    std::vector<Known> known;
+
+    cudaError_t eval_bounds(const FxBounds& B, int nb) {
+        cudaError_t e = cudaMemsetAsync(w.acc, 0, 3 * nb * sizeof(unsigned long long), s);
         if (e != cudaSuccess) return e;
         if (ns) {
             const size_t warps = (ns + (32 / G) - 1) / (32 / G);
-            const unsigned grid = (unsigned)((warps * 32 + kFxThreads - 1) / kFxThreads);
+            const dim3 grid((unsigned)((warps * 32 + kFxThreads - 1) / kFxThreads), (unsigned)nb);
             const double* rd = double_radius ? w.rads_d : nullptr;
             TraceScope tr("fxr_eval", s);
 #define FX_EVAL(TT, GG) \
-    k_fxr_eval<TT, GG><<<grid, kFxThreads, 0, s>>>((const TT*)x, ns, stride, bs, w.rads, w.meds, rd, eb, w.acc)
+    k_fxr_eval<TT, GG><<<grid, kFxThreads, 0, s>>>((const TT*)x, ns, stride, bs, w.rads, w.meds, rd, B, w.acc)
             if (dtype == 0) {
                 switch (G) {
                     case 1: FX_EVAL(float, 1); break;
@@ -348,14 +397,38 @@ struct FxSample {
 #undef FX_EVAL
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
-        unsigned long long h[3] = {0, 0, 0};
-        if ((e = cudaMemcpyAsync(h, w.acc, sizeof h, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+        unsigned long long h[3 * kFxBounds] = {};
+        if ((e = cudaMemcpyAsync(h, w.acc, 3 * nb * sizeof h[0], cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-        *sc = (size_t)h[0];
-        *sr = (size_t)h[1];
-        *sl = (size_t)h[2];
-        *cr = fx_model(dtype, bs, n, nden, *sc, *sr, *sl);
+        for (int i = 0; i < nb; i++) known.push_back({B.eb[i], {h[3 * i], h[3 * i + 1], h[3 * i + 2]}});
         return cudaSuccess;
+    }
+
+    // Bounds a bracket search may visit from eb on (steps of `stride` either
+    // way), and those a bisection of [l, r] may (three levels below r's half).
+    static std::vector<float> bracket_ahead(float eb, int stride, int steps) {
+        std::vector<float> v;
+        float lo = eb, hi = eb;
+        for (int i = 0; i < steps; i++) {
+            v.push_back(lo = lo / stride);
+            v.push_back(hi = hi * stride);
+        }
+        return v;
+    }
+    static std::vector<float> bisect_ahead(float l, float r, int depth = 4) {
+        std::vector<std::pair<float, float>> level{{l, r}};
+        std::vector<float> v;
+        for (int d = 0; d < depth; d++) {
+            std::vector<std::pair<float, float>> next;
+            for (auto& q : level) {
+                const float m = (q.first + q.second) / 2;
+                v.push_back(m);
+                next.push_back({m, q.second});
+                next.push_back({q.first, m});
+            }
+            level.swap(next);
+        }
+        return v;
     }
 };
 
@@ -388,7 +461,7 @@ cudaError_t fxr_bound(int dtype, const void* d_x, size_t n, int bs, float target
     int k = 0;
     size_t sr = 0, sl = 0, sc = 0;
     float CR = 0;
-    if ((e = S.eval(errorBound, &CR, &sr, &sl, &sc)) != cudaSuccess) return e;
+    if ((e = S.eval(errorBound, &CR, &sr, &sl, &sc, FxSample::bracket_ahead(errorBound, stride, 4))) != cudaSuccess) return e;
     sumReqNbBytes[k] = sr; sum_actual_leadNumbers[k] = sl; errorBounds[k] = errorBound; ratios[k] = CR; k++;
     if (fabs(targetCompressionRatio - CR) < tolerance) { *eb_out = errorBound; return cudaSuccess; }
     float left_error = 0, right_error = 0, result_error = 0;
@@ -420,7 +493,8 @@ cudaError_t fxr_bound(int dtype, const void* d_x, size_t n, int bs, float target
     if (foundFlag == 0) {
         for (int i = 0; i < nbIterations; i++) {
             errorBound = (left_error + right_error) / 2;
-            if ((e = S.eval(errorBound, &CR, &sr, &sl, &sc)) != cudaSuccess) return e;
+            if ((e = S.eval(errorBound, &CR, &sr, &sl, &sc, FxSample::bisect_ahead(left_error, right_error))) != cudaSuccess)
+                return e;
             int appeared = 0;
             for (int j = 0; j < k; j++)
                 if (sumReqNbBytes[j] == sr && sum_actual_leadNumbers[j] == sl) { appeared = 1; break; }
@@ -463,7 +537,7 @@ cudaError_t fxr_bound_unbuffered(int dtype, const void* d_x, size_t n, int bs, f
     float errorBound = initErrorBound;
     size_t sr, sl, sc;
     float CR = 0;
-    if ((e = S.eval(errorBound, &CR, &sr, &sl, &sc)) != cudaSuccess) return e;
+    if ((e = S.eval(errorBound, &CR, &sr, &sl, &sc, FxSample::bracket_ahead(errorBound, 8, 4))) != cudaSuccess) return e;
     const int nbIterations = 15;
     if (fabs(targetCompressionRatio - CR) < tolerance) { *eb_out = errorBound; return cudaSuccess; }
     float left_error = 0, right_error = 0, result_error = 0;
@@ -504,7 +578,8 @@ cudaError_t fxr_bound_unbuffered(int dtype, const void* d_x, size_t n, int bs, f
     if (foundFlag == 0) {
         for (int i = 0; i < nbIterations; i++) {
             errorBound = (left_error + right_error) / 2;
-            if ((e = S.eval(errorBound, &CR, &sr, &sl, &sc)) != cudaSuccess) return e;
+            if ((e = S.eval(errorBound, &CR, &sr, &sl, &sc, FxSample::bisect_ahead(left_error, right_error))) != cudaSuccess)
+                return e;
             if (fabs(CR - targetCompressionRatio) < targetTolerance || fabs(CR - preCR) < targetTolerance / 2) {
                 foundFlag = 1;
                 result_error = errorBound;
