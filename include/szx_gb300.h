@@ -291,7 +291,7 @@ int SZxG_batch_fixed_rate(SZxG_Batch* batch, const SZxG_Mlp* mlp, const float* t
  * Returns the number of kernels reported. */
 /* Failure detection (no counterpart in the reference): runs the device-wide
  * look-back the codecs use to place variable-length payloads (scan 0: the
- * encoders' 64-bit status words; scan 1: the decoders' 32-bit words) over
+ * encoders' 64-bit status words; scan 1: the words of the decoders' index) over
  * ntiles (<= 4096) one-warp tiles, tile t contributing t + 1, with tile
  * `withheld` (-1: none) never publishing, and waits bounded by spinLimit
  * polls.  Returns SZXG_ERR_LOOKBACK when a wait gave up, else SZXG_OK with

@@ -42,7 +42,6 @@ namespace szxg {
 constexpr int kEncTileBytes = 16384;
 constexpr int kEncWarpsPerSm = 24;
 constexpr int kSizeThreads = 256;
-constexpr int kWinRepolls = 32;   // window re-reads before the global look-back walk
 constexpr int kIdxThreads = 256;
 constexpr int kIdxItems = 8;   // items per thread in the index scans
 
@@ -390,15 +389,6 @@ __device__ __forceinline__ void enc_block_emit(uint8_t* stg, uint32_t loc, int l
     }
 }
 
-// Lane-predicated claim of the next tile: the reply is waited for where `next`
-// is used, not at the end of a branch.
-__device__ __forceinline__ void claim_tile(unsigned long long& next, unsigned long long* ctr, bool take) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p atom.relaxed.gpu.global.add.u64 %0, [%1], 1;\n\t}"
-                 : "+l"(next)
-                 : "l"(ctr), "r"((uint32_t)take)
-                 : "memory");
-}
-
 template <typename T, int G, int TBYTES = kEncTileBytes>
 struct EncTile {
     static constexpr int E = EncCfg<T>::E;
@@ -420,7 +410,7 @@ struct EncTile {
     static constexpr int kDynSmem = 4 * kBuf;
     static_assert(kGroups <= 8 && kBlocks % kBpw == 0, "one block group per warp");
     static_assert(kBlocks <= 64, "a tile's sizes are scanned as two warp-wide halves");
-    static_assert(kBlocks * kMaxPay < 32767, "a tile's byte count + 1 fits 15 bits of the aggregate words");
+    static_assert(kBlocks * kMaxPay < 65535, "a tile's byte count + 1 fits the 16-bit aggregate words");
     static_assert(kIn % 512 == 0 && kBuf % 64 == 0, "swizzled chunks stay inside the tile, runs on 64-byte boundaries");
     static_assert(kThreads % 32 == 0, "a thread's chunks keep one swizzle phase");
 };
@@ -451,12 +441,9 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     constexpr int BPW = TL::kBpw;
     constexpr int NGRP = TB / BPW;
     extern __shared__ __align__(128) uint8_t dsm[];
-    __shared__ __align__(16) uint16_t s_w16[kLbWin + 8];   // look-back window (16-bit aggregates)
-    __shared__ int s_an_t, s_wlo;                          // placement anchor tile; window's first tile
-    __shared__ unsigned long long s_an_incl;               // the anchor's inclusive prefix
-    __shared__ int s_an_f, s_wok;                          // its field; window state
     __shared__ uint32_t s_size[TB], s_med[TB];
     __shared__ uint8_t s_state[TB];
+    __shared__ PlaceWin s_win;
     __shared__ uint32_t s_agg[4];
     __shared__ int s_tile[4];           // launch-wide tile index of each ring position (-1: none left)
     __shared__ int s_fld[4];            // its field
@@ -522,43 +509,9 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     };
 
     unsigned long long nnc_cta = 0;   // warp kMetaWarp lane 0, single field: non-constant blocks of this CTA's tiles
-    // Placement (warp 0).  A tile's offset is the inclusive prefix of this
-    // CTA's previous tile (the anchor, known here) plus the aggregates of the
-    // tiles claimed between the two, read from the field's 16-bit aggregate
-    // words: a window of at most kLbWin of them is copied into shared memory
-    // an iteration before it is needed.  No anchor in the same field within
-    // kLbWin tiles, or an aggregate not yet published, falls back to the
-    // global look-back over the 64-bit status words.
-    // (the anchor and window state live in shared memory: warp 0 alone uses
-    // them, lane 0 writes, and registers stay free for the statistics)
-    if (threadIdx.x == 0) {
-        s_an_t = -1;
-        s_an_f = -1;
-        s_an_incl = 0;
-    }
+    if (threadIdx.x == 0) s_win.init();
     auto agg16_of = [&](const BlkField* F) {
         return (uint16_t*)(FV(F, st_enc) + enc_tile_words(FV(F, nb)));
-    };
-    auto win_issue = [&](const BlkField* F, int f, int t) {
-        int ok = 0;
-        int lo = 0;
-        const int an_t = s_an_t;
-        if (t > 0 && an_t >= 0 && s_an_f == f && an_t < t && t - an_t - 1 <= kLbWin) {
-            if (t - an_t == 1) {
-                ok = 2;
-            } else {
-                lo = (an_t + 1) & ~7;
-                const int units = (t - lo + 7) >> 3;
-                const uint16_t* src = agg16_of(F) + lo;
-                for (int u = lane; u < units; u += 32) cp_async16(&s_w16[8 * u], src + 8 * u);
-                ok = 1;
-            }
-        }
-        if (lane == 0) {
-            s_wlo = lo;
-            s_wok = ok;
-        }
-        __syncwarp();
     };
     // one warp: sizes, medians and state bits of tile t's blocks, by block
     constexpr int kMetaWarp = TL::kWarps - 2;
@@ -590,70 +543,16 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
     // warp 0: place tile t of field f, ring position r: its offset in the payload, the capacity check, the field's payload total
     auto place = [&](const BlkField* F, int f, int t, int r) {
         const uint32_t agg = s_agg[r];
-        unsigned long long base = 0;
-        if (t > 0) {
-            const int ok = s_wok;
-            const int an_t = s_an_t;
-            const unsigned long long an_incl = s_an_incl;
-            bool placed = false;
-            if (ok == 2) {
-                base = an_incl;
-                placed = true;
-            } else if (ok == 1) {
-                // Sum of the aggregates an_t + 1 .. t - 1, eight to a 16-byte
-                // read (two reads a lane at most) and a redux across the warp;
-                // the words outside that range count as 1, published and empty.
-                const int lo = s_wlo;
-                const int units = (t - lo + 7) >> 3;
-                const int first = an_t + 1 - lo, last = t - lo;
-                cp_async_wait_all();
-                __syncwarp();
-                for (int attempt = 0;; attempt++) {
-                    uint32_t sum = 0, pub = 0x80008000u;
-                    for (int u = lane; u < units; u += 32) {
-                        const uint4 q = *(const uint4*)&s_w16[8 * u];
-                        uint32_t w[4] = {q.x, q.y, q.z, q.w};
-                        if (u == 0 || u == units - 1) {
-#pragma unroll
-                            for (int i = 0; i < 8; i++) {
-                                const int at = 8 * u + i, sh = 16 * (i & 1);
-                                if (at < first || at >= last) w[i >> 1] = (w[i >> 1] & ~(0xFFFFu << sh)) | (1u << sh);
-                            }
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            sum += (w[i] & 0xFFFFu) + (w[i] >> 16);
-                            pub &= w[i] + 0x7FFF7FFFu;   // bit 15 of a half: it is not zero
-                        }
-                        sum -= 8;
-                    }
-                    if (__all_sync(0xffffffffu, (pub & 0x80008000u) == 0x80008000u)) {
-                        base = an_incl + __reduce_add_sync(0xffffffffu, sum);
-                        placed = true;
-                        break;
-                    }
-                    // a window with aggregates not yet published is copied again
-                    // (one round trip each) a few times before the global walk
-                    if (attempt == kWinRepolls) break;
-                    __nanosleep(64);
-                    const uint32_t* src = (const uint32_t*)(agg16_of(F) + lo);
-                    __syncwarp();
-                    for (int u = lane; u < units; u += 32) *(uint4*)&s_w16[8 * u] = ld_volatile_v4(src + 4 * u);
-                    __syncwarp();
-                }
-            }
-            if (!placed) base = prefix_resolve(FV(F, st_enc), t, agg, a.err);   // publishes t's inclusive prefix
-            else if (lane == 0) st_volatile64(&FV(F, st_enc)[t], kS64Inc | ((base + agg) & kS64Val));
-        }
+        unsigned long long base;
+        if (!s_win.offset(agg16_of(F), t, &base)) base = prefix_resolve(FV(F, st_enc), t, agg, a.err);   // (publishes)
+        else if (t > 0 && lane == 0) st_volatile64(&FV(F, st_enc)[t], kS64Inc | ((base + agg) & kS64Val));
         if (lane == 0) {
             const bool cap_ok = base + agg <= FV(F, payload_cap);
             if (!cap_ok) atomicExch(a.err, kErrCapacity);
             if (t == (int)FV(F, enc_tiles) - 1) FV(F, tot)->payload_bytes = base + agg;
             s_base[r & 1] = base;
             s_skip[r & 1] = !cap_ok;
-            s_an_t = t;
-            s_an_f = f;
-            s_an_incl = base + agg;
+            s_win.anchor(f, t, base + agg);
         }
         __syncwarp();
     };
@@ -714,7 +613,7 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
         }
         __syncthreads();   // statistics in (T_j's input is dead)
         // warp 0: T_{j-1}'s look-back window, in flight during the emission
-        if (warp == 0 && t1 >= 0) win_issue(fld(f1), f1, t1);
+        if (warp == 0 && t1 >= 0) s_win.issue(agg16_of(fld(f1)), f1, t1);
         // every warp: the tile's block offsets (two warp-wide halves)
         const bool in0 = lane < TB;
         const uint32_t sz0 = in0 ? s_size[lane] : 0;

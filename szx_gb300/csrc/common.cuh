@@ -209,14 +209,11 @@ __device__ __forceinline__ void split_reqlen(int reqLength, int* R, int* s) {
     *s = rb ? 8 - rb : 0;
 }
 
-__device__ __forceinline__ uint32_t bswap32(uint32_t v) { return __byte_perm(v, 0, 0x0123); }
 // 16 lead codes as stored (4 to a byte, MSB first), one bit of each pair set:
 // moved to value order, value e's bit (its pair's low one) to position 2e+1
 __device__ __forceinline__ uint32_t vorder(uint32_t m) { return __byte_perm(__brev(m), 0, 0x0123); }
 // byte i of x, zero-extended
 __device__ __forceinline__ uint32_t byte_of(uint32_t x, int i) { return __byte_perm(x, 0, 0x4440 | i); }
-// top `n8 / 8` bytes of a 32-bit word set (n8 = 8 * bytes, 0..24)
-__device__ __forceinline__ uint32_t top_bytes_mask(uint32_t n8) { return __funnelshift_r(0u, 0xFFFFFFFFu, n8); }
 
 // ------------------------------------------------------------------ warp scans
 
@@ -247,11 +244,6 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
 }
 __device__ __forceinline__ void st_release(unsigned long long* p, unsigned long long v) {
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_acquire32(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
 }
 
 // ------------------------------------------------------------------ decoupled look-back
@@ -381,9 +373,6 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, uint32_t coun
 }
 __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
 // Raise the transaction count the current phase waits for, without arriving.
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, uint32_t bytes) {
     asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
@@ -416,26 +405,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t pari
     return false;
 }
 
-// ------------------------------------------------------------------ wide look-back
-//
-// Tile status as one 32-bit word: [31:30] flag (0 empty, 1 aggregate,
-// 2 inclusive), [29:23] the tile's second count (<= 127), [22:0] the tile's
-// byte count (< 8 MiB).  Inclusive prefixes (64-bit) live in side arrays
-// written before the inclusive flag is released.  A walking warp reads 8
-// consecutive status words per lane (two 16-byte loads), i.e. 256
-// predecessors per memory round trip: the rate at which tiles can be placed
-// is then (256 / round-trip latency) instead of 32 / latency, which is what
-// lets a look-back over 16-32 KiB tiles keep up with HBM3e.
-struct TileStatus32 {
-    uint32_t* st;                  // [ntiles + 8], zeroed before the launch
-    unsigned long long* inc_a;     // [ntiles]
-    unsigned long long* inc_b;     // [ntiles]
-};
-constexpr uint32_t kSt32Agg = 1u << 30, kSt32Inc = 2u << 30;
-
-__device__ __forceinline__ void st_volatile32(uint32_t* p, uint32_t v) {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ uint4 ld_volatile_v4(const uint32_t* p) {
     uint4 v;
     asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -443,192 +412,6 @@ __device__ __forceinline__ uint4 ld_volatile_v4(const uint32_t* p) {
                  : "l"(p)
                  : "memory");
     return v;
-}
-
-// Second-value policies of the wide look-back.
-// SumPolicy: the 7-bit field is a count, prefixes add.
-struct SumPolicy {
-    static __device__ __forceinline__ unsigned long long contrib(uint32_t f, long long) { return f; }
-    static __device__ __forceinline__ unsigned long long op(unsigned long long x, unsigned long long y) { return x + y; }
-    static __device__ __forceinline__ unsigned long long reduce(unsigned long long v) { return warp_sum(v); }
-};
-
-// Whole warp.  agg_a < 2^23 (a sum), agg_b < 128 (combined by Policy).
-// Returns the exclusive prefixes.
-template <typename Policy = SumPolicy>
-__device__ __forceinline__ void lookback_wide(TileStatus32 s, long long tile, uint32_t agg_a, uint32_t agg_b,
-                                              unsigned long long* ex_a, unsigned long long* ex_b, int* err,
-                                              unsigned limit = kSpinLimit) {
-    const unsigned lane = lane_id();
-    const uint32_t packed = (agg_b << 23) | (agg_a & 0x7FFFFFu);
-    const unsigned long long self_b = Policy::contrib(agg_b, tile);
-    if (tile == 0) {
-        if (lane == 0) {
-            __stcg(&s.inc_a[0], (unsigned long long)agg_a);
-            __stcg(&s.inc_b[0], self_b);
-            __threadfence();
-            st_volatile32(&s.st[0], kSt32Inc | packed);
-        }
-        *ex_a = 0;
-        *ex_b = 0;
-        return;
-    }
-    if (lane == 0) st_volatile32(&s.st[tile], kSt32Agg | packed);
-    unsigned long long pa = 0, pb = 0;
-    long long g0 = ((tile - 1) >> 3) << 3;   // group of 8 holding the nearest predecessor
-    unsigned spins = 0;
-    bool failed = false;
-    while (true) {
-        const long long g = g0 - 8 * (long long)lane;
-        uint32_t w[8];
-        if (g >= 0) {
-            uint4 a = ld_volatile_v4(s.st + g), b = ld_volatile_v4(s.st + g + 4);
-            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; j++) w[j] = kSt32Inc;   // before tile 0: an inclusive zero
-        }
-        // nearest inclusive predecessor in this lane (highest index), and the
-        // readiness / combination of the aggregates above it
-        int inc_j = -1;
-        bool ready = true;
-        uint32_t sa = 0;
-        unsigned long long sb = 0;
-#pragma unroll
-        for (int j = 7; j >= 0; j--) {
-            const long long u = g + j;
-            const bool pred = u < tile;
-            const uint32_t f = w[j] & 0xC0000000u;
-            if (pred && inc_j < 0) {
-                if (f == kSt32Inc) inc_j = j;
-                else {
-                    ready = ready && f != 0;
-                    sa += w[j] & 0x7FFFFFu;
-                    sb = Policy::op(sb, Policy::contrib((w[j] >> 23) & 0x7Fu, u));
-                }
-            }
-        }
-        const unsigned inc_mask = __ballot_sync(0xffffffffu, inc_j >= 0);
-        const unsigned stop = inc_mask ? (unsigned)__ffs(inc_mask) - 1 : 31u;
-        const unsigned window = stop == 31u ? 0xffffffffu : ((1u << (stop + 1)) - 1);
-        if (__ballot_sync(0xffffffffu, !ready) & window) {
-            if (++spins > limit) { failed = true; break; }
-            __nanosleep(spins < 64 ? 32 : 256);
-            continue;
-        }
-        unsigned long long va = 0, vb = 0;
-        if (lane <= stop) { va = sa; vb = sb; }
-        if (lane == stop && inc_j >= 0 && g + inc_j >= 0) {
-            __threadfence();
-            va += __ldcg(&s.inc_a[g + inc_j]);
-            vb = Policy::op(vb, __ldcg(&s.inc_b[g + inc_j]));
-        }
-        pa += warp_sum(va);
-        pb = Policy::op(pb, Policy::reduce(vb));
-        if (inc_mask) break;
-        g0 -= 256;
-    }
-    if (failed && lane == 0) atomicExch(err, kErrLookback);
-    if (lane == 0) {
-        __stcg(&s.inc_a[tile], pa + agg_a);
-        __stcg(&s.inc_b[tile], Policy::op(pb, self_b));
-        __threadfence();
-        st_volatile32(&s.st[tile], kSt32Inc | packed);
-    }
-    *ex_a = pa;
-    *ex_b = pb;
-}
-
-// The wide look-back in two halves, so a tile's aggregate can be published
-// well before its prefix is needed (software-pipelined placement).
-template <typename Policy = SumPolicy>
-__device__ __forceinline__ void lookback_publish(TileStatus32 s, long long tile, uint32_t agg_a, uint32_t agg_b) {
-    if (lane_id() != 0) return;
-    const uint32_t packed = (agg_b << 23) | (agg_a & 0x7FFFFFu);
-    if (tile == 0) {
-        __stcg(&s.inc_a[0], (unsigned long long)agg_a);
-        __stcg(&s.inc_b[0], Policy::contrib(agg_b, 0));
-        __threadfence();
-        st_volatile32(&s.st[0], kSt32Inc | packed);
-    } else {
-        st_volatile32(&s.st[tile], kSt32Agg | packed);
-    }
-}
-
-// Whole warp; the tile's aggregate must already be published.
-template <typename Policy = SumPolicy>
-__device__ __forceinline__ void lookback_resolve(TileStatus32 s, long long tile, uint32_t agg_a, uint32_t agg_b,
-                                                 unsigned long long* ex_a, unsigned long long* ex_b, int* err,
-                                                 unsigned limit = kSpinLimit) {
-    const unsigned lane = lane_id();
-    if (tile == 0) {
-        *ex_a = 0;
-        *ex_b = 0;
-        return;
-    }
-    const uint32_t packed = (agg_b << 23) | (agg_a & 0x7FFFFFu);
-    const unsigned long long self_b = Policy::contrib(agg_b, tile);
-    unsigned long long pa = 0, pb = 0;
-    long long g0 = ((tile - 1) >> 3) << 3;
-    unsigned spins = 0;
-    bool failed = false;
-    while (true) {
-        const long long g = g0 - 8 * (long long)lane;
-        uint32_t w[8];
-        if (g >= 0) {
-            uint4 a = ld_volatile_v4(s.st + g), b = ld_volatile_v4(s.st + g + 4);
-            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; j++) w[j] = kSt32Inc;
-        }
-        int inc_j = -1;
-        bool ready = true;
-        uint32_t sa = 0;
-        unsigned long long sb = 0;
-#pragma unroll
-        for (int j = 7; j >= 0; j--) {
-            const long long u = g + j;
-            const bool pred = u < tile;
-            const uint32_t f = w[j] & 0xC0000000u;
-            if (pred && inc_j < 0) {
-                if (f == kSt32Inc) inc_j = j;
-                else {
-                    ready = ready && f != 0;
-                    sa += w[j] & 0x7FFFFFu;
-                    sb = Policy::op(sb, Policy::contrib((w[j] >> 23) & 0x7Fu, u));
-                }
-            }
-        }
-        const unsigned inc_mask = __ballot_sync(0xffffffffu, inc_j >= 0);
-        const unsigned stop = inc_mask ? (unsigned)__ffs(inc_mask) - 1 : 31u;
-        const unsigned window = stop == 31u ? 0xffffffffu : ((1u << (stop + 1)) - 1);
-        if (__ballot_sync(0xffffffffu, !ready) & window) {
-            if (++spins > limit) { failed = true; break; }
-            __nanosleep(spins < 64 ? 32 : 256);
-            continue;
-        }
-        unsigned long long va = 0, vb = 0;
-        if (lane <= stop) { va = sa; vb = sb; }
-        if (lane == stop && inc_j >= 0 && g + inc_j >= 0) {
-            __threadfence();
-            va += __ldcg(&s.inc_a[g + inc_j]);
-            vb = Policy::op(vb, __ldcg(&s.inc_b[g + inc_j]));
-        }
-        pa += warp_sum(va);
-        pb = Policy::op(pb, Policy::reduce(vb));
-        if (inc_mask) break;
-        g0 -= 256;
-    }
-    if (failed && lane == 0) atomicExch(err, kErrLookback);
-    if (lane == 0) {
-        __stcg(&s.inc_a[tile], pa + agg_a);
-        __stcg(&s.inc_b[tile], Policy::op(pb, self_b));
-        __threadfence();
-        st_volatile32(&s.st[tile], kSt32Inc | packed);
-    }
-    *ex_a = pa;
-    *ex_b = pb;
 }
 
 // ------------------------------------------------------------------ inline-prefix look-back
@@ -702,12 +485,6 @@ __device__ __forceinline__ unsigned long long prefix_resolve(unsigned long long*
     return pa;
 }
 
-// Tiles a placement window of the blocked encoder reaches back (2 KiB of
-// 16-bit counts): a CTA's previous tile is one launch's CTAs back on average
-// (456), further for a CTA that lags; 512 sent a third of the lagging CTAs'
-// tiles to the global walk.
-constexpr int kLbWin = 1024;
-
 // One pass of cta_copy_realign for a word phase of WS: 16 destination bytes
 // are words WS .. WS+4 of two 16-byte staging chunks, shifted by rs bits.
 // sp: shared address of the first of n full destination chunks' staging chunk.
@@ -772,4 +549,113 @@ __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.w
 __device__ __forceinline__ void st_relaxed16(uint16_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u16 [%0], %1;" ::"l"(p), "h"((unsigned short)v) : "memory");
 }
+
+// Lane-predicated claim of the next tile: the reply is waited for where `next`
+// is used, not at the end of a branch.
+__device__ __forceinline__ void claim_tile(unsigned long long& next, unsigned long long* ctr, bool take) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p atom.relaxed.gpu.global.add.u64 %0, [%1], 1;\n\t}"
+                 : "+l"(next)
+                 : "l"(ctr), "r"((uint32_t)take)
+                 : "memory");
+}
+
+// ------------------------------------------------------------------ placement window
+//
+// How the persistent encoders place a tile: its offset is the inclusive prefix
+// of this CTA's previous tile (the anchor, known here) plus the byte counts of
+// the tiles claimed between the two, read from 16-bit words (count + 1, 0: not
+// yet published) that one warp copies into shared memory well before it needs
+// them.  A tile without an anchor within kLbWin tiles of the same field, or
+// with counts still missing after a few re-reads, falls back to the global
+// look-back over the 64-bit status words (prefix_resolve), which every
+// placement keeps valid by publishing its inclusive prefix.
+//
+// kLbWin (2 KiB of counts): a CTA's previous tile is one launch's CTAs back on
+// average (456 or 608), further for a CTA that lags; 512 sent a third of the
+// lagging CTAs' tiles to the global walk.
+constexpr int kLbWin = 1024;
+constexpr int kWinRepolls = 32;   // window re-reads before the global look-back walk
+struct PlaceWin {   // shared memory; one warp's own
+    __align__(16) uint16_t w16[kLbWin + 8];
+    unsigned long long an_incl;   // the anchor's inclusive prefix
+    int an_t, an_f, lo, ok;       // anchor tile (-1: none), its field; the window's first tile and state
+    __device__ __forceinline__ void init() {   // one thread
+        an_t = -1;
+        an_f = -1;
+        an_incl = 0;
+        ok = 0;
+    }
+    __device__ __forceinline__ void anchor(int f, int t, unsigned long long incl) {   // lane 0
+        an_t = t;
+        an_f = f;
+        an_incl = incl;
+    }
+    // whole warp: start copying the window of tile t of field f (counts agg)
+    __device__ __forceinline__ void issue(const uint16_t* agg, int f, int t) {
+        const int lane = (int)lane_id(), a = an_t;
+        int state = 0, first = 0;
+        if (t > 0 && a >= 0 && an_f == f && a < t && t - a - 1 <= kLbWin) {
+            if (t - a == 1) {
+                state = 2;
+            } else {
+                first = (a + 1) & ~7;
+                const int units = (t - first + 7) >> 3;
+                for (int u = lane; u < units; u += 32) cp_async16(&w16[8 * u], agg + first + 8 * u);
+                state = 1;
+            }
+        }
+        if (lane == 0) {
+            lo = first;
+            ok = state;
+        }
+        __syncwarp();
+    }
+    // whole warp: tile t's offset from the window, false when it has to come
+    // from the global look-back
+    __device__ __forceinline__ bool offset(const uint16_t* agg, int t, unsigned long long* base) {
+        *base = 0;
+        if (t == 0) return true;
+        const int state = ok, at0 = an_t;
+        const unsigned long long incl = an_incl;
+        *base = incl;
+        if (state == 2) return true;
+        if (state != 1) return false;
+        // Sum of the counts of tiles an_t + 1 .. t - 1, eight to a 16-byte
+        // read and a redux across the warp; the words outside that range count
+        // as 1, published and empty.
+        const int lane = (int)lane_id(), l = lo, units = (t - l + 7) >> 3, first = at0 + 1 - l, last = t - l;
+        cp_async_wait_all();
+        __syncwarp();
+        for (int attempt = 0;; attempt++) {
+            uint32_t sum = 0, least = ~0u;
+            for (int u = lane; u < units; u += 32) {
+                const uint4 q = *(const uint4*)&w16[8 * u];
+                uint32_t w[4] = {q.x, q.y, q.z, q.w};
+                if (u == 0 || u == units - 1) {
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const int at = 8 * u + i, sh = 16 * (i & 1);
+                        if (at < first || at >= last) w[i >> 1] = (w[i >> 1] & ~(0xFFFFu << sh)) | (1u << sh);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    sum = __dp2a_lo(w[i], 0x0101u, sum);
+                    least = __vminu2(least, w[i]);
+                }
+                sum -= 8;
+            }
+            if (__all_sync(0xffffffffu, (least & 0xFFFFu) != 0 && least >= 0x10000u)) {
+                *base = incl + __reduce_add_sync(0xffffffffu, sum);
+                return true;
+            }
+            if (attempt == kWinRepolls) return false;
+            __nanosleep(64);
+            const uint32_t* src = (const uint32_t*)(agg + l);
+            __syncwarp();
+            for (int u = lane; u < units; u += 32) *(uint4*)&w16[8 * u] = ld_volatile_v4(src + 4 * u);
+            __syncwarp();
+        }
+    }
+};
 }  // namespace szxg

@@ -10,7 +10,7 @@
 // the whole array: each value's lead code depends only on its predecessor, so
 // codes are data-parallel; mid-byte positions need a device-wide prefix sum
 // (encoder: decoupled look-back over 4096-value tiles, placed from the CTA's
-// own previous tile and a window of status words).  Decoding must also find,
+// own previous tile and a window of counts).  Decoding must also find,
 // for every value, the last earlier value that stored each of the top three
 // byte lanes -- possibly many tiles back.  The lead codes alone give every
 // tile's byte count and its last writers, so the decoder needs no look-back:
@@ -47,39 +47,6 @@ __device__ __forceinline__ uint32_t cta_excl_sum32(uint32_t v, uint32_t* tot, ui
     }
     *tot = t;
     return pre + incl - v;
-}
-
-// Copy [sh, sh+n) of a 16-aligned shared buffer to global dst (dst % 16 == sh).
-__device__ __forceinline__ void cta_copy_out(const uint8_t* stage, uint32_t sh, uint32_t n, uint8_t* dst) {
-    uint8_t* gbase = dst - sh;
-    const uint32_t end = sh + n, nch = (end + 15) >> 4;
-    for (uint32_t c = threadIdx.x; c < nch; c += blockDim.x) {
-        uint32_t lo = c << 4;
-        if (lo >= sh && lo + 16 <= end) *(uint4*)(gbase + lo) = *(const uint4*)(stage + lo);
-    }
-    // partial head chunk: threads 0-15, partial tail chunk: threads 16-31
-    if (threadIdx.x < 32) {
-        const uint32_t last = nch - 1;
-        const uint32_t c = threadIdx.x < 16 ? 0 : last;
-        const bool part = threadIdx.x < 16 ? (sh > 0 || end < 16) : (last > 0 && (end & 15) != 0);
-        const uint32_t b = (c << 4) + (threadIdx.x & 15);
-        if (part && b >= sh && b < end) gbase[b] = stage[b];
-    }
-}
-
-// Stage [src, src+n) into a 16-aligned shared buffer at offset src % 16; bytes
-// outside [s0, s1) are never read.
-__device__ __forceinline__ void cta_copy_in(uint8_t* stage, const uint8_t* src, uint32_t n, const uint8_t* s0,
-                                            const uint8_t* s1) {
-    const uint32_t sh = (uint32_t)((uintptr_t)src & 15);
-    const uint8_t* gbase = src - sh;
-    const uint32_t nch = (sh + n + 15) >> 4;
-    for (uint32_t c = threadIdx.x; c < nch; c += blockDim.x) {
-        const uint8_t* lo = gbase + (c << 4);
-        if (lo >= s0 && lo + 16 <= s1) *(uint4*)(stage + (c << 4)) = __ldg((const uint4*)lo);
-        else
-            for (int j = 0; j < 16; j++) stage[(c << 4) + j] = (lo + j >= s0 && lo + j < s1) ? lo[j] : 0;
-    }
 }
 
 template <typename T>
@@ -140,31 +107,27 @@ struct NbEncArgs {
     unsigned long long n, ntiles, cap;
     const CodecParams* params;
     uint8_t* out;
-    TileStatus32 st;
+    unsigned long long* st;   // look-back status words [ntiles + 4], zeroed
+    uint16_t* agg;            // counts + 1 [ntiles + 16], zeroed
     unsigned long long* tile_ctr;
     int* err;
     StreamResult* res;
 };
 
 // One pass over the input in tiles of kNbTile values taken from an atomic
-// counter, one tile ahead.  Per tile T_j: the values (loaded during the
-// previous iteration), shifted words and lead codes (one XOR chain over the
-// whole array: a thread's first value's predecessor is the previous
-// thread's last, or the value before the tile), a CTA scan of the
-// stored-byte counts, the tile's byte count published to the look-back, the
-// lead codes written to their fixed place, the mid bytes emitted into one of
-// three shared staging buffers with byte stores at tile-local offsets.
-// T_{j-2} is placed two iterations late, so that the other CTAs' tiles
-// claimed before it have normally published their counts: its offset is the
-// inclusive prefix of this CTA's previous tile (known here) plus the counts
-// of the tiles claimed in between, read from a window of status words copied
-// in with cp.async during the emission (a window with unpublished words is
-// copied again a few times, then the global look-back takes over); then the
-// CTA copies T_{j-2}'s bytes out, realigned.  Two barriers per tile: the
-// scan's and the one that hands the placement to the copy-out.
-constexpr int kNbWin = 1024;   // status words per placement window (4 KiB)
-constexpr int kNbRepolls = 32;
-
+// counter, one tile ahead.  Iteration j, between two CTA barriers: the values
+// of T_j (loaded during the previous iteration), differences and lead codes
+// (one XOR chain over the whole array: a thread's first value's predecessor is
+// the previous thread's last, or the value before the tile), a CTA scan of the
+// stored-byte counts | barrier | the tile's byte count published, the lead
+// codes to their fixed place, the mid bytes into one of three shared staging
+// buffers, the next tile's loads; then warp 0 places T_{j-1} (PlaceWin; its
+// window was copied in during the emission) while the other warps copy T_{j-2}
+// to its place | barrier | the bytes of the words that threads share.
+// Bound by the instruction rate and the two barriers, 244 us at 2^27 float32
+// values (512 MiB read, 129 us at the copy rate).  With the placement of
+// T_{j-2} between the barriers, followed by a status word beside a prefix array
+// and a fence, the seven other warps waited for warp 0 half the time: 395 us.
 template <typename T>
 constexpr int nb_stage_bytes() { return ((kNbTile * (int)sizeof(T) + 48) + 15) / 16 * 16; }
 
@@ -176,12 +139,12 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
     constexpr int W = EL::W;
     extern __shared__ __align__(16) uint8_t nb_dyn[];   // three staging buffers of nb_stage_bytes<T>()
     auto stage = [&](int k) { return nb_dyn + ((unsigned)k % 3u) * nb_stage_bytes<T>(); };
-    __shared__ __align__(16) uint32_t s_win[kNbWin + 8];
+    __shared__ PlaceWin s_win;
     __shared__ uint32_t s_sum[8];
-    __shared__ long long s_tile[2];
+    __shared__ int s_tile[2];
     __shared__ uint32_t s_total[3];
-    __shared__ unsigned long long s_base;
-    __shared__ int s_skip;
+    __shared__ unsigned long long s_base[2];
+    __shared__ int s_skip[2];
     const T* x = (const T*)a.x;
     const CodecParams P = *a.params;
     // szx/src/szx_float.cc:1514-1535 / szx_double.cc:1615-1636
@@ -200,90 +163,18 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
     const int lane = threadIdx.x & 31;
     const int down = 8 * W - reqLength;
     const uint32_t guard = 0x80u << s, s4 = (uint32_t)(31 + s) * 0x01010101u, R4 = (uint32_t)R * 0x01010101u;
-    const long long nt = (long long)a.ntiles;
-    // warp 0's placement state: anchor tile and its inclusive prefix; window
-    long long an_t = -1;
-    unsigned long long an_incl = 0;
-    long long w_lo = 0;
-    int w_ok = 0;
-    long long pend_t = -1;   // a tile placed from the window, its inclusive prefix not yet published
-    uint32_t pend_agg = 0;
-    auto publish = [&]() {
-        if (pend_t > 0 && lane == 0) {
-            __stcg(&a.st.inc_a[pend_t], an_incl);
-            __stcg(&a.st.inc_b[pend_t], 0ull);
-            __threadfence();
-            st_volatile32(&a.st.st[pend_t], kSt32Inc | (pend_agg & 0x7FFFFFu));
-        }
-        pend_t = -1;
-    };
-    // warp 0: copy the status words of the tiles between the anchor and t
-    auto win_issue = [&](long long t) {
-        w_ok = 0;
-        if (an_t >= 0 && an_t < t && t - an_t - 1 <= kNbWin) {
-            if (t - an_t == 1) {
-                w_ok = 2;
-            } else {
-                w_lo = (an_t + 1) & ~3ll;
-                const int units = (int)((t - w_lo + 3) >> 2);
-                for (int u = lane; u < units; u += 32) cp_async16(&s_win[4 * u], a.st.st + w_lo + 4 * u);
-                w_ok = 1;
-            }
-        }
-    };
-    // warp 0: offset of tile t (count agg), its inclusive prefix published
-    auto place = [&](long long t, uint32_t agg) {
-        unsigned long long base = 0;
-        bool placed = t == 0;
-        if (!placed && w_ok == 2) {
-            base = an_incl;
-            placed = true;
-        } else if (!placed && w_ok == 1) {
-            // counts of tiles an_t + 1 .. t - 1, four status words to a read
-            const int units = (int)((t - w_lo + 3) >> 2);
-            const int lo = (int)(an_t + 1 - w_lo), hi = (int)(t - w_lo);
-            cp_async_wait_all();
-            __syncwarp();
-            for (int attempt = 0;; attempt++) {
-                uint32_t sum = 0;
-                bool ready = true;
-                for (int u = lane; u < units; u += 32) {
-                    const uint4 q = *(const uint4*)&s_win[4 * u];
-                    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int at = 4 * u + i;
-                        if (at >= lo && at < hi) {
-                            ready = ready && w[i] >= kSt32Agg;
-                            sum += w[i] & 0x7FFFFFu;
-                        }
-                    }
-                }
-                if (__all_sync(0xffffffffu, ready)) {
-                    base = an_incl + __reduce_add_sync(0xffffffffu, sum);
-                    placed = true;
-                    break;
-                }
-                if (attempt == kNbRepolls) break;
-                __nanosleep(128);
-                __syncwarp();
-                for (int u = lane; u < units; u += 32) *(uint4*)&s_win[4 * u] = ld_volatile_v4(a.st.st + w_lo + 4 * u);
-                __syncwarp();
-            }
-        }
-        if (!placed) {
-            unsigned long long dummy;
-            lookback_resolve(a.st, t, agg, 0, &base, &dummy, a.err);   // publishes t's inclusive prefix
-        } else if (t > 0) {
-            pend_t = t;   // published after the barrier, off the CTA's critical path
-            pend_agg = agg;
-        }
-        an_t = t;
-        an_incl = base + agg;
+    const int nt = (int)a.ntiles;
+    // warp 0: tile t (count agg, iteration k) placed, the header and result with the last tile
+    auto place = [&](int t, int k) {
+        const uint32_t agg = s_total[(unsigned)k % 3u];
+        unsigned long long base;
+        if (!s_win.offset(a.agg, t, &base)) base = prefix_resolve(a.st, t, agg, a.err);   // (publishes)
+        else if (t > 0 && lane == 0) st_volatile64(&a.st[t], kS64Inc | ((base + agg) & kS64Val));
         if (lane == 0) {
-            s_base = base;
+            s_win.anchor(0, t, base + agg);
+            s_base[k & 1] = base;
             const bool ok = base + agg <= mid_cap;
-            s_skip = !ok;
+            s_skip[k & 1] = !ok;
             if (!ok) atomicExch(a.err, kErrCapacity);
             if (t == nt - 1) {
                 uint8_t* h = a.out + kNbShift;
@@ -291,7 +182,7 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
                 h[4] = (uint8_t)reqLength;
                 h[5] = (uint8_t)(med_stored >> 24); h[6] = (uint8_t)(med_stored >> 16);
                 h[7] = (uint8_t)(med_stored >> 8); h[8] = (uint8_t)med_stored;
-                for (int k = 0; k < 8; k++) h[9 + k] = (uint8_t)(L >> (56 - 8 * k));
+                for (int q = 0; q < 8; q++) h[9 + q] = (uint8_t)(L >> (56 - 8 * q));
                 StreamResult r;
                 r.offset = kNbShift;
                 r.size = 17 + L + base + agg;
@@ -301,23 +192,30 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
                 *a.res = r;
             }
         }
+        __syncwarp();
     };
-    if (threadIdx.x == 0) s_tile[0] = (long long)atomicAdd(a.tile_ctr, 1ull);
+    if (threadIdx.x == 0) {
+        s_win.init();
+        const unsigned long long g = atomicAdd(a.tile_ctr, 1ull);
+        s_tile[0] = g < a.ntiles ? (int)g : -1;
+    }
     __syncthreads();
-    long long tile = s_tile[0];
-    long long t1 = -1, t2 = -1;   // T_{j-1}, T_{j-2}: staged, T_{j-2} placed in this iteration
+    int tile = s_tile[0], t1 = -1, t2 = -1;   // T_j, T_{j-1}, T_{j-2}; -1: none
+    const bool taker = threadIdx.x == kNbThreads - 32;   // the last warp claims the tiles
     T v[kNbPer];
     T before = (T)0;     // lane 0: the value before its first one
-    auto fetch = [&](long long t) {
+    auto fetch = [&](int t) {
         const unsigned long long first = (unsigned long long)t * kNbTile + threadIdx.x * kNbPer;
         load16<T>(x, first, a.n, v);
         before = (lane == 0 && first > 0 && first - 1 < a.n) ? x[first - 1] : (T)0;
     };
-    if (tile < nt) fetch(tile);
-    int it = 0;
-    for (; tile < nt; it++) {
-        // the next tile, claimed now and read after the scan's barriers
-        if (threadIdx.x == 0) s_tile[(it + 1) & 1] = (long long)atomicAdd(a.tile_ctr, 1ull);
+    if (tile >= 0) fetch(tile);
+    // (after the last tile two more iterations place and copy out what is staged)
+    for (int it = 0; tile >= 0 || t1 >= 0 || t2 >= 0; it++) {
+        const bool live = tile >= 0;
+        // the next tile's claim; the reply is used before the scan's barrier
+        unsigned long long gc = ~0ull;
+        claim_tile(gc, a.tile_ctr, taker && live);
         const unsigned long long first = (unsigned long long)tile * kNbTile + threadIdx.x * kNbPer;
         U d[kNbPer];
         const T dprev = EL::sub(before, med);
@@ -362,12 +260,22 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
             mine = __dp4a(c4, 0x01010101u, mine);
             codes |= ((ldb * 0x40100401u) >> 24) << (8 * k);   // 4 leads -> one byte, MSB first
         }
+        if (taker) s_tile[(it + 1) & 1] = gc < a.ntiles ? (int)gc : -1;
         uint32_t total;
         const uint32_t ex = cta_excl_sum32(mine, &total, s_sum);   // one barrier
-        if (threadIdx.x < 32) lookback_publish(a.st, tile, total, 0);
-        if (threadIdx.x == 0) s_total[it % 3] = total;
-        // T_{j-2}'s window, in flight during the emission
-        if (threadIdx.x < 32 && t2 >= 0) win_issue(t2);
+        if (threadIdx.x < 32) {
+            if (live) {
+                if (lane == 0) {
+                    s_total[(unsigned)it % 3u] = total;
+                    st_relaxed16(a.agg + tile, total + 1);
+                }
+                prefix_publish(a.st, tile, total);
+            }
+            // T_{j-1}'s window, in flight during the emission
+            if (t1 >= 0) s_win.issue(a.agg, 0, t1);
+        }
+        RunOut o;
+        if (live) {
         // lead codes: 4 bytes per thread, at their fixed place
         const unsigned long long lb = first >> 2;
         if (lb + 4 <= L && ((uintptr_t)(lead + lb) & 3) == 0) *(uint32_t*)(lead + lb) = codes;
@@ -377,7 +285,6 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
         // mid bytes: each value's low (R - lead) bytes of its required bits, at
         // tile-local offsets: whole words now, the bytes of the words that
         // threads share after the barrier below
-        RunOut o;
         o.start(stage(it), ex);
 #pragma unroll
         for (int k = 0; k < kNbPer / 4; k++) {
@@ -394,33 +301,21 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
                 }
             }
         }
-        // the next tile's values are in flight during the placement
-        const long long next = s_tile[(it + 1) & 1];
-        if (next < nt) fetch(next);
-        if (threadIdx.x < 32 && t2 >= 0) place(t2, s_total[(it - 2) % 3]);
-        __syncthreads();   // T_j's whole words staged; T_{j-2}'s offset known
-        o.finish(stage(it), ex);   // (read by T_j's copy-out, two iterations on)
-        if (threadIdx.x < 32) publish();
-        if (t2 >= 0 && !s_skip) cta_copy_realign(stage(it - 2), s_total[(it - 2) % 3], mid + s_base, threadIdx.x, kNbThreads);
-        // no barrier here: the next writes of T_{j-2}'s buffer (T_{j+1}'s
-        // emission), of s_base / s_skip (the next placement) and of s_sum /
-        // s_total all come after the next iteration's scan barrier
+        }
+        // the next tile's values are in flight during the placement and the copy-out
+        const int next = s_tile[(it + 1) & 1];
+        if (next >= 0) fetch(next);
+        if (threadIdx.x < 32) {
+            if (t1 >= 0) place(t1, it - 1);
+        } else if (t2 >= 0 && !s_skip[it & 1]) {
+            cta_copy_realign(stage(it + 1), s_total[(unsigned)(it + 1) % 3u], mid + s_base[it & 1], threadIdx.x - 32,
+                             kNbThreads - 32);
+        }
+        __syncthreads();   // T_j's whole words staged; T_{j-1}'s offset known, T_{j-2}'s buffer free
+        if (live) o.finish(stage(it), ex);   // (read by T_j's copy-out, two iterations on)
         t2 = t1;
         t1 = tile;
         tile = next;
-    }
-    // the CTA's last two tiles, oldest first
-    for (int back = 2; back >= 1; back--) {
-        const long long t = back == 2 ? t2 : t1;
-        if (t < 0) continue;
-        __syncthreads();   // the last copy-out has read s_base / s_skip
-        if (threadIdx.x < 32) {
-            win_issue(t);
-            place(t, s_total[(it - back) % 3]);
-        }
-        __syncthreads();
-        if (threadIdx.x < 32) publish();
-        if (!s_skip) cta_copy_realign(stage(it - back), s_total[(it - back) % 3], mid + s_base, threadIdx.x, kNbThreads);
     }
 }
 
@@ -432,11 +327,13 @@ size_t nonblocked_bound(int dtype, size_t n) {
 ClearList nonblocked_enc_clear(const Workspace& ws, size_t n) {
     const size_t ntiles = (n + kNbTile - 1) / kNbTile;
     ClearList c{};
-    c.p[0] = ws.st32;
-    c.bytes[0] = sizeof(uint32_t) * (ntiles + 8);
+    c.p[0] = ws.st32;   // the 16-bit counts
+    c.bytes[0] = (2 * (ntiles + 16) + 3) & ~size_t(3);
     c.p[1] = ws.totals;
     c.bytes[1] = kWsHeaderClear;
-    c.n = 2;
+    c.p[2] = ws.st_word;
+    c.bytes[2] = sizeof(unsigned long long) * (ntiles + 4);
+    c.n = 3;
     return c;
 }
 
@@ -444,11 +341,13 @@ cudaError_t launch_nonblocked_encode(int dtype, const void* x, size_t n, uint8_t
                                      const Workspace& ws, cudaStream_t s, bool cleared, StreamResult* res_out) {
     if (n == 0 || cap < nonblocked_bound(dtype, n) - 64) return cudaErrorInvalidValue;
     const size_t ntiles = (n + kNbTile - 1) / kNbTile;
+    if (ntiles > 0x7FFFFFFF) return cudaErrorInvalidValue;
     cudaError_t e;
     if (!cleared && (e = launch_ws_clear(nonblocked_enc_clear(ws, n), s)) != cudaSuccess) return e;
     NbEncArgs a;
     a.x = x; a.n = n; a.ntiles = ntiles; a.cap = cap; a.params = ws.params; a.out = d_out;
-    a.st = TileStatus32{ws.st32, ws.st_agg2, ws.st_inc2};
+    a.st = ws.st_word;
+    a.agg = (uint16_t*)ws.st32;
     a.tile_ctr = &ws.counters[0];
     a.err = ws.err;
     a.res = res_out ? res_out : ws.result;

@@ -42,7 +42,6 @@ template <typename T, int G>
 struct Chunks {
     static constexpr int E = EncCfg<T>::E;
     static constexpr int NC = E / 4;                  // chunks per lane
-    static constexpr int CB = 4 * (int)sizeof(T);     // bytes per chunk
     // first value of the lane's k-th chunk
     static __device__ __forceinline__ int first(int sl, int k) { return 4 * (sl + k * G); }
 };

@@ -23,9 +23,8 @@ namespace szxg {
 namespace {
 
 // scan 0: the 64-bit status words of the encoders' placement (prefix_resolve);
-// scan 1: the 32-bit words with an inclusive side array (lookback_wide) of the
-//         decoders and the non-blocked layout.
-__global__ void k_selftest_lookback(int scan, unsigned long long* st64, TileStatus32 st32, int ntiles, int withheld,
+// scan 1: the words with side arrays (lookback) of the decoders' index.
+__global__ void k_selftest_lookback(int scan, unsigned long long* st64, TileStatus st, int ntiles, int withheld,
                                     unsigned limit, unsigned long long* prefix, int* err) {
     const long long tile = blockIdx.x;
     if (tile >= ntiles || tile == withheld) return;   // the withheld tile never publishes
@@ -36,7 +35,7 @@ __global__ void k_selftest_lookback(int scan, unsigned long long* st64, TileStat
         p = prefix_resolve(st64, tile, agg, err, limit);
     } else {
         unsigned long long dummy = 0;
-        lookback_wide(st32, tile, (uint32_t)agg, 0u, &p, &dummy, err, limit);
+        lookback(st, tile, agg, 0, &p, &dummy, err, limit);
     }
     if (lane_id() == 0) prefix[tile] = p;
 }
@@ -55,8 +54,7 @@ extern "C" int SZxG_selftest_lookback(int scan, int ntiles, int withheld, unsign
     cudaStream_t s = (cudaStream_t)stream;
     const size_t n = (size_t)ntiles;
     auto a256 = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t o32 = a256(8 * (n + 8)), oinc = o32 + a256(4 * (n + 8)), opre = oinc + a256(16 * n),
-                 oerr = opre + a256(8 * n), bytes = oerr + 256;
+    const size_t ost = a256(8 * (n + 8)), opre = ost + a256(24 * n), oerr = opre + a256(8 * n), bytes = oerr + 256;
     unsigned char* b = nullptr;
     if (cudaMalloc(&b, bytes) != cudaSuccess) {
         cudaGetLastError();
@@ -64,16 +62,16 @@ extern "C" int SZxG_selftest_lookback(int scan, int ntiles, int withheld, unsign
         return SZXG_ERR_CUDA;
     }
     unsigned long long* st64 = (unsigned long long*)b;          // [n + 8]
-    TileStatus32 st32;
-    st32.st = (uint32_t*)(b + o32);                             // [n + 8]
-    st32.inc_a = (unsigned long long*)(b + oinc);               // [n]
-    st32.inc_b = st32.inc_a + n;                                // [n]
+    TileStatus st;
+    st.word = (unsigned long long*)(b + ost);                   // [n] each
+    st.agg2 = st.word + n;
+    st.inc2 = st.agg2 + n;
     unsigned long long* d_prefix = (unsigned long long*)(b + opre);
     int* d_err = (int*)(b + oerr);
     int rc = SZXG_OK;
     cudaError_t e = cudaMemsetAsync(b, 0, bytes, s);
     if (e == cudaSuccess) {
-        k_selftest_lookback<<<ntiles, kWarp, 0, s>>>(scan, st64, st32, ntiles, withheld, spinLimit, d_prefix, d_err);
+        k_selftest_lookback<<<ntiles, kWarp, 0, s>>>(scan, st64, st, ntiles, withheld, spinLimit, d_prefix, d_err);
         e = cudaGetLastError();
     }
     int h_err = 0;

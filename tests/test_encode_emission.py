@@ -76,3 +76,20 @@ def test_non_blocked_streams_at_emission_edges(szx, dt, n):
             buf[off:off + n] = torch.from_numpy(x).cuda()
             codec.compress(buf[off:off + n], szx.ABS, eb)
             assert codec.stream_bytes().cpu().numpy().tobytes() == O.compress(1, x, eb, 128), (name, off)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("tiles", [2, 3, 700, 4 * 608])
+def test_non_blocked_placement(szx, dt, tiles):
+    """Tiles placed from the CTA's previous one: fewer tiles than CTAs, each CTA
+    with one to several, a window beyond the counts' end, byte counts of tiles
+    from nothing stored to every byte."""
+    n = tiles * 4096 - 5
+    rng = np.random.default_rng(5)
+    x = rng.normal(size=n).astype(dt)
+    for t in rng.choice(tiles, tiles // 2, replace=False):
+        x[t * 4096:(t + 1) * 4096] = 0.25
+    import torch
+    codec = szx.DeviceCodec(1, dt, n)
+    codec.compress(torch.from_numpy(x).cuda(), szx.ABS, 1e-12)
+    assert codec.stream_bytes().cpu().numpy().tobytes() == O.compress(1, x, 1e-12, 128)
