@@ -187,8 +187,8 @@ int SZxG_decompress_host_into(int fastMode, int dataType, const unsigned char* b
  *
  * SZxG_batch_create plans the batch once: it checks the fields, lays out
  * every field's scratch, allocates it (one cudaMalloc) and uploads the field
- * table.  SZxG_batch_run then only enqueues memsets, kernels and (optionally)
- * a device-to-device copy of the per-field results on `stream`, so it can be
+ * table.  SZxG_batch_run then only enqueues kernels and (optionally) a
+ * device-to-device copy of the per-field results on `stream`, so it can be
  * captured into a CUDA graph and replayed; the fields' buffers must stay
  * valid while the plan is used.  Runs of one plan must not overlap. */
 typedef struct {
@@ -220,7 +220,8 @@ void SZxG_batch_destroy(SZxG_Batch* batch);
 /* Launch shapes by field-size class (no counterpart in the reference).  A
  * batch groups its fields by size class -- the first entry whose maxValues is
  * >= the field's value count, the last entry for larger fields -- and codes
- * each class with one persistent launch per kernel of that class's shape:
+ * each run of neighbouring classes of one shape with one persistent launch
+ * per kernel of that shape:
  * encoder tile variant (0: 16 KiB of input per tile, 8 warps per CTA; 1:
  * 8 KiB, 4 warps -- float blocks of 65..128 values only, else as 0) and CTAs
  * per SM of the encoder and the decoder (0: as many as fit).  Shapes change
@@ -251,8 +252,8 @@ int SZxG_batch_set_bounds(SZxG_Batch* batch, int nActive, const int* fieldIndex,
 
 /* ---------------------------------------------------------------- fixed rate, learned
  * A small network predicts the bound that gives a target compression ratio
- * from 32 features of every 10th block; real compress passes of the whole
- * batch judge it (float fields, blockSize 128).  Features of a field, row
+ * from 32 features of every 10th block; the streams' exact sizes at the bound,
+ * measured over the whole batch, judge it (float fields, blockSize 128).  Features of a field, row
  * layout of X (SZXG_FXR_FEATURES floats): see szx_gb300/csrc/learned.cu. */
 #define SZXG_FXR_FEATURES 32
 typedef struct SZxG_Mlp SZxG_Mlp;
@@ -276,10 +277,10 @@ int SZxG_mlp_train(SZxG_Mlp* mlp, const float* d_X, const float* d_y, size_t n, 
  * sampled range (synchronous). */
 int SZxG_batch_features(SZxG_Batch* batch, int nRows, const int* fieldOfRow, const float* targetRatio, float* d_X,
                         float* h_range, void* stream);
-/* Choose every field's bound for targetRatio[f] within `tolerance` by real
- * compress passes of the plan (mlp NULL: plain bisection; else prediction,
- * one re-targeted prediction, then bisection), leaving the chosen streams in
- * the fields' buffers.  Outputs per field: bound, achieved ratio, passes. */
+/* Choose every field's bound for targetRatio[f] within `tolerance` by passes
+ * that measure the exact size each field's stream has at a bound (mlp NULL:
+ * plain bisection; else prediction, one re-targeted prediction, then
+ * bisection), then code the fields at the chosen bounds into their buffers.  Outputs per field: bound, achieved ratio, passes. */
 int SZxG_batch_fixed_rate(SZxG_Batch* batch, const SZxG_Mlp* mlp, const float* targetRatio, float tolerance,
                           int maxPasses, float* eb, float* ratio, int* passes, SZxG_StreamInfo* d_info,
                           void* stream);
@@ -291,7 +292,7 @@ int SZxG_batch_fixed_rate(SZxG_Batch* batch, const SZxG_Mlp* mlp, const float* t
  * Returns the number of kernels reported. */
 /* Failure detection (no counterpart in the reference): runs the device-wide
  * look-back the codecs use to place variable-length payloads (scan 0: the
- * encoders' 64-bit status words; scan 1: the words of the decoders' index) over
+ * 64-bit status words; scan 1: the encoders' placement window before them) over
  * ntiles (<= 4096) one-warp tiles, tile t contributing t + 1, with tile
  * `withheld` (-1: none) never publishing, and waits bounded by spinLimit
  * polls.  Returns SZXG_ERR_LOOKBACK when a wait gave up, else SZXG_OK with

@@ -85,11 +85,7 @@ Workspace ws_carve(void* base, int layout, int dtype, size_t n, int bs) {
     w.counters = (unsigned long long*)(h + 512);
     w.st32 = (uint32_t*)(b + L.st32);
     w.st_word = (unsigned long long*)(b + L.st);
-    w.st_agg2 = w.st_word + L.status_tiles;
-    w.st_inc2 = w.st_agg2 + L.status_tiles;
     w.st2_word = (unsigned long long*)(b + L.st2);
-    w.st2_agg2 = w.st2_word + L.status2_tiles;
-    w.st2_inc2 = w.st2_agg2 + L.status2_tiles;
     w.partials = b + L.partials;
     w.o_scr = (uint16_t*)(b + L.o);
     w.m_scr = (uint32_t*)(b + L.m);

@@ -14,8 +14,7 @@
 // Fields are grouped by size class, and neighbouring classes of one launch
 // shape share a launch (a table of value-count bounds, each with
 // its launch shape: encoder tile size and CTAs per SM of the encoder and the
-// decoder), and each class is one persistent launch per kernel with its own
-// shape.  The table comes from the tuning file written by the project's
+// decoder): one persistent launch per kernel and shape.  The table comes from the tuning file written by the project's
 // autotuner (szx_gb300/tune.py: tuning/batch_shapes.txt next to the
 // library, or the file SZXG_TUNING_FILE names), or from
 // SZxG_set_launch_shapes; with neither, one class with the default shape.
@@ -23,7 +22,7 @@
 //
 // This file plans a batch (layout of the per-field scratch in one
 // allocation, the field table and tile map on the device) and runs it as a
-// handful of memsets and launches that a CUDA graph can capture.
+// handful of launches that a CUDA graph can capture.
 #include <dlfcn.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -250,6 +249,7 @@ static SZxG_Batch* create_decode(int fastMode, int dataType, int blockSize, int 
     const size_t o_map = off; off += a256(4 * dec_tiles_all);
     const size_t o_zero = off;
     const size_t o_err = off; off += a256(sizeof(int) * nf);
+    auto words_of = [](size_t tiles) { return (tiles + 7) & ~size_t(3); };   // look-back words: 4 more, in fours
     std::vector<size_t> o_st(nf), o_p(nf), o_rw(nf), ta(nf), tbw(nf);
     for (size_t f = 0; f < nf; f++) {
         const SZxG_Field& F = fields[f];
@@ -258,7 +258,7 @@ static SZxG_Batch* create_decode(int fastMode, int dataType, int blockSize, int 
         const size_t nb = (F.nbEle + blockSize - 1) / blockSize, nw = (nb + 31) / 32;
         ta[f] = (nb + kIdxPerTile - 1) / kIdxPerTile;
         tbw[f] = (nw + kIdxPerTile - 1) / kIdxPerTile;
-        o_st[f] = off; off += a256(3 * 8 * (ta[f] + tbw[f]));
+        o_st[f] = off; off += a256(8 * (words_of(ta[f]) + words_of(tbw[f])));
     }
     const size_t zero_bytes = off - o_zero;
     for (size_t f = 0; f < nf; f++) {
@@ -302,9 +302,8 @@ static SZxG_Batch* create_decode(int fastMode, int dataType, int blockSize, int 
             D.P = (unsigned long long*)(base + o_p[f]);
             D.RW = (uint32_t*)(base + o_rw[f]);
             unsigned long long* st = (unsigned long long*)(base + o_st[f]);
-            for (int q = 0; q < 3; q++) D.stA[q] = st + q * ta[f];
-            st += 3 * ta[f];
-            for (int q = 0; q < 3; q++) D.stB[q] = st + q * tbw[f];
+            D.stA = st;
+            D.stB = st + words_of(ta[f]);
             D.idxA_tiles = ta[f]; D.idxB_tiles = tbw[f];
             D.idx_tile0 = P.idx_total; P.idx_total += ta[f] + tbw[f];
             D.dec_tiles = (D.nb + tb - 1) / tb;

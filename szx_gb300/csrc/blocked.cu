@@ -11,12 +11,14 @@
 //
 // GB300 design
 // * Encode is ONE pass over the input.  Persistent CTAs take tiles of blocks
-//   from an atomic counter and pipeline them over three shared-memory buffers
-//   filled by TMA bulk copies.  A block is handled by a segment of G lanes
-//   (16 float / 8 double values per lane) in a chunk-interleaved layout; the
-//   tile's payload bytes are placed by a decoupled look-back whose 64-bit
-//   status words carry the inclusive prefix inline, and each tile's payloads
-//   are emitted into shared memory and written with aligned 16-byte stores.
+//   from an atomic counter and pipeline them over four shared-memory buffers
+//   filled by cp.async.  A block is handled by a segment of G lanes, each with
+//   a run of consecutive values (16 float / 8 double, 64 bytes, swizzled in
+//   16-byte chunks so that neither the fill nor the runs meet bank conflicts);
+//   a lane's stored bytes are then one run of the payload, written as whole
+//   words.  One warp places a tile from its CTA's previous tile and a window
+//   of byte counts while the others copy the tile before it out in aligned
+//   16-byte stores.
 // * The payload region is written at a fixed position (as if no block were
 //   non-constant); the stream then starts 2*nnc (mode 3/4) or 4*nnc (mode 2)
 //   bytes into the buffer, so that header, size index, state bits and
@@ -24,10 +26,10 @@
 //   exactly where the payload region begins.  Nothing is ever moved.
 // * Decode scans the size index and the state bits once (payload offsets by
 //   non-constant rank, rank at each 32-block state word); then a producer
-//   warp per CTA stages each tile's payload range by TMA into a ring of
-//   buffers while eight consumer warps decode G lanes per block, with the
-//   bytes carried from earlier values resolved by a packed "last writer"
-//   scan over 4-value chunks.
+//   warp per CTA stages each tile's payload range by a bulk copy into a ring
+//   of buffers while eight consumer warps decode G lanes per block, the bytes
+//   inherited from earlier lanes resolved by one "last writer" scan over the
+//   lanes' summaries.
 #include "common.cuh"
 #include "kernels.h"
 #include "segment.cuh"
@@ -35,10 +37,12 @@
 namespace szxg {
 
 // Encoder tiles: ~16 KiB of input per tile, as many warps as the tile has
-// block groups (at least 4), 24 warps per SM.  Measured on 512^3 fp32: 8 KiB
-// tiles in 4-warp CTAs (6 per SM) encode in 0.396 ms against 0.380 ms -- the
-// extra look-backs and tile claims cost more than the extra barrier domains
-// save.
+// block groups (at least 4), 24 warps per SM.  An earlier form of the encoder
+// took 0.396 ms for 512^3 fp32 with 8 KiB tiles in 4-warp CTAs (6 per SM)
+// against 0.380 ms -- the extra look-backs and tile claims cost more than the
+// extra barrier domains save.  Four CTAs of 8 warps with a three-buffer ring
+// (64 registers) took 462 us against 281 us: the loads are issued too late and
+// the double variants spill.
 constexpr int kEncTileBytes = 16384;
 constexpr int kEncWarpsPerSm = 24;
 constexpr int kSizeThreads = 256;
@@ -417,21 +421,25 @@ struct EncTile {
 
 // One pass over the input.  A CTA works through its tiles T_j in a ring of
 // four shared-memory buffers; iteration j, between two CTA barriers:
-//   TMA load of T_{j+1} (into the buffer T_{j-3} left); warp 0 places T_{j-2}
-//   from the look-back window copied in during iteration j-1; statistics of
-//   T_j's blocks (registers)  |  barrier  |  window copy for T_{j-1}; every
-//   warp scans T_j's block sizes for its own blocks' offsets (warp 0
-//   publishes T_j's byte count) and emits them into T_j's buffer in place
-//   (its input is dead); copy-out of T_{j-2} to its place in the payload
-//   region  |  barrier.
+//   barrier (T_j's values are in)  |  cp.async of T_{j+1} into the buffer
+//   T_{j-3} left; statistics of T_j's blocks (registers)  |  barrier  |  the
+//   window copy for T_{j-1}; every warp scans T_j's block sizes for its own
+//   blocks' offsets (warp 0 publishes T_j's byte count) and emits them into
+//   T_j's buffer in place (its input is dead); then warp 0 places T_{j-1}
+//   while the other warps copy T_{j-2} out, one of them T_j's block tables.
 // Every global round trip of a tile -- input load, tile claim, look-back --
-// thus has a whole iteration to complete.  Tile ids come from an atomic
-// counter, taken in increasing order two tiles ahead (the look-back stays
-// deadlock-free with any number of resident CTAs).  The look-back window
-// holds the 512 nearest predecessors, which normally reach back to this
-// CTA's own previous tile (already placed); otherwise it falls back to the
-// global walk.  A segment of G lanes owns one block from its statistics to
-// its emission.
+// thus has most of an iteration to complete, and nothing waits for warp 0.
+// Tile ids come from an atomic counter, taken in increasing order two tiles
+// ahead (the look-back stays deadlock-free with any number of resident CTAs).
+// A segment of G lanes owns one block from its statistics to its emission.
+//
+// Bound by the instructions of the statistics and the emission (issue 65 %):
+// 50 warp instructions per 32 floats, 124 per 32 doubles.  2^27 floats, REL
+// 1e-3, blocks of 128: 281 us (512 MiB in, 129 us with the stream at the copy
+// rate); 2^28 doubles in blocks of 256: 1363 us (490).  Before -- lanes over
+// interleaved 4-value chunks, byte stores, doubles on the FP64 pipe (two lanes
+// a clock and SM here), T_{j-2} placed by warp 0 while the others waited --
+// 363 and 2791 us.
 template <typename T, int G, bool MULTI, int TBYTES = kEncTileBytes>
 __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G, TBYTES>::kMinCtas)
     k_blocked_encode(EncArgs a) {
@@ -766,9 +774,13 @@ cudaError_t launch_blocked_sizes(const SizeItem* d_items, int ni, unsigned long 
 // compacts them: an assemble tile covers kAsmWords state words (32 blocks
 // each), the non-constant rank of its first block comes from an inline-prefix
 // look-back over the tiles' popcounts, and each block then writes its size
-// (non-constant, by rank) or its median (constant, by constant rank).
+// (non-constant, by rank) or its median (constant, by constant rank).  The
+// sizes and medians are loaded before the look-back, not behind it: 2^20
+// blocks 25.3 -> 21 us, those of float64 55 -> 39.  (The index's CTA-wide
+// look-back: 22.4.)
 constexpr int kAsmThreads = 256;
 constexpr int kAsmWords = (int)(kAsmBlocksPerTile / 32);
+constexpr int kAsmItems = (int)kAsmBlocksPerTile / kAsmThreads;   // blocks a thread
 
 struct AsmArgs {
     BlkField one;                // the field when nf == 1
@@ -805,7 +817,7 @@ __device__ __forceinline__ void asm_header(const BlkField* F, int layout, unsign
     *F->res = r;
 }
 
-__global__ void __launch_bounds__(kAsmThreads) k_blocked_assemble(AsmArgs a) {
+__global__ void __launch_bounds__(kAsmThreads, 4) k_blocked_assemble(AsmArgs a) {
     pdl_start();
     __shared__ uint32_t s_word[kAsmWords], s_pre[kAsmWords];
     __shared__ uint32_t s_wsum[kAsmThreads / 32];
@@ -858,7 +870,24 @@ __global__ void __launch_bounds__(kAsmThreads) k_blocked_assemble(AsmArgs a) {
         const uint32_t pc = __popc(word);
         const uint32_t incl = warp_inclusive_sum(pc);
         if (lane == 31) s_wsum[warp] = incl;
+        if (tid < kAsmWords) s_word[tid] = word;
         __syncthreads();
+        // every block's size or median, in flight during the look-back
+        const unsigned long long b0 = (unsigned long long)t * kAsmWords * 32;
+        uint32_t val[kAsmItems];
+#pragma unroll
+        for (int k = 0; k < kAsmItems; k++) {
+            const int lb = k * kAsmThreads + tid;
+            const unsigned long long b = b0 + lb;
+            val[k] = 0;
+            if (b < nb) {
+                if ((s_word[lb >> 5] >> (31 - (lb & 31))) & 1u) {
+                    if (ra) val[k] = F->size_blk[b];
+                } else {
+                    val[k] = F->med_blk[b];
+                }
+            }
+        }
         uint32_t wpre = 0, agg = 0;
 #pragma unroll
         for (int k = 0; k < kAsmThreads / 32; k++) {
@@ -866,10 +895,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_blocked_assemble(AsmArgs a) {
             wpre += k < warp ? v : 0u;
             agg += v;
         }
-        if (tid < kAsmWords) {
-            s_word[tid] = word;
-            s_pre[tid] = wpre + incl - pc;
-        }
+        if (tid < kAsmWords) s_pre[tid] = wpre + incl - pc;
         if (warp == 0) {
             prefix_publish(F->st_asm, t, agg);
             const unsigned long long base = prefix_resolve(F->st_asm, t, agg, a.err);
@@ -877,9 +903,8 @@ __global__ void __launch_bounds__(kAsmThreads) k_blocked_assemble(AsmArgs a) {
         }
         __syncthreads();
         const unsigned long long base = s_base;
-        const unsigned long long b0 = (unsigned long long)t * kAsmWords * 32;
-#pragma unroll 4
-        for (int k = 0; k < kAsmWords * 32 / kAsmThreads; k++) {
+#pragma unroll
+        for (int k = 0; k < kAsmItems; k++) {
             const int lb = k * kAsmThreads + tid;
             const unsigned long long b = b0 + lb;
             if (b >= nb) break;
@@ -888,7 +913,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_blocked_assemble(AsmArgs a) {
             const unsigned long long rank = base + s_pre[lb >> 5] + (bit ? __popc(wd >> (32 - bit)) : 0);
             if ((wd >> (31 - bit)) & 1u) {
                 if (ra) {
-                    const uint16_t v = F->size_blk[b];
+                    const uint16_t v = (uint16_t)val[k];
                     if (o_aligned) {
                         *(uint16_t*)(O + 2 * rank) = v;   // little-endian u16
                     } else {
@@ -897,7 +922,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_blocked_assemble(AsmArgs a) {
                     }
                 }
             } else {
-                const uint32_t v = F->med_blk[b];
+                const uint32_t v = val[k];
                 uint8_t* q = M + 4 * (b - rank);
                 if (a.layout == kRandomAccessNative) {
                     q[0] = (uint8_t)v; q[1] = (uint8_t)(v >> 8); q[2] = (uint8_t)(v >> 16); q[3] = (uint8_t)(v >> 24);
@@ -1244,75 +1269,115 @@ __global__ void k_blocked_parse_fields(const DecField* F, int nf, unsigned long 
 }
 
 // CTA-wide exclusive sum over kIdxThreads threads.
-__device__ __forceinline__ unsigned long long cta_exclusive_sum(unsigned long long v, unsigned long long* total,
-                                                                unsigned long long* smem /*[8]*/) {
+__device__ __forceinline__ uint32_t cta_exclusive_sum(uint32_t v, uint32_t* total, uint32_t* smem /*[8]*/) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned long long incl = warp_inclusive_sum(v);
+    const uint32_t incl = warp_inclusive_sum(v);
     if (lane == 31) smem[warp] = incl;
     __syncthreads();
-    unsigned long long wpre = 0, tot = 0;
+    uint32_t wpre = 0, tot = 0;
 #pragma unroll
     for (int w = 0; w < kIdxThreads / 32; w++) {
-        unsigned long long x = smem[w];
+        const uint32_t x = smem[w];
         if (w < warp) wpre += x;
         tot += x;
     }
-    __syncthreads();
     *total = tot;
     return wpre + incl - v;
+}
+
+// N words at any byte address, from the aligned words that hold them; the
+// caller's bytes end at `end`.  False when the last aligned word passes it.
+template <int N>
+__device__ __forceinline__ bool load_words(const uint8_t* p, const uint8_t* end, uint32_t (&w)[N]) {
+    const uint32_t sh = (uint32_t)((uintptr_t)p & 3);
+    const uint32_t* q = (const uint32_t*)(p - sh);
+    if ((const uint8_t*)(q + N + (sh != 0)) > end) return false;
+    uint32_t a[N + 1];
+#pragma unroll
+    for (int i = 0; i < N; i++) a[i] = __ldg(q + i);
+    a[N] = sh ? __ldg(q + N) : 0u;
+#pragma unroll
+    for (int i = 0; i < N; i++) w[i] = __funnelshift_r(a[i], a[i + 1], 8 * sh);
+    return true;
 }
 
 // Two independent exclusive scans:
 //   family A: payload offsets  P[k] = sum O[0..k)          (k < nnc)
 //   family B: rank words       RW[w] = popcount(state < 32w) (w < ceil(nb/32))
-// One tile (kIdxPerTile items) of either, by the whole CTA.
+// One tile (kIdxPerTile items, kIdxItems consecutive ones a thread) of either,
+// by the whole CTA.  st: the family's status words.
+//
+// Bound by latency: 2^20 blocks are 528 tiles, all resident, 2 + 8 MB of
+// traffic.  With items loaded a byte at a time, results stored 8 bytes at a
+// time and a look-back by one warp, 32 words and two dependent loads a round,
+// it took 21.6 us (between events); words, 32-byte stores and inline prefixes
+// alone 22.7, with the look-back over 1024 words at once 15.7.
 __device__ __forceinline__ void index_tile(const uint8_t* s, const BlockedHdr& h, unsigned long long* P, uint32_t* RW,
-                                           TileStatus st, bool famA, long long lt, unsigned long long len, int* err,
-                                           unsigned long long* sm, unsigned long long* s_base) {
-    static_assert((unsigned long long)kIdxThreads * kIdxItems == kIdxPerTile, "index tile size");
-    const unsigned long long nw = (h.nb + 31) / 32;
+                                           unsigned long long* st, bool famA, long long lt, unsigned long long len,
+                                           int* err, uint32_t* sm, unsigned long long* s_base) {
+    static_assert((unsigned long long)kIdxThreads * kIdxItems == kIdxPerTile && kIdxItems == 8, "index tile size");
+    const unsigned long long nw = (h.nb + 31) / 32, items = famA ? h.nnc : nw;
     const unsigned long long first = (unsigned long long)lt * kIdxPerTile + threadIdx.x * kIdxItems;
-    unsigned long long vals[kIdxItems];
-    unsigned long long mine = 0;
+    const bool all = first + kIdxItems <= items;
+    uint32_t vals[kIdxItems];
+    uint32_t w4[4], w8[8];
+    if (famA && all && load_words<4>(s + h.o_off + 2 * first, s + len, w4)) {
 #pragma unroll
-    for (int i = 0; i < kIdxItems; i++) {
-        unsigned long long k = first + i;
-        unsigned long long v = 0;
-        if (famA) {
-            if (k < h.nnc) v = (unsigned long long)s[h.o_off + 2 * k] | ((unsigned long long)s[h.o_off + 2 * k + 1] << 8);
-        } else if (k < nw) {
-            uint32_t w = 0;
-            for (int j = 0; j < 4; j++) {
-                unsigned long long bi = 4 * k + j;
-                w = (w << 8) | (bi < h.sb ? s[h.s_off + bi] : 0u);
-            }
-            v = __popc(w);
-        }
-        vals[i] = v;
-        mine += v;
-    }
-    unsigned long long tot;
-    unsigned long long ex = cta_exclusive_sum(mine, &tot, sm);
-    if (threadIdx.x < 32) {
-        unsigned long long ba, bb;
-        lookback(st, lt, tot, 0, &ba, &bb, err);
-        if (threadIdx.x == 0) *s_base = ba;
-    }
-    __syncthreads();
-    unsigned long long run = *s_base + ex;
+        for (int i = 0; i < kIdxItems; i++) vals[i] = (w4[i >> 1] >> (16 * (i & 1))) & 0xFFFFu;
+    } else if (!famA && 4 * (first + kIdxItems) <= h.sb && load_words<8>(s + h.s_off + 4 * first, s + len, w8)) {
 #pragma unroll
-    for (int i = 0; i < kIdxItems; i++) {
-        unsigned long long k = first + i;
-        if (famA) {
-            if (k < h.nnc) P[k] = run;
-            if (k == h.nnc - 1) {
-                P[h.nnc] = run + vals[i];
-                if (h.q_off + run + vals[i] > len) atomicExch(err, kErrStream);
+        for (int i = 0; i < kIdxItems; i++) vals[i] = __popc(w8[i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kIdxItems; i++) {
+            const unsigned long long k = first + i;
+            uint32_t v = 0;
+            if (famA) {
+                if (k < h.nnc) v = (uint32_t)s[h.o_off + 2 * k] | ((uint32_t)s[h.o_off + 2 * k + 1] << 8);
+            } else if (k < nw) {
+                for (int j = 0; j < 4; j++) {
+                    const unsigned long long bi = 4 * k + j;
+                    v += bi < h.sb ? __popc((uint32_t)s[h.s_off + bi]) : 0;
+                }
             }
-        } else if (k < nw) {
-            RW[k] = (uint32_t)run;
+            vals[i] = v;
         }
-        run += vals[i];
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (int i = 0; i < kIdxItems; i++) mine += vals[i];
+    uint32_t tot;
+    const uint32_t ex = cta_exclusive_sum(mine, &tot, sm);
+    if (threadIdx.x < 32) prefix_publish(st, lt, tot);
+    const unsigned long long run0 = prefix_resolve_cta<kIdxThreads / 32>(st, lt, tot, err, s_base) + ex;
+    if (famA) {
+        unsigned long long run = run0;
+        double q[kIdxItems];   // (a store's type: the offsets' bits)
+#pragma unroll
+        for (int i = 0; i < kIdxItems; i++) {
+            const unsigned long long k = first + i;
+            q[i] = __longlong_as_double((long long)run);
+            if (!all && k < h.nnc) P[k] = run;
+            run += vals[i];
+            if (k + 1 == h.nnc) {
+                P[h.nnc] = run;
+                if (h.q_off + run > len) atomicExch(err, kErrStream);
+            }
+        }
+        if (all) {
+            st_v8((double*)(P + first), q);
+            st_v8((double*)(P + first) + 4, q + 4);
+        }
+    } else {
+        uint32_t run = (uint32_t)run0;
+        float q[kIdxItems];
+#pragma unroll
+        for (int i = 0; i < kIdxItems; i++) {
+            q[i] = __uint_as_float(run);
+            if (!all && first + i < nw) RW[first + i] = run;
+            run += vals[i];
+        }
+        if (all) st_v8((float*)(RW + first), q);
     }
     __syncthreads();
 }
@@ -1320,13 +1385,13 @@ __device__ __forceinline__ void index_tile(const uint8_t* s, const BlockedHdr& h
 // The scans of one stream in one persistent launch (family A first).
 __global__ void __launch_bounds__(kIdxThreads) k_blocked_index(const uint8_t* s, const BlockedHdr* hp,
                                                                unsigned long long* P, uint32_t* RW,
-                                                               TileStatus stA, TileStatus stB,
+                                                               unsigned long long* stA, unsigned long long* stB,
                                                                unsigned long long* ctr, int* err,
                                                                unsigned long long len, int famA) {
     pdl_start();
-    __shared__ unsigned long long sm[8];
+    __shared__ uint32_t sm[8];
     __shared__ long long s_tile;
-    __shared__ unsigned long long s_base;
+    __shared__ unsigned long long s_base[8];
     const BlockedHdr h = *hp;
     if (!h.ok) return;
     const unsigned long long nw = (h.nb + 31) / 32;
@@ -1338,7 +1403,7 @@ __global__ void __launch_bounds__(kIdxThreads) k_blocked_index(const uint8_t* s,
         long long t = s_tile;
         if (t >= TA + TBt) break;
         const bool fa = t < TA;
-        index_tile(s, h, P, RW, fa ? stA : stB, fa, fa ? t : t - TA, len, err, sm, &s_base);
+        index_tile(s, h, P, RW, fa ? stA : stB, fa, fa ? t : t - TA, len, err, sm, s_base);
     }
 }
 
@@ -1348,10 +1413,10 @@ __global__ void __launch_bounds__(kIdxThreads) k_blocked_index(const uint8_t* s,
 __global__ void __launch_bounds__(kIdxThreads) k_blocked_index_fields(const DecField* F, int nf,
                                                                       unsigned long long total,
                                                                       unsigned long long* ctr) {
-    __shared__ unsigned long long sm[8];
+    __shared__ uint32_t sm[8];
     __shared__ long long s_tile;
     __shared__ int s_f;
-    __shared__ unsigned long long s_base;
+    __shared__ unsigned long long s_base[8];
     for (;;) {
         if (threadIdx.x == 0) {
             const long long g = (long long)atomicAdd(ctr, 1ull);
@@ -1374,8 +1439,7 @@ __global__ void __launch_bounds__(kIdxThreads) k_blocked_index_fields(const DecF
         const long long lt = fa ? local : local - (long long)D.idxA_tiles;
         const long long TA = (long long)((h.nnc + kIdxPerTile - 1) / kIdxPerTile);
         if (h.ok && (!fa || lt < TA)) {
-            const TileStatus st = fa ? TileStatus{D.stA[0], D.stA[1], D.stA[2]} : TileStatus{D.stB[0], D.stB[1], D.stB[2]};
-            index_tile(D.s, h, D.P, D.RW, st, fa, lt, D.len, D.err, sm, &s_base);
+            index_tile(D.s, h, D.P, D.RW, fa ? D.stA : D.stB, fa, lt, D.len, D.err, sm, s_base);
         }
         __syncthreads();
     }
@@ -1468,10 +1532,15 @@ __device__ __forceinline__ void dec_segment(uint32_t p, int len, T* ob, int vec,
 // reads the tile's state bits and first rank, the payload offsets of its
 // non-constant blocks and the medians of its constant blocks, checks them,
 // and stages the tile's payload bytes (one contiguous range) into a ring of
-// kDecStages shared-memory buffers with a TMA bulk copy.  Eight consumer
+// kDecStages shared-memory buffers with a bulk copy.  Eight consumer
 // warps decode a tile per step, G lanes per block, and write the values with
-// 16-byte stores.  Full/empty mbarriers hand the buffers back and forth; every
+// 32-byte stores.  Full/empty mbarriers hand the buffers back and forth; every
 // wait is bounded and reports kErrLookback instead of hanging.
+//
+// Bound by the integer pipe for floats (2^27 values: 179 us, 129 us of
+// traffic; 240 us before the run decoder) and by the FP64 add for doubles
+// (2^28 values: 737 us, 427 us of FP64 pipe and 522 us of traffic; 1117 us
+// before the NaN check left that pipe).
 constexpr int kDecWarps = 8;
 constexpr int kDecThreadsP = (kDecWarps + 1) * 32;
 constexpr int kDecStages = 3;
@@ -1554,7 +1623,7 @@ __global__ void __launch_bounds__(kDecThreadsP, kDecCtasPerSm) k_blocked_decode(
     auto field_of = [&](long long g) { return (int)a.tile_field[g]; };
 
     // The producer's copy of a tile's payload range [sa, sa + nbytes) of the
-    // stream [sbeg, send): one TMA copy of the 16-byte chunks it touches, and
+    // stream [sbeg, send): one bulk copy of the 16-byte chunks it touches, and
     // plain copies of the ends where a chunk would pass the stream's.  Byte x
     // goes to stage + kFront + (x - (sa & ~15)).
     auto copy_range = [&](uint8_t* stage, const uint8_t* src, unsigned long long nbytes, const uint8_t* sbeg,
@@ -1996,8 +2065,7 @@ cudaError_t launch_blocked_decode(int layout, int dtype, const uint8_t* d_stream
         const size_t cap = (size_t)sm_count() * 4;
         TraceScope tr("blocked_index", s);
         if ((e = launch_after(k_blocked_index, (unsigned)(tiles < cap ? tiles : cap), kIdxThreads, 0, s, d_stream, ws.bhdr,
-                              ws.p_off, ws.rank_w, TileStatus{ws.st_word, ws.st_agg2, ws.st_inc2},
-                              TileStatus{ws.st2_word, ws.st2_agg2, ws.st2_inc2}, &ws.counters[0], ws.err,
+                              ws.p_off, ws.rank_w, ws.st_word, ws.st2_word, &ws.counters[0], ws.err,
                               (unsigned long long)len, m2 ? 0 : 1)) != cudaSuccess)
             return e;
     }

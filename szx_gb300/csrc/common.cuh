@@ -235,30 +235,14 @@ __device__ __forceinline__ V warp_sum(V v) {
     return v;
 }
 
-// ------------------------------------------------------------------ acquire/release
-
-__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
 // ------------------------------------------------------------------ decoupled look-back
 //
 // Single-pass exclusive prefix over tiles (Merrill & Garland, "Single-pass
-// Parallel Prefix Scan with Decoupled Look-back", NVR-2016-002).  The status
-// word of a tile packs a 2-bit flag over a 62-bit byte count; a second 64-bit
-// count (e.g. non-constant blocks) travels in side arrays written before the
-// flag is released.  Tiles are taken in order from an atomic counter, so every
-// predecessor is running or done and the look-back always ends; the spin is
-// still capped and reports through *err instead of hanging.
+// Parallel Prefix Scan with Decoupled Look-back", NVR-2016-002).  Tiles are
+// taken in order from an atomic counter, so every predecessor is running or
+// done and the look-back always ends; the spin is still capped and reports
+// through *err instead of hanging.
 
-constexpr unsigned long long kFlagAgg = 1ull << 62;
-constexpr unsigned long long kFlagInc = 2ull << 62;
-constexpr unsigned long long kValMask = (1ull << 62) - 1;
 constexpr unsigned kSpinLimit = 1u << 22;   // polls before giving up (~1 s with backoff)
 // Every look-back below takes its poll limit as a last argument (default
 // kSpinLimit); the failure-detection self-test (selftest.cu) passes a small
@@ -266,18 +250,6 @@ constexpr unsigned kSpinLimit = 1u << 22;   // polls before giving up (~1 s with
 
 enum : int { kErrNone = 0, kErrLookback = 1, kErrCapacity = 2, kErrStream = 3 };
 
-struct TileStatus {
-    unsigned long long* word;     // [ntiles] flag|bytes
-    unsigned long long* agg2;     // [ntiles] second count, aggregate
-    unsigned long long* inc2;     // [ntiles] second count, inclusive
-};
-
-// Combine rules for the second value.
-struct SumOp {
-    static __device__ __forceinline__ unsigned long long id() { return 0; }
-    static __device__ __forceinline__ unsigned long long op(unsigned long long x, unsigned long long y) { return x + y; }
-    static __device__ __forceinline__ unsigned long long warp_reduce(unsigned long long v) { return warp_sum(v); }
-};
 // Three 21-bit fields combined by max each (latest tile index + 1, 0 = none).
 struct Max3x21Op {
     static __device__ __forceinline__ unsigned long long id() { return 0; }
@@ -296,69 +268,6 @@ struct Max3x21Op {
         return v;
     }
 };
-
-// Called by one whole warp.  Publishes the tile's aggregate (a, b), walks back
-// over predecessors and returns the exclusive prefix.  Lane 0 of the warp
-// publishes; all lanes get the result.  `a` is always a sum; `b` combines by Op.
-template <typename Op = SumOp>
-__device__ __forceinline__ void lookback(TileStatus st, long long tile, unsigned long long a,
-                                         unsigned long long b, unsigned long long* ex_a,
-                                         unsigned long long* ex_b, int* err, unsigned limit = kSpinLimit) {
-    const unsigned lane = lane_id();
-    if (tile == 0) {
-        if (lane == 0) {
-            st.inc2[0] = b;
-            __threadfence();
-            st_release(&st.word[0], kFlagInc | (a & kValMask));
-        }
-        *ex_a = 0;
-        *ex_b = Op::id();
-        return;
-    }
-    if (lane == 0) {
-        st.agg2[tile] = b;
-        __threadfence();
-        st_release(&st.word[tile], kFlagAgg | (a & kValMask));
-    }
-    unsigned long long pa = 0, pb = Op::id();
-    long long base = tile - 1;
-    unsigned spins = 0;
-    bool failed = false;
-    while (true) {
-        // lane l inspects predecessor base - l; tiles below 0 read as an
-        // inclusive prefix of zero, so the walk always stops.
-        long long t = base - (long long)lane;
-        unsigned long long w = kFlagInc;
-        if (t >= 0) w = ld_acquire(&st.word[t]);
-        unsigned long long flag = w & ~kValMask;
-        unsigned inc_mask = __ballot_sync(0xffffffffu, flag == kFlagInc);
-        unsigned stop = inc_mask ? (unsigned)__ffs(inc_mask) - 1 : 31u;
-        unsigned window = stop == 31u ? 0xffffffffu : ((1u << (stop + 1)) - 1);
-        unsigned not_ready = __ballot_sync(0xffffffffu, flag == 0) & window;
-        if (not_ready) {
-            if (++spins > limit) { failed = true; break; }
-            __nanosleep(spins < 64 ? 32 : 256);
-            continue;
-        }
-        unsigned long long va = 0, vb = Op::id();
-        if (t >= 0 && lane <= stop) {
-            va = w & kValMask;
-            vb = (flag == kFlagInc) ? __ldcg(&st.inc2[t]) : __ldcg(&st.agg2[t]);
-        }
-        pa += warp_sum(va);
-        pb = Op::op(Op::warp_reduce(vb), pb);
-        if (inc_mask) break;
-        base -= 32;
-    }
-    if (failed && lane == 0) atomicExch(err, kErrLookback);
-    if (lane == 0) {
-        st.inc2[tile] = Op::op(pb, b);
-        __threadfence();
-        st_release(&st.word[tile], kFlagInc | ((pa + a) & kValMask));
-    }
-    *ex_a = pa;
-    *ex_b = pb;
-}
 
 // ------------------------------------------------------------------ TMA bulk copies + mbarriers
 //
@@ -482,6 +391,64 @@ __device__ __forceinline__ unsigned long long prefix_resolve(unsigned long long*
     }
     if (failed && lane == 0) atomicExch(err, kErrLookback);
     if (lane == 0) st_volatile64(&st[tile], kS64Inc | ((pa + agg) & kS64Val));
+    return pa;
+}
+
+// The same by the whole CTA, WARPS windows of 128 predecessors in one memory
+// round trip; every thread gets the prefix.  For grids of fewer than 128 *
+// WARPS CTAs that hold one tile each: the tiles without an inclusive prefix are
+// then fewer than the windows reach (read again until one is seen).  sm: WARPS
+// words; a barrier lies between two calls.
+template <int WARPS>
+__device__ __forceinline__ unsigned long long prefix_resolve_cta(unsigned long long* st, long long tile,
+                                                                 unsigned long long agg, int* err,
+                                                                 unsigned long long* sm) {
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    const long long g0 = (((tile - 1) >> 2) << 2) - 128 * (long long)warp, g = g0 - 4 * (long long)lane;
+    unsigned long long pa = 0;
+    bool done = false;
+    unsigned spins = 0;
+    for (unsigned round = 0; !done && round < kSpinLimit; round++) {   // (the same rounds in every thread)
+        if (round) __syncthreads();   // (the sums of the round before are read)
+        unsigned long long mine = kS64Inc;   // this warp's window: its sum, and kS64Inc where a prefix ends it
+        while (tile > 0 && g0 >= 0) {
+            unsigned long long w[4] = {kS64Inc, kS64Inc, kS64Inc, kS64Inc};
+            if (g >= 0) ld_volatile_v2x2(st + g, w);
+            bool inc = false, ready = true;
+            unsigned long long sa = 0;
+#pragma unroll
+            for (int j = 3; j >= 0; j--) {
+                const unsigned long long f = w[j] & ~kS64Val;
+                if (g + j < tile && !inc) {
+                    sa += w[j] & kS64Val;
+                    inc = f == kS64Inc;
+                    ready = ready && f != 0;
+                }
+            }
+            const unsigned inc_mask = __ballot_sync(0xffffffffu, inc);
+            const unsigned stop = inc_mask ? (unsigned)__ffs(inc_mask) - 1 : 31u;
+            if (!(__ballot_sync(0xffffffffu, !ready) & (0xffffffffu >> (31 - stop)))) {
+                mine = (inc_mask ? kS64Inc : 0ull) | (warp_sum(lane <= stop ? sa : 0ull) & kS64Val);
+                break;
+            }
+            if (++spins > kSpinLimit) {
+                if (lane == 0) atomicExch(err, kErrLookback);
+                break;
+            }
+            __nanosleep(spins < 64 ? 32 : 256);
+        }
+        if (lane == 0) sm[warp] = mine;
+        __syncthreads();
+        pa = 0;
+#pragma unroll
+        for (int k = 0; k < WARPS; k++) {
+            const unsigned long long v = sm[k];
+            if (!done) pa += v & kS64Val;
+            done = done || (v & ~kS64Val) != 0;
+        }
+    }
+    if (!done && threadIdx.x == 0) atomicExch(err, kErrLookback);
+    if (threadIdx.x == 0 && tile > 0) st_volatile64(&st[tile], kS64Inc | ((pa + agg) & kS64Val));
     return pa;
 }
 

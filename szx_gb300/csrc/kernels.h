@@ -88,8 +88,8 @@ struct DecField {
     BlockedHdr* hdr;                             // parsed header
     unsigned long long* P;                       // [nb + 1] payload offsets by non-constant rank
     uint32_t* RW;                                // [nb / 32 + 2] rank at each 32-block state word
-    unsigned long long* stA[3];                  // offset-scan look-back: word, agg2, inc2 [idxA_tiles], zeroed
-    unsigned long long* stB[3];                  // rank-scan look-back [idxB_tiles], zeroed
+    unsigned long long* stA;                     // offset-scan look-back words [idxA_tiles + 4], zeroed, 16-aligned
+    unsigned long long* stB;                     // rank-scan look-back words [idxB_tiles + 4], the same
     unsigned long long idx_tile0, idxA_tiles, idxB_tiles;   // launch-wide first index tile, tiles per scan
     unsigned long long dec_tile0, dec_tiles;     // launch-wide first decode tile, decode tiles
     int* err;                                    // this stream's error word, zeroed
@@ -111,11 +111,7 @@ struct Workspace {
     unsigned long long* counters;   // 4 tile counters
     uint32_t* st32;                 // 32-bit tile status words ([status_tiles + 16])
     unsigned long long* st_word;    // tile status words (family A)
-    unsigned long long* st_agg2;
-    unsigned long long* st_inc2;
     unsigned long long* st2_word;   // tile status (family B)
-    unsigned long long* st2_agg2;
-    unsigned long long* st2_inc2;
     void* partials;                 // range-pass partials
     uint16_t* o_scr;                // payload sizes by non-constant rank
     uint32_t* m_scr;                // median bits by constant rank

@@ -7,11 +7,11 @@
 // 1/64 of a binade) corrected by a small MLP: from 32 features of the sampled
 // blocks the network predicts by how much the whole field's ratio will miss
 // the target at the sampled curve's crossing, log2(real / target), and the
-// bound is the sampled crossing for the target divided by that miss.  A real
-// compress pass (of the whole batch of fields at once) judges the bound, a
+// bound is the sampled crossing for the target divided by that miss.  A pass
+// that measures the exact stream sizes (of all fields at once) judges it, a
 // field that misses by more than the tolerance gets one refined bound (the
 // sampled crossing re-targeted by the miss it measured), and plain bisection
-// over real compress passes is the fallback after that -- and, run alone, the
+// over such passes is the fallback after that -- and, run alone, the
 // baseline.
 //
 // Features of a (field, target) row (float data, blocks of 128 values, every
@@ -1120,9 +1120,9 @@ int SZxG_batch_features(SZxG_Batch* b, int nRows, const int* fieldOfRow, const f
 }
 
 // Pick every field's bound so that its stream reaches targetRatio[f] within
-// `tolerance` (relative), judged by real compress passes of the batch; the
-// streams of the chosen bounds are left in the fields' buffers and their
-// results in d_info (when not NULL).  Bounds are searched as y =
+// `tolerance` (relative), judged by the streams' exact sizes; the streams of
+// the chosen bounds are left in the fields' buffers and their results in
+// d_info (when not NULL).  Bounds are searched as y =
 // log2(bound / sampled range) in [-28, 1].
 //   mlp == NULL: plain bisection.
 //   otherwise: the sampled crossing for the target divided by the network's

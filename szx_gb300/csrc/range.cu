@@ -3,6 +3,8 @@
 // bound conversion of SZx_fast_compress_args (szx/src/szx.cc:249-253,
 // :277-287, :304-308, :332-340), done in one launch: grid-stride partials,
 // then the last CTA to finish reduces them and derives the codec parameters.
+// A field of up to 2 MiB takes one cluster of eight CTAs instead
+// (k_range_small), which also does the call's clears: one launch fewer.
 //
 // The reference's sequential scan (`if (min > v) min = v; else if (max < v)
 // max = v;` starting from x[0]) keeps the FIRST element that reaches the

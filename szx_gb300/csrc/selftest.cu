@@ -23,20 +23,29 @@ namespace szxg {
 namespace {
 
 // scan 0: the 64-bit status words of the encoders' placement (prefix_resolve);
-// scan 1: the words with side arrays (lookback) of the decoders' index.
-__global__ void k_selftest_lookback(int scan, unsigned long long* st64, TileStatus st, int ntiles, int withheld,
+// scan 1: the placement window (PlaceWin) both encoders try first, anchored at
+//         tile 1, and the same words behind it.
+__global__ void k_selftest_lookback(int scan, unsigned long long* st64, uint16_t* counts, int ntiles, int withheld,
                                     unsigned limit, unsigned long long* prefix, int* err) {
     const long long tile = blockIdx.x;
     if (tile >= ntiles || tile == withheld) return;   // the withheld tile never publishes
     const unsigned long long agg = (unsigned long long)tile + 1;
+    if (lane_id() == 0) st_relaxed16(counts + tile, (uint32_t)agg + 1);
+    prefix_publish(st64, tile, agg);
     unsigned long long p = 0;
-    if (scan == 0) {
-        prefix_publish(st64, tile, agg);
-        p = prefix_resolve(st64, tile, agg, err, limit);
-    } else {
-        unsigned long long dummy = 0;
-        lookback(st, tile, agg, 0, &p, &dummy, err, limit);
+    bool placed = false;
+    if (scan == 1) {
+        __shared__ PlaceWin win;
+        if (lane_id() == 0) {
+            win.init();
+            if (tile > 1 && withheld != 1) win.anchor(0, 1, 3);   // tiles 0 and 1: one byte and two
+        }
+        __syncwarp();
+        win.issue(counts, 0, (int)tile);
+        placed = win.offset(counts, (int)tile, &p);
+        if (placed && tile > 0 && lane_id() == 0) st_volatile64(&st64[tile], kS64Inc | ((p + agg) & kS64Val));
     }
+    if (!placed) p = prefix_resolve(st64, tile, agg, err, limit);
     if (lane_id() == 0) prefix[tile] = p;
 }
 
@@ -54,7 +63,7 @@ extern "C" int SZxG_selftest_lookback(int scan, int ntiles, int withheld, unsign
     cudaStream_t s = (cudaStream_t)stream;
     const size_t n = (size_t)ntiles;
     auto a256 = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t ost = a256(8 * (n + 8)), opre = ost + a256(24 * n), oerr = opre + a256(8 * n), bytes = oerr + 256;
+    const size_t ocnt = a256(8 * (n + 8)), opre = ocnt + a256(2 * (n + 16)), oerr = opre + a256(8 * n), bytes = oerr + 256;
     unsigned char* b = nullptr;
     if (cudaMalloc(&b, bytes) != cudaSuccess) {
         cudaGetLastError();
@@ -62,16 +71,13 @@ extern "C" int SZxG_selftest_lookback(int scan, int ntiles, int withheld, unsign
         return SZXG_ERR_CUDA;
     }
     unsigned long long* st64 = (unsigned long long*)b;          // [n + 8]
-    TileStatus st;
-    st.word = (unsigned long long*)(b + ost);                   // [n] each
-    st.agg2 = st.word + n;
-    st.inc2 = st.agg2 + n;
+    uint16_t* counts = (uint16_t*)(b + ocnt);                    // [n + 16]
     unsigned long long* d_prefix = (unsigned long long*)(b + opre);
     int* d_err = (int*)(b + oerr);
     int rc = SZXG_OK;
     cudaError_t e = cudaMemsetAsync(b, 0, bytes, s);
     if (e == cudaSuccess) {
-        k_selftest_lookback<<<ntiles, kWarp, 0, s>>>(scan, st64, st, ntiles, withheld, spinLimit, d_prefix, d_err);
+        k_selftest_lookback<<<ntiles, kWarp, 0, s>>>(scan, st64, counts, ntiles, withheld, spinLimit, d_prefix, d_err);
         e = cudaGetLastError();
     }
     int h_err = 0;

@@ -12,7 +12,7 @@
 
 The reference's fixed-rate mode searches an analytic model of every 10th
 block (szx/src/szx_float.cc:684-832, 921-949); here the decision is judged by
-compressing the field for real.
+the exact size of the field's stream.
 """
 from __future__ import annotations
 

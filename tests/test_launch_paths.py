@@ -80,3 +80,30 @@ def test_captured_in_a_graph(szx, mode, n):
         assert codec.stream_bytes().cpu().numpy().tobytes() == O.fast_compress_args(mode, v, 1, 0.0, 1e-3, 128)
         z = O.decompress(mode, np.float32, s.cpu().numpy().tobytes(), n)
         assert dec.status() == 0 and np.array_equal(y.cpu().numpy().view(np.uint8), z.view(np.uint8))
+
+
+@pytest.mark.parametrize("mode", [2, 3, 4])
+@pytest.mark.parametrize("nb", [16385, 9 * 2048, 9 * 2048 + 1, 65536 + 7])
+def test_index_at_every_byte_alignment(szx, mode, nb):
+    """The persistent index over streams at any address: whole, partial and
+    missing last tiles of either scan, no coded block, none but coded ones, and
+    a coded few whose index ends right before the payloads."""
+    import torch
+    bs, n = 4, 4 * nb - 1
+    rng = np.random.default_rng(nb)
+    noise = rng.normal(size=n).astype(np.float32)
+    some = np.where(np.repeat(rng.random(nb) < 0.3, bs)[:n], noise, np.float32(2.5))
+    few = np.full(n, 1.5, np.float32)
+    few[n - 9:] = noise[:9]
+    for x in (noise, some, few, np.zeros(n, np.float32)):
+        want = O.compress(mode, x, 1e-3, bs)
+        z = O.decompress(mode, np.float32, want, n)
+        for off in range(4):
+            buf = torch.empty(off + len(want), dtype=torch.uint8, device="cuda")
+            s = buf[off:]
+            s.copy_(torch.frombuffer(bytearray(want), dtype=torch.uint8))
+            codec = szx.DeviceCodec(mode, np.float32, n, bs)
+            codec.ws.random_(0, 256)
+            y = codec.decompress(s, n)
+            assert codec.status() == 0
+            assert np.array_equal(y.cpu().numpy().view(np.uint8), z.view(np.uint8)), off
