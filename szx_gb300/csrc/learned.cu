@@ -152,35 +152,42 @@ __device__ __forceinline__ float probe_bound(float range, int m) {
     return __fmul_rn(__fmul_rn(range, c_frac64[fr]), pow2_int((m - fr) / 64));
 }
 
-// last index i in [0, n) with key[i] <= g (key ascending, key[0] <= g)
-template <typename K>
-__device__ __forceinline__ int upper_index(const K* key, size_t stride_bytes, int n, unsigned long long g) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        const unsigned long long k = *(const unsigned long long*)((const uint8_t*)key + (size_t)mid * stride_bytes);
-        if (k <= g) lo = mid;
-        else hi = mid - 1;
+// Whole warp, 32 keys a step: the last index i in [0, n) with key[i] <= g (key
+// ascending, key[0] <= g).
+__device__ __forceinline__ int upper_index_warp(const unsigned long long* key, size_t stride_bytes, int n,
+                                                unsigned long long g) {
+    int lo = 0;
+    while (n > 1) {
+        const int step = (n + 31) / 32, at = (int)(threadIdx.x & 31) * step;
+        const bool le = at < n &&
+                        *(const unsigned long long*)((const uint8_t*)key + (size_t)(lo + at) * stride_bytes) <= g;
+        const int c = __popc(__ballot_sync(0xffffffffu, le)) - 1;   // (key[lo] <= g)
+        lo += c * step;
+        n = min(step, n - c * step);
     }
     return lo;
 }
 
-// Sampled min / max of every field (one warp per tile of sampled blocks).
+// Sampled min / max of every field (one warp per tile of sampled blocks, whose
+// loads are all in flight together).
 template <int BS>
 __global__ void k_lfx_range(const LfxField* F, int nf, unsigned long long tiles, uint32_t* mm) {
     const int lane = threadIdx.x & 31;
     const unsigned long long w0 = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
     const unsigned long long nw = (gridDim.x * (unsigned long long)blockDim.x) >> 5;
     for (unsigned long long g = w0; g < tiles; g += nw) {
-        const int f = upper_index(&F[0].tile0, sizeof(LfxField), nf, g);
+        const int f = upper_index_warp(&F[0].tile0, sizeof(LfxField), nf, g);
         const LfxField D = F[f];
         const unsigned long long k0 = (g - D.tile0) * kTileBlocks;
         const unsigned long long k1 = min(k0 + kTileBlocks, D.ns);
         uint32_t lo = 0xFFFFFFFFu, hi = 0u;
-        for (unsigned long long k = k0; k < k1; k++) {
-            const float* p = D.x + k * kRate * BS;
-            for (int i = lane; i < BS; i += 32) {
-                const float v = p[i];
+#pragma unroll
+        for (int q = 0; q < kTileBlocks; q++) {
+            if (k0 + q >= k1) break;
+            const float* p = D.x + (k0 + q) * kRate * BS;
+#pragma unroll
+            for (int i = 0; i < BS / 32; i++) {
+                const float v = p[lane + 32 * i];
                 if (v == v) {
                     lo = min(lo, ord_f32(v));
                     hi = max(hi, ord_f32(v));
@@ -202,10 +209,8 @@ __device__ __forceinline__ float lfx_range_of(const uint32_t* mm, int f) {
     return __fsub_rn(f32_ord(hi), f32_ord(lo));
 }
 
-// Values 4*lane .. 4*lane+3 of sampled block k (128 values) and the block's
-// radius and median as the codec computes them.
-__device__ __forceinline__ void lfx_block(const float* x, unsigned long long k, int lane, float v[4], float* r,
-                                          float* med, int off = 0) {
+// Values 4*lane .. 4*lane+3 of sampled block k (128 values).
+__device__ __forceinline__ void lfx_load(const float* x, unsigned long long k, int lane, float v[4], int off = 0) {
     const float* p = x + (k * kRate + off) * 128 + 4 * lane;
     if (((uintptr_t)x & 15) == 0) {
         const float4 q = *(const float4*)p;
@@ -214,6 +219,10 @@ __device__ __forceinline__ void lfx_block(const float* x, unsigned long long k, 
 #pragma unroll
         for (int i = 0; i < 4; i++) v[i] = p[i];
     }
+}
+
+// The block's radius and median as the codec computes them.
+__device__ __forceinline__ void lfx_stats(const float v[4], float* r, float* med) {
     float mn = fminf(fminf(v[0], v[1]), fminf(v[2], v[3]));
     float mx = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
 #pragma unroll
@@ -252,34 +261,25 @@ __device__ __forceinline__ uint32_t lfx_bytes_nc(const float v[4], float med, in
     return st + (lane == 0 ? 5u + 128 / 4 : 0u);
 }
 
-// Add the block's bytes at every bound eb[0..N) to bytes[]: a
-// constant block costs its 4-byte median; a non-constant block's count
-// depends on the bound only through its reqLength, which changes only where
-// the bound crosses a power of two, so it is computed once per distinct key.
-// r is the same in every lane: all lanes take the same branches.
-template <int N>
-__device__ __forceinline__ void lfx_block_bytes(const float v[4], float r, float med, const float* eb,
-                                                uint32_t* bytes, int lane) {
-    int last = -1;
-    uint32_t cached = 0;
-#pragma unroll
-    for (int j = 0; j < N; j++) {
-        if (r <= eb[j]) {
-            bytes[j] += lane == 0 ? 4u : 0u;
-        } else {
-            const int key = lfx_req_key(eb[j], r);
-            if (key != last) {
-                cached = lfx_bytes_nc(v, med, key, lane);
-                last = key;
-            }
-            bytes[j] += cached;
-        }
+// Add the block's bytes at the bound of this lane to *bytes (lanes without a
+// bound: eb infinite).  A constant block costs its 4-byte median; a
+// non-constant block's count depends on the bound only through its reqLength,
+// which changes only where the bound crosses a power of two, so the warp
+// counts it once per distinct key.  (Every lane going through all 16 bounds:
+// ~500 instructions a block, and 16 sums to reduce per tile.)
+__device__ __forceinline__ void lfx_block_bytes(const float v[4], float r, float med, float eb, uint32_t* bytes,
+                                                int lane) {
+    const bool coded = !(r <= eb);
+    const int key = lfx_req_key(eb, r);
+    if (!coded) *bytes += 4u;
+    unsigned left = __ballot_sync(0xffffffffu, coded);
+    while (left) {
+        const int k = __shfl_sync(0xffffffffu, key, __ffs(left) - 1);
+        const uint32_t n = __reduce_add_sync(0xffffffffu, lfx_bytes_nc(v, med, k, lane));
+        const bool hit = coded && key == k;
+        if (hit) *bytes += n;
+        left &= ~__ballot_sync(0xffffffffu, hit);
     }
-}
-
-__device__ __forceinline__ void lfx_flush(unsigned long long* dst, uint32_t v, int lane) {
-    v = __reduce_add_sync(0xffffffffu, v);
-    if (lane == 0 && v) atomicAdd(dst, (unsigned long long)v);
 }
 
 // Per-field sums (slots A_*) over every kCoarseStep-th sampled block: their
@@ -292,31 +292,33 @@ __global__ void __launch_bounds__(256) k_lfx_accumulate(const LfxField* F, int n
     const unsigned long long w0 = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
     const unsigned long long nw = (gridDim.x * (unsigned long long)blockDim.x) >> 5;
     for (unsigned long long g = w0; g < tiles; g += nw) {
-        const int f = upper_index(&F[0].tile0, sizeof(LfxField), nf, g);
+        const int f = upper_index_warp(&F[0].tile0, sizeof(LfxField), nf, g);
         const LfxField D = F[f];
         const float range = lfx_range_of(mm, f);
-        float eb[kProbes];
-#pragma unroll
-        for (int j = 0; j < kProbes; j++) eb[j] = __fmul_rn(range, c_probe[j]);
-        uint32_t bytes[kProbes], zero = 0, nsb = 0;
-#pragma unroll
-        for (int j = 0; j < kProbes; j++) bytes[j] = 0;
+        const float eb = lane < kProbes ? __fmul_rn(range, c_probe[lane]) : __int_as_float(0x7f800000);
         const unsigned long long k0 = (g - D.tile0) * kTileBlocks;
         const unsigned long long k1 = min(k0 + kTileBlocks, D.ns);
-        for (unsigned long long k = k0; k < k1; k += kCoarseStep) {
-            float v[4], r, med;
-            lfx_block(D.x, k, lane, v, &r, &med);
-            if (lane == 0) {
-                nsb++;
-                zero += r == 0.f;
-            }
-            lfx_block_bytes<kProbes>(v, r, med, eb, bytes, lane);
+        constexpr int NB = kTileBlocks / kCoarseStep;
+        float v[NB][4];
+#pragma unroll
+        for (int q = 0; q < NB; q++)
+            if (k0 + kCoarseStep * q < k1) lfx_load(D.x, k0 + kCoarseStep * q, lane, v[q]);
+        uint32_t bytes = 0, zero = 0, nsb = 0;
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            if (k0 + kCoarseStep * q >= k1) break;
+            float r, med;
+            lfx_stats(v[q], &r, &med);
+            nsb++;
+            zero += r == 0.f;
+            lfx_block_bytes(v[q], r, med, eb, &bytes, lane);
         }
         unsigned long long* a = acc + (size_t)f * kAcc;
-        lfx_flush(a + A_NS, nsb, lane);
-#pragma unroll
-        for (int j = 0; j < kProbes; j++) lfx_flush(a + A_BYTES + j, bytes[j], lane);
-        lfx_flush(a + A_ZERO, zero, lane);
+        if (lane < kProbes) atomicAdd(a + A_BYTES + lane, (unsigned long long)bytes);
+        if (lane == 0) {
+            atomicAdd(a + A_NS, (unsigned long long)nsb);
+            if (zero) atomicAdd(a + A_ZERO, (unsigned long long)zero);
+        }
     }
 }
 
@@ -382,6 +384,12 @@ __global__ void k_lfx_center2(const LfxField* F, const unsigned long long* racc,
 
 // Per-row byte sums at 16 probes m = mstart[r] + stride * k into racc[r][slot..]:
 // items (row, tile of the row's field).
+//
+// Bound by the instructions a sampled block takes and by latency at both ends
+// of a tile (39 K sampled blocks of 24 fields of 2^18..2^23 values are 8 warps
+// a scheduler).  A lane to a bound, one count per distinct key, a tile's loads
+// together, the field found 32 keys a step: 34 -> 18 us a launch; the range
+// pass 31 -> 21, the coarse sums 37 -> 26.
 __global__ void __launch_bounds__(256) k_lfx_probe(const LfxField* F, const uint32_t* mm, int nrows, const int* rows,
                                                    const int* mstart, int stride, const unsigned long long* rtile0,
                                                    unsigned long long items, unsigned long long* racc, int slot,
@@ -390,28 +398,29 @@ __global__ void __launch_bounds__(256) k_lfx_probe(const LfxField* F, const uint
     const unsigned long long w0 = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
     const unsigned long long nw = (gridDim.x * (unsigned long long)blockDim.x) >> 5;
     for (unsigned long long g = w0; g < items; g += nw) {
-        const int r = upper_index(rtile0, sizeof(unsigned long long), nrows, g);
+        const int r = upper_index_warp(rtile0, sizeof(unsigned long long), nrows, g);
         const int f = rows[r];
         const LfxField D = F[f];
         const float range = lfx_range_of(mm, f);
         const int m0 = mstart[r];
-        float eb[kFine];
-#pragma unroll
-        for (int k = 0; k < kFine; k++) eb[k] = probe_bound(range, m0 + stride * k);
-        uint32_t bytes[kFine];
-#pragma unroll
-        for (int k = 0; k < kFine; k++) bytes[k] = 0;
+        const float eb = lane < kFine ? probe_bound(range, m0 + stride * lane) : __int_as_float(0x7f800000);
         // the second sample's blocks are tiled like the first's (ns2 <= ns)
         const unsigned long long k0 = (g - rtile0[r]) * kTileBlocks;
         const unsigned long long k1 = min(k0 + kTileBlocks, off ? D.ns2 : D.ns);
-        for (unsigned long long k = k0; k < k1; k++) {
-            float v[4], rr, med;
-            lfx_block(D.x, k, lane, v, &rr, &med, off);
-            lfx_block_bytes<kFine>(v, rr, med, eb, bytes, lane);
-        }
-        unsigned long long* a = racc + (size_t)r * kRowAcc + slot;
+        // the tile's loads are all in flight together
+        float v[kTileBlocks][4];
 #pragma unroll
-        for (int j = 0; j < kFine; j++) lfx_flush(a + j, bytes[j], lane);
+        for (int q = 0; q < kTileBlocks; q++)
+            if (k0 + q < k1) lfx_load(D.x, k0 + q, lane, v[q], off);
+        uint32_t bytes = 0;
+#pragma unroll
+        for (int q = 0; q < kTileBlocks; q++) {
+            if (k0 + q >= k1) break;
+            float rr, med;
+            lfx_stats(v[q], &rr, &med);
+            lfx_block_bytes(v[q], rr, med, eb, &bytes, lane);
+        }
+        if (lane < kFine && bytes) atomicAdd(racc + (size_t)r * kRowAcc + slot + lane, (unsigned long long)bytes);
     }
 }
 

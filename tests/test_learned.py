@@ -106,6 +106,32 @@ def test_features_match_oracle(L):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nf", [1, 33, 1100])
+def test_features_of_many_small_fields(L, nf):
+    """Sampled blocks from none to a few tiles and a part of one per field, and
+    field tables of one, two and three levels of the search for a tile's field."""
+    import torch
+    rng = np.random.default_rng(nf)
+    xs = []
+    for f in range(nf):
+        n = int(rng.integers(1, 21)) * 1280 - int(rng.integers(0, 1290))
+        x = rng.normal(size=max(n, 1)) * 10.0 ** rng.integers(-3, 3)
+        xs.append((np.round(x, 1) if f % 3 else np.cumsum(x)).astype(np.float32))
+    b = L.Batch([torch.tensor(x, device="cuda") for x in xs])
+    rows = np.arange(nf)[::-1].copy()
+    tg = np.exp2(rng.uniform(1, 6, nf)).astype(np.float32)
+    X, rg = b.features(rows, tg)
+    X = X.cpu().numpy().astype(np.float64)
+    for r, (f, t) in enumerate(zip(rows, tg)):
+        want_rng, acc = OL.sums(xs[f])
+        assert rg[f] == want_rng, f
+        mq = OL.center(acc, t)
+        mu = int(round(X[r, 4] * 64))
+        np.testing.assert_allclose(X[r], OL.features(xs[f], t, mq, mu), rtol=1e-5, atol=2e-6, err_msg=f"field {f}")
+    b.close()
+
+
+@pytest.mark.gpu
 def test_network_forward_and_gradient_match_oracle(L):
     import torch
     rng = np.random.default_rng(4)
