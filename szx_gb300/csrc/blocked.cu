@@ -436,7 +436,7 @@ struct EncTile {
 // Bound by the instructions of the statistics and the emission (issue 65 %):
 // 50 warp instructions per 32 floats, 124 per 32 doubles.  2^27 floats, REL
 // 1e-3, blocks of 128: 281 us (512 MiB in, 129 us with the stream at the copy
-// rate); 2^28 doubles in blocks of 256: 1363 us (490).  Before -- lanes over
+// rate); 2^28 doubles in blocks of 64: 1355 us (490).  Before -- lanes over
 // interleaved 4-value chunks, byte stores, doubles on the FP64 pipe (two lanes
 // a clock and SM here), T_{j-2} placed by warp 0 while the others waited --
 // 363 and 2791 us.
@@ -776,7 +776,7 @@ cudaError_t launch_blocked_sizes(const SizeItem* d_items, int ni, unsigned long 
 // look-back over the tiles' popcounts, and each block then writes its size
 // (non-constant, by rank) or its median (constant, by constant rank).  The
 // sizes and medians are loaded before the look-back, not behind it: 2^20
-// blocks 25.3 -> 21 us, those of float64 55 -> 39.  (The index's CTA-wide
+// blocks 25.5 -> 20.5 us, 2^22 blocks 55 -> 38.  (The index's CTA-wide
 // look-back: 22.4.)
 constexpr int kAsmThreads = 256;
 constexpr int kAsmWords = (int)(kAsmBlocksPerTile / 32);
@@ -1349,6 +1349,8 @@ __device__ __forceinline__ void index_tile(const uint8_t* s, const BlockedHdr& h
     uint32_t tot;
     const uint32_t ex = cta_exclusive_sum(mine, &tot, sm);
     if (threadIdx.x < 32) prefix_publish(st, lt, tot);
+    // (a workspace need not be aligned to a sector)
+    const bool wide = all && ((uintptr_t)(famA ? (const void*)P : (const void*)RW) & 31) == 0;
     const unsigned long long run0 = prefix_resolve_cta<kIdxThreads / 32>(st, lt, tot, err, s_base) + ex;
     if (famA) {
         unsigned long long run = run0;
@@ -1357,14 +1359,14 @@ __device__ __forceinline__ void index_tile(const uint8_t* s, const BlockedHdr& h
         for (int i = 0; i < kIdxItems; i++) {
             const unsigned long long k = first + i;
             q[i] = __longlong_as_double((long long)run);
-            if (!all && k < h.nnc) P[k] = run;
+            if (!wide && k < h.nnc) P[k] = run;
             run += vals[i];
             if (k + 1 == h.nnc) {
                 P[h.nnc] = run;
                 if (h.q_off + run > len) atomicExch(err, kErrStream);
             }
         }
-        if (all) {
+        if (wide) {
             st_v8((double*)(P + first), q);
             st_v8((double*)(P + first) + 4, q + 4);
         }
@@ -1374,10 +1376,10 @@ __device__ __forceinline__ void index_tile(const uint8_t* s, const BlockedHdr& h
 #pragma unroll
         for (int i = 0; i < kIdxItems; i++) {
             q[i] = __uint_as_float(run);
-            if (!all && first + i < nw) RW[first + i] = run;
+            if (!wide && first + i < nw) RW[first + i] = run;
             run += vals[i];
         }
-        if (all) st_v8((float*)(RW + first), q);
+        if (wide) st_v8((float*)(RW + first), q);
     }
     __syncthreads();
 }

@@ -337,6 +337,11 @@ constexpr unsigned long long kS64Agg = 1ull << 62, kS64Inc = 2ull << 62, kS64Val
 __device__ __forceinline__ void st_volatile64(unsigned long long* p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+__device__ __forceinline__ unsigned long long ld_volatile64(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void ld_volatile_v2x2(const unsigned long long* p, unsigned long long (&w)[4]) {
     unsigned long long a, b, c, d;
     asm volatile("ld.relaxed.gpu.global.v2.u64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
@@ -398,7 +403,8 @@ __device__ __forceinline__ unsigned long long prefix_resolve(unsigned long long*
 // round trip; every thread gets the prefix.  For grids of fewer than 128 *
 // WARPS CTAs that hold one tile each: the tiles without an inclusive prefix are
 // then fewer than the windows reach (read again until one is seen).  sm: WARPS
-// words; a barrier lies between two calls.
+// words; a barrier lies between two calls.  st needs the alignment of its words
+// only: a decoder's workspace may lie at any multiple of 8.
 template <int WARPS>
 __device__ __forceinline__ unsigned long long prefix_resolve_cta(unsigned long long* st, long long tile,
                                                                  unsigned long long agg, int* err,
@@ -413,7 +419,14 @@ __device__ __forceinline__ unsigned long long prefix_resolve_cta(unsigned long l
         unsigned long long mine = kS64Inc;   // this warp's window: its sum, and kS64Inc where a prefix ends it
         while (tile > 0 && g0 >= 0) {
             unsigned long long w[4] = {kS64Inc, kS64Inc, kS64Inc, kS64Inc};
-            if (g >= 0) ld_volatile_v2x2(st + g, w);
+            if (g >= 0) {
+                if (((uintptr_t)st & 15) == 0) {
+                    ld_volatile_v2x2(st + g, w);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) w[j] = ld_volatile64(st + g + j);
+                }
+            }
             bool inc = false, ready = true;
             unsigned long long sa = 0;
 #pragma unroll

@@ -107,3 +107,21 @@ def test_index_at_every_byte_alignment(szx, mode, nb):
             y = codec.decompress(s, n)
             assert codec.status() == 0
             assert np.array_equal(y.cpu().numpy().view(np.uint8), z.view(np.uint8)), off
+
+
+@pytest.mark.parametrize("mode", [1, 2, 3, 4])
+@pytest.mark.parametrize("skew", [8, 16])
+def test_decode_workspace_at_any_word(szx, mode, skew):
+    """A decompress workspace needs the alignment of its words, no more."""
+    import torch
+    for n in (300_000, 40_000 * 16 + 3):
+        x = field(np.float32, n, 5)
+        want = O.compress(mode, x, 1e-3, 16)
+        codec = szx.DeviceCodec(mode, np.float32, n, 16)
+        ws = torch.empty(codec.wsb + 64, dtype=torch.uint8, device="cuda").random_(0, 256)
+        codec.ws = ws[skew:skew + codec.wsb]
+        s = torch.frombuffer(bytearray(want), dtype=torch.uint8).cuda()
+        y = codec.decompress(s, n)
+        assert codec.status() == 0
+        z = O.decompress(mode, np.float32, want, n)
+        assert np.array_equal(y.cpu().numpy().view(np.uint8), z.view(np.uint8)), n
