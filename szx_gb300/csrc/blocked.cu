@@ -1285,22 +1285,6 @@ __device__ __forceinline__ uint32_t cta_exclusive_sum(uint32_t v, uint32_t* tota
     return wpre + incl - v;
 }
 
-// N words at any byte address, from the aligned words that hold them; the
-// caller's bytes end at `end`.  False when the last aligned word passes it.
-template <int N>
-__device__ __forceinline__ bool load_words(const uint8_t* p, const uint8_t* end, uint32_t (&w)[N]) {
-    const uint32_t sh = (uint32_t)((uintptr_t)p & 3);
-    const uint32_t* q = (const uint32_t*)(p - sh);
-    if ((const uint8_t*)(q + N + (sh != 0)) > end) return false;
-    uint32_t a[N + 1];
-#pragma unroll
-    for (int i = 0; i < N; i++) a[i] = __ldg(q + i);
-    a[N] = sh ? __ldg(q + N) : 0u;
-#pragma unroll
-    for (int i = 0; i < N; i++) w[i] = __funnelshift_r(a[i], a[i + 1], 8 * sh);
-    return true;
-}
-
 // Two independent exclusive scans:
 //   family A: payload offsets  P[k] = sum O[0..k)          (k < nnc)
 //   family B: rank words       RW[w] = popcount(state < 32w) (w < ceil(nb/32))

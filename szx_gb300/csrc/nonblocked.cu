@@ -404,22 +404,36 @@ __device__ __forceinline__ uint32_t lead_word(const uint8_t* lead, unsigned long
     return w;
 }
 
-// Lead word of values [first, first + 16): one 4-byte load when aligned.
-__device__ __forceinline__ uint32_t lead_word16(const uint8_t* lead, unsigned long long first,
-                                                unsigned long long L) {
+// Lead word of values [first, first + 16), as the two aligned words that hold
+// it: joined by lead_join() where it is used, so that a word loaded ahead is
+// not waited for.  (The codes start 17 bytes into the stream: at no word
+// boundary where the stream itself starts at one.)
+__device__ __forceinline__ void lead_load(const uint8_t* lead, unsigned long long first, unsigned long long L,
+                                          uint32_t& a, uint32_t& b) {
     const unsigned long long lb = first >> 2;
-    if (lb + 4 <= L && ((uintptr_t)(lead + lb) & 3) == 0) return __ldg((const uint32_t*)(lead + lb));
-    return lead_word(lead, lb, L);
+    const uint32_t sh = (uint32_t)((uintptr_t)(lead + lb) & 3);
+    if (lb + 8 <= L) {
+        const uint32_t* q = (const uint32_t*)(lead + lb - sh);
+        a = __ldg(q);
+        b = __ldg(q + 1);
+    } else {
+        const uint32_t w = lead_word(lead, lb, L);
+        a = w << (8 * sh);
+        b = __funnelshift_l(w, 0u, 8 * sh);
+    }
+}
+__device__ __forceinline__ uint32_t lead_join(const uint8_t* lead, uint32_t a, uint32_t b) {
+    return __funnelshift_r(a, b, 8 * (uint32_t)((uintptr_t)lead & 3));   // (words lie whole words into the codes)
 }
 
 // Per tile (one warp): its mid-byte count (tcnt[t]) and, for each of the top
 // three byte lanes, where in the tile's mid bytes the last value storing that
 // lane put it (aux[3t+2], 3x21 bits, position+1, 0 = none).  A lane takes 8
-// consecutive 16-code words (two 16-byte loads), so the tile takes one warp
-// scan; each word costs its three masks, their population counts (a value
+// consecutive 16-code words, so the tile takes one warp scan; each word costs its three masks, their population counts (a value
 // stores max(R - lead, 0) bytes = the number of k < R with lead <= k) and the
 // last word of each mask that is not empty.  (One word per lane and eight
-// scans a tile: 59 us at 2^27 values.)
+// scans a tile: 59 us at 2^27 values; codes that start at no word boundary, the
+// usual case, were read a byte at a time: 46 us, 33 as words.)
 // The CTA's eight tiles form a group: aux[3t] / aux[3t+1] get the tile's
 // exclusive prefix within its group (bytes; latest writer tiles, 3x21 bits,
 // tile+1), gsum[g] / gwr[g] the group's totals.  Independent per group: no
@@ -458,9 +472,9 @@ __global__ void __launch_bounds__(kNbThreads) k_nb_count(const uint8_t* __restri
             const uint4 a = __ldg((const uint4*)lp), b = __ldg((const uint4*)lp + 1);
             cw[0] = a.x; cw[1] = a.y; cw[2] = a.z; cw[3] = a.w;
             cw[4] = b.x; cw[5] = b.y; cw[6] = b.z; cw[7] = b.w;
-        } else {
+        } else if (first + kWords * kNbPer > h.n || !load_words<kWords>(lp, s + len, cw)) {
 #pragma unroll
-            for (int j = 0; j < kWords; j++) cw[j] = lead_word16(lead, first + kNbPer * j, h.L);
+            for (int j = 0; j < kWords; j++) cw[j] = lead_word(lead, (first >> 2) + 4 * j, h.L);
         }
         uint32_t mine = 0, lastw[3] = {0, 0, 0}, lastc[3] = {0, 0, 0};   // per byte lane: its last word and the bytes before it
         int lastn[3] = {0, 0, 0};
@@ -690,9 +704,9 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2)
     };
     // a tile's words: lead codes (per thread), group prefix + offset in the
     // group, carried bytes, byte count
-    auto words = [&](long long t, uint32_t& cd, unsigned long long& ga, unsigned long long& la, uint32_t& cy,
-                     uint32_t& tot) {
-        cd = lead_word16(lead, (unsigned long long)t * kNbTile + threadIdx.x * kNbPer, h.L);
+    auto words = [&](long long t, uint32_t& ca, uint32_t& cb, unsigned long long& ga, unsigned long long& la,
+                     uint32_t& cy, uint32_t& tot) {
+        lead_load(lead, (unsigned long long)t * kNbTile + threadIdx.x * kNbPer, h.L, ca, cb);
         ga = gsum[t / kTpg];
         la = aux[3 * t];
         cy = (uint32_t)aux[3 * t + 1];
@@ -701,15 +715,20 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2)
     const long long G = gridDim.x;
     uint32_t cd0, cy0, tot0, cd1 = 0, cy1 = 0, tot1 = 0;
     unsigned long long ga0, la0, ga1 = 0, la1 = 0;
-    words(tile, cd0, ga0, la0, cy0, tot0);
-    if (tile + G < ntiles) words(tile + G, cd1, ga1, la1, cy1, tot1);
+    uint32_t ca, cb = 0;
+    words(tile, ca, cb, ga0, la0, cy0, tot0);
+    cd0 = lead_join(lead, ca, cb);
+    if (tile + G < ntiles) {
+        words(tile + G, ca, cb, ga1, la1, cy1, tot1);
+        cd1 = lead_join(lead, ca, cb);
+    }
     copy_in(0, ga0 + la0, tot0);
     for (int it = 0;; it++) {
         const bool more = tile + G < ntiles;
         // the words of the tile after next, in flight during this tile
-        uint32_t cd2 = 0, cy2 = 0, tot2 = 0;
+        uint32_t ca2 = 0, cb2 = 0, cy2 = 0, tot2 = 0;
         unsigned long long ga2 = 0, la2 = 0;
-        if (tile + 2 * G < ntiles) words(tile + 2 * G, cd2, ga2, la2, cy2, tot2);
+        if (tile + 2 * G < ntiles) words(tile + 2 * G, ca2, cb2, ga2, la2, cy2, tot2);
         const uint32_t codes = cd0, carry = cy0;
         const unsigned long long base = ga0 + la0;
         const unsigned long long first = (unsigned long long)tile * kNbTile + threadIdx.x * kNbPer;
@@ -762,7 +781,7 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2)
         // barrier that follows that copy
         tile += G;
         cd0 = cd1; ga0 = ga1; la0 = la1; cy0 = cy1; tot0 = tot1;
-        cd1 = cd2; ga1 = ga2; la1 = la2; cy1 = cy2; tot1 = tot2;
+        cd1 = lead_join(lead, ca2, cb2); ga1 = ga2; la1 = la2; cy1 = cy2; tot1 = tot2;
     }
     cp_async_wait_all();
 }

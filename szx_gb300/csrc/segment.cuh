@@ -416,6 +416,22 @@ __device__ __forceinline__ void st_v8(double* p, const double* v) {
                  : "memory");
 }
 
+// N words at any byte address, from the aligned words that hold them; the
+// caller's bytes end at `end`.  False when the last aligned word passes it.
+template <int N>
+__device__ __forceinline__ bool load_words(const uint8_t* p, const uint8_t* end, uint32_t (&w)[N]) {
+    const uint32_t sh = (uint32_t)((uintptr_t)p & 3);
+    const uint32_t* q = (const uint32_t*)(p - sh);
+    if ((const uint8_t*)(q + N + (sh != 0)) > end) return false;
+    uint32_t a[N + 1];
+#pragma unroll
+    for (int i = 0; i < N; i++) a[i] = __ldg(q + i);
+    a[N] = sh ? __ldg(q + N) : 0u;
+#pragma unroll
+    for (int i = 0; i < N; i++) w[i] = __funnelshift_r(a[i], a[i + 1], 8 * sh);
+    return true;
+}
+
 // ------------------------------------------------------------------ runs, decoded
 
 // Lead-byte tables (a lead byte holds 4 codes, MSB first): 8 * the four leads

@@ -125,3 +125,21 @@ def test_decode_workspace_at_any_word(szx, mode, skew):
         assert codec.status() == 0
         z = O.decompress(mode, np.float32, want, n)
         assert np.array_equal(y.cpu().numpy().view(np.uint8), z.view(np.uint8)), n
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_non_blocked_stream_at_every_byte_alignment(szx, dt):
+    """Lead codes loaded as words around any address: fields of less than a
+    word of codes, ends of every kind, whole and partial tiles and groups."""
+    import torch
+    for n in (1, 15, 17, 32, 33, 127, 4095, 4096 + 16, 8 * 4096, 9 * 4096 + 37):
+        x = field(dt, max(n, 4), 11)[:n]
+        want = O.compress(1, x, 1e-3, 128)
+        z = O.decompress(1, dt, want, n)
+        codec = szx.DeviceCodec(1, dt, n)
+        for off in range(16):
+            buf = torch.empty(off + len(want), dtype=torch.uint8, device="cuda")
+            buf[off:].copy_(torch.frombuffer(bytearray(want), dtype=torch.uint8))
+            y = codec.decompress(buf[off:], n)
+            assert codec.status() == 0
+            assert np.array_equal(y.cpu().numpy().view(np.uint8), z.view(np.uint8)), (n, off)
