@@ -380,7 +380,9 @@ cudaError_t launch_nonblocked_encode(int dtype, const void* x, size_t n, uint8_t
 
 // ------------------------------------------------------------------ decode
 
-__device__ NonBlockedHdr parse_nb(const uint8_t* s, unsigned long long len, unsigned long long n) {
+// W: bytes of a value.  A reqLength above its bits is refused here, for every kernel of the decode (they test ok alone,
+// and find the counting kernel's tables complete).
+__device__ NonBlockedHdr parse_nb(const uint8_t* s, unsigned long long len, unsigned long long n, int W) {
     NonBlockedHdr r = {};
     r.n = n;
     r.ok = 0;
@@ -391,7 +393,7 @@ __device__ NonBlockedHdr parse_nb(const uint8_t* s, unsigned long long len, unsi
         r.reqLength = s[4];
         r.median = __uint_as_float(((uint32_t)s[5] << 24) | ((uint32_t)s[6] << 16) | ((uint32_t)s[7] << 8) | s[8]);
         r.mid_off = 17 + L;
-        r.ok = L == (n + 3) / 4 && r.mid_off <= len && r.reqLength >= 1 && r.reqLength <= 64;
+        r.ok = L == (n + 3) / 4 && r.mid_off <= len && r.reqLength >= 1 && r.reqLength <= 8 * W;
         r.mid_len = r.ok ? len - r.mid_off : 0;
     }
     return r;
@@ -451,12 +453,12 @@ __global__ void __launch_bounds__(kNbThreads) k_nb_count(const uint8_t* __restri
     __shared__ uint32_t s_cnt[kTpg];
     __shared__ unsigned long long s_own[kTpg];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const NonBlockedHdr h = parse_nb(s, len, n);   // (every thread: the same loads, from cache)
+    const NonBlockedHdr h = parse_nb(s, len, n, W);   // (every thread: the same loads, from cache)
     if (blockIdx.x == 0 && threadIdx.x == 0) {     // for the kernels that follow
         *hp = h;
         *err = h.ok ? kErrNone : kErrStream;
     }
-    if (!h.ok || h.reqLength > 8 * W) return;
+    if (!h.ok) return;
     const int R = run_bytes<T>(h.reqLength);
     const unsigned long long ntiles = (h.n + kNbTile - 1) / kNbTile;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -674,7 +676,6 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2)
     __shared__ uint32_t lut_ld[512];
     const NonBlockedHdr h = *hp;
     if (!h.ok) return;
-    if (h.reqLength > 8 * W) return;
     const int R = run_bytes<T>(h.reqLength);
     const long long ntiles = (long long)((h.n + kNbTile - 1) / kNbTile);
     long long tile = blockIdx.x;
