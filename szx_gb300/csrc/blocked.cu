@@ -1456,15 +1456,20 @@ __device__ __forceinline__ void dec_segment(uint32_t p, int len, T* ob, int vec,
     constexpr int E = EncCfg<T>::E;
     constexpr int NC = E / 4;
     const int sl = (int)(lane_id() & (G - 1));
-    const int reqLength = (int)lds8(p);
+    int reqLength = (int)lds8(p);
     const uint32_t mb = (lds8(p + 1) << 24) | (lds8(p + 2) << 16) | (lds8(p + 3) << 8) | lds8(p + 4);
-    const int R = run_bytes<T>(reqLength);
     const int Lb = FULL ? G * NC : (len + 3) / 4;
     const int nv = FULL ? E : (len - E * sl < 0 ? 0 : (len - E * sl < E ? len - E * sl : E));   // the lane's values
     // the lane's lead bytes, chunk k in byte k
     const uint32_t lp = p + 5 + NC * sl;
     uint32_t codes = __funnelshift_r(lds32(lp & ~3u), lds32((lp & ~3u) + 4), 8 * lp);
     if constexpr (NC == 2) codes &= 0xFFFFu;
+    int R = (reqLength + 7) >> 3;
+    if (!__all_sync(0xffffffffu, plain_req<T>(reqLength))) {   // (one vote: no lane pays for what no encoder here writes)
+        reqLength = clamp_req<T>(reqLength);
+        R = run_bytes(reqLength);
+        if (one_byte_req(reqLength)) codes = one_byte_codes(codes);
+    }
     const RunLeads<E> leads(codes, nv, R);
     const uint32_t incl = seg_inclusive_sum<G>(leads.bytes());
     const uint32_t q0 = p + 5 + (uint32_t)Lb + incl - leads.bytes();   // the run's first byte

@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(kNbThreads) k_nb_count(const uint8_t* __restri
         *err = h.ok ? kErrNone : kErrStream;
     }
     if (!h.ok) return;
-    const int R = run_bytes<T>(h.reqLength);
+    const int R = run_bytes(h.reqLength);
     const unsigned long long ntiles = (h.n + kNbTile - 1) / kNbTile;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long tile = (long long)blockIdx.x * kTpg + warp;
@@ -477,6 +477,10 @@ __global__ void __launch_bounds__(kNbThreads) k_nb_count(const uint8_t* __restri
         } else if (first + kWords * kNbPer > h.n || !load_words<kWords>(lp, s + len, cw)) {
 #pragma unroll
             for (int j = 0; j < kWords; j++) cw[j] = lead_word(lead, (first >> 2) + 4 * j, h.L);
+        }
+        if (one_byte_req(h.reqLength)) {
+#pragma unroll
+            for (int j = 0; j < kWords; j++) cw[j] = one_byte_codes(cw[j]);
         }
         uint32_t mine = 0, lastw[3] = {0, 0, 0}, lastc[3] = {0, 0, 0};   // per byte lane: its last word and the bytes before it
         int lastn[3] = {0, 0, 0};
@@ -669,14 +673,13 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2)
     constexpr int kTpg = kNbThreads / 32;
     using EL = Elem<T>;
     using U = typename EL::U;
-    constexpr int W = EL::W;
     extern __shared__ __align__(16) uint8_t nb_dyn[];   // two staging buffers of nb_dec_stage_bytes<T>()
     __shared__ uint32_t s_sum[8];
     __shared__ uint32_t s_wv[8], s_wm[8];   // per warp: last written top bytes, their byte mask
     __shared__ uint32_t lut_ld[512];
     const NonBlockedHdr h = *hp;
     if (!h.ok) return;
-    const int R = run_bytes<T>(h.reqLength);
+    const int R = run_bytes(h.reqLength);
     const long long ntiles = (long long)((h.n + kNbTile - 1) / kNbTile);
     long long tile = blockIdx.x;
     if (tile >= ntiles) return;
@@ -730,7 +733,10 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2)
         uint32_t ca2 = 0, cb2 = 0, cy2 = 0, tot2 = 0;
         unsigned long long ga2 = 0, la2 = 0;
         if (tile + 2 * G < ntiles) words(tile + 2 * G, ca2, cb2, ga2, la2, cy2, tot2);
-        const uint32_t codes = cd0, carry = cy0;
+        uint32_t codes = cd0;
+        const uint32_t carry = cy0;
+        // (R first: with the one test the loop spills and takes 226 us at 2^27 values, not 210)
+        if (R == 2 && one_byte_req(h.reqLength)) codes = one_byte_codes(codes);
         const unsigned long long base = ga0 + la0;
         const unsigned long long first = (unsigned long long)tile * kNbTile + threadIdx.x * kNbPer;
         const int nv = first >= h.n ? 0 : (h.n - first < kNbPer ? (int)(h.n - first) : kNbPer);

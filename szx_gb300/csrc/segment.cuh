@@ -437,7 +437,7 @@ __device__ __forceinline__ bool load_words(const uint8_t* p, const uint8_t* end,
 // Lead-byte tables (a lead byte holds 4 codes, MSB first): 8 * the four leads
 // as bytes, value 0 in byte 0; at 256 + c the same with leads cut at 2.  A
 // value stores max(R - lead, 0) bytes, so 8 * R less the entry is its stored
-// bits, from the second table where R is 2 (no stream has a smaller one).
+// bits, from the second table where R is 2 (the decoders turn R = 1 into it).
 __device__ __forceinline__ void lead_table_init(uint32_t* lut) {
     for (int c = threadIdx.x; c < 256; c += blockDim.x) {
         uint32_t a = 0, b = 0;
@@ -463,11 +463,23 @@ __device__ __forceinline__ uint32_t lds8(uint32_t a) {
     return v;
 }
 
-// Stored bytes of a value at lead 0, kept in range for streams that are not valid.
+// The run decoder below takes R = 2 bytes a value at least, what this library's
+// encoders write (reqLength from 9).  A value of one byte is one of two whose
+// top byte is always its predecessor's, zero before the first: every lead one
+// higher, cut at 2.  Four codes to a byte, any number of bytes.
+__device__ __forceinline__ bool one_byte_req(int reqLength) { return reqLength <= 8; }
+__device__ __forceinline__ uint32_t one_byte_codes(uint32_t c) { return 0x55555555u + ((c | c >> 1) & 0x55555555u); }
+// Stored bytes of a value at lead 0; reqLength 1 .. 8 * sizeof(T).
+__device__ __forceinline__ int run_bytes(int reqLength) { return reqLength <= 8 ? 2 : (reqLength + 7) >> 3; }
+// A block's reqLength byte is taken as it comes, and decoded without reading
+// outside the block's largest size: 0 as 8, one above the type's bits as all
+// bytes shifted by what its low three bits say.
 template <typename T>
-__device__ __forceinline__ int run_bytes(int reqLength) {
-    const int R = (reqLength + 7) >> 3;
-    return R < 2 ? 2 : (R > Elem<T>::W ? Elem<T>::W : R);
+__device__ __forceinline__ bool plain_req(int reqLength) { return (uint32_t)(reqLength - 9) <= 8u * sizeof(T) - 9u; }
+template <typename T>
+__device__ __forceinline__ int clamp_req(int reqLength) {
+    constexpr int B = 8 * (int)sizeof(T);
+    return reqLength == 0 ? 8 : (reqLength > B ? B - (-reqLength & 7) : reqLength);
 }
 
 // The lead codes of a run of up to E (at most 16) values as masks, value e's
@@ -511,10 +523,11 @@ struct RunLeads {
 };
 
 // One pass over a run: cur, the values' bits less the median, and v, their
-// sums with it.  q0: shared address of the run's first stored byte (the reads
-// start up to eight bytes before it); carry: the top 32 bits of the value before
-// (three bytes of them count).  Returns whether a sum may be a NaN: the x86
-// rules then decide (nan_rule).  FULL: nv is E.
+// sums with it.  reqLength: 1 .. 8 * sizeof(T), R its run_bytes(); q0: shared
+// address of the run's first stored byte (the reads start up to eight bytes
+// before it); carry: the top 32 bits of the value before (three bytes of them
+// count).  Returns whether a sum may be a NaN: the x86 rules then decide
+// (nan_rule).  FULL: nv is E.
 template <typename T, int E, bool FULL>
 __device__ __forceinline__ bool run_decode(uint32_t codes, int nv, int R, int reqLength, uint32_t q0, uint32_t carry,
                                            T med, const uint32_t* lut_ld, typename Elem<T>::U (&cur)[E], T (&v)[E]) {
@@ -527,7 +540,7 @@ __device__ __forceinline__ bool run_decode(uint32_t codes, int nv, int R, int re
     const uint32_t R8 = (uint32_t)R * 0x08080808u;
     unsigned long long nan2 = 0;
     if constexpr (sizeof(T) == 4) {
-        const int down = reqLength > 32 ? 0 : (reqLength < 1 ? 31 : 32 - reqLength);   // `run` ends in the value's required bits
+        const int down = 32 - reqLength;   // `run` ends in the value's required bits
         // (the shift by `down` is a multiplication: the integer pipe sets the pace, the FMA pipe has room)
         const uint32_t scale = 1u << down;
         uint32_t run = carry >> (32 - 8 * R);
@@ -563,7 +576,7 @@ __device__ __forceinline__ bool run_decode(uint32_t codes, int nv, int R, int re
                 : "=f"(v[e]), "=f"(v[e + 1]), "+l"(nan2)
                 : "r"(cur[e]), "r"(cur[e + 1]), "f"(med), "f"(0.0f));
     } else {
-        const int s = reqLength & 7 ? 8 - (reqLength & 7) : 0;
+        const int s = 8 * R - reqLength;
         const U keep = ~(U)0 << (8 * (W - R));
         uint32_t prev = carry;   // the previous value's top 32 bits
 #pragma unroll
