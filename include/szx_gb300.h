@@ -292,8 +292,10 @@ int SZxG_batch_fixed_rate(SZxG_Batch* batch, const SZxG_Mlp* mlp, const float* t
  * Returns the number of kernels reported. */
 /* Failure detection (no counterpart in the reference): runs the device-wide
  * look-back the codecs use to place variable-length payloads (scan 0: the
- * 64-bit status words; scan 1: the encoders' placement window before them) over
- * ntiles (<= 4096) one-warp tiles, tile t contributing t + 1, with tile
+ * 64-bit status words, by one warp; scan 1: the encoders' placement window
+ * before them; scan 2: the decoders' index, by a whole CTA; scan 3: the same
+ * with status words that start 8 bytes behind a 16-byte boundary) over ntiles
+ * (<= 4096) tiles, tile t contributing t + 1, with tile
  * `withheld` (-1: none) never publishing, and waits bounded by spinLimit
  * polls.  Returns SZXG_ERR_LOOKBACK when a wait gave up, else SZXG_OK with
  * prefix[t] = t(t+1)/2 (host array of ntiles, may be NULL).  Synchronous. */

@@ -246,7 +246,9 @@ __device__ __forceinline__ V warp_sum(V v) {
 constexpr unsigned kSpinLimit = 1u << 22;   // polls before giving up (~1 s with backoff)
 // Every look-back below takes its poll limit as a last argument (default
 // kSpinLimit); the failure-detection self-test (selftest.cu) passes a small
-// one and withholds a tile, so the give-up path runs for real.
+// one and withholds a tile, so the give-up path runs for real.  (The placement
+// window has no waits of its own: it is read again kWinRepolls times, then one
+// of them takes over.)
 
 enum : int { kErrNone = 0, kErrLookback = 1, kErrCapacity = 2, kErrStream = 3 };
 
@@ -408,13 +410,14 @@ __device__ __forceinline__ unsigned long long prefix_resolve(unsigned long long*
 template <int WARPS>
 __device__ __forceinline__ unsigned long long prefix_resolve_cta(unsigned long long* st, long long tile,
                                                                  unsigned long long agg, int* err,
-                                                                 unsigned long long* sm) {
+                                                                 unsigned long long* sm,
+                                                                 unsigned limit = kSpinLimit) {
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     const long long g0 = (((tile - 1) >> 2) << 2) - 128 * (long long)warp, g = g0 - 4 * (long long)lane;
     unsigned long long pa = 0;
     bool done = false;
     unsigned spins = 0;
-    for (unsigned round = 0; !done && round < kSpinLimit; round++) {   // (the same rounds in every thread)
+    for (unsigned round = 0; !done && round < limit; round++) {   // (the same rounds in every thread)
         if (round) __syncthreads();   // (the sums of the round before are read)
         unsigned long long mine = kS64Inc;   // this warp's window: its sum, and kS64Inc where a prefix ends it
         while (tile > 0 && g0 >= 0) {
@@ -444,7 +447,7 @@ __device__ __forceinline__ unsigned long long prefix_resolve_cta(unsigned long l
                 mine = (inc_mask ? kS64Inc : 0ull) | (warp_sum(lane <= stop ? sa : 0ull) & kS64Val);
                 break;
             }
-            if (++spins > kSpinLimit) {
+            if (++spins > limit) {   // (its window counts as an empty prefix: the walk ends, the error stands)
                 if (lane == 0) atomicExch(err, kErrLookback);
                 break;
             }

@@ -8,7 +8,7 @@
 // SZXG_ERR_LOOKBACK in the call's error word instead of hanging the GPU.
 //
 // SZxG_selftest_lookback runs the same look-back functions the codecs use over
-// ntiles one-warp tiles (tile t contributes t + 1 bytes), with one tile
+// ntiles one-warp or one-CTA tiles (tile t contributes t + 1 bytes), with one tile
 // `withheld` that never publishes, and a small poll limit.  The tile after the
 // withheld one waits, gives up after `spinLimit` polls, and the call reports
 // SZXG_ERR_LOOKBACK; with nothing withheld it returns every tile's exclusive
@@ -49,6 +49,22 @@ __global__ void k_selftest_lookback(int scan, unsigned long long* st64, uint16_t
     if (lane_id() == 0) prefix[tile] = p;
 }
 
+// scan 2: the CTA-wide look-back of the decoders' index (prefix_resolve_cta),
+//         256 threads a tile; scan 3: the same with the status words 8 bytes
+//         behind a 16-byte boundary, where they are read one at a time.
+constexpr int kSelfCta = 256;
+__global__ void __launch_bounds__(kSelfCta) k_selftest_lookback_cta(unsigned long long* st64, int ntiles, int withheld,
+                                                                    unsigned limit, unsigned long long* prefix,
+                                                                    int* err) {
+    __shared__ unsigned long long sm[kSelfCta / kWarp];
+    const long long tile = blockIdx.x;
+    if (tile >= ntiles || tile == withheld) return;
+    const unsigned long long agg = (unsigned long long)tile + 1;
+    if (threadIdx.x < kWarp) prefix_publish(st64, tile, agg);
+    const unsigned long long p = prefix_resolve_cta<kSelfCta / kWarp>(st64, tile, agg, err, sm, limit);
+    if (threadIdx.x == 0) prefix[tile] = p;
+}
+
 }  // namespace
 }  // namespace szxg
 
@@ -56,7 +72,7 @@ using namespace szxg;
 
 extern "C" int SZxG_selftest_lookback(int scan, int ntiles, int withheld, unsigned spinLimit,
                                       unsigned long long* prefix, void* stream) {
-    if ((scan != 0 && scan != 1) || ntiles < 1 || ntiles > 4096 || withheld >= ntiles || spinLimit < 1) {
+    if (scan < 0 || scan > 3 || ntiles < 1 || ntiles > 4096 || withheld >= ntiles || spinLimit < 1) {
         set_last_error(SZXG_ERR_ARG);
         return SZXG_ERR_ARG;
     }
@@ -77,7 +93,11 @@ extern "C" int SZxG_selftest_lookback(int scan, int ntiles, int withheld, unsign
     int rc = SZXG_OK;
     cudaError_t e = cudaMemsetAsync(b, 0, bytes, s);
     if (e == cudaSuccess) {
-        k_selftest_lookback<<<ntiles, kWarp, 0, s>>>(scan, st64, counts, ntiles, withheld, spinLimit, d_prefix, d_err);
+        if (scan < 2)
+            k_selftest_lookback<<<ntiles, kWarp, 0, s>>>(scan, st64, counts, ntiles, withheld, spinLimit, d_prefix, d_err);
+        else   // (scan 3 starts a word later: the n + 8 words hold what is read past the last tile's all the same)
+            k_selftest_lookback_cta<<<ntiles, kSelfCta, 0, s>>>(st64 + (scan == 3), ntiles, withheld, spinLimit, d_prefix,
+                                                                d_err);
         e = cudaGetLastError();
     }
     int h_err = 0;
