@@ -64,6 +64,7 @@
 #include "../../include/szx_gb300.h"
 #include "batch.h"
 #include "common.cuh"
+#include "size_pass.h"
 
 using namespace szxg;
 
@@ -86,6 +87,9 @@ constexpr int kSizeAhead = 7;           // sizes a pass measures of one field: t
 constexpr int kAheadFrom = 2;           // passes of a field before its later bounds are measured ahead
 constexpr unsigned long long kAheadSteps = 1ull << 17;   // steps of 512 values a launch with such bounds may have
                                                          // (2^26 values: ~55 us, about what another pass's round trip costs)
+constexpr size_t kAheadItems = 512;     // sizes from which a pass asks for no more of them: the host's work on one is a
+                                        // fraction of a us, a round trip 20 (1000 fields of 2^12..2^16 values, bisection:
+                                        // 1.01 ms, 1.39 with four times as many; 50 fields: 0.43 and 0.44)
 constexpr double kBracketStop = 1.0 / 1024;   // searches stop on a measured bracket this narrow
 
 // parameter offsets
@@ -1330,53 +1334,38 @@ int SZxG_batch_fixed_rate(SZxG_Batch* b, const SZxG_Mlp* mlp, const float* targe
     // nothing; the streams are coded once, at the chosen bounds.  Beside the
     // next bound of a field that has missed twice a pass measures the bounds
     // that would follow either outcome, two deep, while that stays a small part
-    // of a launch (kAheadSteps): a search that runs on then takes three
+    // of a launch (kAheadSteps, kAheadItems): a search that runs on then takes three
     // decisions per launch and round trip.  Decisions, bounds and pass counts
     // are those of the one-by-one search.  (24 fields of 2^18..2^23 values,
     // ratio 16: up to ten passes, each of which coded its fields, 2267 us.)
     const unsigned long long hdr = b->mode == kBlocked ? 13 : 20, per_nnc = b->mode == kBlocked ? 0 : 2;
-    struct Asked { float eb; double cr; };
-    auto same = [](float x, float y) { return memcmp(&x, &y, sizeof x) == 0; };   // (a NaN bound is found again too)
-    std::vector<std::vector<Asked>> known(nf);
-    auto find = [&](int f, float eb) -> const Asked* {
-        for (const Asked& a : known[f])
-            if (same(a.eb, eb)) return &a;
-        return nullptr;
-    };
+    KnownRatios known(nf);
+    SizePass pass(nf);
+    const std::vector<SizeItem>& items = pass.items;
     std::vector<uint8_t> up;
     std::vector<unsigned long long> sums;
-    std::vector<SizeItem> items;
-    std::vector<int> owner;
+    std::vector<Search> level, next;
     for (;;) {
-        items.clear();
-        owner.clear();
-        unsigned long long steps = 0;
-        auto ask = [&](int f, float eb) {
-            for (size_t k = 0; k < items.size(); k++)
-                if (owner[k] == f && same(items[k].eb, eb)) return;
-            const unsigned long long n = b->tab[f].n;
-            items.push_back({(const float*)b->tab[f].x, n, steps, eb, 0});
-            owner.push_back(f);
-            steps += (n + 511) / 512;
-        };
+        pass.clear();
         for (int f = 0; f < nf; f++) {
             if (st[f].done || st[f].passes >= maxPasses) continue;
-            ask(f, bound_of(f, st[f]));
+            pass.ask(f, (const float*)b->tab[f].x, b->tab[f].n, bound_of(f, st[f]));
         }
-        for (int f = 0; f < nf; f++) {
+        for (int f = 0; f < nf && items.size() < kAheadItems; f++) {
             if (st[f].done || st[f].passes < kAheadFrom || st[f].passes + 1 >= maxPasses) continue;
             const unsigned long long own = (b->tab[f].n + 511) / 512;
-            const int deep = steps + 6 * own <= kAheadSteps ? 2 : steps + 2 * own <= kAheadSteps ? 1 : 0;
+            const int deep = pass.steps + 6 * own <= kAheadSteps ? 2 : pass.steps + 2 * own <= kAheadSteps ? 1 : 0;
             // both outcomes of this bound, and both of each of those (a miss is a miss, by any factor)
-            std::vector<Search> level{st[f]};
+            pass.begin_turn();
+            level.assign(1, st[f]);
             for (int d = 0; d < deep; d++) {
-                std::vector<Search> next;
+                next.clear();
                 for (const Search& S : level)
                     for (int side = 0; side < 2; side++) {
                         Search Q = S;
                         judge(f, Q, bound_of(f, S), (double)tgt[f] * (side ? 8.0 * (1.0 + tolerance) : 0.125 / (1.0 + tolerance)));
                         if (Q.done || Q.passes >= maxPasses) continue;
-                        ask(f, bound_of(f, Q));
+                        pass.ask_more(f, (const float*)b->tab[f].x, b->tab[f].n, bound_of(f, Q));
                         next.push_back(Q);
                     }
                 level.swap(next);
@@ -1389,15 +1378,15 @@ int SZxG_batch_fixed_rate(SZxG_Batch* b, const SZxG_Mlp* mlp, const float* targe
         unsigned long long* d_acc = (unsigned long long*)(b->lfx->size_in + ib);
         sums.resize(2 * ni);
         e = cudaMemcpyAsync(b->lfx->size_in, up.data(), up.size(), cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = launch_blocked_sizes((const SizeItem*)b->lfx->size_in, (int)ni, steps, d_acc, s);
+        if (e == cudaSuccess) e = launch_blocked_sizes((const SizeItem*)b->lfx->size_in, (int)ni, pass.steps, d_acc, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(sums.data(), d_acc, 16 * ni, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return fail_code(e);
         for (size_t k = 0; k < ni; k++) {
-            const int f = owner[k];
+            const int f = pass.owner[k];
             const unsigned long long n = b->tab[f].n, nb = b->tab[f].nb, pay = sums[2 * k], nnc = sums[2 * k + 1];
             const unsigned long long size = hdr + per_nnc * nnc + (nb + 7) / 8 + 4 * (nb - nnc) + pay;
-            known[f].push_back({items[k].eb, (double)n * 4.0 / (double)size});
+            known.add(f, items[k].eb, (double)n * 4.0 / (double)size);
         }
         // every field as far as its measured bounds take it
         std::vector<int> fl, fw;
@@ -1406,11 +1395,12 @@ int SZxG_batch_fixed_rate(SZxG_Batch* b, const SZxG_Mlp* mlp, const float* targe
             Search& S = st[f];
             while (!S.done && S.passes < maxPasses) {
                 const float eb = bound_of(f, S);
-                const Asked* a = find(f, eb);
-                if (!a) break;
-                if (!judge(f, S, eb, a->cr)) continue;
+                const double* found = known.find(f, eb);
+                if (!found) break;
+                const double cr = *found;
+                if (!judge(f, S, eb, cr)) continue;
                 // re-aim the sampled crossing by the miss this pass measured
-                t2[f] = (float)((double)aim[f] * std::min(std::max((double)tgt[f] / a->cr, 0.25), 4.0));
+                t2[f] = (float)((double)aim[f] * std::min(std::max((double)tgt[f] / cr, 0.25), 4.0));
                 if (!(t2[f] > 0.f) || !std::isfinite(t2[f])) t2[f] = aim[f];
                 double yw;
                 if (window_crossing(f, t2[f], yw)) {
