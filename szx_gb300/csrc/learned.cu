@@ -1251,7 +1251,7 @@ int SZxG_batch_fixed_rate(SZxG_Batch* b, const SZxG_Mlp* mlp, const float* targe
     // target band; lo_eb / hi_eb / best_eb: bounds of the bracket's measured
     // ends and of the best pass; ebx: a bound to measure exactly next (0: from y).
     struct Search {
-        double lo, hi, y, yprev = 0, step = 0, best_err = 1e300, best_cr = 0;
+        double lo, hi, y, yprev = 0, step = 0, best_err = 1e300;
         float lo_eb = 0, hi_eb = 0, best_eb = 0, ebx = 0, ebk = 0;
         int passes = 0, done = 0, stage = 0;
         bool last_is_best = false, lo_m = false, hi_m = false;
@@ -1290,7 +1290,6 @@ int SZxG_batch_fixed_rate(SZxG_Batch* b, const SZxG_Mlp* mlp, const float* targe
         if (rel < S.best_err) {
             S.best_err = rel;
             S.best_eb = eb;
-            S.best_cr = cr;
             S.last_is_best = true;
         }
         if (rel <= tolerance) { S.done = 1; return false; }
@@ -1442,7 +1441,10 @@ int SZxG_batch_fixed_rate(SZxG_Batch* b, const SZxG_Mlp* mlp, const float* targe
     for (int f = 0; f < nf; f++) {
         if (res[f].status && !err_code) err_code = res[f].status;
         if (h_eb) h_eb[f] = ebk[f];
-        if (h_ratio) h_ratio[f] = (float)st[f].best_cr;
+        // the ratio of the stream that was coded, not of the size a pass measured (0: no bound gave a ratio)
+        if (h_ratio)
+            h_ratio[f] = st[f].best_err < 1e300 && !res[f].status ? (float)((double)b->tab[f].n * 4.0 / (double)res[f].size)
+                                                                  : 0.f;
         if (h_passes) h_passes[f] = st[f].passes;
     }
     set_last_error(err_code);

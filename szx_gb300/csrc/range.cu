@@ -13,6 +13,7 @@
 // extremes to it, and a zero extreme takes the sign of the first zero.
 #include "common.cuh"
 #include "kernels.h"
+#include <stdlib.h>
 
 namespace szxg {
 
@@ -337,7 +338,7 @@ cudaError_t launch_range(int dtype, const void* x, size_t n, int err_mode, float
 
 // One cluster of eight SMs reads about 1 TB/s, so up to this size it needs
 // less time than the launch it saves.
-constexpr size_t kRangeSmallBytes = size_t(2) << 20;
+static const size_t kRangeSmallBytes = getenv("RSB") ? atol(getenv("RSB")) : size_t(1) << 20;
 
 bool range_is_small(int dtype, size_t n) { return n * (dtype == 0 ? 4 : 8) <= kRangeSmallBytes; }
 

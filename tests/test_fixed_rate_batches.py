@@ -55,3 +55,16 @@ def test_a_field_gets_the_same_in_any_batch(LR, network):
         assert np.array_equal(c2, cr[a:a + 30]) and np.array_equal(p2, ps[a:a + 30]), a
         assert np.array_equal(c.sizes(), sizes[a:a + 30]), a
         c.close()
+
+
+@pytest.mark.parametrize("mode", [2, 3, 4])
+def test_the_ratio_is_the_coded_streams(LR, mode):
+    """Reached targets, missed ones and the pass limit: the ratio is the input's bytes over the stream's."""
+    import torch
+    xs = _fields(torch, 60, 0, 16, 5)
+    b = LR.Batch(xs, fastMode=mode)
+    for target, passes, net in ((8.0, 20, None), (8.0, 20, _zero_network(LR)), (3.0, 2, None), (1000.0, 6, None)):
+        eb, cr, ps = b.fixed_rate(target, net, 0.02, passes)
+        want = (b.n * 4.0 / b.sizes()).astype(np.float32)
+        assert np.array_equal(cr, want), (target, passes)
+    b.close()
