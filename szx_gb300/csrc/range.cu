@@ -3,7 +3,7 @@
 // bound conversion of SZx_fast_compress_args (szx/src/szx.cc:249-253,
 // :277-287, :304-308, :332-340), done in one launch: grid-stride partials,
 // then the last CTA to finish reduces them and derives the codec parameters.
-// A field of up to 2 MiB takes one cluster of eight CTAs instead
+// A field of up to 512 KiB takes one cluster of eight CTAs instead
 // (k_range_small), which also does the call's clears: one launch fewer.
 //
 // The reference's sequential scan (`if (min > v) min = v; else if (max < v)
@@ -13,7 +13,6 @@
 // extremes to it, and a zero extreme takes the sign of the first zero.
 #include "common.cuh"
 #include "kernels.h"
-#include <stdlib.h>
 
 namespace szxg {
 
@@ -336,9 +335,12 @@ cudaError_t launch_range(int dtype, const void* x, size_t n, int err_mode, float
     return cudaGetLastError();
 }
 
-// One cluster of eight SMs reads about 1 TB/s, so up to this size it needs
-// less time than the launch it saves.
-static const size_t kRangeSmallBytes = getenv("RSB") ? atol(getenv("RSB")) : size_t(1) << 20;
+// One cluster of eight SMs reads about 1 TB/s, and up to this size it needs no
+// more time than the launch it saves.  A whole compress, one cluster against
+// clear and grid (us, REL 1e-3): float64 256 KiB 22.6 and 24.6, 512 KiB 24.6 and
+// 24.7, 1 MiB 26.7 and 24.6, 2 MiB 31.5 and 28.8; float32 512 KiB 20.6 and 20.6,
+// 768 KiB 22.5 and 21.6, 2 MiB 26.8 and 24.6.
+constexpr size_t kRangeSmallBytes = size_t(512) << 10;
 
 bool range_is_small(int dtype, size_t n) { return n * (dtype == 0 ? 4 : 8) <= kRangeSmallBytes; }
 
