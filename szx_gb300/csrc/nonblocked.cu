@@ -218,9 +218,17 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
         claim_tile(gc, a.tile_ctr, taker && live);
         const unsigned long long first = (unsigned long long)tile * kNbTile + threadIdx.x * kNbPer;
         U d[kNbPer];
-        const T dprev = EL::sub(before, med);
+        T dprev = (T)0;
+        // (no double subtractions in the two iterations after the last tile: they held the FP64 pipe as long as a tile's
+        // do, 15.9 instead of 13.8 us for 2^18 doubles, a tile a CTA; for floats the branch spills)
+        if (sizeof(T) == 4 || live) {
+            dprev = EL::sub(before, med);
+            sub_run(v, med, d);
+        } else {
+#pragma unroll
+            for (int e = 0; e < kNbPer; e++) d[e] = 0;
+        }
         U d_l0 = first > 0 ? EL::bits(dprev) : (U)0;   // lane 0: the value before its first one
-        sub_run(v, med, d);
         bool bad = lane == 0 && first > 0 && inf_or_nan(dprev);
         if constexpr (sizeof(T) == 4) {
             float hn = __uint_as_float(d[0]);
