@@ -241,7 +241,11 @@ __global__ void __launch_bounds__(kNbThreads, sizeof(T) == 4 ? 4 : 2) k_nb_encod
         }
         if (__any_sync(0xffffffffu, bad)) {
 #pragma unroll
-            for (int e = 0; e < kNbPer; e++) d[e] = EL::bits(xsub(v[e], med));
+            for (int e = 0; e < kNbPer; e++) {
+                // (doubles: the subtraction is done, an infinity among the differences stands)
+                if constexpr (sizeof(T) == 4) d[e] = EL::bits(xsub(v[e], med));
+                else if ((d[e] & 0x7FFFFFFFFFFFFFFFull) > 0x7FF0000000000000ull) d[e] = EL::bits(nan_rule(v[e], med));
+            }
             if (lane == 0 && first > 0) d_l0 = EL::bits(xsub(before, med));
         }
         // lead codes from the top 32 bits, as in the blocked encoder
