@@ -175,8 +175,34 @@ __device__ __forceinline__ bool enc_minmax_fast(const T (&v)[EncCfg<T>::E], int 
     return odd;
 }
 
-// The same with every rule of the reference's sequential scan
-// (szx/src/szx_float.cc:322-345), for the warps that met an odd value: NaNs
+// Floats: what the extremes above leave open of the reference's sequential
+// scan (szx/src/szx_float.cc:322-345).  They ignored the NaNs, as the scan does
+// unless the block's first value is one; a zero extreme takes the sign of the
+// first zero.  In registers, like the differences below: the loops over shared
+// memory that doubles take cost 2^23 floats with NaNs in one of a hundred values
+// 55 us a compress, 38.6 now (51.2 before the runs; 35.2 without NaNs), and their
+// code spilled beside the float loop (2^27 values: 282 -> 275 us).
+template <int G, bool FULL>
+__device__ __forceinline__ void enc_minmax_rules(const float (&v)[EncCfg<float>::E], int len, float& mn, float& mx) {
+    constexpr int E = EncCfg<float>::E;
+    const int f = E * (int)(lane_id() & (G - 1));
+    if (__any_sync(0xffffffffu, is_zero(mn) || is_zero(mx))) {
+        int zi = 1 << 30;   // 2 * index + sign of the first zero
+#pragma unroll
+        for (int e = E - 1; e >= 0; e--)
+            if (is_zero(v[e]) && (FULL || f + e < len)) zi = 2 * (f + e) + (int)(__float_as_uint(v[e]) >> 31);
+#pragma unroll
+        for (int d = G / 2; d > 0; d >>= 1) zi = min(zi, __shfl_xor_sync(0xffffffffu, zi, d, G));
+        const float zero = __uint_as_float((uint32_t)zi << 31);
+        if (is_zero(mn)) mn = zero;
+        if (is_zero(mx)) mx = zero;
+    }
+    const float x0 = __shfl_sync(0xffffffffu, v[0], 0, G);
+    if (len > 0 && isnan(x0)) mn = mx = x0;
+}
+
+// Doubles, with every rule of the scan
+// (szx/src/szx_double.cc:973-1030), for the warps that met an odd value: NaNs
 // are skipped unless the block's first value is one, a zero extreme has the
 // sign of the first zero.  Values come from shared memory again, one at a
 // time: this is the rare path, and small code beside the encoder's loop
@@ -256,7 +282,10 @@ __device__ __forceinline__ void enc_block_stats(uint8_t* tile, uint32_t e0, int 
     else load_run<T, G>(tile, e0, vec, v);
     T mn, mx;
     bool special = enc_minmax_fast<T, G, FULL>(v, len, mn, mx);
-    if (__any_sync(0xffffffffu, special)) special = enc_minmax_exact<T, G>(tile, e0, len, mn, mx);
+    if (__any_sync(0xffffffffu, special)) {
+        if constexpr (sizeof(T) == 4) enc_minmax_rules<G, FULL>(v, len, mn, mx);
+        else special = enc_minmax_exact<T, G>(tile, e0, len, mn, mx);
+    }
     int state;
     float radius_f, median_f;
     if constexpr (sizeof(T) == 4) {
@@ -289,13 +318,18 @@ __device__ __forceinline__ void enc_block_stats(uint8_t* tile, uint32_t e0, int 
     else med = xf2d(median_f);
     // differences from the median (szx/src/szx_float.cc:88-92); x86 NaN rules only where a NaN can arise
     U d[E];
-    if (__any_sync(0xffffffffu, special)) {
+    if (sizeof(T) == 8 && __any_sync(0xffffffffu, special)) {
         enc_diff_exact<T, G>(tile, e0, len, med);
         load_run<T, G>(tile, e0, vec, v);
 #pragma unroll
         for (int e = 0; e < E; e++) d[e] = EL::bits(v[e]);
     } else {
         sub_run(v, med, d);
+        if (sizeof(T) == 4 && __any_sync(0xffffffffu, special)) {
+#pragma unroll
+            for (int e = 0; e < E; e++)
+                if (isnan(EL::of(d[e]))) d[e] = EL::bits(nan_rule(v[e], med));
+        }
     }
     // Lead codes: leading identical bytes of the words shifted right by s with
     // the previous value's, capped at 3 -- (leading zeros of the XOR + s) / 8,
@@ -435,7 +469,7 @@ struct EncTile {
 //
 // Bound by the instructions of the statistics and the emission (issue 65 %):
 // 50 warp instructions per 32 floats, 124 per 32 doubles.  2^27 floats, REL
-// 1e-3, blocks of 128: 281 us (512 MiB in, 129 us with the stream at the copy
+// 1e-3, blocks of 128: 275 us (512 MiB in, 129 us with the stream at the copy
 // rate); 2^28 doubles in blocks of 64: 1355 us (490).  Before -- lanes over
 // interleaved 4-value chunks, byte stores, doubles on the FP64 pipe (two lanes
 // a clock and SM here), T_{j-2} placed by warp 0 while the others waited --
@@ -673,7 +707,9 @@ __global__ void __launch_bounds__(EncTile<T, G, TBYTES>::kThreads, EncTile<T, G,
 // contiguous range of 4-block steps (2 KiB, copied a step ahead into its own
 // two buffers), no placement, no barriers.  An item is a field and a bound;
 // acc[2 i] / [2 i + 1] gain its coded blocks' payload bytes and their number.
-__global__ void __launch_bounds__(kSizeThreads) k_blocked_sizes(const SizeItem* items, int ni,
+// (Four CTAs an SM, 64 registers: 263 us in the batch of 24 fields, 284 at two
+// CTAs and the 120 registers it takes unasked.)
+__global__ void __launch_bounds__(kSizeThreads, 4) k_blocked_sizes(const SizeItem* items, int ni,
                                                                 unsigned long long steps, unsigned long long* acc) {
     constexpr int G = 8, BS = 128, STEP = 4 * BS;   // values per step
     __shared__ __align__(512) uint8_t buf[kSizeThreads / 32][2][STEP * 4];
