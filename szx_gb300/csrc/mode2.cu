@@ -214,6 +214,7 @@ __global__ void __launch_bounds__(kM2Threads) k_m2_walk(const uint8_t* s, const 
     __shared__ uint32_t s_place[kM2Places], s_more[kM2Places], s_exit[kM2Places];   // more: blocks to the end, kM2No: none
     const BlockedHdr h = *hp;
     const unsigned long long j = blockIdx.x;
+    const int nthr = (int)blockDim.x;   // kM2Threads, or fewer where the candidates are few (m2_walk_threads)
     if (!h.ok) return;
     const uint8_t* P = s + h.q_off;
     const unsigned long long L = g.len - h.q_off, x0 = j * g.seg;
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(kM2Threads) k_m2_walk(const uint8_t* s, const 
     const int bs = (int)h.bs;
     const uint32_t end = seg < S.len ? seg : S.len;   // a walk is through when it stands here or beyond
     // candidates: a valid reqLength (the last four bytes of the region start no block)
-    for (uint32_t c0 = 0; c0 < ms; c0 += kM2Threads) {
+    for (uint32_t c0 = 0; c0 < ms; c0 += (uint32_t)nthr) {
         const uint32_t c = c0 + threadIdx.x;
         const bool in = c < ms, ok = in && c + 5 <= S.len && m2_valid_req(S.buf[S.ph + c], W);
         if (in && !ok) tab[c] = kM2Dead;
@@ -259,7 +260,7 @@ __global__ void __launch_bounds__(kM2Threads) k_m2_walk(const uint8_t* s, const 
         return true;
     };
     const uint32_t t0 = kM2Reach * ms < end ? kM2Reach * ms : end;
-    for (int i = threadIdx.x; i < n; i += kM2Threads) {
+    for (int i = threadIdx.x; i < n; i += nthr) {
         const uint32_t c = s_cand[i];
         uint32_t p = c, k = 0, pos = kM2No;
         if (walk(p, k, t0)) {
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(kM2Threads) k_m2_walk(const uint8_t* s, const 
     const uint32_t mask = m2_lead_mask((int)lane_id(), bs);
     uint32_t* list = lists + j * (unsigned long long)g.list;   // [0] the place, [1] blocks listed, then their offsets
     if (threadIdx.x == 0) list[0] = np ? s_place[0] : kM2No;
-    for (int i = threadIdx.x >> 5; i < np; i += kM2Threads / 32) {
+    for (int i = threadIdx.x >> 5; i < np; i += nthr / 32) {
         uint32_t p = s_place[i], k = 0;
         while (p < end) {
             if (i == 0 && lane_id() == 0) list[2 + k] = p;   // (a whole block's payload is at least its header and lead bytes)
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(kM2Threads) k_m2_walk(const uint8_t* s, const 
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += kM2Threads) {
+    for (int i = threadIdx.x; i < n; i += nthr) {
         const uint32_t c = s_cand[i] & 0xFFFFu;
         uint32_t k = s_cand[i] >> 16, p = s_pos[i];
         bool alive = p != kM2No;
@@ -482,6 +483,12 @@ __global__ void k_m2_serial(const uint8_t* s, const BlockedHdr* hp, M2Geom g, in
 namespace {
 
 int m2_maxsize(int dtype, int bs) { return 5 + (bs + 3) / 4 + (dtype == 0 ? 4 : 8) * bs; }
+// Threads of a segment's walk.  A segment of small blocks has few candidates and
+// few bytes, and one warp a segment keeps up to 32 of them on an SM instead of
+// eight: decode of 2^22 floats in blocks of 2 / 3 / 8 / 32 values 515 / 374 / 170
+// / 88 us with 256 threads, 312 / 226 / 114 / 75 with 32; blocks of 64 (277
+// bytes) 52 and 60, 24 doubles (203 bytes) 118 and 140.
+unsigned m2_walk_threads(int maxsize) { return maxsize <= 160 ? 32u : (unsigned)kM2Threads; }
 // Words of a segment's block list: place, count, and as many blocks of the smallest payload as a segment holds.
 int m2_list_words(int dtype, int bs) { return 3 + 32 * m2_maxsize(dtype, bs) / (5 + (bs + 3) / 4); }
 
@@ -545,7 +552,7 @@ cudaError_t launch_m2_offsets(int dtype, const uint8_t* d_stream, size_t len, si
     }
     {
         TraceScope tr("m2_walk", s);
-        e = launch_after(k_m2_walk, (unsigned)g.nseg, kM2Threads, dyn, s, d_stream, ws.bhdr, g, W, cnt_tab, exit_lo, exit_hi,
+        e = launch_after(k_m2_walk, (unsigned)g.nseg, m2_walk_threads(ms), dyn, s, d_stream, ws.bhdr, g, W, cnt_tab, exit_lo, exit_hi,
                          lists);
     }
     if (e == cudaSuccess)
