@@ -53,8 +53,11 @@ static WsLayout ws_layout(int layout, int dtype, size_t n, int bs) {
     size_t off = 0;
     L.hdr = off; off += 4096;
     L.st32 = off; off += a256(4 * (L.status_tiles + 16));
-    L.st = off; off += a256(8 * (3 * L.status_tiles > blocked_status_words(nb) ? 3 * L.status_tiles : blocked_status_words(nb)));
-    L.st2 = off; off += a256(3 * 8 * L.status2_tiles);
+    // fastMode 1: a word a tile and four read past the last (encode), two words a group of eight tiles, the second from
+    // status_tiles on (decode); blocked: both encode look-backs, more than the index's word a tile and four
+    const size_t st_nb = L.status_tiles + (L.status_tiles + 7) / 8 + 4, st_blk = blocked_status_words(nb);
+    L.st = off; off += a256(8 * (st_nb > st_blk ? st_nb : st_blk));
+    L.st2 = off; off += a256(8 * (L.status2_tiles + 4));
     L.partials = off; off += a256(4096 * 24);
     L.o = off; off += a256(2 * L.blocks);
     L.m = off; off += a256(4 * L.blocks);

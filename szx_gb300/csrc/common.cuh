@@ -264,11 +264,6 @@ struct Max3x21Op {
         }
         return r;
     }
-    static __device__ __forceinline__ unsigned long long warp_reduce(unsigned long long v) {
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, d));
-        return v;
-    }
 };
 
 // ------------------------------------------------------------------ TMA bulk copies + mbarriers

@@ -110,8 +110,8 @@ struct Workspace {
     int* err;
     unsigned long long* counters;   // 4 tile counters
     uint32_t* st32;                 // 32-bit tile status words ([status_tiles + 16])
-    unsigned long long* st_word;    // tile status words (family A)
-    unsigned long long* st2_word;   // tile status (family B)
+    unsigned long long* st_word;    // tile status words (encoders; decode index, family A; fastMode-1 group totals)
+    unsigned long long* st2_word;   // tile status words (decode index, family B)
     void* partials;                 // range-pass partials
     uint16_t* o_scr;                // payload sizes by non-constant rank
     uint32_t* m_scr;                // median bits by constant rank
