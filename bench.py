@@ -491,8 +491,9 @@ def make_batch_fields(nf, seed, device):
 
 def run_fixed_rate(args, wl):
     """C5: fixed-rate selection for 500 fields x 3 targets -- the learned path
-    (sampled model + network, judged by real compress passes) against plain
-    bisection over real compress passes, on the same GPU and plan."""
+    (sampled model + network) against plain bisection, on the same GPU and plan.
+    Both judge a bound by the exact size of its stream, which a pass measures
+    without coding it, and code every field once, at the bound they choose."""
     import numpy as np
     import torch
 

@@ -194,9 +194,9 @@ cudaError_t launch_ws_clear(const ClearList& c, cudaStream_t s) {
 }
 
 // Enqueue compress; the result record lands in res_out (device; default
-// ws.result).  One launch (for a small field the value-range pass itself) clears what the passes expect zeroed (the
-// value-range pass's ticket and the result record among it), so the
-// value-range pass and the encoder skip their own clears.
+// ws.result).  One launch clears what the passes expect zeroed, the value-range
+// pass's ticket and the result record among it; for a small field the
+// value-range pass does so itself.  The passes skip their own clears.
 static int enqueue_compress(int mode, int dtype, const void* d_x, size_t n, int bs, int err_mode, float abs_eb,
                             float rel, uint8_t* d_out, size_t cap, const Workspace& ws, cudaStream_t s,
                             StreamResult* res_out = nullptr) {

@@ -11,13 +11,13 @@
 // counter, so a field's tiles are always acquired before any later field's,
 // which is all the per-field look-back needs to make progress.
 //
-// Fields are grouped by size class, and neighbouring classes of one launch
-// shape share a launch (a table of value-count bounds, each with
-// its launch shape: encoder tile size and CTAs per SM of the encoder and the
-// decoder): one persistent launch per kernel and shape.  The table comes from the tuning file written by the project's
-// autotuner (szx_gb300/tune.py: tuning/batch_shapes.txt next to the
-// library, or the file SZXG_TUNING_FILE names), or from
-// SZxG_set_launch_shapes; with neither, one class with the default shape.
+// Fields are grouped by size class: a table of value-count bounds, each with a
+// launch shape (encoder tile size, CTAs per SM of the encoder and the decoder).
+// Neighbouring classes of one shape share one persistent launch per kernel.
+// The table comes from the tuning file written by the project's autotuner
+// (szx_gb300/tune.py: tuning/batch_shapes.txt next to the library, or the file
+// SZXG_TUNING_FILE names), or from SZxG_set_launch_shapes; with neither, one
+// class with the default shape.
 // The shape never changes a stream: only how the work is cut and spread.
 //
 // This file plans a batch (layout of the per-field scratch in one

@@ -75,8 +75,10 @@ constexpr int kH = 64;              // hidden width
 constexpr int kProbes = 16;         // coarse probes, y = -1.5 j (j = 1..16)
 constexpr int kFine = 16;           // fine probes, y = yq + (k - 8) / 4
 constexpr int kRate = 10;           // every 10th block sampled
-constexpr int kTileBlocks = 8;      // sampled blocks per warp tile (a multiple of kCoarseStep): with 32 the few, long
-                                    // tiles of 24 fields of 2^18..2^23 values left the passes waiting on latency
+// Sampled blocks per warp tile (a multiple of kCoarseStep).  A feature call with 8 and with 32: 24 fields of 2^18..2^23
+// values 239 and 299 us (few, long tiles wait on latency), 2000 of 2^14..2^22 1517 and 1970 (a tile's loads are in
+// flight together), 8000 of 2^10..2^12 316 and 359.
+constexpr int kTileBlocks = 8;
 constexpr int kCoarseStep = 4;      // the coarse curve uses every 4th sampled block (every 40th block)
 constexpr int kAcc = 18;            // per field, over the coarse blocks: count, bytes[16], radius-0 blocks
 constexpr int A_NS = 0, A_BYTES = 1, A_ZERO = 17;

@@ -443,11 +443,12 @@ __device__ __forceinline__ uint32_t lead_join(const uint8_t* lead, uint32_t a, u
 // Per tile (one warp): its mid-byte count (tcnt[t]) and, for each of the top
 // three byte lanes, where in the tile's mid bytes the last value storing that
 // lane put it (aux[3t+2], 3x21 bits, position+1, 0 = none).  A lane takes 8
-// consecutive 16-code words, so the tile takes one warp scan; each word costs its three masks, their population counts (a value
-// stores max(R - lead, 0) bytes = the number of k < R with lead <= k) and the
-// last word of each mask that is not empty.  (One word per lane and eight
-// scans a tile: 59 us at 2^27 values; codes that start at no word boundary, the
-// usual case, were read a byte at a time: 46 us, 33 as words.)
+// consecutive 16-code words, so the tile takes one warp scan.  A word costs its
+// three masks, their population counts (a value stores max(R - lead, 0) bytes,
+// the number of k < R with lead <= k) and the last word of each mask that is
+// not empty.  (One word per lane and eight scans a tile: 59 us at 2^27 values;
+// codes that start at no word boundary, the usual case, were read a byte at a
+// time: 46 us, 33 as words.)
 // The CTA's eight tiles form a group: aux[3t] / aux[3t+1] get the tile's
 // exclusive prefix within its group (bytes; latest writer tiles, 3x21 bits,
 // tile+1), gsum[g] / gwr[g] the group's totals.  Independent per group: no

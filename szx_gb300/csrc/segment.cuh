@@ -1,6 +1,7 @@
 // Segment helpers shared by the blocked codec kernels: a block of up to G*E
 // values is handled by a segment of G lanes of a warp (G a power of two),
-// E = 16 float / 8 double values per lane, in chunks of 4 values.
+// E = 16 float / 8 double values per lane: a run of consecutive values (codec)
+// or chunks of 4 values dealt out in turn (constant blocks, fixed-rate sampling).
 #pragma once
 #include "common.cuh"
 
