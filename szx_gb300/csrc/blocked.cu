@@ -1564,9 +1564,9 @@ __device__ __forceinline__ void dec_segment(uint32_t p, int len, T* ob, int vec,
 // 32-byte stores.  Full/empty mbarriers hand the buffers back and forth; every
 // wait is bounded and reports kErrLookback instead of hanging.
 //
-// Bound by the integer pipe for floats (2^27 values: 179 us, 129 us of
+// Bound by the integer pipe for floats (2^27 values: 177 us, 129 us of
 // traffic; 240 us before the run decoder) and by the FP64 add for doubles
-// (2^28 values: 737 us, 427 us of FP64 pipe and 522 us of traffic; 1117 us
+// (2^28 values: 727 us, 427 us of FP64 pipe and 522 us of traffic; 1117 us
 // before the NaN check left that pipe).
 constexpr int kDecWarps = 8;
 constexpr int kDecThreadsP = (kDecWarps + 1) * 32;

@@ -124,7 +124,7 @@ struct NbEncArgs {
 // buffers, the next tile's loads; then warp 0 places T_{j-1} (PlaceWin; its
 // window was copied in during the emission) while the other warps copy T_{j-2}
 // to its place | barrier | the bytes of the words that threads share.
-// Bound by the instruction rate and the two barriers, 244 us at 2^27 float32
+// Bound by the instruction rate and the two barriers, 242 us at 2^27 float32
 // values (512 MiB read, 129 us at the copy rate).  With the placement of
 // T_{j-2} between the barriers, followed by a status word beside a prefix array
 // and a fence, the seven other warps waited for warp 0 half the time: 395 us.
